@@ -86,48 +86,40 @@ __device__ __forceinline__ uint64_t block_rule(uint64_t V, uint32_t rk, uint32_t
 // is (A, B): (0,0) empty, (0,1) solid, (1,0) sand, (1,1) water.
 // ---------------------------------------------------------------------------
 
-// bit-sliced u < c for the 8-bit numbers u whose bit w is plane p[w]
-template <uint32_t C>
-__device__ __forceinline__ uint32_t lt_const(const uint32_t (&p)[8]) {
-    uint32_t lt = 0, eq = 0xFFFFFFFFu;
-#pragma unroll
-    for (int w = 7; w >= 0; --w) {
-        if ((C >> w) & 1u) {
-            lt |= eq & ~p[w];
-            eq &= p[w];
-        } else {
-            eq &= ~p[w];
-        }
-    }
-    return lt;
-}
-
 // Chooses among up to three ordered candidate masks c1..c3 for the blocks in
-// `mov`; r = draw(n) with n = the number of candidates, from the slot's random
-// words P_w = plane(rk, g, s, w) (draw(2) = P_0; draw(3) compares u = sum_w
-// P_w << w with 85 and 170).  Outputs destination masks.
+// `mov` (each has at least one): the r-th candidate, r = draw(n) with n their
+// number, from the slot's random words P_w = plane(rk, g, s, w).  draw(2) =
+// P_0; draw(3) compares u = sum_w P_w << w with 85 and 170.  Outputs
+// destination masks, one candidate per block of `mov`.
+//
+// The comparisons run from the lowest bit up, so no word is kept: with ge the
+// answer for the bits below, a constant's bits 1 then 0 turn it into p1 | (p0 &
+// ge) and its bits 0 then 1 into p1 & (p0 | ge); 85 = 0b01010101 and 170 =
+// 0b10101010 repeat one of the two four times, one three-input operation per
+// pair of words and constant.
 __device__ __forceinline__ void bs_select(uint32_t mov, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t rk,
                                           uint32_t g, uint32_t s, uint32_t& d1, uint32_t& d2, uint32_t& d3) {
     const uint32_t two = (c1 & c2) | (c1 & c3) | (c2 & c3);
-    const uint32_t three = c1 & c2 & c3;
-    uint32_t r1 = 0, r2 = 0;
+    uint32_t past1 = 0, past2 = 0;  // blocks that pass over their first (and second) candidate
     if (mov & two) {
+        const uint32_t three = c1 & c2 & c3;
         const uint32_t p0 = plane(rk, g, s, 0u);
-        r1 = p0 & two & ~three;
+        past1 = two & ~three & p0;
         if (mov & three) {
-            uint32_t p[8];
-            p[0] = p0;
+            uint32_t ge85 = 0xFFFFFFFFu, ge170 = 0xFFFFFFFFu;
 #pragma unroll
-            for (uint32_t w = 1; w < 8u; ++w) p[w] = plane(rk, g, s, w);
-            const uint32_t lt85 = lt_const<85u>(p), lt170 = lt_const<170u>(p);
-            r1 |= three & ~lt85 & lt170;
-            r2 = three & ~lt170;
+            for (uint32_t w = 0; w < 8u; w += 2u) {
+                const uint32_t lo = w ? plane(rk, g, s, w) : p0, hi = plane(rk, g, s, w + 1u);
+                ge85 = hi | (lo & ge85);
+                ge170 = hi & (lo | ge170);
+            }
+            past1 |= three & ge85;
+            past2 = three & ge170;
         }
     }
-    const uint32_t r0 = ~(r1 | r2);
-    d1 = mov & r0 & c1;
-    d2 = mov & ((r0 & ~c1 & c2) | (r1 & c1 & c2));
-    d3 = mov & ((r0 & ~c1 & ~c2 & c3) | (r1 & c3 & (c1 ^ c2)) | r2);
+    d1 = mov & c1 & ~past1;
+    d2 = mov & c2 & ((c1 & past1 & ~past2) | (~c1 & ~past1));
+    d3 = mov & ~d1 & ~d2;
 }
 
 // The three other columns of q, in increasing order.
@@ -146,6 +138,15 @@ __device__ __forceinline__ uint32_t activity_mask(const uint32_t (&A)[8], const 
 
 // Runs one step of the rule on 32 blocks.  A[s], B[s] in/out per slot s.
 // Returns the mask of blocks that changed.
+//
+// Bound: the integer instructions of the eight dependent slots, most of them
+// the draws' hashes (each slot's words are drawn when any of a warp's 1024
+// blocks needs them).  A top slot chooses once for its diagonal and its
+// sideways moves together, since a block has candidates of one kind only:
+// with a choice for each, the same words were hashed twice.  One choice a slot
+// and the comparison from the lowest bit up: 2048 settled worlds' segment and
+// snapshot 1260 -> 1073 us, two segments of 512 fresh worlds 2545 -> 2309 us,
+// the 512^3 byte step 67.8 -> 64.6 us while everything falls.
 __device__ __forceinline__ uint32_t bs_rule(uint32_t (&A)[8], uint32_t (&B)[8], uint32_t rk, uint32_t g) {
     // Only the empty and water planes change as slots are visited.  A slot
     // acts exactly on the particles it held at the start (A[s]): a particle
@@ -169,41 +170,48 @@ __device__ __forceinline__ uint32_t bs_rule(uint32_t (&A)[8], uint32_t (&B)[8], 
         const uint32_t act = A[s] & active;
         if (!act) continue;
         const uint32_t wat = W[s];  // on the acting blocks: the slot's own water, untouched so far
-        uint32_t fall = 0, dg1 = 0, dg2 = 0, dg3 = 0, side;
+        // the other cells of the slot's own layer (where water moves sideways) and,
+        // for a top slot, of the layer below; a particle takes a diagonal when
+        // there is one, so one choice serves both: the candidates of a block are
+        // its diagonal ones, or its sideways ones when it has no diagonal
+        uint32_t c1 = E[base + other_col(q, 0)], c2 = E[base + other_col(q, 1)], c3 = E[base + other_col(q, 2)];
+        uint32_t fall = 0, down = 0, rest = act;
         if (s < 4) {
-            const int b = 4 + q;
-            fall = act & E[b];
-            const uint32_t rest = act & ~E[b];
-            const uint32_t c1 = E[4 + other_col(q, 0)], c2 = E[4 + other_col(q, 1)], c3 = E[4 + other_col(q, 2)];
-            const uint32_t any = c1 | c2 | c3;
-            bs_select(rest & any, c1, c2, c3, rk, g, (uint32_t)s, dg1, dg2, dg3);
-            side = rest & ~any & wat;
-        } else {
-            side = act & wat;
+            const uint32_t g1 = E[4 + other_col(q, 0)], g2 = E[4 + other_col(q, 1)], g3 = E[4 + other_col(q, 2)];
+            fall = act & E[4 + q];
+            rest = act & ~E[4 + q];
+            down = g1 | g2 | g3;  // the blocks with a diagonal
+            c1 = g1 | (c1 & ~down);
+            c2 = g2 | (c2 & ~down);
+            c3 = g3 | (c3 & ~down);
         }
-        const uint32_t e1 = E[base + other_col(q, 0)], e2 = E[base + other_col(q, 1)],
-                       e3 = E[base + other_col(q, 2)];
-        uint32_t sd1 = 0, sd2 = 0, sd3 = 0;
-        const uint32_t smov = side & (e1 | e2 | e3);
-        if (smov) bs_select(smov, e1, e2, e3, rk, g, (uint32_t)s, sd1, sd2, sd3);
-        const uint32_t moved = fall | dg1 | dg2 | dg3 | smov;
+        const uint32_t mov = rest & (down | wat) & (c1 | c2 | c3);
+        const uint32_t moved = fall | mov;
         if (!moved) continue;
         changed |= moved;
         W[s] &= ~moved;
         E[s] |= moved;
-        auto put = [&](int t, uint32_t m) {
-            E[t] &= ~m;
-            W[t] |= m & wat;
-        };
+        uint32_t d1 = 0, d2 = 0, d3 = 0;
+        if (mov) bs_select(mov, c1, c2, c3, rk, g, (uint32_t)s, d1, d2, d3);
         if (s < 4) {
-            put(4 + q, fall);
-            put(4 + other_col(q, 0), dg1);
-            put(4 + other_col(q, 1), dg2);
-            put(4 + other_col(q, 2), dg3);
+            E[4 + q] &= ~fall;
+            W[4 + q] |= fall & wat;
+            const uint32_t dw = down & wat;
+            E[4 + other_col(q, 0)] &= ~(d1 & down);
+            W[4 + other_col(q, 0)] |= d1 & dw;
+            E[4 + other_col(q, 1)] &= ~(d2 & down);
+            W[4 + other_col(q, 1)] |= d2 & dw;
+            E[4 + other_col(q, 2)] &= ~(d3 & down);
+            W[4 + other_col(q, 2)] |= d3 & dw;
         }
-        put(base + other_col(q, 0), sd1);
-        put(base + other_col(q, 1), sd2);
-        put(base + other_col(q, 2), sd3);
+        // only water moves sideways (down is empty for a bottom slot)
+        const uint32_t sw = ~down;
+        E[base + other_col(q, 0)] &= ~(d1 & sw);
+        W[base + other_col(q, 0)] |= d1 & sw;
+        E[base + other_col(q, 1)] &= ~(d2 & sw);
+        W[base + other_col(q, 1)] |= d2 & sw;
+        E[base + other_col(q, 2)] &= ~(d3 & sw);
+        W[base + other_col(q, 2)] |= d3 & sw;
     }
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
