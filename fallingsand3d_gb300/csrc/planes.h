@@ -55,16 +55,6 @@ constexpr int kMetaWorlds = 1 + 2 * kAllClasses;
 constexpr int kMetaInts = kMetaWorlds + 1;
 // smallest class that holds a world of these dims, -1 if none does
 int resident_class(int X, int Y, int Z);
-// Whether a call of n steps on one world of class cls takes them in one
-// resident launch (one CTA or cluster: its load, store and launch paid once
-// per call, then about 3-4.3 us per step up to 112^3) rather than n launches
-// of the per-step kernel (each step on the whole GPU, about 6.2-7.4 us).
-// Measured crossovers: 64^3 at 3-4 steps per call, 80^3 at 5, 96^3 at 7-8,
-// 112^3 at 11; 128^3 (a cluster) the per-step kernel at 1 and 8 steps per
-// call (7.1 against 9.8-22 us resident).
-inline bool prefer_resident(int cls, int n_steps, int64_t cells) {
-    return cls >= 0 && n_steps >= 4 && cells <= 1500000 && (int64_t)n_steps * 120000 >= cells;
-}
 // largest plane buffer (bytes) one CTA can hold; 0 if unavailable
 int smem_world_limit();
 constexpr int kErrInts = 4;  // size of the error record a resident launch is given
@@ -175,6 +165,25 @@ fs3d_status layer_flags_from_cells(const uint4* rows, uint8_t* lflags, int X, in
                                    cudaStream_t st);
 // one step (w.t) of the world; counts as for launch_plane_step
 fs3d_status launch_plane_step_skip(const PlaneWorld& w, uint8_t* rflags, int* counts, cudaStream_t st);
+// ---- many steps of one world in one launch over the whole GPU (slab.cu)
+struct SlabPlan {
+    int zs = 0;          // slabs cut along z (else along y)
+    int ctas = 0;        // slabs
+    int threads = 0;     // per CTA
+    int smem = 0;        // dynamic shared memory per CTA
+    size_t scratch = 0;  // device scratch a launch needs (256-byte aligned; the launch clears it)
+};
+// how a world would be cut; false if its slabs do not fit in shared memory
+bool slab_plan(int X, int Y, int Z, SlabPlan* out);
+// whether a call of n steps takes them in one such launch rather than in n
+// launches of the per-step kernel
+bool prefer_slabs(int X, int Y, int Z, int n_steps, SlabPlan* out);
+// w.steps steps from w.t; rflags as for launch_plane_step_skip (kept from call
+// to call), err as for launch_plane_segment_resident
+fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_t* rflags, void* scratch, int* err,
+                               cudaStream_t st);
+void set_slab_tx_extra(uint32_t bytes);  // test hook, as set_inject_tx_extra
+
 fs3d_status planes_hash_async(const uint4* rows, const uint8_t* statics, int X, int Y, int Z,
                               unsigned long long* out_dev, cudaStream_t st);
 // whole-grid hashes of njobs worlds in one launch: out_dev[j] for jobs[j]

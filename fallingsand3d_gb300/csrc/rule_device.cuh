@@ -86,41 +86,79 @@ __device__ __forceinline__ uint64_t block_rule(uint64_t V, uint32_t rk, uint32_t
 // is (A, B): (0,0) empty, (0,1) solid, (1,0) sand, (1,1) water.
 // ---------------------------------------------------------------------------
 
-// Chooses among up to three ordered candidate masks c1..c3 for the blocks in
+// Choosing among up to three ordered candidate masks c1..c3 for the blocks in
 // `mov` (each has at least one): the r-th candidate, r = draw(n) with n their
 // number, from the slot's random words P_w = plane(rk, g, s, w).  draw(2) =
-// P_0; draw(3) compares u = sum_w P_w << w with 85 and 170.  Outputs
-// destination masks, one candidate per block of `mov`.
+// P_0; draw(3) compares u = sum_w P_w << w with 85 and 170.
 //
 // The comparisons run from the lowest bit up, so no word is kept: with ge the
 // answer for the bits below, a constant's bits 1 then 0 turn it into p1 | (p0 &
 // ge) and its bits 0 then 1 into p1 & (p0 | ge); 85 = 0b01010101 and 170 =
 // 0b10101010 repeat one of the two four times, one three-input operation per
 // pair of words and constant.
-__device__ __forceinline__ void bs_select(uint32_t mov, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t rk,
-                                          uint32_t g, uint32_t s, uint32_t& d1, uint32_t& d2, uint32_t& d3) {
-    const uint32_t two = (c1 & c2) | (c1 & c3) | (c2 & c3);
-    uint32_t past1 = 0, past2 = 0;  // blocks that pass over their first (and second) candidate
-    if (mov & two) {
-        const uint32_t three = c1 & c2 & c3;
-        const uint32_t p0 = plane(rk, g, s, 0u);
-        past1 = two & ~three & p0;
-        if (mov & three) {
-            uint32_t ge85 = 0xFFFFFFFFu, ge170 = 0xFFFFFFFFu;
+__device__ __forceinline__ void draw3(uint32_t rk, uint32_t g, uint32_t s, uint32_t p0, uint32_t& ge85,
+                                      uint32_t& ge170) {
+    ge85 = ge170 = 0xFFFFFFFFu;
 #pragma unroll
-            for (uint32_t w = 0; w < 8u; w += 2u) {
-                const uint32_t lo = w ? plane(rk, g, s, w) : p0, hi = plane(rk, g, s, w + 1u);
-                ge85 = hi | (lo & ge85);
-                ge170 = hi & (lo | ge170);
-            }
-            past1 |= three & ge85;
-            past2 = three & ge170;
-        }
+    for (uint32_t w = 0; w < 8u; w += 2u) {
+        const uint32_t lo = w ? plane(rk, g, s, w) : p0, hi = plane(rk, g, s, w + 1u);
+        ge85 = hi | (lo & ge85);
+        ge170 = hi & (lo | ge170);
     }
+}
+
+// Destination masks, one candidate per block of `mov`, from the blocks that
+// pass over their first candidate (past1) and their second too (past2).
+__device__ __forceinline__ void bs_pick(uint32_t mov, uint32_t c1, uint32_t c2, uint32_t past1, uint32_t past2,
+                                        uint32_t& d1, uint32_t& d2, uint32_t& d3) {
     d1 = mov & c1 & ~past1;
     d2 = mov & c2 & ((c1 & past1 & ~past2) | (~c1 & ~past1));
     d3 = mov & ~d1 & ~d2;
 }
+
+// A row-pair word's draws, hashed where a slot needs them (throughput: about
+// half of the slots of a settled warp need none).
+struct LazyDraws {
+    static constexpr bool kReady = false;
+    uint32_t rk, g;
+    __device__ __forceinline__ void select(uint32_t mov, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t s, uint32_t& d1,
+                                           uint32_t& d2, uint32_t& d3) const {
+        const uint32_t two = (c1 & c2) | (c1 & c3) | (c2 & c3);
+        uint32_t past1 = 0, past2 = 0;
+        if (mov & two) {
+            const uint32_t three = c1 & c2 & c3;
+            const uint32_t p0 = plane(rk, g, s, 0u);
+            past1 = two & ~three & p0;
+            if (mov & three) {
+                uint32_t ge85, ge170;
+                draw3(rk, g, s, p0, ge85, ge170);
+                past1 |= three & ge85;
+                past2 = three & ge170;
+            }
+        }
+        bs_pick(mov, c1, c2, past1, past2, d1, d2, d3);
+    }
+};
+
+// The draws of all eight slots, hashed beforehand: they depend on the world's
+// seed, the step and the place only, so a caller that has to wait for cells
+// hashes them meanwhile, and the slots' serial chain runs without branches.
+struct ReadyDraws {
+    static constexpr bool kReady = true;
+    uint32_t p0[8], ge85[8], ge170[8];
+    __device__ __forceinline__ void fill(uint32_t rk, uint32_t g) {
+#pragma unroll
+        for (uint32_t s = 0; s < 8u; ++s) {
+            p0[s] = plane(rk, g, s, 0u);
+            draw3(rk, g, s, p0[s], ge85[s], ge170[s]);
+        }
+    }
+    __device__ __forceinline__ void select(uint32_t mov, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t s, uint32_t& d1,
+                                           uint32_t& d2, uint32_t& d3) const {
+        const uint32_t two = (c1 & c2) | (c1 & c3) | (c2 & c3), three = c1 & c2 & c3;
+        bs_pick(mov, c1, c2, (three & ge85[s]) | (two & ~three & p0[s]), three & ge170[s], d1, d2, d3);
+    }
+};
 
 // The three other columns of q, in increasing order.
 __host__ __device__ constexpr int other_col(int q, int n) { return n < q ? n : n + 1; }
@@ -147,7 +185,8 @@ __device__ __forceinline__ uint32_t activity_mask(const uint32_t (&A)[8], const 
 // and the comparison from the lowest bit up: 2048 settled worlds' segment and
 // snapshot 1260 -> 1073 us, two segments of 512 fresh worlds 2545 -> 2309 us,
 // the 512^3 byte step 67.8 -> 64.6 us while everything falls.
-__device__ __forceinline__ uint32_t bs_rule(uint32_t (&A)[8], uint32_t (&B)[8], uint32_t rk, uint32_t g) {
+template <class Draws>
+__device__ __forceinline__ uint32_t bs_rule(uint32_t (&A)[8], uint32_t (&B)[8], const Draws& draws) {
     // Only the empty and water planes change as slots are visited.  A slot
     // acts exactly on the particles it held at the start (A[s]): a particle
     // only ever moves into an empty cell, so a cell's own particle is still
@@ -168,7 +207,7 @@ __device__ __forceinline__ uint32_t bs_rule(uint32_t (&A)[8], uint32_t (&B)[8], 
     for (int s = 0; s < 8; ++s) {
         const int q = s & 3, base = s & 4;
         const uint32_t act = A[s] & active;
-        if (!act) continue;
+        if (!Draws::kReady && !act) continue;
         const uint32_t wat = W[s];  // on the acting blocks: the slot's own water, untouched so far
         // the other cells of the slot's own layer (where water moves sideways) and,
         // for a top slot, of the layer below; a particle takes a diagonal when
@@ -187,12 +226,12 @@ __device__ __forceinline__ uint32_t bs_rule(uint32_t (&A)[8], uint32_t (&B)[8], 
         }
         const uint32_t mov = rest & (down | wat) & (c1 | c2 | c3);
         const uint32_t moved = fall | mov;
-        if (!moved) continue;
+        if (!Draws::kReady && !moved) continue;
         changed |= moved;
         W[s] &= ~moved;
         E[s] |= moved;
         uint32_t d1 = 0, d2 = 0, d3 = 0;
-        if (mov) bs_select(mov, c1, c2, c3, rk, g, (uint32_t)s, d1, d2, d3);
+        if (Draws::kReady || mov) draws.select(mov, c1, c2, c3, (uint32_t)s, d1, d2, d3);
         if (s < 4) {
             E[4 + q] &= ~fall;
             W[4 + q] |= fall & wat;
@@ -222,6 +261,10 @@ __device__ __forceinline__ uint32_t bs_rule(uint32_t (&A)[8], uint32_t (&B)[8], 
     return changed;
 }
 
+
+__device__ __forceinline__ uint32_t bs_rule(uint32_t (&A)[8], uint32_t (&B)[8], uint32_t rk, uint32_t g) {
+    return bs_rule(A, B, LazyDraws{rk, g});
+}
 
 // The half block at the right end of an odd-phase row (x = X-1 present,
 // x = X outside) has only its dx=0 column: cells r = layer*2 + dz with bit r
@@ -297,11 +340,12 @@ __device__ __forceinline__ void rowpair_slots(const uint4 (&q)[4], int o, int gl
 // carried in (x = -1 is solid), and the left lane receives its new bit 31
 // back; when the row width is a multiple of 64 (`half_at_end`) the last lane
 // also runs the half block at x = 64*nw - 1.
-__device__ __forceinline__ void rowpair_core(uint4 (&q)[4], bool has, int o, uint32_t rk, int gl, int G, int nw,
+template <class Draws>
+__device__ __forceinline__ void rowpair_core(uint4 (&q)[4], bool has, int o, const Draws& draws, int gl, int G, int nw,
                                              bool half_at_end) {
     uint32_t A[8], B[8];
     rowpair_slots(q, o, gl, G, A, B);
-    if (has) bs_rule(A, B, rk, (uint32_t)gl);
+    if (has) bs_rule(A, B, draws);
     if (o == 0) {
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
@@ -338,6 +382,11 @@ __device__ __forceinline__ void rowpair_core(uint4 (&q)[4], bool has, int o, uin
         }
         q[a] = make_uint4(A[s0 + 1], (A[s0] >> 1) | (na << 31), B[s0 + 1], (B[s0] >> 1) | (nb << 31));
     }
+}
+
+__device__ __forceinline__ void rowpair_core(uint4 (&q)[4], bool has, int o, uint32_t rk, int gl, int G, int nw,
+                                             bool half_at_end) {
+    rowpair_core(q, has, o, LazyDraws{rk, (uint32_t)gl}, gl, G, nw, half_at_end);
 }
 
 // Whether lane gl's blocks of a block row-pair (q as for rowpair_core, only

@@ -1,13 +1,13 @@
 // fs3d_run_device: n steps of a caller-owned device byte grid through the bit
 // plane kernels.  The grid is converted once into 2-bit planes (scratch), the
-// steps run there (all of them in one resident launch when the world fits in
+// steps run there (all of them in one launch when the world's slabs fit in
 // shared memory, one per-step launch each otherwise), and the planes are
 // converted back.  Static cells never change, so their byte values are read
 // back from the caller's grid itself.  Rows wider than 2048 cells take the
 // byte kernels instead.
 //
-// A resident launch whose bulk copy does not land within its bounded wait
-// leaves the grid as it was and sets a sticky per-device word; while it is
+// A launch whose bulk copy (or a neighbour slab's result) does not arrive
+// within its bounded wait leaves the grid as it was and sets a sticky per-device word; while it is
 // set, later runs on the device leave their grids unchanged too, and
 // fs3d_run_device_check reports FS3D_ERR_TIMEOUT and clears it.
 #include <chrono>
@@ -26,7 +26,7 @@ using namespace fs3d;
 
 namespace {
 
-static __device__ __align__(16) int g_run_device_err[kErrInts];  // the resident kernel's error record
+static __device__ __align__(16) int g_run_device_err[kErrInts];  // the multi-step kernel's error record
 
 constexpr int kMaxDevices = 64;
 struct ErrAddr {
@@ -56,15 +56,6 @@ fs3d_status run_error_word(int** out) {
     return FS3D_OK;
 }
 
-// device scratch of one run: the planes and the one-world step tables
-struct RunScratch {
-    uint4* rows = nullptr;
-    PlaneWorld* desc = nullptr;
-    int* ints = nullptr;  // meta (1 + 2*classes), order[0], counter
-};
-
-constexpr int kOrder = kMetaInts, kCounter = kOrder + 1, kInts = kCounter + 1;
-
 }  // namespace
 
 extern "C" fs3d_status fs3d_run_device(uint8_t* grid_dev, int X, int Y, int Z, uint64_t seed, uint64_t t0,
@@ -74,26 +65,21 @@ extern "C" fs3d_status fs3d_run_device(uint8_t* grid_dev, int X, int Y, int Z, u
     cudaStream_t st = (cudaStream_t)stream;
     if (n_steps == 0) return FS3D_OK;
     if (X > kPlaneMaxX) return launch_step_bytes(grid_dev, X, Y, Z, seed, t0, n_steps, st);
-    const int nw = plane_nw(X), lg = plane_lg(nw);
-    // a resident launch, or the per-step kernel (prefer_resident)
-    const int cls = prefer_resident(resident_class(X, Y, Z), n_steps, (int64_t)X * Y * Z) ? resident_class(X, Y, Z) : -1;
-    // worlds too large for shared memory, and short calls: the per-step
-    // kernel that skips settled row-pairs (per-row flags in the scratch)
+    const int nw = plane_nw(X);
+    SlabPlan plan;
+    const bool slabs = prefer_slabs(X, Y, Z, n_steps, &plan);
     int* err = nullptr;
     {
         const fs3d_status se = run_error_word(&err);
         if (se != FS3D_OK) return se;
     }
-    RunScratch sc;
-    uint8_t* rflags = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&sc.rows, plane_bytes(X, Y, Z), st);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&sc.desc, sizeof(PlaneWorld), st);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&sc.ints, sizeof(int) * kInts, st);
-    // per-row flags for the per-step kernel, per-layer flags for a resident launch
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&rflags, cls < 0 ? (size_t)Y * Z : layer_flag_bytes(Y), st);
-    fs3d_status s = e == cudaSuccess ? FS3D_OK : cuda_fail(e, "fs3d_run_device scratch");
+    // one block of scratch: the planes, the row flags, the slabs' scratch
+    const size_t rows_b = (plane_bytes(X, Y, Z) + 255) & ~(size_t)255, flags_b = ((size_t)Y * Z + 255) & ~(size_t)255;
+    char* scratch = nullptr;
+    FS3D_CUDA(cudaMallocAsync((void**)&scratch, rows_b + flags_b + (slabs ? plan.scratch : 0), st));
+    uint8_t* rflags = reinterpret_cast<uint8_t*>(scratch + rows_b);
     PlaneWorld d{};
-    d.rows = sc.rows;
+    d.rows = reinterpret_cast<uint4*>(scratch);
     d.seed = seed;
     d.t = t0;
     d.X = X;
@@ -101,33 +87,20 @@ extern "C" fs3d_status fs3d_run_device(uint8_t* grid_dev, int X, int Y, int Z, u
     d.Z = Z;
     d.nw = nw;
     d.steps = n_steps;
-    d.lg = lg;
-    if (cls >= 0) d.lflags = rflags;  // set from the cells below: no dense first steps
-    int ints[kInts] = {};
-    if (cls >= 0) ints[1 + cls] = 1;
-    // pageable sources: staged before each call returns
-    if (s == FS3D_OK) e = cudaMemcpyAsync(sc.desc, &d, sizeof(d), cudaMemcpyHostToDevice, st);
-    if (s == FS3D_OK && e == cudaSuccess) e = cudaMemcpyAsync(sc.ints, ints, sizeof(ints), cudaMemcpyHostToDevice, st);
-    if (s == FS3D_OK && e != cudaSuccess) s = cuda_fail(e, "fs3d_run_device tables");
-    if (s == FS3D_OK) s = planes_from_bytes(grid_dev, X, Y, Z, sc.rows, st);
-    if (s == FS3D_OK) {
-        if (cls >= 0) {
-            s = layer_flags_from_cells(sc.rows, rflags, X, Y, Z, t0, st);
-            if (s == FS3D_OK)
-                s = launch_plane_segment_resident(cls, sc.desc, sc.ints + kOrder, sc.ints, sc.ints + kCounter, err, st);
-        } else {
-            s = init_row_flags(sc.rows, rflags, X, Y, Z, t0, st);
-            for (int a = 0; a < n_steps && s == FS3D_OK; ++a) {
-                d.t = t0 + (uint64_t)a;
-                s = launch_plane_step_skip(d, rflags, nullptr, st);
-            }
+    d.lg = plane_lg(nw);
+    fs3d_status s = planes_from_bytes(grid_dev, X, Y, Z, d.rows, st);
+    if (s == FS3D_OK) s = init_row_flags(d.rows, rflags, X, Y, Z, t0, st);
+    if (s == FS3D_OK && slabs) {
+        s = launch_plane_slabs(d, plan, rflags, scratch + rows_b + flags_b, err, st);
+    } else {
+        for (int a = 0; a < n_steps && s == FS3D_OK; ++a) {
+            d.t = t0 + (uint64_t)a;
+            s = launch_plane_step_skip(d, rflags, nullptr, st);
         }
     }
     // a recorded failure (this run's or an earlier one's) leaves the grid as it was
-    if (s == FS3D_OK) s = planes_to_bytes(sc.rows, grid_dev, X, Y, Z, grid_dev, st, err);
-    // only what was allocated (the allocations stop at the first failure)
-    for (void* p : {(void*)sc.rows, (void*)sc.desc, (void*)sc.ints, (void*)rflags})
-        if (p) cudaFreeAsync(p, st);
+    if (s == FS3D_OK) s = planes_to_bytes(d.rows, grid_dev, X, Y, Z, grid_dev, st, err);
+    cudaFreeAsync(scratch, st);
     return s;
 }
 

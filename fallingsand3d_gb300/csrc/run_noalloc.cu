@@ -40,17 +40,13 @@ namespace {
 constexpr size_t kNoAllocPlaneBytes = (size_t)64 << 20;
 constexpr int kMaxDevices = 64;
 
-// scratch layout: [planes][one-world descriptor][ints][sticky error record][row flags]
-constexpr size_t kDescOff = kNoAllocPlaneBytes;
-constexpr size_t kIntsOff = kDescOff + 256;
-constexpr int kOrder = kMetaInts, kCounter = kOrder + 1, kInts = kCounter + 1;
-constexpr size_t kErrOff = kIntsOff + 256;  // set by a timed-out copy, cleared by fs3d_run_device_check only
+// scratch layout: [planes, then the slabs' scratch where it fits][sticky error record][row flags]
+constexpr size_t kErrOff = kNoAllocPlaneBytes;  // set by a timed-out copy, cleared by fs3d_run_device_check only
 constexpr size_t kFlagsOff = kErrOff + 256;
 // one byte per row of the per-step kernel: a world of at most 64 MiB of
 // planes has at most 4 Mi rows (one 16-byte word each at the least)
 constexpr size_t kNoAllocFlagBytes = kNoAllocPlaneBytes / sizeof(uint4);
 constexpr size_t kScratchBytes = kFlagsOff + kNoAllocFlagBytes;
-static_assert(kInts * sizeof(int) <= 256, "ints region");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -61,19 +57,6 @@ struct ScratchAddr {
 };
 ScratchAddr g_scratch_addr[kMaxDevices];
 std::mutex g_scratch_mu;
-
-// Writes the one-world tables into the scratch and clears the work counter
-// (the array keeps whatever the previous call left; the sticky error record
-// is left alone).
-__global__ void k_noalloc_tables(PlaneWorld d, int cls, unsigned char* base) {
-    PlaneWorld* desc = reinterpret_cast<PlaneWorld*>(base + kDescOff);
-    int* ints = reinterpret_cast<int*>(base + kIntsOff);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *desc = d;
-        for (int a = 0; a < kInts; ++a) ints[a] = 0;
-        if (cls >= 0) ints[1 + cls] = 1;
-    }
-}
 
 }  // namespace
 
@@ -119,14 +102,15 @@ extern "C" fs3d_status fs3d_run_device_noalloc(uint8_t* grid_dev, int X, int Y, 
         return set_error(FS3D_ERR_INVALID_ARG,
                          "fs3d_run_device_noalloc: world too large for the static scratch (planes of at most "
                          "64 MiB, about 268 M cells, and rows of at most 2048 cells)");
-    const int nw = plane_nw(X), lg = plane_lg(nw);
-    // a resident launch, or the per-step kernel (prefer_resident)
-    const int cls = prefer_resident(resident_class(X, Y, Z), n_steps, (int64_t)X * Y * Z) ? resident_class(X, Y, Z) : -1;
     if (n_steps == 0) return FS3D_OK;
     unsigned char* base = nullptr;
     fs3d_status s = noalloc_scratch_base(&base);
     if (s != FS3D_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
+    // all the steps in one launch (its scratch behind the planes), or one launch a step
+    const size_t rows_b = (plane_bytes(X, Y, Z) + 255) & ~(size_t)255;
+    SlabPlan plan;
+    const bool slabs = prefer_slabs(X, Y, Z, n_steps, &plan) && rows_b + plan.scratch <= kNoAllocPlaneBytes;
     uint4* rows = reinterpret_cast<uint4*>(base);
     PlaneWorld d{};
     d.rows = rows;
@@ -135,28 +119,19 @@ extern "C" fs3d_status fs3d_run_device_noalloc(uint8_t* grid_dev, int X, int Y, 
     d.X = X;
     d.Y = Y;
     d.Z = Z;
-    d.nw = nw;
+    d.nw = plane_nw(X);
     d.steps = n_steps;
-    d.lg = lg;
-    uint8_t* flags = base + kFlagsOff;  // per-row flags (per-step kernel) or per-layer flags (resident launch)
-    if (cls >= 0) d.lflags = flags;     // set from the cells below: no dense first steps
-    k_noalloc_tables<<<1, 32, 0, st>>>(d, cls, base);
-    FS3D_CHECK_LAUNCH("noalloc tables launch");
-    PlaneWorld* desc = reinterpret_cast<PlaneWorld*>(base + kDescOff);
-    int* ints = reinterpret_cast<int*>(base + kIntsOff);
+    d.lg = plane_lg(d.nw);
+    uint8_t* rflags = base + kFlagsOff;
     int* err = reinterpret_cast<int*>(base + kErrOff);
     s = planes_from_bytes(grid_dev, X, Y, Z, rows, st);
-    if (s == FS3D_OK) {
-        if (cls >= 0) {
-            s = layer_flags_from_cells(rows, flags, X, Y, Z, t0, st);
-            if (s == FS3D_OK) s = launch_plane_segment_resident(cls, desc, ints + kOrder, ints, ints + kCounter, err, st);
-        } else {
-            uint8_t* rflags = flags;
-            s = init_row_flags(rows, rflags, X, Y, Z, t0, st);
-            for (int a = 0; a < n_steps && s == FS3D_OK; ++a) {
-                d.t = t0 + (uint64_t)a;
-                s = launch_plane_step_skip(d, rflags, nullptr, st);
-            }
+    if (s == FS3D_OK) s = init_row_flags(rows, rflags, X, Y, Z, t0, st);
+    if (s == FS3D_OK && slabs) {
+        s = launch_plane_slabs(d, plan, rflags, base + rows_b, err, st);
+    } else {
+        for (int a = 0; a < n_steps && s == FS3D_OK; ++a) {
+            d.t = t0 + (uint64_t)a;
+            s = launch_plane_step_skip(d, rflags, nullptr, st);
         }
     }
     // static cells never change: their values are read back from the grid

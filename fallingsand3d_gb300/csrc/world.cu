@@ -24,32 +24,24 @@ struct fs3d_world {
     uint8_t* bytes = nullptr;    // BYTES: the state
     uint4* rows = nullptr;       // PLANES: the state
     uint8_t* statics = nullptr;  // PLANES: initial bytes when some cell holds a material >= 4
-    PlaneWorld* desc = nullptr;  // PLANES: one-world descriptor of the resident kernels
-    int* aux = nullptr;          // resident tables, see kAux*
-    int cls = -1;        // resident class (-1: stepped by the per-step kernel)
+    void* slab_scratch = nullptr;  // PLANES: scratch of the whole-GPU multi-step launches (worlds that fit them)
+    int* err = nullptr;            // PLANES: error record of those launches (kErrInts ints)
     unsigned long long* hash_dev = nullptr;
     uint32_t* brickmap = nullptr;  // render: per-frame occupancy of 8x8x8 bricks
     int* brick_counts = nullptr;   // PLANES render: non-empty cells per brick, kept by the per-step kernel
     bool counts_valid = false;     // brick_counts match the planes
-    // change flags kept from one call to the next: per row (Y*Z bytes) for the
-    // per-step kernel, per layer (Y bytes, padded) for a resident launch
+    // change flags per row (Y*Z bytes), kept from one call to the next
     uint8_t* rflags = nullptr;
     bool flags_ok = false;  // rflags describe the state at step flags_t
     uint64_t flags_t = 0;
-    uint8_t* lflags = nullptr;  // resident class only
-    bool lflags_ok = false;     // lflags describe the state at step lflags_t
-    uint64_t lflags_t = 0;
     int64_t cells() const { return (int64_t)X * Y * Z; }
 };
 
 namespace {
 
-// layout of fs3d_world::aux (device ints)
-constexpr int kAuxMeta = 0;                              // kMetaInts ints
-constexpr int kAuxOrder = kMetaInts;      // order[0] = 0
-constexpr int kAuxCounter = kAuxOrder + 1;
-constexpr int kAuxErr = (kAuxCounter + 2) & ~1;   // kErrInts ints, 8-byte aligned
-constexpr int kAuxInts = kAuxErr + kErrInts;
+// plane bytes from which a rendered world keeps brick counts (the per-step
+// kernel's cost of keeping them against a frame's pass over the planes)
+constexpr size_t kCountsPlaneBytes = (size_t)1800 << 10;
 
 bool dims_ok(int X, int Y, int Z) {
     return X > 0 && Y > 0 && Z > 0 && X <= (1 << 16) && Y <= (1 << 16) && Z <= (1 << 16);
@@ -83,13 +75,12 @@ void destroy(fs3d_world* w) {
     cudaFree(w->bytes);
     cudaFree(w->rows);
     cudaFree(w->statics);
-    cudaFree(w->desc);
-    cudaFree(w->aux);
+    cudaFree(w->slab_scratch);
+    cudaFree(w->err);
     cudaFree(w->hash_dev);
     cudaFree(w->brickmap);
     cudaFree(w->brick_counts);
     cudaFree(w->rflags);
-    cudaFree(w->lflags);
     if (w->stream) cudaStreamDestroy(w->stream);
     delete w;
 }
@@ -155,16 +146,12 @@ fs3d_status fs3d_world_create(const uint8_t* grid_host, int X, int Y, int Z, uin
     } else {
         e = cudaMalloc((void**)&w->rows, plane_bytes(X, Y, Z));
         if (e != cudaSuccess) return fail(e, "cudaMalloc(planes)");
-        e = cudaMalloc((void**)&w->desc, sizeof(PlaneWorld));
-        // resident tables: meta (one world in its class), order {0}, work counter, error record
-        int aux[kAuxInts] = {};
-        w->cls = resident_class(X, Y, Z);
-        if (w->cls >= 0) aux[1 + w->cls] = 1;
-        if (e == cudaSuccess) e = cudaMalloc((void**)&w->aux, sizeof(aux));
-        if (e == cudaSuccess) e = cudaMemcpy(w->aux, aux, sizeof(aux), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return fail(e, "cudaMalloc/copy(step tables)");
+        if (e == cudaSuccess) e = cudaMalloc((void**)&w->err, sizeof(int) * kErrInts);
+        if (e == cudaSuccess) e = cudaMemset(w->err, 0, sizeof(int) * kErrInts);
+        if (e != cudaSuccess) return fail(e, "cudaMalloc(error record)");
+        SlabPlan plan;
         e = cudaMalloc((void**)&w->rflags, (size_t)Y * Z);
-        if (e == cudaSuccess && w->cls >= 0) e = cudaMalloc((void**)&w->lflags, layer_flag_bytes(Y));
+        if (e == cudaSuccess && slab_plan(X, Y, Z, &plan)) e = cudaMalloc(&w->slab_scratch, plan.scratch);
         if (e != cudaSuccess) return fail(e, "cudaMalloc(change flags)");
     }
     s = upload(w, grid_host);
@@ -195,52 +182,40 @@ fs3d_status fs3d_world_step(fs3d_world* w, int n_steps) {
         d.steps = n_steps;
         d.lg = plane_lg(nw);
         s = FS3D_OK;
-        // one resident launch, or one per-step launch per step (prefer_resident)
-        const bool resident = prefer_resident(w->cls, n_steps, w->cells());
-        if (!resident) {
-            // one launch per step, settled row-pairs skipped; the row flags
-            // carry over from the previous call when nothing else touched the
-            // world since.  Once a frame has counted the bricks, the kernel
-            // keeps the counts exact, so later frames read no pass over the planes
-            if (!w->flags_ok || w->flags_t != w->step) {
-                s = init_row_flags(w->rows, w->rflags, w->X, w->Y, w->Z, w->step, w->stream);
-                w->flags_ok = s == FS3D_OK;
-            }
-            int* counts = w->counts_valid ? w->brick_counts : nullptr;
-            int launched = 0;
-            while (s == FS3D_OK && launched < n_steps) {
-                d.t = w->step + (uint64_t)launched;
-                s = launch_plane_step_skip(d, w->rflags, counts, w->stream);
-                if (s == FS3D_OK) ++launched;
-            }
-            w->step += (uint64_t)launched;  // the steps that went out before a failed launch still count
-            if (s == FS3D_OK)
+        // settled row-pairs are skipped; the row flags carry over from the
+        // previous call when nothing else touched the world since
+        if (!w->flags_ok || w->flags_t != w->step) {
+            s = init_row_flags(w->rows, w->rflags, w->X, w->Y, w->Z, w->step, w->stream);
+            w->flags_ok = s == FS3D_OK;
+        }
+        // one launch for all the steps, or one per-step launch per step (prefer_slabs)
+        SlabPlan plan;
+        if (w->slab_scratch && prefer_slabs(w->X, w->Y, w->Z, n_steps, &plan)) {
+            if (s == FS3D_OK) s = launch_plane_slabs(d, plan, w->rflags, w->slab_scratch, w->err, w->stream);
+            w->counts_valid = false;  // the next frame recounts
+            if (s == FS3D_OK) {
+                w->step += (uint64_t)n_steps;
                 w->flags_t = w->step;
-            else
+            } else {
                 w->flags_ok = false;
+            }
             return s;
         }
-        // the world fits in shared memory (one CTA or a cluster): all n steps
-        // in one launch, the layer flags kept from the previous call (or set
-        // from the cells); the descriptor's pageable source is staged before
-        // the call returns
-        if (!w->lflags_ok || w->lflags_t != w->step) {
-            s = layer_flags_from_cells(w->rows, w->lflags, w->X, w->Y, w->Z, w->step, w->stream);
-            w->lflags_ok = s == FS3D_OK;
+        // once a frame has counted the bricks, the per-step kernel keeps the
+        // counts exact, so later frames read no pass over the planes
+        int* counts = w->counts_valid ? w->brick_counts : nullptr;
+        int launched = 0;
+        while (s == FS3D_OK && launched < n_steps) {
+            d.t = w->step + (uint64_t)launched;
+            s = launch_plane_step_skip(d, w->rflags, counts, w->stream);
+            if (s == FS3D_OK) ++launched;
         }
-        d.lflags = w->lflags;
-        if (s == FS3D_OK) {
-            const cudaError_t ce = cudaMemcpyAsync(w->desc, &d, sizeof(d), cudaMemcpyHostToDevice, w->stream);
-            s = ce == cudaSuccess ? FS3D_OK : cuda_fail(ce, "fs3d_world_step descriptor");
-        }
+        w->step += (uint64_t)launched;  // the steps that went out before a failed launch still count
         if (s == FS3D_OK)
-            s = launch_plane_segment_resident(w->cls, w->desc, w->aux + kAuxOrder, w->aux + kAuxMeta,
-                                              w->aux + kAuxCounter, w->aux + kAuxErr, w->stream);
-        if (s == FS3D_OK)
-            w->lflags_t = w->step + (uint64_t)n_steps;
+            w->flags_t = w->step;
         else
-            w->lflags_ok = false;
-        w->counts_valid = false;  // the next frame recounts
+            w->flags_ok = false;
+        return s;
     }
     if (s == FS3D_OK) w->step += (uint64_t)n_steps;
     return s;
@@ -250,14 +225,15 @@ fs3d_status fs3d_world_sync(fs3d_world* w, int64_t timeout_ns) {
     if (!w) return set_error(FS3D_ERR_INVALID_ARG, "fs3d_world_sync: NULL world");
     fs3d_status s = bounded_wait(w->stream, timeout_ns);
     if (s != FS3D_OK) return s;
-    if (w->aux) {
+    if (w->err) {
         int err[kErrInts] = {};
-        FS3D_CUDA(cudaMemcpy(err, w->aux + kAuxErr, sizeof(err), cudaMemcpyDeviceToHost));
+        FS3D_CUDA(cudaMemcpy(err, w->err, sizeof(err), cudaMemcpyDeviceToHost));
         if (err[0]) {
             uint64_t t_fail = 0;
             memcpy(&t_fail, err + 2, sizeof(t_fail));
-            FS3D_CUDA(cudaMemset(w->aux + kAuxErr, 0, sizeof(err)));
+            FS3D_CUDA(cudaMemset(w->err, 0, sizeof(err)));
             w->counts_valid = false;
+            w->flags_ok = false;
             // the failed launch and every launch after it stepped nothing: the
             // state is the one the failed launch started from
             w->step = t_fail;
@@ -292,7 +268,6 @@ fs3d_status fs3d_world_write(fs3d_world* w, const uint8_t* g) {
     if (!w || !g) return set_error(FS3D_ERR_INVALID_ARG, "fs3d_world_write: bad args");
     w->counts_valid = false;
     w->flags_ok = false;
-    w->lflags_ok = false;
     return upload(w, g);
 }
 
@@ -397,7 +372,8 @@ fs3d_status fs3d_render(fs3d_world* w, const fs3d_camera* cam, int W, int H, int
     if (mode == FS3D_RENDER_DDA && !w->brickmap)
         FS3D_CUDA(cudaMalloc((void**)&w->brickmap, brickmap_bytes(w->X, w->Y, w->Z)));
     // planes worlds stepped by the per-step kernel keep exact brick counts
-    if (mode == FS3D_RENDER_DDA && w->layout == FS3D_LAYOUT_PLANES && w->cls < 0 && !w->brick_counts)
+    if (mode == FS3D_RENDER_DDA && w->layout == FS3D_LAYOUT_PLANES && !w->brick_counts &&
+        plane_bytes(w->X, w->Y, w->Z) > kCountsPlaneBytes)
         FS3D_CUDA(cudaMalloc((void**)&w->brick_counts, brick_count_bytes(w->X, w->Y, w->Z)));
     if (!out_on_device) FS3D_CUDA(cudaMallocAsync((void**)&dst, bytes, w->stream));
     fs3d_status s;
