@@ -10,48 +10,75 @@
 
 namespace fs3d {
 
-// bits 0, 8, 16, 24 -> bits 0..3
-__device__ __forceinline__ uint32_t gather_lo4(uint32_t m) { return (m * 0x10204080u) >> 28; }
-// bits 0..3 -> bit 0 of bytes 0..3
-__device__ __forceinline__ uint32_t spread4(uint32_t n) { return (n * 0x00204081u) & 0x01010101u; }
-
-// Four cells (one byte each) -> nibbles of A (sand or water) and B (water or solid).
-__device__ __forceinline__ void classify4(uint32_t v, uint32_t& a4, uint32_t& b4) {
+// Every byte of v with a static material (>= 4) turned into a solid's code (1).
+__device__ __forceinline__ uint32_t statics_to_solid(uint32_t v) {
     const uint32_t big = v & 0xFCFCFCFCu;
-    if (big) {
-        const uint32_t nz = ((big & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | big;  // bit 7 set iff byte >= 4
-        const uint32_t m = ((nz & 0x80808080u) >> 7) * 0xFFu;
-        v = (v & ~m) | (0x01010101u & m);
-    }
-    a4 = gather_lo4((v >> 1) & 0x01010101u);
-    b4 = gather_lo4(v & 0x01010101u);
+    const uint32_t nz = ((big & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | big;  // bit 7 set iff the byte is >= 4
+    const uint32_t m = ((nz & 0x80808080u) >> 7) * 0xFFu;
+    return (v & ~m) | (0x01010101u & m);
 }
 
-// 64 cells (16 little-endian words, cell 4k + i in byte i of word k) -> plane word
-__device__ __forceinline__ uint4 bytes_to_planes64(const uint32_t (&w)[16]) {
-    uint32_t ae = 0, ao = 0, be = 0, bo = 0;
+// The bytes of four words, transposed: byte g of q[i] = byte i of p[g].
+__device__ __forceinline__ void transpose4(const uint32_t (&p)[4], uint32_t (&q)[4]) {
+    const uint32_t a = __byte_perm(p[0], p[1], 0x5140), b = __byte_perm(p[2], p[3], 0x5140);
+    const uint32_t c = __byte_perm(p[0], p[1], 0x7362), d = __byte_perm(p[2], p[3], 0x7362);
+    q[0] = __byte_perm(a, b, 0x5410);
+    q[1] = __byte_perm(a, b, 0x7632);
+    q[2] = __byte_perm(c, d, 0x5410);
+    q[3] = __byte_perm(c, d, 0x7632);
+}
+
+// Four words of a 16-cell piece (codes 0..3 in their bytes) in one: byte i
+// holds the codes of cells i, 4 + i, 8 + i, 12 + i from its low bits up.
+// Multiply-adds, which leave the logic unit free (it bounds the byte step).
+__device__ __forceinline__ uint32_t pack_piece(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
+    return w0 + 4u * (w1 + 4u * (w2 + 4u * w3));
+}
+
+// The four packed pieces of 64 cells -> plane word.  After the transposition
+// byte g of t[i] holds cells 16g + i, + 4 + i, + 8 + i, + 12 + i: an even i
+// gives even cells, whose plane bits are 8g + 2j + i/2 for j = 0..3.
+__device__ __forceinline__ uint4 pieces_to_planes(const uint32_t (&p)[4]) {
+    uint32_t t[4];
+    transpose4(p, t);
+    return make_uint4(((t[0] >> 1) & 0x55555555u) | (t[2] & 0xAAAAAAAAu), ((t[1] >> 1) & 0x55555555u) | (t[3] & 0xAAAAAAAAu),
+                      (t[0] & 0x55555555u) | ((t[2] << 1) & 0xAAAAAAAAu), (t[1] & 0x55555555u) | ((t[3] << 1) & 0xAAAAAAAAu));
+}
+
+// and back
+__device__ __forceinline__ void planes_to_pieces(const uint4& q, uint32_t (&p)[4]) {
+    const uint32_t t[4] = {(q.z & 0x55555555u) | ((q.x << 1) & 0xAAAAAAAAu), (q.w & 0x55555555u) | ((q.y << 1) & 0xAAAAAAAAu),
+                           ((q.z >> 1) & 0x55555555u) | (q.x & 0xAAAAAAAAu), ((q.w >> 1) & 0x55555555u) | (q.y & 0xAAAAAAAAu)};
+    transpose4(t, p);
+}
+
+// word j (cells 4j .. 4j + 3) of a packed piece
+__device__ __forceinline__ uint32_t piece_word(uint32_t p, int j) { return (p >> (2 * j)) & 0x03030303u; }
+__device__ __forceinline__ uint4 piece_bytes(uint32_t p) {
+    return make_uint4(piece_word(p, 0), piece_word(p, 1), piece_word(p, 2), piece_word(p, 3));
+}
+
+// 64 cells (16 little-endian words, cell 4k + i in byte i of word k) -> plane
+// word; `big`: some byte is a static material
+__device__ __forceinline__ uint4 bytes_to_planes64(const uint32_t (&w)[16], bool big) {
+    uint32_t p[4];
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
-        uint32_t a, b;
-        classify4(__byte_perm(w[2 * p], w[2 * p + 1], 0x6420), a, b);  // x = 8p, 8p+2, 8p+4, 8p+6
-        ae |= a << (4 * p);
-        be |= b << (4 * p);
-        classify4(__byte_perm(w[2 * p], w[2 * p + 1], 0x7531), a, b);  // x = 8p+1, +3, +5, +7
-        ao |= a << (4 * p);
-        bo |= b << (4 * p);
+    for (int g = 0; g < 4; ++g) {
+        uint32_t v[4] = {w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]};
+        if (big)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = statics_to_solid(v[j]);
+        p[g] = pack_piece(v[0], v[1], v[2], v[3]);
     }
-    return make_uint4(ae, ao, be, bo);
+    return pieces_to_planes(p);
 }
 
 // plane word -> the codes of its 64 cells as 16 little-endian words
 __device__ __forceinline__ void planes_to_words64(const uint4& q, uint32_t (&w)[16]) {
+    uint32_t p[4];
+    planes_to_pieces(q, p);
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
-        const uint32_t ve = (spread4((q.x >> (4 * p)) & 0xFu) << 1) | spread4((q.z >> (4 * p)) & 0xFu);
-        const uint32_t vo = (spread4((q.y >> (4 * p)) & 0xFu) << 1) | spread4((q.w >> (4 * p)) & 0xFu);
-        w[2 * p] = __byte_perm(ve, vo, 0x5140);      // x = 8p, 8p+1, 8p+2, 8p+3
-        w[2 * p + 1] = __byte_perm(ve, vo, 0x7362);  // x = 8p+4 .. 8p+7
-    }
+    for (int k = 0; k < 16; ++k) w[k] = piece_word(p[k >> 2], k & 3);
 }
 
 // Loads n (1..64) bytes from p into 16 words; cells past n read as solid (1).

@@ -41,7 +41,7 @@ namespace fs3d {
 __device__ __forceinline__ uint4 chunk_to_planes(const uint8_t* row, int X, int w, bool& big) {
     uint32_t v[16];
     load_chunk64(row + 64 * w, min(64, X - 64 * w), v, big);
-    return bytes_to_planes64(v);
+    return bytes_to_planes64(v, big);
 }
 
 __device__ __forceinline__ void planes_to_chunk(const uint4& q, const uint8_t* statics_row, uint8_t* row, int X,
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kConvBlock) k_bytes_to_planes_multi(const Conv
         uint32_t v[16];
         bool big;
         load_chunk64(staging + at.pos, at.n, v, big);
-        jb.rows[at.lu] = bytes_to_planes64(v);
+        jb.rows[at.lu] = bytes_to_planes64(v, big);
         if (big) atomicOr(flags + j, 1);  // holds a static material >= 4: keep its bytes
     }
 }

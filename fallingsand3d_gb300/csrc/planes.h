@@ -205,7 +205,6 @@ fs3d_status launch_plane_step(const PlaneWorld* worlds, const PlaneItem* items, 
 fs3d_status launch_advance_worlds(PlaneWorld* worlds, const int* meta, cudaStream_t st);
 
 // byte-grid kernels (step_bytes.cu)
-bool rows16_ok(const void* grid, int X);
 fs3d_status launch_step_bytes(uint8_t* grid, int X, int Y, int Z, uint64_t seed, uint64_t t0, int n_steps,
                               cudaStream_t st);
 fs3d_status hash_bytes_async(const uint8_t* g, int64_t n, unsigned long long* out_dev, cudaStream_t st);

@@ -1,20 +1,21 @@
 // Drop-in step on a canonical uint8 grid in device memory (FS3D-rule v1).
 //
-// Two kernels, both in place (Margolus blocks of one step are disjoint):
+// All in place (Margolus blocks of one step are disjoint):
+//  * k_step_rows: rows of at most 2048 cells in whole 16-byte pieces.  A lane
+//    owns 64 cells of each of the four rows of a block row-pair, turns them
+//    into plane words in registers, runs the shared bit-sliced row-pair step
+//    (32 blocks per 32-bit operation) and writes back the pieces that changed;
+//    k_step_ragged: the same for rows of any length and alignment, through
+//    shared memory.
+//  * k_step_rows16: longer rows of whole 16-byte pieces.
 //  * k_step_simple: one thread per 2x2x2 block, byte loads; any dims.
-//  * k_step_rows16: X % 16 == 0.  A thread owns a 16-byte chunk of x in the
-//    four rows (2 y x 2 z) of one block row-pair, loads them as uint4, checks
-//    each block for possible motion with byte-parallel tests, runs the rule
-//    only on blocks that can move and stores uint4 rows back.  In the odd
-//    phase the blocks start at odd x, so one block straddles each chunk
-//    boundary: the chunk on the left owns it, receives the neighbour's first
-//    byte through a warp shuffle and hands the updated byte back the same way;
-//    across a warp boundary the owner reads/writes that byte itself and the
-//    right-hand thread stores only bytes 1..15.  Every cell is read for
-//    computation and written by exactly one thread, so there is no race.
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "fs3d_common.h"
+#include "planes.h"
+#include "bulk_device.cuh"
 #include "conv_device.cuh"
 #include "rule_device.cuh"
 
@@ -50,7 +51,17 @@ __global__ void k_step_simple(uint8_t* __restrict__ grid, int X, int Y, int Z, i
 }
 
 // ---------------------------------------------------------------------------
-// vectorised kernel (X % 16 == 0, grid 16-byte aligned)
+// vectorised kernel for rows of more than 2048 cells (X % 16 == 0, grid 16-byte
+// aligned).  A thread owns a 16-byte chunk of x in the four rows (2 y x 2 z) of
+// one block row-pair, loads them as uint4, checks each block for possible
+// motion with byte-parallel tests, runs the rule only on blocks that can move
+// and stores uint4 rows back.  In the odd phase the blocks start at odd x, so
+// one block straddles each chunk boundary: the chunk on the left owns it,
+// receives the neighbour's first byte through a warp shuffle and hands the
+// updated byte back the same way; across a warp boundary the owner
+// reads/writes that byte itself and the right-hand thread stores only bytes
+// 1..15.  Every cell is read for computation and written by exactly one
+// thread, so there is no race.
 // ---------------------------------------------------------------------------
 struct Row16 {
     uint32_t w[4];
@@ -196,106 +207,285 @@ __global__ void __launch_bounds__(256) k_step_rows16(uint8_t* __restrict__ grid,
 }
 
 // ---------------------------------------------------------------------------
-// bit-sliced byte kernel (X % 64 == 0, X <= 2048, grid 16-byte aligned)
-//
-// A lane owns 64 cells of each of the four rows of a block row-pair (16 uint4
-// loads), turns them into plane words in registers, runs the shared
-// bit-sliced row-pair step (32 blocks per 32-bit operation) and writes back
-// only the 16-byte pieces whose cells changed class.
+// bit-sliced byte kernel (X <= 2048)
 // ---------------------------------------------------------------------------
 
-// Merges the new class of every changed cell of one 16-byte piece u (word
-// pairs 2u, 2u+1 of a 64-cell chunk) into its bytes.  Only empty, sand and
-// water cells change, and their byte is their code (A << 1) | B.
-__device__ __forceinline__ uint4 merge_piece(uint4 v, int u, uint32_t che, uint32_t cho, const uint4& n) {
-    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+// bytes of a static material in v, as a byte mask
+__device__ __forceinline__ uint32_t static_bytes(uint32_t v) {
+    const uint32_t big = v & 0xFCFCFCFCu;
+    return (((((big & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | big) & 0x80808080u) >> 7) * 0xFFu;
+}
+
+// New bytes of a chunk (w: the cells' codes), but static materials keep their old byte.
+__device__ __forceinline__ void merge_statics(const uint32_t (&old)[16], uint32_t (&w)[16]) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int p = 2 * u + h;
-        const uint32_t ce = (che >> (4 * p)) & 0xFu, co = (cho >> (4 * p)) & 0xFu;
-        const uint32_t ve = (spread4((n.x >> (4 * p)) & 0xFu) << 1) | spread4((n.z >> (4 * p)) & 0xFu);
-        const uint32_t vo = (spread4((n.y >> (4 * p)) & 0xFu) << 1) | spread4((n.w >> (4 * p)) & 0xFu);
-        const uint32_t me = spread4(ce) * 0xFFu, mo = spread4(co) * 0xFFu;
-        const uint32_t m0 = __byte_perm(me, mo, 0x5140), m1 = __byte_perm(me, mo, 0x7362);
-        w[2 * h] = (w[2 * h] & ~m0) | (__byte_perm(ve, vo, 0x5140) & m0);
-        w[2 * h + 1] = (w[2 * h + 1] & ~m1) | (__byte_perm(ve, vo, 0x7362) & m1);
+    for (int k = 0; k < 16; ++k) {
+        const uint32_t keep = static_bytes(old[k]);
+        w[k] = (w[k] & ~keep) | (old[k] & keep);
     }
-    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// ---- rows of whole 16-byte pieces
+
+// the n cells (a multiple of 16) at p, 16-byte aligned; cells past n as solid
+__device__ __forceinline__ void load_pieces(const uint8_t* p, int n, uint32_t (&w)[16]) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        uint4 v = make_uint4(0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u);
+        if (16 * u < n) v = reinterpret_cast<const uint4*>(p)[u];
+        w[4 * u] = v.x;
+        w[4 * u + 1] = v.y;
+        w[4 * u + 2] = v.z;
+        w[4 * u + 3] = v.w;
+    }
+}
+
+__device__ __forceinline__ bool any_static(const uint32_t (&w)[16]) {
+    uint32_t any = 0;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) any |= w[k];
+    return (any & 0xFCFCFCFCu) != 0;
 }
 
 // `rev` walks the row-pairs from the top: consecutive steps alternate, so a
-// step starts on the rows the previous one touched last (still in L2).  The
-// loaded bytes are not kept across the rule (that would cost 64 registers);
-// the 16-byte pieces with changed cells are read again (L1) when merging.
-#ifndef FS3D_ROWS64_CTAS_PER_SM
-#define FS3D_ROWS64_CTAS_PER_SM 6  // register cap: 6 CTAs of 128 threads per SM (measured best)
+// step starts on the rows the previous one touched last (still in L2).
+//
+// Bound: HBM (2 B a cell).  512^3 while everything falls: 43.4 us a step (6.2
+// TB/s); 64.6 us when the conversions were byte tests and multiply-gathers,
+// whose instructions then bound it (26 M warp instructions of the logic unit,
+// two cycles each); now they are packed multiply-adds and byte transpositions.
+#ifndef FS3D_ROWS_CTAS_PER_SM
+#define FS3D_ROWS_CTAS_PER_SM 6  // register cap: 6 CTAs of 128 threads per SM (measured best)
 #endif
-__global__ void __launch_bounds__(128, FS3D_ROWS64_CTAS_PER_SM)
-    k_step_rows64(uint8_t* __restrict__ grid, int X, int Y, int Z, int o,
-                                                       uint32_t sk, int lg, int rev) {
-    const int NC = X >> 6, G = 1 << lg, per = 32 >> lg;
+__global__ void __launch_bounds__(128, FS3D_ROWS_CTAS_PER_SM)
+    k_step_rows(uint8_t* __restrict__ grid, int X, int Y, int Z, int o, uint32_t sk, int lg, int rev) {
+    const int nw = (X + 63) >> 6, G = 1 << lg, per = 32 >> lg;
     const int NBZ = nblocks(Z, o), NRP = nblocks(Y, o) * NBZ;
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
     const int warps = (gridDim.x * blockDim.x) >> 5;
-    const int n_items = (NRP + per - 1) / per;
+    const int n_items = (NRP + per - 1) / per, n = min(64, X - 64 * gl);
     for (int it0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it0 < n_items; it0 += warps) {
         const int it = rev ? n_items - 1 - it0 : it0;
         const int rp = it * per + (lane >> lg);
         const bool valid = rp < NRP;  // every lane takes part in the row-pair step
         const int j = valid ? rp / NBZ : 0, k = valid ? rp - j * NBZ : 0;
-        const uint32_t rk = rowkey(sk, (uint32_t)j, (uint32_t)k);
         const int y0 = 2 * j - o, z0 = 2 * k - o;
-        const bool has = valid && gl < NC;
+        const bool has = valid && gl < nw;
         uint4 q[4], q0[4];
-        uint4* ptr[4];
-        bool in[4];
-        // Settled-work skip: without a sand or water cell nothing can move, and
-        // a byte without bit 1 (values 0, 1, 4, 5, ...) is neither.  The test is
-        // warp-uniform, so the cells a lane borrows from its neighbour for the
-        // straddling blocks are covered too.  The loads hit L1 again below.
-        uint32_t part = 0;
+        uint8_t* ptr[4];
+        bool in[4], big[4];
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             const int y = (a < 2) ? y0 + 1 : y0, z = z0 + (a & 1);
             in[a] = has && y >= 0 && y < Y && z >= 0 && z < Z;
-            ptr[a] = reinterpret_cast<uint4*>(in[a] ? grid + ((int64_t)y * Z + z) * X + 64 * gl : grid);
-            if (in[a])
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const uint4 v = ptr[a][u];
-                    part |= v.x | v.y | v.z | v.w;
-                }
-        }
-        if (__all_sync(0xFFFFFFFFu, (part & 0x02020202u) == 0u)) continue;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
+            ptr[a] = grid + (in[a] ? ((int64_t)y * Z + z) * X + 64 * gl : 0);
+            q[a] = make_uint4(0u, 0u, 0xFFFFFFFFu, 0xFFFFFFFFu);
+            big[a] = false;
             if (in[a]) {
                 uint32_t w[16];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const uint4 v = ptr[a][u];
-                    w[4 * u] = v.x;
-                    w[4 * u + 1] = v.y;
-                    w[4 * u + 2] = v.z;
-                    w[4 * u + 3] = v.w;
-                }
-                q[a] = bytes_to_planes64(w);
-            } else {
-                q[a] = make_uint4(0u, 0u, 0xFFFFFFFFu, 0xFFFFFFFFu);
+                load_pieces(ptr[a], n, w);
+                big[a] = any_static(w);
+                q[a] = bytes_to_planes64(w, big[a]);
             }
             q0[a] = q[a];
         }
-        rowpair_core(q, has, o, rk, gl, G, NC, true);
+        // without a sand or water cell nothing moves; the test is warp-uniform,
+        // so the cells a lane borrows from its neighbour are covered too
+        if (!__any_sync(0xFFFFFFFFu, (q[0].x | q[0].y | q[1].x | q[1].y | q[2].x | q[2].y | q[3].x | q[3].y) != 0u)) continue;
+        rowpair_core(q, has, o, rowkey(sk, (uint32_t)j, (uint32_t)k), gl, G, nw, (X & 63) == 0);
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             if (!in[a]) continue;
-            const uint32_t che = (q[a].x ^ q0[a].x) | (q[a].z ^ q0[a].z);
-            const uint32_t cho = (q[a].y ^ q0[a].y) | (q[a].w ^ q0[a].w);
-            if (!(che | cho)) continue;
+            // bit m: cell 2m or 2m + 1 changed; piece u holds bits 8u .. 8u + 7
+            const uint32_t ch = (q[a].x ^ q0[a].x) | (q[a].z ^ q0[a].z) | (q[a].y ^ q0[a].y) | (q[a].w ^ q0[a].w);
+            if (!ch) continue;
+            uint32_t w[16];
+            planes_to_words64(q[a], w);
+            if (big[a]) {
+                uint32_t old[16];
+                load_pieces(ptr[a], n, old);
+                merge_statics(old, w);
+            }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                if (((che | cho) >> (8 * u)) & 0xFFu) ptr[a][u] = merge_piece(ptr[a][u], u, che, cho, q[a]);
+                if ((ch >> (8 * u)) & 0xFFu)
+                    reinterpret_cast<uint4*>(ptr[a])[u] = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
         }
+    }
+}
+
+// ---- rows of any length and alignment
+//
+// A warp takes consecutive row-pairs along z of one block layer: their rows in
+// one y layer are one span of bytes, so the two spans come in (and go back,
+// when a cell changed) as coalesced 16-byte pieces, with single bytes at their
+// ends, and lie in shared memory between; every byte of them belongs to this
+// warp alone in this step.  A lane reads its 64 cells there as words shifted
+// to its row's alignment.  (Words straight from global memory, 64 bytes apart
+// from lane to lane, took 15 us a step on 75x61x93; one thread per block 7.0.)
+constexpr int kSpanBytes = 4096 + 16;  // 2 * (32 >> lg) rows of at most 64 << lg cells, at any alignment
+
+// [g, g + n) between global memory and shared memory at sm, which is congruent
+// to g modulo 16; by T threads (id: which of them)
+template <bool STORE, int T>
+__device__ __forceinline__ void move_span(uint8_t* g, uint8_t* sm, int n, int id) {
+    const int head = (int)(-(intptr_t)reinterpret_cast<uintptr_t>(g) & 15);
+    const int h = head < n ? head : n, body = (n - h) & ~15, t = h + body;
+    const int i0 = id < h ? id : (id >= 16 && t + id - 16 < n ? t + id - 16 : -1);  // a single byte at either end
+    if (i0 >= 0) {
+        if (STORE) g[i0] = sm[i0];
+        else sm[i0] = g[i0];
+    }
+    for (int i = h + 16 * id; i < t; i += 16 * T) {
+        if (STORE) *reinterpret_cast<uint4*>(g + i) = *reinterpret_cast<const uint4*>(sm + i);
+        else *reinterpret_cast<uint4*>(sm + i) = *reinterpret_cast<const uint4*>(g + i);
+    }
+}
+
+// the n cells at shared-memory address p, cells past n as solid
+__device__ __forceinline__ void read_cells(const uint8_t* p, int n, uint32_t (&w)[16]) {
+    const uint32_t m = smem_u32(p) & 3u;
+    const uint32_t* pa = reinterpret_cast<const uint32_t*>(p - m);
+    uint32_t lo = pa[0];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const int left = n - 4 * k;  // cells of the row from this word on
+        uint32_t hi = 0;
+        if (left + (int)m > 4) hi = pa[k + 1];
+        w[k] = __funnelshift_r(lo, hi, 8 * m);
+        lo = hi;
+        if (left < 4) {
+            const uint32_t keep = left <= 0 ? 0u : (1u << (8 * left)) - 1u;
+            w[k] = (w[k] & keep) | (0x01010101u & ~keep);
+        }
+    }
+}
+
+// The first n of 64 cells (w) to shared-memory address p: aligned words whole,
+// the chunk's ends byte by byte (a word there may hold another lane's cells).
+__device__ __forceinline__ void write_cells(uint8_t* p, int n, const uint32_t (&w)[16]) {
+    const int m = (int)(smem_u32(p) & 3u);
+    uint32_t tail = 0;  // the word with the chunk's last cells
+#pragma unroll
+    for (int i = 0; i <= 16; ++i) {
+        const uint32_t before = i > 0 ? w[i - 1] : 0u, now = i < 16 ? w[i] : 0u;
+        const uint32_t word = m ? __funnelshift_r(before, now, 8 * (4 - m)) : now;
+        const int at = 4 * i - m;
+        if (at >= 0 && at + 4 <= n) *reinterpret_cast<uint32_t*>(p + at) = word;
+        else if (at < n && at > 0) tail = word;
+    }
+    const int e = (n + m) & ~3;  // offset (from p - m) of the word holding the last cells
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        if (c >= m && m && c - m < n) p[c - m] = (uint8_t)(w[0] >> (8 * (c - m)));
+        if (e > 0 && e - m + c < n) p[e - m + c] = (uint8_t)(tail >> (8 * c));
+        if (e == 0 && !m && c < n) p[c] = (uint8_t)(w[0] >> (8 * c));
+    }
+}
+
+// The row loops are not unrolled, with the planes in shared memory between: a
+// small world's launch runs each instruction once per SM, and fetching 3000
+// straight-line instructions took 14 us a step.  SPLIT: four warps share an
+// item, each converting one row of every pair (the rule is one warp's), for
+// worlds of fewer items than warps that could run: 75x61x93 11 us a step with
+// a warp an item.
+struct RaggedItem {
+    uint8_t span[2][kSpanBytes];
+    uint4 planes[4][32];
+    uint32_t ch[4][32];  // bit m: cell 2m or 2m + 1 of the lane's row changed
+    uint8_t big[4][32];  // the lane's row holds a static material
+};
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(128, 5)
+    k_step_ragged(uint8_t* __restrict__ grid, int X, int Y, int Z, int o, uint32_t sk, int lg) {
+    constexpr int T = SPLIT ? 128 : 32;  // threads of an item
+    __shared__ __align__(16) RaggedItem items[SPLIT ? 1 : 4];
+    const int nw = (X + 63) >> 6, G = 1 << lg, per = 32 >> lg;
+    const int NBY = nblocks(Y, o), NBZ = nblocks(Z, o), chunks = (NBZ + per - 1) / per;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), n = min(64, X - 64 * gl), id = threadIdx.x & (T - 1);
+    const int takers = gridDim.x * (128 / T), n_items = NBY * chunks;
+    RaggedItem& W = items[threadIdx.x / T];
+    auto sync = [] {
+        if (SPLIT) __syncthreads();
+        else __syncwarp();
+    };
+    for (int it = (int)((blockIdx.x * 128u + threadIdx.x) / T); it < n_items; it += takers) {
+        const int j = it / chunks, k0 = (it - j * chunks) * per, k = k0 + (lane >> lg);
+        const int y0 = 2 * j - o, z0 = 2 * k - o;
+        const int zs = max(2 * k0 - o, 0), ze = min(2 * (k0 + per) - o, Z);  // the item's rows
+        const int bytes = (ze - zs) * X;
+        auto layer_in = [&](int l) { return y0 + l >= 0 && y0 + l < Y; };
+        auto layer = [&](int l) { return grid + ((int64_t)(y0 + l) * Z + zs) * X; };
+        // where the layer's span lies in shared memory: congruent to its address modulo 16
+        auto held = [&](int l) { return W.span[l] + (reinterpret_cast<uintptr_t>(layer(l)) & 15u); };
+#pragma unroll
+        for (int l = 0; l < 2; ++l)
+            if (layer_in(l)) move_span<false, T>(layer(l), held(l), bytes, id);
+        sync();
+        const bool has = k < NBZ && gl < nw;
+        // row a of the pair: y0 + 1 for a < 2, z0 + (a & 1)
+        auto row_in = [&](int a) {
+            const int z = z0 + (a & 1);
+            return has && layer_in(a < 2 ? 1 : 0) && z >= 0 && z < Z;
+        };
+        auto row = [&](int a) { return held(a < 2 ? 1 : 0) + (z0 + (a & 1) - zs) * X + 64 * gl; };
+        bool part = false;
+#pragma unroll 1
+        for (int a = id >> 5; a < 4; a += T / 32) {
+            uint4 v = make_uint4(0u, 0u, 0xFFFFFFFFu, 0xFFFFFFFFu);
+            bool b = false;
+            if (row_in(a)) {
+                uint32_t w[16];
+                read_cells(row(a), n, w);
+                b = any_static(w);
+                v = bytes_to_planes64(w, b);
+            }
+            part = part || (v.x | v.y) != 0u;
+            W.planes[a][lane] = v;
+            W.big[a][lane] = b;
+        }
+        // without a sand or water cell nothing moves
+        const bool some = SPLIT ? __syncthreads_or(part) != 0 : __any_sync(0xFFFFFFFFu, part) != 0;
+        bool any = false;
+        if (some) {
+            if (id < 32) {
+                uint4 q[4];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) q[a] = W.planes[a][lane];
+                rowpair_core(q, has, o, rowkey(sk, (uint32_t)j, (uint32_t)k), gl, G, nw, (X & 63) == 0);
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    const uint4 q0 = W.planes[a][lane];
+                    W.planes[a][lane] = q[a];
+                    W.ch[a][lane] = (q[a].x ^ q0.x) | (q[a].z ^ q0.z) | (q[a].y ^ q0.y) | (q[a].w ^ q0.w);
+                }
+            }
+            sync();
+#pragma unroll 1
+            for (int a = id >> 5; a < 4; a += T / 32) {
+                if (!row_in(a) || !W.ch[a][lane]) continue;
+                any = true;
+                uint8_t* p = row(a);
+                uint32_t w[16];
+                planes_to_words64(W.planes[a][lane], w);
+                if (W.big[a][lane]) {
+                    uint32_t old[16];
+                    read_cells(p, n, old);
+                    merge_statics(old, w);
+                }
+                write_cells(p, n, w);
+            }
+            // (and every thread's bytes are in place)
+            any = SPLIT ? __syncthreads_or(any) != 0 : __any_sync(0xFFFFFFFFu, any) != 0;
+            if (!SPLIT) __syncwarp();
+            if (any) {
+#pragma unroll
+                for (int l = 0; l < 2; ++l)
+                    if (layer_in(l)) move_span<true, T>(layer(l), held(l), bytes, id);
+            }
+        }
+        sync();
     }
 }
 
@@ -344,30 +534,27 @@ static int sm_count() {
     return n;
 }
 
+fs3d_status launch_step_simple(uint8_t* grid, int X, int Y, int Z, uint64_t seed, uint64_t t0, int n_steps,
+                               cudaStream_t st);
+
 static int grid_for(int64_t work, int threads, int per_sm) {
     const int64_t need = (work + threads - 1) / threads;
     const int64_t cap = (int64_t)sm_count() * per_sm;
     return (int)(need < cap ? (need > 0 ? need : 1) : cap);
 }
 
-bool rows16_ok(const void* grid, int X) {
+// rows of whole 16-byte pieces
+static bool rows_aligned(const void* grid, int X) {
     return (X % 16) == 0 && (reinterpret_cast<uintptr_t>(grid) & 15u) == 0;
 }
 
-bool rows64_ok(const void* grid, int X) {
-    return (X % 64) == 0 && X <= 2048 && (reinterpret_cast<uintptr_t>(grid) & 15u) == 0;
-}
+// most items per SM that k_step_ragged splits over four warps each (one wave of CTAs)
+constexpr int kSplitItemsPerSm = 4;
 
-static int rows64_lg(int X) {
-    int lg = 0;
-    while ((1 << lg) < (X >> 6)) ++lg;
-    return lg;
-}
-
-static int rows64_ctas_per_sm() {
+static int rows_ctas_per_sm() {
     static const int n = [] {
         int v = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_step_rows64, 128, 0) != cudaSuccess || v < 1) v = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_step_rows, 128, 0) != cudaSuccess || v < 1) v = 1;
         return v;
     }();
     return n;
@@ -375,22 +562,34 @@ static int rows64_ctas_per_sm() {
 
 fs3d_status launch_step_bytes(uint8_t* grid, int X, int Y, int Z, uint64_t seed, uint64_t t0, int n_steps,
                               cudaStream_t st) {
+    const bool a16 = rows_aligned(grid, X);
+    // rows longer than a warp's 32 words, or more row-pairs than an int counts
+    const bool wide = X > kPlaneMaxX || (int64_t)nblocks(Y, 1) * nblocks(Z, 1) >= (int64_t)1 << 30;
+    if (wide && !a16) return launch_step_simple(grid, X, Y, Z, seed, t0, n_steps, st);
+    if (wide) {
+        for (int a = 0; a < n_steps; ++a) {
+            const uint64_t t = t0 + (uint64_t)a;
+            const int o = (int)(t & 1u);
+            const int64_t units = (int64_t)(X >> 4) * nblocks(Y, o) * nblocks(Z, o);
+            k_step_rows16<<<grid_for(units, 256, 8), 256, 0, st>>>(grid, X, Y, Z, o, stepkey(seed, t));
+            FS3D_CHECK_LAUNCH("step kernel launch");
+        }
+        return FS3D_OK;
+    }
+    const int lg = plane_lg(plane_nw(X)), per = 32 >> lg;
     for (int a = 0; a < n_steps; ++a) {
         const uint64_t t = t0 + (uint64_t)a;
         const int o = (int)(t & 1u);
-        const uint32_t sk = stepkey(seed, t);
-        if (rows64_ok(grid, X)) {
-            const int lg = rows64_lg(X);
-            const int per = 32 >> lg;
+        if (a16) {
             const int64_t items = ((int64_t)nblocks(Y, o) * nblocks(Z, o) + per - 1) / per;
-            k_step_rows64<<<grid_for(items * 32, 128, rows64_ctas_per_sm()), 128, 0, st>>>(grid, X, Y, Z, o, sk,
-                                                                                          lg, (int)(a & 1));
-        } else if (rows16_ok(grid, X)) {
-            const int64_t units = (int64_t)(X >> 4) * nblocks(Y, o) * nblocks(Z, o);
-            k_step_rows16<<<grid_for(units, 256, 8), 256, 0, st>>>(grid, X, Y, Z, o, sk);
+            k_step_rows<<<grid_for(items * 32, 128, rows_ctas_per_sm()), 128, 0, st>>>(grid, X, Y, Z, o, stepkey(seed, t),
+                                                                                       lg, (int)(a & 1));
         } else {
-            const int64_t nb = (int64_t)nblocks(X, o) * nblocks(Y, o) * nblocks(Z, o);
-            k_step_simple<<<grid_for(nb, 256, 8), 256, 0, st>>>(grid, X, Y, Z, o, sk);
+            const int64_t items = (int64_t)nblocks(Y, o) * ((nblocks(Z, o) + per - 1) / per);
+            if (items <= (int64_t)sm_count() * kSplitItemsPerSm)
+                k_step_ragged<true><<<(unsigned)items, 128, 0, st>>>(grid, X, Y, Z, o, stepkey(seed, t), lg);
+            else
+                k_step_ragged<false><<<grid_for(items * 32, 128, 5), 128, 0, st>>>(grid, X, Y, Z, o, stepkey(seed, t), lg);
         }
         FS3D_CHECK_LAUNCH("step kernel launch");
     }
