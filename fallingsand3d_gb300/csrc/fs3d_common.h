@@ -66,6 +66,31 @@ void note_launch(uint64_t n = 1);
 // in another (after cudaDeviceReset, for example).
 bool current_context_id(unsigned long long* id);
 
+// ---- chained launches: a kernel that begins with chain_wait() may be launched
+// with launch_chained(), so that its CTAs are placed and its first instructions
+// fetched while the kernel before it in the stream still runs (programmatic
+// dependent launch).  chain_wait() returns once that kernel has run and its
+// writes are visible; nothing in global memory may be touched before it.
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+cudaError_t launch_chained(void (*fn)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(block);
+    lc.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, fn, static_cast<P>(args)...);
+}
+#endif
+
 }  // namespace fs3d
 
 #define FS3D_CUDA(call)                                              \

@@ -387,6 +387,7 @@ __device__ __forceinline__ bool rows_changed_recently(const uint8_t* __restrict_
 // 118 us per step against 133 us, 123 us at four CTAs)
 __global__ void __launch_bounds__(256, 3) k_plane_step_skip(const PlaneWorld w, uint8_t* __restrict__ rflags,
                                                         int* counts) {
+    chain_wait();
     const uint64_t t = w.t;
     const int o = (int)(t & 1u);
     const int lane = threadIdx.x & 31;
@@ -1311,8 +1312,9 @@ fs3d_status launch_plane_step_skip(const PlaneWorld& w, uint8_t* rflags, int* co
     const int64_t need = ((nrp + per - 1) / per + 7) / 8;  // eight warps per CTA
     const int64_t cap = (int64_t)sm_count_public() * per_sm;
     const int grid = (int)(need < 1 ? 1 : (need < cap ? need : cap));
-    k_plane_step_skip<<<grid, 256, 0, st>>>(w, rflags, counts);
-    FS3D_CHECK_LAUNCH("plane step (settled skip) launch");
+    const cudaError_t e = launch_chained(k_plane_step_skip, (unsigned)grid, 256, st, w, rflags, counts);
+    if (e != cudaSuccess) return cuda_fail(e, "plane step (settled skip) launch");
+    note_launch();
     return FS3D_OK;
 }
 

@@ -259,6 +259,7 @@ __device__ __forceinline__ bool any_static(const uint32_t (&w)[16]) {
 #endif
 __global__ void __launch_bounds__(128, FS3D_ROWS_CTAS_PER_SM)
     k_step_rows(uint8_t* __restrict__ grid, int X, int Y, int Z, int o, uint32_t sk, int lg, int rev) {
+    chain_wait();
     const int nw = (X + 63) >> 6, G = 1 << lg, per = 32 >> lg;
     const int NBZ = nblocks(Z, o), NRP = nblocks(Y, o) * NBZ;
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
@@ -399,6 +400,7 @@ struct RaggedItem {
 template <bool SPLIT>
 __global__ void __launch_bounds__(128, 5)
     k_step_ragged(uint8_t* __restrict__ grid, int X, int Y, int Z, int o, uint32_t sk, int lg) {
+    chain_wait();
     constexpr int T = SPLIT ? 128 : 32;  // threads of an item
     __shared__ __align__(16) RaggedItem items[SPLIT ? 1 : 4];
     const int nw = (X + 63) >> 6, G = 1 << lg, per = 32 >> lg;
@@ -580,18 +582,21 @@ fs3d_status launch_step_bytes(uint8_t* grid, int X, int Y, int Z, uint64_t seed,
     for (int a = 0; a < n_steps; ++a) {
         const uint64_t t = t0 + (uint64_t)a;
         const int o = (int)(t & 1u);
+        cudaError_t e;
         if (a16) {
             const int64_t items = ((int64_t)nblocks(Y, o) * nblocks(Z, o) + per - 1) / per;
-            k_step_rows<<<grid_for(items * 32, 128, rows_ctas_per_sm()), 128, 0, st>>>(grid, X, Y, Z, o, stepkey(seed, t),
-                                                                                       lg, (int)(a & 1));
+            e = launch_chained(k_step_rows, grid_for(items * 32, 128, rows_ctas_per_sm()), 128, st, grid, X, Y, Z, o,
+                               stepkey(seed, t), lg, a & 1);
         } else {
             const int64_t items = (int64_t)nblocks(Y, o) * ((nblocks(Z, o) + per - 1) / per);
             if (items <= (int64_t)sm_count() * kSplitItemsPerSm)
-                k_step_ragged<true><<<(unsigned)items, 128, 0, st>>>(grid, X, Y, Z, o, stepkey(seed, t), lg);
+                e = launch_chained(k_step_ragged<true>, (unsigned)items, 128, st, grid, X, Y, Z, o, stepkey(seed, t), lg);
             else
-                k_step_ragged<false><<<grid_for(items * 32, 128, 5), 128, 0, st>>>(grid, X, Y, Z, o, stepkey(seed, t), lg);
+                e = launch_chained(k_step_ragged<false>, grid_for(items * 32, 128, 5), 128, st, grid, X, Y, Z, o,
+                                   stepkey(seed, t), lg);
         }
-        FS3D_CHECK_LAUNCH("step kernel launch");
+        if (e != cudaSuccess) return cuda_fail(e, "step kernel launch");
+        note_launch();
     }
     return FS3D_OK;
 }
