@@ -1132,33 +1132,30 @@ fs3d_status admit_many_impl(fs3d_batch* b, int n, const fs3d_world_spec* specs, 
     if (!pa.flags) return set_error(FS3D_ERR_CUDA, "fs3d_batch_admit_many: page-locked flag buffer");
     // one staging buffer, one copy per run of contiguous grids, one conversion launch for all
     std::vector<ConvJob> jobs((size_t)k);
-    std::vector<int64_t> unit_off((size_t)k);
     std::vector<uint4*> rows((size_t)k, nullptr);
-    int64_t bytes_total = 0, units = 0;
+    int64_t bytes_total = 0, blocks = 0;
     for (int a = 0; a < k; ++a) {
         const fs3d_world_spec& p = specs[a];
         ConvJob& j = jobs[(size_t)a];
         j.statics = nullptr;
         j.static_flag = nullptr;
         j.static_src = nullptr;
-        j.byte_off = bytes_total;
         j.X = p.X;
         j.Y = p.Y;
         j.Z = p.Z;
         j.nw = plane_nw(p.X);
-        unit_off[(size_t)a] = units;
         pa.tickets.push_back(0);
         pa.byte_off.push_back(bytes_total);
         pa.cells.push_back((int64_t)p.X * p.Y * p.Z);
         bytes_total += ((int64_t)p.X * p.Y * p.Z + 15) / 16 * 16;
-        units += (int64_t)p.Y * p.Z * j.nw;
+        blocks += conv_blocks(p.Y, p.Z, j.nw, kConvChunks);
     }
-    const size_t jobs_bytes = sizeof(ConvJob) * (size_t)k, off_bytes = sizeof(int64_t) * (size_t)k;
-    const size_t flags_off = (jobs_bytes + off_bytes + 15) / 16 * 16;
+    const size_t jobs_bytes = sizeof(ConvJob) * (size_t)k;
+    const size_t flags_off = (jobs_bytes + 15) / 16 * 16;
     const size_t copy_off = (flags_off + sizeof(int) * (size_t)k + 15) / 16 * 16;
     const size_t copy_bytes = sizeof(CopyJob) * (size_t)k + sizeof(int64_t) * (size_t)k;
-    const size_t bj_off = (copy_off + copy_bytes + 15) / 16 * 16;  // the conversion's job of each unit block
-    const size_t table_bytes = bj_off + sizeof(int) * (size_t)conv_blocks(units);
+    const size_t bj_off = (copy_off + copy_bytes + 15) / 16 * 16;  // the conversion's blocks
+    const size_t table_bytes = bj_off + sizeof(ConvBlock) * (size_t)blocks;
     // the grid uploads run on their own stream: the next admission's upload
     // does not wait for this one's conversion (which waits for free SMs)
     cudaStream_t up = b->upload;
@@ -1213,16 +1210,15 @@ fs3d_status admit_many_impl(fs3d_batch* b, int n, const fs3d_world_spec* specs, 
             const int64_t c_prev = (int64_t)specs[e_run - 1].X * specs[e_run - 1].Y * specs[e_run - 1].Z;
             const uintptr_t g = reinterpret_cast<uintptr_t>(specs[e_run].grid);
             if (specs[e_run].grid != specs[e_run - 1].grid + c_prev ||
-                run_bytes != jobs[(size_t)e_run].byte_off - jobs[(size_t)a].byte_off || g + (uintptr_t)c > rs + rn)
+                run_bytes != pa.byte_off[(size_t)e_run] - pa.byte_off[(size_t)a] || g + (uintptr_t)c > rs + rn)
                 break;
             run_bytes += c;
             ++e_run;
         }
         if (!dv || e_run - a > 1) {
-            e = cudaMemcpyAsync(staging + jobs[(size_t)a].byte_off, specs[a].grid, (size_t)run_bytes, cudaMemcpyDefault,
-                                up);
+            e = cudaMemcpyAsync(staging + pa.byte_off[(size_t)a], specs[a].grid, (size_t)run_bytes, cudaMemcpyDefault, up);
         } else {
-            copies.push_back(CopyJob{dv, staging + jobs[(size_t)a].byte_off, cells});
+            copies.push_back(CopyJob{dv, staging + pa.byte_off[(size_t)a], cells});
             chunk_off.push_back(chunks);
             chunks += (cells + 15) / 16;
         }
@@ -1232,6 +1228,7 @@ fs3d_status admit_many_impl(fs3d_batch* b, int n, const fs3d_world_spec* specs, 
     for (int a = 0; a < k; ++a) {
         ConvJob& j = jobs[(size_t)a];
         j.rows = rows[(size_t)a];
+        j.bytes = staging + pa.byte_off[(size_t)a];
         j.lflags = reinterpret_cast<uint8_t*>(j.rows) + plane_bytes(j.X, j.Y, j.Z);
         j.t0b = (uint32_t)specs[a].start_step & 0xFFu;
         max_Y = std::max(max_Y, j.Y);
@@ -1245,7 +1242,6 @@ fs3d_status admit_many_impl(fs3d_batch* b, int n, const fs3d_world_spec* specs, 
         if (uploaded) cudaEventDestroy(uploaded);
     }
     ConvJob* jobs_dev = static_cast<ConvJob*>(pa.table);
-    int64_t* off_dev = reinterpret_cast<int64_t*>(static_cast<char*>(pa.table) + jobs_bytes);
     int* flags_dev = reinterpret_cast<int*>(static_cast<char*>(pa.table) + flags_off);
     pa.flags_dev = flags_dev;
     CopyJob* copies_dev = reinterpret_cast<CopyJob*>(static_cast<char*>(pa.table) + copy_off);
@@ -1260,20 +1256,20 @@ fs3d_status admit_many_impl(fs3d_batch* b, int n, const fs3d_world_spec* specs, 
         } else {
             char* h = b->host_chunks[(size_t)ci].p;
             memcpy(h, jobs.data(), jobs_bytes);
-            memcpy(h + jobs_bytes, unit_off.data(), off_bytes);
             memset(h + flags_off, 0, copy_off - flags_off);
             if (!copies.empty()) {
                 memcpy(h + copy_off, copies.data(), sizeof(CopyJob) * copies.size());
                 memcpy(h + copy_off + sizeof(CopyJob) * (size_t)k, chunk_off.data(), sizeof(int64_t) * chunk_off.size());
             }
-            conv_block_jobs(unit_off.data(), k, units, reinterpret_cast<int*>(h + bj_off));
+            ConvBlock* hb = reinterpret_cast<ConvBlock*>(h + bj_off);
+            for (int a = 0; a < k; ++a) hb += conv_fill_blocks(a, specs[a].Y, specs[a].Z, jobs[(size_t)a].nw, kConvChunks, hb);
             e = upload_chunk(b, ci, pa.table, image, b->side);
         }
     }
     if (e != cudaSuccess) s = cuda_fail(e, "fs3d_batch_admit_many upload");
     if (s == FS3D_OK) s = copy_many(copies_dev, chunk_dev, (int)copies.size(), chunks, b->side);
-    const int* bj_dev = reinterpret_cast<const int*>(static_cast<char*>(pa.table) + bj_off);
-    if (s == FS3D_OK) s = planes_from_bytes_multi(jobs_dev, off_dev, bj_dev, k, units, staging, flags_dev, b->side);
+    const ConvBlock* bj_dev = reinterpret_cast<const ConvBlock*>(static_cast<char*>(pa.table) + bj_off);
+    if (s == FS3D_OK) s = planes_from_bytes_multi(jobs_dev, bj_dev, blocks, flags_dev, b->side);
     // layer flags from the cells: the first two steps evaluate only the row-pairs that can change
     if (s == FS3D_OK) s = layer_flags_from_cells_multi(jobs_dev, k, max_Y, b->side);
     // segments may start once the planes are written
@@ -1409,10 +1405,27 @@ fs3d_status retire_many_impl(fs3d_batch* b, int n, const uint64_t* tickets, uint
     std::shared_ptr<CUevent_st> copied;  // recorded after the copy kernel (download stream), if one ran
     fs3d_batch::StagingSlot* rb_slot = nullptr;  // the read-back's staging buffer
     if (grids_out) {
+        // outputs in this device's memory are written by the conversion itself;
+        // the others go through the staging bytes (in call order, so that
+        // outputs lying back to back stay so there)
         std::vector<ConvJob> jobs;
-        std::vector<int64_t> unit_off;
+        std::vector<int64_t> byte_off;  // in the staging bytes; -1: converted in place
         std::vector<int> who;
-        int64_t bytes_total = 0, units = 0;
+        int64_t bytes_total = 0, blocks = 0;
+        // (the last allocation that held an output, so that one lookup serves a buffer of many)
+        uintptr_t local_lo = 1, local_hi = 0;
+        auto local = [&](const uint8_t* p, int64_t n) {
+            const uintptr_t u = reinterpret_cast<uintptr_t>(p);
+            if (u >= local_lo && u + (uintptr_t)n <= local_hi) return true;
+            uintptr_t rs = 0;
+            size_t rn = 0;
+            if (!device_local(p)) return false;
+            if (alloc_range(p, &rs, &rn)) {
+                local_lo = rs;
+                local_hi = rs + rn;
+            }
+            return true;
+        };
         for (int a = 0; a < n; ++a) {
             if (!grids_out[a]) continue;
             const BWorld& w = its[(size_t)a]->second;
@@ -1427,29 +1440,35 @@ fs3d_status retire_many_impl(fs3d_batch* b, int n, const uint64_t* tickets, uint
                     j.static_src = pa->staging + pa->byte_off[(size_t)w.admit_index];
                     if (std::find(readers.begin(), readers.end(), pa) == readers.end()) readers.push_back(pa);
                 }
-            j.byte_off = bytes_total;
             j.X = w.X;
             j.Y = w.Y;
             j.Z = w.Z;
             j.nw = w.nw;
+            j.magic = conv_magic(w.X);
+            const int64_t cells = (int64_t)w.X * w.Y * w.Z;
+            const bool direct = local(grids_out[a], cells);
+            j.bytes = direct ? grids_out[a] : nullptr;
             jobs.push_back(j);
-            unit_off.push_back(units);
+            byte_off.push_back(direct ? -1 : bytes_total);
             who.push_back(a);
-            bytes_total += ((int64_t)w.X * w.Y * w.Z + 15) / 16 * 16;
-            units += (int64_t)w.Y * w.Z * w.nw;
+            if (!direct) bytes_total += (cells + 15) / 16 * 16;
+            blocks += conv_blocks(w.Y, w.Z, w.nw, kConvChunksBack);
         }
         const int k = (int)jobs.size();
         if (k) {
             const size_t jobs_bytes = sizeof(ConvJob) * (size_t)k;
-            const size_t copy_off = (jobs_bytes + sizeof(int64_t) * (size_t)k + 15) / 16 * 16;
+            const size_t copy_off = (jobs_bytes + 15) / 16 * 16;
             const size_t bj_off = (copy_off + (sizeof(CopyJob) + sizeof(int64_t)) * (size_t)k + 15) / 16 * 16;
-            const size_t table_bytes = bj_off + sizeof(int) * (size_t)conv_blocks(units);
+            const size_t table_bytes = bj_off + sizeof(ConvBlock) * (size_t)blocks;
             cudaError_t e = cudaSuccess;
-            rb_slot = take_slot(b->rb_ring, b->rb_turn, (size_t)bytes_total, rb, &e);
-            staging = rb_slot->p;
+            if (bytes_total > 0) {
+                rb_slot = take_slot(b->rb_ring, b->rb_turn, (size_t)bytes_total, rb, &e);
+                staging = rb_slot->p;
+                for (int q = 0; q < k; ++q)
+                    if (byte_off[(size_t)q] >= 0) jobs[(size_t)q].bytes = staging + byte_off[(size_t)q];
+            }
             if (e == cudaSuccess) e = stream_alloc(&table, table_bytes, rb);
             ConvJob* jobs_dev = static_cast<ConvJob*>(table);
-            int64_t* off_dev = reinterpret_cast<int64_t*>(static_cast<char*>(table) + jobs_bytes);
             // the copy jobs are only known below: the table goes up in one
             // page-locked image once they are
             if (e != cudaSuccess) s = cuda_fail(e, "fs3d_batch_retire_many upload");
@@ -1462,17 +1481,24 @@ fs3d_status retire_many_impl(fs3d_batch* b, int n, const uint64_t* tickets, uint
             char* h = ci >= 0 ? b->host_chunks[(size_t)ci].p : nullptr;
             if (h) {
                 memcpy(h, jobs.data(), jobs_bytes);
-                memcpy(h + jobs_bytes, unit_off.data(), sizeof(int64_t) * (size_t)k);
-                conv_block_jobs(unit_off.data(), k, units, reinterpret_cast<int*>(h + bj_off));
+                ConvBlock* hb = reinterpret_cast<ConvBlock*>(h + bj_off);
+                for (int q = 0; q < k; ++q) {
+                    const ConvJob& j = jobs[(size_t)q];
+                    hb += conv_fill_blocks(q, j.Y, j.Z, j.nw, kConvChunksBack, hb);
+                }
             }
             std::vector<CopyJob> copies;
             std::vector<int64_t> chunk_off;
             int64_t chunks = 0;
             std::vector<std::pair<int, int64_t>> runs;  // (first job, bytes) of each copy-engine run
-            // outputs the device can address are written by one copy kernel,
-            // pageable ones take a copy call each; outputs lying back to back
-            // go back in one copy-engine transfer per run
+            // other outputs the device can address are written by one copy
+            // kernel, pageable ones take a copy call each; outputs lying back to
+            // back go back in one copy-engine transfer per run
             for (int q = 0; q < k && s == FS3D_OK;) {
+                if (byte_off[(size_t)q] < 0) {
+                    ++q;
+                    continue;
+                }
                 uint8_t* out = grids_out[who[(size_t)q]];
                 const BWorld& w = its[(size_t)who[(size_t)q]]->second;
                 const int64_t cells = (int64_t)w.X * w.Y * w.Z;
@@ -1482,7 +1508,7 @@ fs3d_status retire_many_impl(fs3d_batch* b, int n, const uint64_t* tickets, uint
                 uintptr_t rs = 0;
                 size_t rn = 0;
                 const bool ranged = dv && alloc_range(out, &rs, &rn);
-                while (ranged && e_run < k) {
+                while (ranged && e_run < k && byte_off[(size_t)e_run] >= 0) {
                     const BWorld& w2 = its[(size_t)who[(size_t)e_run]]->second;
                     const BWorld& w1 = its[(size_t)who[(size_t)e_run - 1]]->second;
                     // back to back in both, with no staging padding in between
@@ -1492,7 +1518,7 @@ fs3d_status retire_many_impl(fs3d_batch* b, int n, const uint64_t* tickets, uint
                     const int64_t c1 = (int64_t)w1.X * w1.Y * w1.Z;
                     const uintptr_t g = reinterpret_cast<uintptr_t>(grids_out[who[(size_t)e_run]]);
                     if (grids_out[who[(size_t)e_run]] != grids_out[who[(size_t)e_run - 1]] + c1 ||
-                        run_bytes != jobs[(size_t)e_run].byte_off - jobs[(size_t)q].byte_off ||
+                        run_bytes != byte_off[(size_t)e_run] - byte_off[(size_t)q] ||
                         g + (uintptr_t)((int64_t)w2.X * w2.Y * w2.Z) > rs + rn)
                         break;
                     run_bytes += (int64_t)w2.X * w2.Y * w2.Z;
@@ -1501,7 +1527,7 @@ fs3d_status retire_many_impl(fs3d_batch* b, int n, const uint64_t* tickets, uint
                 if (!dv || e_run - q > 1) {
                     runs.emplace_back(q, run_bytes);
                 } else {
-                    copies.push_back(CopyJob{staging + jobs[(size_t)q].byte_off, dv, cells});
+                    copies.push_back(CopyJob{staging + byte_off[(size_t)q], dv, cells});
                     chunk_off.push_back(chunks);
                     chunks += (cells + 15) / 16;
                 }
@@ -1518,8 +1544,8 @@ fs3d_status retire_many_impl(fs3d_batch* b, int n, const uint64_t* tickets, uint
                 e = upload_chunk(b, ci, table, image, rb);
                 if (e != cudaSuccess) s = cuda_fail(e, "fs3d_batch_retire_many upload");
             }
-            const int* bj_dev = reinterpret_cast<const int*>(static_cast<char*>(table) + bj_off);
-            if (s == FS3D_OK) s = planes_to_bytes_multi(jobs_dev, off_dev, bj_dev, k, units, staging, rb);
+            const ConvBlock* bj_dev = reinterpret_cast<const ConvBlock*>(static_cast<char*>(table) + bj_off);
+            if (s == FS3D_OK) s = planes_to_bytes_multi(jobs_dev, bj_dev, blocks, rb);
             if (s == FS3D_OK) read = record_read(rb);
             // the downloads run on their own stream: the next read-back's
             // conversion does not wait for this one's copies over the host link
@@ -1530,7 +1556,7 @@ fs3d_status retire_many_impl(fs3d_batch* b, int n, const uint64_t* tickets, uint
             cudaStream_t dl = b->download;
             for (size_t r = 0; r < runs.size() && s == FS3D_OK; ++r) {
                 const int q = runs[r].first;
-                e = cudaMemcpyAsync(grids_out[who[(size_t)q]], staging + jobs[(size_t)q].byte_off, (size_t)runs[r].second,
+                e = cudaMemcpyAsync(grids_out[who[(size_t)q]], staging + byte_off[(size_t)q], (size_t)runs[r].second,
                                     cudaMemcpyDefault, dl);
                 if (e != cudaSuccess) s = cuda_fail(e, "fs3d_batch_retire_many readback");
             }

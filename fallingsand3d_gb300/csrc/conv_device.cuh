@@ -45,10 +45,16 @@ __device__ __forceinline__ uint4 pieces_to_planes(const uint32_t (&p)[4]) {
                       (t[0] & 0x55555555u) | ((t[2] << 1) & 0xAAAAAAAAu), (t[1] & 0x55555555u) | ((t[3] << 1) & 0xAAAAAAAAu));
 }
 
-// and back
+// and back: byte u of t[0..3] are the bytes of packed piece u
+__device__ __forceinline__ void planes_transposed(const uint4& q, uint32_t (&t)[4]) {
+    t[0] = (q.z & 0x55555555u) | ((q.x << 1) & 0xAAAAAAAAu);
+    t[1] = (q.w & 0x55555555u) | ((q.y << 1) & 0xAAAAAAAAu);
+    t[2] = ((q.z >> 1) & 0x55555555u) | (q.x & 0xAAAAAAAAu);
+    t[3] = ((q.w >> 1) & 0x55555555u) | (q.y & 0xAAAAAAAAu);
+}
 __device__ __forceinline__ void planes_to_pieces(const uint4& q, uint32_t (&p)[4]) {
-    const uint32_t t[4] = {(q.z & 0x55555555u) | ((q.x << 1) & 0xAAAAAAAAu), (q.w & 0x55555555u) | ((q.y << 1) & 0xAAAAAAAAu),
-                           ((q.z >> 1) & 0x55555555u) | (q.x & 0xAAAAAAAAu), ((q.w >> 1) & 0x55555555u) | (q.y & 0xAAAAAAAAu)};
+    uint32_t t[4];
+    planes_transposed(q, t);
     transpose4(t, p);
 }
 
@@ -81,83 +87,18 @@ __device__ __forceinline__ void planes_to_words64(const uint4& q, uint32_t (&w)[
     for (int k = 0; k < 16; ++k) w[k] = piece_word(p[k >> 2], k & 3);
 }
 
-// Loads n (1..64) bytes from p into 16 words; cells past n read as solid (1).
-// Sets *big when a loaded byte is a static material (>= 4).
-__device__ __forceinline__ void load_chunk64(const uint8_t* p, int n, uint32_t (&w)[16], bool& big) {
-    uint32_t any = 0;
-    if (n == 64 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const uint4 v = reinterpret_cast<const uint4*>(p)[u];
-            w[4 * u] = v.x;
-            w[4 * u + 1] = v.y;
-            w[4 * u + 2] = v.z;
-            w[4 * u + 3] = v.w;
-            any |= v.x | v.y | v.z | v.w;
-        }
-    } else if ((reinterpret_cast<uintptr_t>(p) & 3u) == 0) {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            uint32_t v;
-            if (4 * k + 4 <= n) {
-                v = reinterpret_cast<const uint32_t*>(p)[k];
-            } else {
-                v = 0x01010101u;
-                for (int i = 0; i < 4; ++i)
-                    if (4 * k + i < n) v = (v & ~(0xFFu << (8 * i))) | ((uint32_t)p[4 * k + i] << (8 * i));
-            }
-            w[k] = v;
-            any |= v;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            uint32_t v = 0x01010101u;
-            for (int i = 0; i < 4; ++i)
-                if (4 * k + i < n) v = (v & ~(0xFFu << (8 * i))) | ((uint32_t)p[4 * k + i] << (8 * i));
-            w[k] = v;
-            any |= v;
-        }
-    }
-    big = (any & 0xFCFCFCFCu) != 0;
+// codes with a solid's (1) replaced by its static byte
+__device__ __forceinline__ uint32_t with_static(uint32_t codes, uint32_t statics) {
+    const uint32_t m = (codes & ~(codes >> 1) & 0x01010101u) * 0xFFu;
+    return (codes & ~m) | (statics & m);
 }
 
-// Stores the first n (1..64) cells of 16 words to p.
-__device__ __forceinline__ void store_chunk64(uint8_t* p, int n, const uint32_t (&w)[16]) {
-    if (n == 64 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+// cell x of the words w set to byte v (static indexing of w)
+template <int N>
+__device__ __forceinline__ void patch_byte(uint32_t (&w)[N], int x, uint32_t v) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            reinterpret_cast<uint4*>(p)[u] = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
-    } else if ((reinterpret_cast<uintptr_t>(p) & 3u) == 0) {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            if (4 * k + 4 <= n)
-                reinterpret_cast<uint32_t*>(p)[k] = w[k];
-            else
-                for (int i = 0; i < 4; ++i)
-                    if (4 * k + i < n) p[4 * k + i] = (uint8_t)(w[k] >> (8 * i));
-        }
-    } else {
-        for (int x = 0; x < n; ++x) p[x] = (uint8_t)(w[x >> 2] >> (8 * (x & 3)));
-    }
-}
-
-// Replaces the code of every solid cell of the chunk by its static byte
-// (statics_row: the world's static bytes at the chunk's first cell).
-__device__ __forceinline__ void patch_statics64(const uint4& q, const uint8_t* statics_row, int n, uint32_t (&w)[16]) {
-    uint32_t se = ~q.x & q.z, so = ~q.y & q.w;  // solid cells, even and odd
-    while (se) {
-        const int m = __ffs(se) - 1;
-        se &= se - 1;
-        const int x = 2 * m;
-        if (x < n) w[x >> 2] = (w[x >> 2] & ~(0xFFu << (8 * (x & 3)))) | ((uint32_t)statics_row[x] << (8 * (x & 3)));
-    }
-    while (so) {
-        const int m = __ffs(so) - 1;
-        so &= so - 1;
-        const int x = 2 * m + 1;
-        if (x < n) w[x >> 2] = (w[x >> 2] & ~(0xFFu << (8 * (x & 3)))) | ((uint32_t)statics_row[x] << (8 * (x & 3)));
-    }
+    for (int k = 0; k < N; ++k)
+        if (k == x >> 2) w[k] = (w[k] & ~(0xFFu << (8 * (x & 3)))) | (v << (8 * (x & 3)));
 }
 
 }  // namespace fs3d

@@ -27,7 +27,6 @@
 #include "fs3d_common.h"
 #include "pcg.h"
 #include "planes.h"
-#include "conv_device.cuh"
 #include "rule_device.cuh"
 #include "bulk_device.cuh"
 #include "bricks_device.cuh"
@@ -35,52 +34,14 @@
 namespace fs3d {
 
 // ---------------------------------------------------------------------------
-// conversions
+// hashes
 // ---------------------------------------------------------------------------
-// One (row, word) unit: the 64-cell chunk at x = 64w of row r.
-__device__ __forceinline__ uint4 chunk_to_planes(const uint8_t* row, int X, int w, bool& big) {
-    uint32_t v[16];
-    load_chunk64(row + 64 * w, min(64, X - 64 * w), v, big);
-    return bytes_to_planes64(v, big);
-}
-
-__device__ __forceinline__ void planes_to_chunk(const uint4& q, const uint8_t* statics_row, uint8_t* row, int X,
-                                                int w) {
-    uint32_t v[16];
-    planes_to_words64(q, v);
-    const int n = min(64, X - 64 * w);
-    if (statics_row) patch_statics64(q, statics_row + 64 * w, n, v);
-    store_chunk64(row + 64 * w, n, v);
-}
-
-__global__ void k_bytes_to_planes(const uint8_t* __restrict__ g, int X, int Y, int Z, int nw,
-                                  uint4* __restrict__ rows) {
-    const int64_t n = (int64_t)Y * Z * nw;
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-        const int w = (int)(u % nw);
-        const int64_t r = u / nw;
-        bool big;
-        rows[u] = chunk_to_planes(g + r * X, X, w, big);
-    }
-}
-
 // the byte value of one cell of a plane word (static cells from `statics`, or stone)
 __device__ __forceinline__ uint32_t cell_value(const uint4& q, int m, int odd, const uint8_t* statics, int64_t idx) {
     const uint32_t a = ((odd ? q.y : q.x) >> m) & 1u, b = ((odd ? q.w : q.z) >> m) & 1u;
     if (a) return b ? 3u : 2u;
     if (!b) return 0u;
     return statics ? statics[idx] : 1u;
-}
-
-__global__ void k_planes_to_bytes(const uint4* __restrict__ rows, const uint8_t* __restrict__ statics, int X,
-                                  int Y, int Z, int nw, uint8_t* __restrict__ g, const int* skip_if_set) {
-    if (skip_if_set && *(volatile const int*)skip_if_set) return;
-    const int64_t n = (int64_t)Y * Z * nw;
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-        const int w = (int)(u % nw);
-        const int64_t r = u / nw;
-        planes_to_chunk(rows[u], statics ? statics + r * X : nullptr, g + r * X, X, w);
-    }
 }
 
 __global__ void k_hash_planes(const uint4* __restrict__ rows, const uint8_t* __restrict__ statics, int X, int Y,
@@ -129,9 +90,7 @@ __global__ void __launch_bounds__(256) k_hash_planes_many(const HashJob* __restr
     }
 }
 
-// Many worlds per launch (admission and retirement of a batch): job j covers
-// units [unit_off[j], unit_off[j+1]) of (row, word) pairs; its bytes sit at
-// byte_off in one staging buffer.
+// the job j with off[j] <= u < off[j + 1]
 __device__ __forceinline__ int find_job(const int64_t* __restrict__ unit_off, int njobs, int64_t u) {
     int lo = 0, hi = njobs - 1;
     while (lo < hi) {
@@ -142,124 +101,6 @@ __device__ __forceinline__ int find_job(const int64_t* __restrict__ unit_off, in
             hi = mid - 1;
     }
     return lo;
-}
-
-// The job of a unit: the job of its block's first unit (block_job, from the
-// host), then at most a few steps forward (a block of kConvBlock consecutive
-// units spans few worlds).
-__device__ __forceinline__ int unit_job(const int64_t* __restrict__ unit_off, const int* __restrict__ block_job,
-                                        int njobs, int64_t u) {
-    int j = __ldg(block_job + u / kConvBlock);
-    while (j + 1 < njobs && __ldg(unit_off + j + 1) <= u) ++j;
-    return j;
-}
-
-// Read-back: a CTA converts kConvBlock consecutive units per pass.  Their
-// bytes are one contiguous span of the staging buffer (rows are back to back;
-// a span may cross into the next world over at most a few padding bytes), so
-// each thread writes its 64-cell chunk into shared memory and the span goes
-// out in coalesced 16-byte stores (254 µs for 2048 worlds against 290 µs with
-// per-thread stores of rows 16-48 bytes wide).  Rows whose width is not a
-// multiple of 8 (chunks not 8-byte aligned), or spans wider than the buffer
-// (many tiny worlds), take the direct per-thread path.
-constexpr int kConvSpan = kConvBlock * 64 + 64;
-
-struct UnitAt {
-    int j;
-    int64_t lu, r, pos;  // unit within its world, row, first byte in the staging buffer
-    int w, n;            // word within the row, bytes of the chunk
-};
-
-__device__ __forceinline__ UnitAt unit_at(const ConvJob& jb, int j, int64_t lu) {
-    UnitAt a;
-    a.j = j;
-    a.lu = lu;
-    a.w = jb.nw == 1 ? 0 : (int)(lu % jb.nw);
-    a.r = jb.nw == 1 ? lu : lu / jb.nw;
-    a.n = min(64, jb.X - 64 * a.w);
-    a.pos = jb.byte_off + a.r * jb.X + 64 * a.w;
-    return a;
-}
-
-// Stores len bytes (a multiple of 8) from shared memory at sm to global g
-// (8-byte aligned; sm congruent to g modulo 16) in 16-byte pieces with an
-// 8-byte head and tail.
-__device__ __forceinline__ void store_span(uint8_t* g, const uint8_t* sm, uint64_t len) {
-    const uint64_t head = (reinterpret_cast<uintptr_t>(g) & 15u) ? 8u : 0u;
-    const uint64_t body = (len - head) & ~(uint64_t)15;
-    if (threadIdx.x == 0 && head) *reinterpret_cast<uint2*>(g) = *reinterpret_cast<const uint2*>(sm);
-    for (uint64_t o = head + 16u * threadIdx.x; o < head + body; o += 16u * kConvBlock)
-        *reinterpret_cast<uint4*>(g + o) = *reinterpret_cast<const uint4*>(sm + o);
-    const uint64_t t = head + body;
-    if (threadIdx.x == 0 && t < len) *reinterpret_cast<uint2*>(g + t) = *reinterpret_cast<const uint2*>(sm + t);
-}
-
-// Admission: each thread loads and converts its own chunk straight from the
-// staging bytes.  (A version staging the span in shared memory, as the
-// read-back does, took twice as long: a thread's chunk is X bytes apart from
-// its neighbour's, so reading it from shared memory meets 4- to 16-way bank
-// conflicts, and loads no longer overlap the conversion.)
-__global__ void __launch_bounds__(kConvBlock) k_bytes_to_planes_multi(const ConvJob* __restrict__ jobs,
-                                                                      const int64_t* __restrict__ unit_off,
-                                                                      const int* __restrict__ block_job, int njobs,
-                                                                      int64_t total, const uint8_t* __restrict__ staging,
-                                                                      int* flags) {
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < total; u += (int64_t)gridDim.x * blockDim.x) {
-        const int j = unit_job(unit_off, block_job, njobs, u);
-        const ConvJob jb = jobs[j];
-        const UnitAt at = unit_at(jb, j, u - unit_off[j]);
-        uint32_t v[16];
-        bool big;
-        load_chunk64(staging + at.pos, at.n, v, big);
-        jb.rows[at.lu] = bytes_to_planes64(v, big);
-        if (big) atomicOr(flags + j, 1);  // holds a static material >= 4: keep its bytes
-    }
-}
-
-__global__ void __launch_bounds__(kConvBlock) k_planes_to_bytes_multi(const ConvJob* __restrict__ jobs,
-                                                                      const int64_t* __restrict__ unit_off,
-                                                                      const int* __restrict__ block_job, int njobs,
-                                                                      int64_t total, uint8_t* __restrict__ staging) {
-    __shared__ __align__(16) uint8_t span[kConvSpan + 16];
-    __shared__ unsigned long long s_start, s_len;
-    for (int64_t base = (int64_t)blockIdx.x * kConvBlock; base < total; base += (int64_t)gridDim.x * kConvBlock) {
-        const int64_t u = base + threadIdx.x;
-        const bool live = u < total;
-        UnitAt at{};
-        int X = 0;
-        uint32_t v[16];
-        if (live) {
-            const int j = unit_job(unit_off, block_job, njobs, u);
-            const ConvJob jb = jobs[j];
-            X = jb.X;
-            at = unit_at(jb, j, u - unit_off[j]);
-            const uint4 q = jb.rows[at.lu];
-            planes_to_words64(q, v);
-            const uint8_t* st = jb.statics;
-            if (!st && jb.static_flag && *jb.static_flag) st = jb.static_src;
-            if (st) patch_statics64(q, st + at.r * jb.X + 64 * at.w, at.n, v);
-        }
-        if (threadIdx.x == 0) {
-            s_start = (unsigned long long)at.pos;  // unit `base` is live
-            s_len = 0;
-        }
-        __syncthreads();
-        const uint64_t start = s_start;
-        bool direct = live && ((X & 7) != 0 || (uint64_t)at.pos - start + (uint64_t)at.n > (uint64_t)kConvSpan);
-        if (live && !direct) atomicMax(&s_len, (unsigned long long)((uint64_t)at.pos - start + (uint64_t)at.n));
-        direct = __syncthreads_or(direct) != 0;
-        uint8_t* sm = span + (start & 15u);
-        if (direct) {
-            if (live) store_chunk64(staging + at.pos, at.n, v);
-        } else {
-            if (live) store_chunk64(sm + ((uint64_t)at.pos - start), at.n, v);
-            __syncthreads();
-            // the span's padding bytes between two worlds (if any) are written
-            // too: they belong to no world
-            store_span(staging + start, sm, s_len);
-        }
-        __syncthreads();  // the span and s_start are rewritten by the next pass
-    }
 }
 
 // The mixed-size batch world generated straight into planes: stone at y < 2,
@@ -1015,11 +856,6 @@ fs3d_status set_inject_tx_extra(uint32_t bytes) {
     return FS3D_OK;
 }
 
-int smem_world_limit() {
-    init_classes();
-    return g_classes[2].smem;
-}
-
 fs3d_status launch_plane_segment_resident(int cls, const PlaneWorld* worlds, const int* order, const int* meta,
                                           int* counter, int* err, cudaStream_t st,
                                           unsigned long long* processed_cells) {
@@ -1076,22 +912,6 @@ int plane_items_for(int Y, int Z, int nw) {
     const int per = 32 >> plane_lg(nw);
     const int nrp = nblocks(Y, 1) * nblocks(Z, 1);
     return (nrp + per - 1) / per;
-}
-
-fs3d_status planes_from_bytes(const uint8_t* g, int X, int Y, int Z, uint4* rows, cudaStream_t st) {
-    const int nw = plane_nw(X);
-    k_bytes_to_planes<<<conv_grid((int64_t)Y * Z * nw), 256, 0, st>>>(g, X, Y, Z, nw, rows);
-    FS3D_CHECK_LAUNCH("bytes->planes launch");
-    return FS3D_OK;
-}
-
-fs3d_status planes_from_bytes_multi(const ConvJob* jobs, const int64_t* unit_off, const int* block_job, int njobs,
-                                    int64_t total_units, const uint8_t* staging, int* flags, cudaStream_t st) {
-    if (njobs <= 0 || total_units <= 0) return FS3D_OK;
-    k_bytes_to_planes_multi<<<conv_grid(total_units), kConvBlock, 0, st>>>(jobs, unit_off, block_job, njobs,
-                                                                            total_units, staging, flags);
-    FS3D_CHECK_LAUNCH("bytes->planes (many worlds) launch");
-    return FS3D_OK;
 }
 
 // Each warp moves 2 KB blocks: lane l takes the 16-byte chunks 32i + l of its
@@ -1177,6 +997,16 @@ uint8_t* device_view(const void* p) {
     return nullptr;
 }
 
+bool device_local(const void* p) {
+    cudaPointerAttributes a{};
+    int dev = -1;
+    if (!p || cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == dev;
+}
+
 bool alloc_range(const void* p, uintptr_t* start, size_t* bytes) {
     // cuPointerGetAttributes, looked up once through the runtime (no link
     // dependency on the driver library)
@@ -1201,28 +1031,11 @@ bool alloc_range(const void* p, uintptr_t* start, size_t* bytes) {
     return true;
 }
 
-fs3d_status planes_to_bytes_multi(const ConvJob* jobs, const int64_t* unit_off, const int* block_job, int njobs,
-                                  int64_t total_units, uint8_t* staging, cudaStream_t st) {
-    if (njobs <= 0 || total_units <= 0) return FS3D_OK;
-    k_planes_to_bytes_multi<<<conv_grid(total_units), kConvBlock, 0, st>>>(jobs, unit_off, block_job, njobs,
-                                                                            total_units, staging);
-    FS3D_CHECK_LAUNCH("planes->bytes (many worlds) launch");
-    return FS3D_OK;
-}
-
 fs3d_status planes_generate_batch_world(uint64_t world_seed, int X, int Y, int Z, uint4* rows, cudaStream_t st) {
     const int nw = plane_nw(X);
     k_gen_batch_planes<<<conv_grid((int64_t)Y * Z * nw), 256, 0, st>>>(X, Y, Z, nw, batch_world_gen(world_seed),
                                                                        rows);
     FS3D_CHECK_LAUNCH("generate batch world launch");
-    return FS3D_OK;
-}
-
-fs3d_status planes_to_bytes(const uint4* rows, const uint8_t* statics, int X, int Y, int Z, uint8_t* g,
-                            cudaStream_t st, const int* skip_if_set) {
-    const int nw = plane_nw(X);
-    k_planes_to_bytes<<<conv_grid((int64_t)Y * Z * nw), 256, 0, st>>>(rows, statics, X, Y, Z, nw, g, skip_if_set);
-    FS3D_CHECK_LAUNCH("planes->bytes launch");
     return FS3D_OK;
 }
 

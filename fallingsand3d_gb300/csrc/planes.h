@@ -55,8 +55,6 @@ constexpr int kMetaWorlds = 1 + 2 * kAllClasses;
 constexpr int kMetaInts = kMetaWorlds + 1;
 // smallest class that holds a world of these dims, -1 if none does
 int resident_class(int X, int Y, int Z);
-// largest plane buffer (bytes) one CTA can hold; 0 if unavailable
-int smem_world_limit();
 constexpr int kErrInts = 4;  // size of the error record a resident launch is given
 // test hook: resident kernels announce `bytes` more than each bulk copy delivers
 fs3d_status set_inject_tx_extra(uint32_t bytes);
@@ -80,12 +78,12 @@ fs3d_status launch_plane_segment_gm(int cls, const PlaneWorld* worlds, const int
                                     int* counter, int* err, cudaStream_t st, unsigned long long* processed_cells,
                                     bool first = false);
 
-// One world of a many-world conversion: its planes, its static bytes
-// (nullable) and the offset of its canonical bytes in a shared staging buffer.
+// One world of a many-world conversion: its planes, its canonical bytes
+// (admission: read; read-back: written) and its static bytes (nullable).
 struct ConvJob {
     uint4* rows;
     const uint8_t* statics;
-    int64_t byte_off;
+    uint8_t* bytes;
     int32_t X, Y, Z, nw;
     // read-back of a world whose static-material flag has not reached the
     // host yet: when *static_flag is set, its static bytes are at static_src
@@ -95,23 +93,33 @@ struct ConvJob {
     // layer_flags_from_cells_multi; null: none) and its first step's low 8 bits
     uint8_t* lflags = nullptr;
     uint32_t t0b = 0;
+    uint32_t magic = 0;  // read-back: conv_magic(X)
 };
-// bytes -> planes for njobs worlds in one launch; unit_off[j] = sum of Y*Z*nw
-// over jobs before j; block_job[i] = the job of unit kConvBlock*i (from
-// conv_block_jobs); flags[j] |= 1 when world j holds a material >= 4
-constexpr int kConvBlock = 256;  // units per CTA pass of the conversion kernels
-inline int64_t conv_blocks(int64_t total_units) { return (total_units + kConvBlock - 1) / kConvBlock; }
-inline void conv_block_jobs(const int64_t* unit_off, int njobs, int64_t total_units, int* block_job) {
-    int j = 0;
-    for (int64_t i = 0; i < conv_blocks(total_units); ++i) {
-        while (j + 1 < njobs && unit_off[j + 1] <= i * kConvBlock) ++j;
-        block_job[i] = j;
-    }
+// One CTA of a conversion takes whole rows of one world: as many as make
+// `chunks` 64-cell chunks, from row0 on.  Read-backs of many worlds take twice
+// the chunks of the others (a CTA's set-up is a third of its instructions).
+constexpr int kConvThreads = 256, kConvChunks = kConvThreads, kConvChunksBack = 2 * kConvThreads;
+struct ConvBlock {
+    int32_t job;
+    uint32_t row0;
+};
+FS3D_HD int conv_rows(int nw, int chunks) { return chunks / nw; }
+inline int64_t conv_blocks(int Y, int Z, int nw, int chunks) {
+    return ((int64_t)Y * Z + conv_rows(nw, chunks) - 1) / conv_rows(nw, chunks);
 }
-fs3d_status planes_from_bytes_multi(const ConvJob* jobs, const int64_t* unit_off, const int* block_job, int njobs,
-                                    int64_t total_units, const uint8_t* staging, int* flags, cudaStream_t st);
-fs3d_status planes_to_bytes_multi(const ConvJob* jobs, const int64_t* unit_off, const int* block_job, int njobs,
-                                  int64_t total_units, uint8_t* staging, cudaStream_t st);
+// the blocks of job j, written to out; returns how many
+inline int64_t conv_fill_blocks(int j, int Y, int Z, int nw, int chunks, ConvBlock* out) {
+    const int64_t n = conv_blocks(Y, Z, nw, chunks);
+    for (int64_t i = 0; i < n; ++i) out[i] = ConvBlock{j, (uint32_t)(i * conv_rows(nw, chunks))};
+    return n;
+}
+// ConvJob::magic: i / ceil(X / 16) = umulhi(i, magic) for i < 2^16
+inline uint32_t conv_magic(int X) { return 0xFFFFFFFFu / (uint32_t)((X + 15) / 16) + 1u; }
+// bytes -> planes for many worlds in one launch; flags[j] |= 1 when world j
+// holds a material >= 4
+fs3d_status planes_from_bytes_multi(const ConvJob* jobs, const ConvBlock* blocks, int64_t nblocks, int* flags,
+                                    cudaStream_t st);
+fs3d_status planes_to_bytes_multi(const ConvJob* jobs, const ConvBlock* blocks, int64_t nblocks, cudaStream_t st);
 
 // Many byte copies in one launch (each thread moves a 16-byte chunk): used
 // instead of one cudaMemcpyAsync per world when both sides are addressable
@@ -128,6 +136,8 @@ fs3d_status copy_many(const CopyJob* jobs, const int64_t* chunk_off, int njobs, 
 // pointers must be device-addressable (device memory, or the device view of
 // page-locked host memory); pointers not 16-byte aligned take cudaMemcpyAsync.
 cudaError_t copy_small_async(void* dst, const void* src, size_t bytes, cudaStream_t st);
+// Whether p is memory of the current device (which a kernel may write at full rate).
+bool device_local(const void* p);
 // A device-addressable alias of p (itself for device or managed memory, the
 // mapped address for page-locked host memory), or nullptr for pageable memory.
 uint8_t* device_view(const void* p);
