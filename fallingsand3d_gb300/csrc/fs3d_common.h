@@ -77,9 +77,9 @@ __device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template <class... P, class... A>
-cudaError_t launch_chained(void (*fn)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
+cudaError_t launch_chained(void (*fn)(P...), dim3 grid, unsigned block, cudaStream_t st, A... args) {
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(grid);
+    lc.gridDim = grid;
     lc.blockDim = dim3(block);
     lc.stream = st;
     cudaLaunchAttribute attr[1];

@@ -222,15 +222,15 @@ int sm_count_public();
 
 // render (render.cu)
 fs3d_status launch_render_sdf(const fs3d_camera* cam, int W, int H, float* rgba_dev, cudaStream_t st);
-// the DDA kernels take a per-frame brick occupancy bitmap of brickmap_bytes() bytes
+// the DDA kernels take a brick occupancy map of brickmap_bytes() bytes, zeroed before its first frame
 size_t brickmap_bytes(int X, int Y, int Z);
-fs3d_status launch_render_dda_bytes(const uint8_t* g, int X, int Y, int Z, uint32_t* bm_bits, const fs3d_camera* cam,
+fs3d_status launch_render_dda_bytes(const uint8_t* g, int X, int Y, int Z, uint8_t* bits, const fs3d_camera* cam,
                                     int W, int H, float* rgba_dev, cudaStream_t st);
 // brick_counts (nullable): exact per-brick counts of non-empty cells; the
 // frame then derives its brick map from them (rebuild: recount from the
 // planes first) instead of a pass over the planes
 fs3d_status launch_render_dda_planes(const uint4* rows, const uint8_t* statics, int X, int Y, int Z, int nw,
-                                     uint32_t* bm_bits, const fs3d_camera* cam, int W, int H, float* rgba_dev,
+                                     uint8_t* bits, const fs3d_camera* cam, int W, int H, float* rgba_dev,
                                      cudaStream_t st, int* brick_counts = nullptr, bool recount = true);
 size_t brick_count_bytes(int X, int Y, int Z);
 

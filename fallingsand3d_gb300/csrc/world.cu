@@ -27,7 +27,7 @@ struct fs3d_world {
     void* slab_scratch = nullptr;  // PLANES: scratch of the whole-GPU multi-step launches (worlds that fit them)
     int* err = nullptr;            // PLANES: error record of those launches (kErrInts ints)
     unsigned long long* hash_dev = nullptr;
-    uint32_t* brickmap = nullptr;  // render: per-frame occupancy of 8x8x8 bricks
+    uint8_t* brickmap = nullptr;  // render: per-frame occupancy of 8x8x8 bricks
     int* brick_counts = nullptr;   // PLANES render: non-empty cells per brick, kept by the per-step kernel
     bool counts_valid = false;     // brick_counts match the planes
     // change flags per row (Y*Z bytes), kept from one call to the next
@@ -369,8 +369,11 @@ fs3d_status fs3d_render(fs3d_world* w, const fs3d_camera* cam, int W, int H, int
         return set_error(FS3D_ERR_INVALID_ARG, "fs3d_render: bad args");
     float* dst = rgba;
     const size_t bytes = (size_t)W * H * 4 * sizeof(float);
-    if (mode == FS3D_RENDER_DDA && !w->brickmap)
-        FS3D_CUDA(cudaMalloc((void**)&w->brickmap, brickmap_bytes(w->X, w->Y, w->Z)));
+    if (mode == FS3D_RENDER_DDA && !w->brickmap) {
+        const size_t n = brickmap_bytes(w->X, w->Y, w->Z);
+        FS3D_CUDA(cudaMalloc((void**)&w->brickmap, n));
+        FS3D_CUDA(cudaMemsetAsync(w->brickmap, 0, n, w->stream));  // (its counters)
+    }
     // planes worlds stepped by the per-step kernel keep exact brick counts
     if (mode == FS3D_RENDER_DDA && w->layout == FS3D_LAYOUT_PLANES && !w->brick_counts &&
         plane_bytes(w->X, w->Y, w->Z) > kCountsPlaneBytes)
