@@ -68,14 +68,17 @@ bool current_context_id(unsigned long long* id);
 
 // ---- chained launches: a kernel that begins with chain_wait() may be launched
 // with launch_chained(), so that its CTAs are placed and its first instructions
-// fetched while the kernel before it in the stream still runs (programmatic
+// fetched while the kernel before it in the stream ends (programmatic
 // dependent launch).  chain_wait() returns once that kernel has run and its
 // writes are visible; nothing in global memory may be touched before it.
+// chain_go() lets the next kernel's CTAs be placed; it stands at the end of
+// each CTA's work (the end of the kernel does the same): CTAs placed any
+// earlier hold registers that other streams' kernels could use (three 1024^3
+// worlds stepped and drawn in turn: 315 us a pass with chain_go() first, 222
+// with it last; a lone stream's steps take the same either way).
 #ifdef __CUDACC__
-__device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>
 cudaError_t launch_chained(void (*fn)(P...), dim3 grid, unsigned block, cudaStream_t st, A... args) {
     cudaLaunchConfig_t lc = {};

@@ -277,6 +277,7 @@ __global__ void __launch_bounds__(256, 3) k_plane_step_skip(const PlaneWorld w, 
         }
         if (counts && any) count_bricks(counts, w, y0, z0, gl, q, q0, in);
     }
+    chain_go();
 }
 
 // ---------------------------------------------------------------------------

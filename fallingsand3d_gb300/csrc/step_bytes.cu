@@ -277,6 +277,7 @@ __global__ void __launch_bounds__(128, FS3D_ROWS_CTAS_PER_SM)
                     reinterpret_cast<uint4*>(ptr[a])[u] = make_uint4(w[4 * u], w[4 * u + 1], w[4 * u + 2], w[4 * u + 3]);
         }
     }
+    chain_go();
 }
 
 // ---- rows of any length and alignment
@@ -395,6 +396,7 @@ __global__ void __launch_bounds__(128, 5)
         }
         sync();
     }
+    chain_go();
 }
 
 // ---------------------------------------------------------------------------
