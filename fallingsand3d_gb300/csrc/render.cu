@@ -42,10 +42,22 @@ __device__ __forceinline__ void pixel_uv2(int px, int py, int W, int H, float& u
     ux = __fsub_rn(__fmul_rn(u, 2.0f), 1.0f);
     uy = __fsub_rn(__fmul_rn(v, 2.0f), 1.0f);
 }
+// Whether the ray o + t d (d of unit length) stays clear of the ball of radius r
+// about the origin, by far more than the hit distance (0.001) and the march's
+// rounding (relative to |o|) can bridge: marching it would never hit.  False
+// for NaN.
+__device__ __forceinline__ bool passes_by(const float* o, const float* d, float r) {
+    const float along = o[0] * d[0] + o[1] * d[1] + o[2] * d[2];
+    const float x = o[0] - along * d[0], y = o[1] - along * d[1], z = o[2] - along * d[2];
+    const float far = r + 0.01f + 1e-5f * (fabsf(o[0]) + fabsf(o[1]) + fabsf(o[2]));
+    return x * x + y * y + z * z > far * far;
+}
 __device__ __forceinline__ float sdf_world(float x, float y, float z) {
     return __fsub_rn(__fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z))), 0.5f);
 }
 
+// Most of the frame's rays miss the sphere by far (29 us a 1920x1080 frame
+// marching all of them, 64 steps or until t > 1000).
 __global__ void k_render_sdf(CamDev cam, int W, int H, float4* __restrict__ out) {
     const int px = blockIdx.x * blockDim.x + threadIdx.x;
     const int py = blockIdx.y * blockDim.y + threadIdx.y;
@@ -56,7 +68,8 @@ __global__ void k_render_sdf(CamDev cam, int W, int H, float4* __restrict__ out)
     float d[3] = {ux, uy, 1.0f};
     normalize3(d);
     float col = 0.0f, t = 0.0f;
-    for (int it = 0; it < 64; ++it) {
+    const int steps = passes_by(cam.o, d, 0.5f) ? 0 : 64;
+    for (int it = 0; it < steps; ++it) {
         const float p[3] = {__fadd_rn(cam.o[0], __fmul_rn(t, d[0])), __fadd_rn(cam.o[1], __fmul_rn(t, d[1])),
                             __fadd_rn(cam.o[2], __fmul_rn(t, d[2]))};
         const float dist = sdf_world(p[0], p[1], p[2]);
