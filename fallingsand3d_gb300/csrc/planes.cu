@@ -526,6 +526,13 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
     __shared__ int s_count[2];                   // work-list length, by step parity
     constexpr int kKeys = 32;                    // step keys computed together, one per thread
     __shared__ uint32_t s_keys[kKeys];
+    // many dirty layer pairs: each warp lists them once a step, so that a pass
+    // looks its own up (the families of dense steps; settled worlds have one or
+    // two, found from the masks, and the list's round trip made their 2048-world
+    // segment and snapshot 946 us instead of 794)
+    constexpr bool kListed = !GM || NT >= 768;
+    constexpr int kMasked = 96;
+    __shared__ uint8_t s_list[NT / 32][kListed ? kMasked : 1];
     // per phase o: the world's block rows along z, and the multiplier that
     // divides by it (e / n = umulhi(e, m), exact for e, n < 2^16)
     __shared__ uint32_t s_nbz[2], s_magic[2];
@@ -619,12 +626,24 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
             // through the shared list
             uint32_t dm0 = 0, dm1 = 0, dm2 = 0;
             int n_layers;
-            const bool masked = nj <= 96;
+            const bool masked = nj <= kMasked;
+            uint8_t* list = s_list[threadIdx.x >> 5];
             if (masked) {
                 dm0 = __ballot_sync(0xFFFFFFFFu, lane < nj && layer_dirty(v, w, o, tb, j_lo + lane));
                 if (nj > 32) dm1 = __ballot_sync(0xFFFFFFFFu, lane + 32 < nj && layer_dirty(v, w, o, tb, j_lo + 32 + lane));
                 if (nj > 64) dm2 = __ballot_sync(0xFFFFFFFFu, lane + 64 < nj && layer_dirty(v, w, o, tb, j_lo + 64 + lane));
                 n_layers = __popc(dm0) + __popc(dm1) + __popc(dm2);
+                if (kListed) {
+                    __syncwarp();  // the last step's readers are done
+                    const uint32_t dm[3] = {dm0, dm1, dm2};
+                    int at = 0;
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        if ((dm[i] >> lane) & 1u) list[at + __popc(dm[i] & ((1u << lane) - 1u))] = (uint8_t)(32 * i + lane);
+                        at += __popc(dm[i]);
+                    }
+                    __syncwarp();
+                }
             } else {
                 int* cnt = &s_count[s & 1];
                 for (int base = 0; base < nj; base += NT) {
@@ -663,6 +682,8 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
                 if (valid) {
                     if (!masked)
                         jj = (int)jlist[jd];
+                    else if (kListed)
+                        jj = (int)list[jd];
                     else if (jd == 0 && dm0)
                         jj = __ffs(dm0) - 1;
                     else if (jd < __popc(dm0))
