@@ -209,6 +209,10 @@ struct fs3d_batch {
     uint32_t class_mask = ~0u, graph_mask = 0;
     int grid = 0;
     int promote = 0;  // single-CTA resident worlds run this many classes wider (autotuned)
+    // hybrid mode: young worlds of class `spread_from` or wider run in cluster
+    // class `spread` (0: none), chosen with the tables
+    int spread = 0, spread_from = 0;
+    void* edges[kResidentClasses - kSingleCtaClasses] = {};  // the cluster classes' edge buffers (once needed)
     unsigned long long* hash_dev = nullptr;
     unsigned long long* processed_dev = nullptr;  // cell-steps the resident kernels evaluated
     uint64_t segments = 0;
@@ -259,14 +263,17 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
     if (mode == 2) return gm();
     if (mode == 3) {
         if (w.t < kYoungSteps) {
-            // a young world that needs a cluster runs instead from L2 with a
-            // whole SM (768 threads): dense steps keep its warps busy, and no
-            // cluster barrier or y-slab imbalance holds it up.  The smallest
-            // worlds run in 256-thread CTAs: their dense steps take half the
+            // few large young worlds are spread over clusters (choose_spread);
+            // of many, those that need more than one CTA's shared memory run
+            // from L2 with a whole SM (768 threads).  The smallest worlds run in
+            // 256-thread CTAs: their dense steps take half the
             // passes there (2048 fresh worlds: 2.79 ms per first segment
             // against 3.02 ms in 128-thread CTAs; moving the 256-thread worlds
             // up to 768 threads too measured 3.09 ms)
             const int c = smem();
+            if (b->spread && (c < 0 || c >= b->spread_from) &&
+                batch_slabs_fit(w.X, w.Y, w.Z, kClusterSizes[b->spread - kSingleCtaClasses]))
+                return b->spread;
             if (c >= 0 && c < kSingleCtaClasses) return c == 0 ? 1 : c;
             if (w.Y <= 4096) return kResidentClasses + kGmDense;
             return c >= 0 ? c : gm();
@@ -275,6 +282,41 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
         return first >= 0 ? first : smem();
     }
     return -1;
+}
+
+// How the hybrid mode spreads young worlds over clusters.  A large world's
+// dense steps are the segment's longest chain, so where SMs are left over it
+// is spread: every world of a whole SM's class and larger over 8 CTAs when the
+// batch then still fits the SMs, else those larger than one CTA's shared
+// memory over 8 or 4 while the batch fits the SMs twice over.  Beyond that,
+// and in clusters of 2, clusters only take SMs from the other worlds.  Two
+// segments of fresh mixed worlds, none spread / the larger ones / all: 32
+// worlds 1625 / 1076 / 969 us, 64 1482 / 1152 / 1249, 150 1837 / 1284 / 1855,
+// 350 2213 / 1704 / 1975, 512 2304 / 3317 (in clusters of 2) / -.
+void choose_spread(fs3d_batch* b) {
+    b->spread = 0;
+    if (b->cfg.use_smem != 3) return;
+    int large = 0, whole = 0, rest = 0;
+    for (auto& kv : b->worlds) {
+        BWorld& w = kv.second;
+        if (w.done || w.t >= kYoungSteps) continue;
+        if (w.cls_smem == -2) w.cls_smem = resident_class(w.X, w.Y, w.Z);
+        if (w.cls_smem < 0 || w.cls_smem >= kSingleCtaClasses) ++large;
+        else if (w.cls_smem == kSingleCtaClasses - 1) ++whole;
+        else ++rest;  // three to an SM
+    }
+    const int sms = sm_count_public();
+    auto spread = [&](int cs, int from) {
+        for (int c = kSingleCtaClasses; c < kResidentClasses; ++c)
+            if (kClusterSizes[c - kSingleCtaClasses] == cs) b->spread = c;
+        b->spread_from = from;
+    };
+    if (large + whole > 0 && (large + whole) * 8 + rest / 3 <= sms)
+        spread(8, kSingleCtaClasses - 1);
+    else if (large > 0 && large * 8 + whole + rest / 3 <= 2 * sms)
+        spread(8, kSingleCtaClasses);
+    else if (large > 0 && large * 4 + whole + rest / 3 <= 2 * sms)
+        spread(4, kSingleCtaClasses);
 }
 
 fs3d_status wait_stream(cudaStream_t st, int64_t timeout_ns) {
@@ -525,7 +567,12 @@ fs3d_status enqueue_segment(fs3d_batch* b, cudaStream_t a, bool fork, bool with_
     if (mode == 3) s = gm(kGmDense);
     if (mode == 1 || mode == 3)
         for (int c = kResidentClasses - 1; c >= 0 && s == FS3D_OK; --c)
-            if (has(c))
+            if (c >= kSingleCtaClasses) {
+                void* edges = b->edges[c - kSingleCtaClasses];
+                if (has(c) && edges)
+                    s = launch_batch_slabs(c, kClusterSizes[c - kSingleCtaClasses], b->tw.d, b->to.d, b->tn.d, b->counter + c,
+                                           b->err, edges, fork ? b->branch[c] : a, b->processed_dev);
+            } else if (has(c))
                 s = launch_plane_segment_resident(c, b->tw.d, b->to.d, b->tn.d, b->counter + c, b->err,
                                                   fork ? b->branch[c] : a, b->processed_dev);
     if (mode == 2 || mode == 3)
@@ -752,6 +799,7 @@ fs3d_status build_tables(fs3d_batch* b) {
     b->ti.select(b->tab_cur);
     b->tn.select(b->tab_cur);
     b->to.select(b->tab_cur);
+    choose_spread(b);
     // resident class of every running world (-1: stepped by the per-step kernel)
     std::vector<std::pair<int, BWorld*>> run;
     size_t ni = 0, ns = 0;
@@ -834,6 +882,9 @@ fs3d_status build_tables(fs3d_batch* b) {
     uint32_t mask = 0;
     for (int c = 0; c < kAllClasses; ++c)
         if (!by_class[c].empty()) mask |= 1u << c;
+    for (int c = kSingleCtaClasses; c < kResidentClasses; ++c)
+        if (((mask >> c) & 1u) && !b->edges[c - kSingleCtaClasses])
+            FS3D_CUDA(cudaMalloc(&b->edges[c - kSingleCtaClasses], batch_slab_edge_bytes(kClusterSizes[c - kSingleCtaClasses])));
     b->class_mask = mask;
     // admissions complete before the segment reads their planes
     for (auto& ev : b->pending_ready) FS3D_CUDA(cudaStreamWaitEvent(b->stream, ev.get(), 0));
@@ -1885,6 +1936,7 @@ fs3d_status fs3d_batch_destroy(fs3d_batch* b) {
     cudaFree(b->counter);
     cudaFree(b->err);
     cudaFree(b->processed_dev);
+    for (void* p : b->edges) cudaFree(p);
     if (b->fork) cudaEventDestroy(b->fork);
     for (int c = 0; c <= kAllClasses; ++c) {
         if (b->join[c]) cudaEventDestroy(b->join[c]);

@@ -48,6 +48,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, uint64_
 // a test that makes every wait run out stays short.
 constexpr uint64_t kCopyWaitNs = 2000000000ull, kCopyWaitInjectedNs = 20000000ull;
 
+// tells the mbarrier's current phase how many bytes to expect
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
 // one bulk copy whose bytes the mbarrier has been told to expect
 __device__ __forceinline__ void bulk_copy_in(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -60,8 +65,7 @@ __device__ __forceinline__ void bulk_copy_in(void* smem_dst, const void* gsrc, u
 // (`expect` = bytes, or more under the test hook above)
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint32_t expect,
                                           uint64_t* bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(expect)
-                 : "memory");
+    mbar_expect(bar, expect);
     bulk_copy_in(smem_dst, gsrc, bytes, bar);
 }
 

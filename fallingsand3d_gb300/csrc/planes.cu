@@ -18,7 +18,6 @@
 // read for computation and written by exactly one lane.  When X is a multiple
 // of 64 the odd phase has one extra half block per row-pair (cells x = X-1,
 // x = X outside), which the last lane runs with the scalar rule.
-#include <cooperative_groups.h>
 #include <stdint.h>
 
 #include <algorithm>
@@ -373,34 +372,23 @@ __global__ void __launch_bounds__(256) k_row_flags_from_cells(const uint4* __res
 // normal operation.
 static __device__ uint32_t g_inject_tx_extra;
 
-// The rows of one world held in shared memory by the CTAs of a cluster: CTA
-// r holds rows y in [lo_r, hi_r) (lo_r even), stored as ((y - lo_r)*Z + z)*nw
-// + word, followed (at the next 16-byte boundary) by four change buffers of
-// one byte per layer y (buffer t & 3: 1 if step t changed a row of the
-// layer) and a list of up to (hi_r - lo_r)/2 + 2 16-bit layer-pair indices.
-// Step t writes buffer t & 3, reads buffers (t-1) & 3 and (t-2) & 3 and
-// clears buffer (t+1) & 3, so no buffer is both read and written in a step.
-// `left` is the shared memory of CTA r-1 (null for r == 0): the only layer a
-// CTA touches outside its slab is y = lo_r - 1, in the odd phase.
-template <bool CL>
-struct SlabView {
-    uint4* mine;
-    uint4* left;
-    uint8_t* fmine;
-    uint8_t* fleft;
-    int lo, hi, left_lo, Z, nw;
-    __device__ __forceinline__ uint4* at(int y, int z, int g) const {
-        if (!CL || y >= lo) return mine + ((y - lo) * Z + z) * nw + g;
-        return left + ((y - left_lo) * Z + z) * nw + g;
-    }
-    __device__ __forceinline__ uint8_t* flag(int y, uint32_t b) const {
-        if (!CL || y >= lo) return fmine + b * flag_stride(hi - lo) + (y - lo);
-        return fleft + b * flag_stride(lo - left_lo) + (y - left_lo);
-    }
+// One world held by a CTA: its rows, followed in shared memory (at the next
+// 16-byte boundary) by four change buffers of one byte per layer y (buffer t &
+// 3: 1 if step t changed a row of the layer) and a list of up to Y/2 + 2 16-bit
+// layer-pair indices.  Step t writes buffer t & 3, reads buffers (t-1) & 3 and
+// (t-2) & 3 and clears buffer (t+1) & 3, so no buffer is both read and written
+// in a step.
+struct WorldView {
+    uint4* rows;
+    uint8_t* flags;
+    uint32_t stride;  // of the change buffers
+    int Z, nw;
+    __device__ __forceinline__ uint4* at(int y, int z, int g) const { return rows + (y * Z + z) * nw + g; }
+    __device__ __forceinline__ uint8_t* flag(int y, uint32_t b) const { return flags + b * stride + y; }
     __host__ __device__ static __forceinline__ uint32_t flag_stride(int layers) { return ((uint32_t)layers + 15u) & ~15u; }
 };
 
-// shared-memory bytes after a slab's planes: change buffers and the layer list
+// shared-memory bytes after a world's planes: change buffers and the layer list
 __host__ __device__ __forceinline__ uint32_t slab_aux_bytes(uint32_t layers) {
     return 4u * ((layers + 15u) & ~15u) + ((2u * (layers / 2u + 2u) + 15u) & ~15u);
 }
@@ -418,7 +406,7 @@ __device__ __forceinline__ int select_bit(uint32_t m, int n) {
     return pos + (n >= (int)(m & 1u) ? 1 : 0);
 }
 
-// bytes of a slab's planes, rounded up so its change buffers start 16-byte aligned
+// bytes of a world's planes, rounded up so its change buffers start 16-byte aligned
 __host__ __device__ __forceinline__ uint32_t slab_flag_offset(uint32_t plane_bytes) {
     return (plane_bytes + 15u) & ~15u;
 }
@@ -430,8 +418,7 @@ __host__ __device__ __forceinline__ uint32_t slab_flag_offset(uint32_t plane_byt
 // change depends on its cells alone (the rule's activity mask), so it would
 // change nothing again.  A world without kept flags starts with every layer
 // changed at steps t0 - 1 and t0 - 2.
-template <bool CL>
-__device__ __forceinline__ bool layer_dirty(const SlabView<CL>& v, const PlaneWorld& w, int o, uint32_t tb, int j) {
+__device__ __forceinline__ bool layer_dirty(const WorldView& v, const PlaneWorld& w, int o, uint32_t tb, int j) {
     uint32_t dirty = 0;
 #pragma unroll
     for (int a = 0; a < 2; ++a) {
@@ -444,8 +431,7 @@ __device__ __forceinline__ bool layer_dirty(const SlabView<CL>& v, const PlaneWo
 // Evaluates block row-pair (j, k) of a world held in shared memory when `run`
 // is set.  Every lane of the warp calls this together (the odd phase passes
 // carry bits between lanes).  Layers with a changed row get the step's flag.
-template <bool CL>
-__device__ __forceinline__ void slab_rowpair(const SlabView<CL>& v, const PlaneWorld& w, int o, uint32_t sk,
+__device__ __forceinline__ void world_rowpair(const WorldView& v, const PlaneWorld& w, int o, uint32_t sk,
                                              uint32_t tt /* step & 3 */, int j, int k, bool run, int gl,
                                              int G) {
     if (!__any_sync(0xFFFFFFFFu, run)) return;
@@ -470,17 +456,11 @@ __device__ __forceinline__ void slab_rowpair(const SlabView<CL>& v, const PlaneW
         }
 }
 
-// first row of slab r of CS slabs (even, so even-phase row-pairs never straddle)
-__device__ __forceinline__ int slab_lo(int Y, int r, int CS) { return 2 * ((r * ((Y + 1) / 2)) / CS); }
-
-// Persistent resident segment kernel.  A group of CS CTAs (a thread-block
-// cluster when CS > 1) takes worlds of its class, largest first, from
-// `counter`.  Each CTA loads its slab of the world's planes into shared
-// memory with one TMA bulk copy, the group runs the world's segment steps
-// (one CTA / cluster barrier per step: the next phase pairs different rows;
-// the one row a CTA reads from its neighbour travels through distributed
-// shared memory), and each CTA writes its slab back with one TMA bulk store.
-// Worlds are independent, so groups never wait on one another.
+// Persistent resident segment kernel.  A CTA takes worlds of its class, largest
+// first, from `counter`, loads a world's planes into shared memory with one
+// TMA bulk copy, runs its segment steps (one barrier per step: the next phase
+// pairs different rows) and writes it back with one TMA bulk store.  Worlds
+// are independent, so CTAs never wait on one another.
 // meta: [0] per-step items, [1 + c] resident worlds of class c, [1 + kAllClasses + c] their offset in order[].
 // CTAs of each single-CTA class that share an SM (the register cap that lets
 // them: 24 warps of at most 80 registers per SM)
@@ -496,32 +476,22 @@ constexpr int resident_ctas_per_sm() {
 #define FS3D_GM_THREADS_PER_SM 768
 #endif
 constexpr int kGmThreadsPerSm = FS3D_GM_THREADS_PER_SM;
-template <int NT, bool CL, bool GM = false>
-__global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resident_ctas_per_sm<NT>()))
+template <int NT, bool GM = false>
+__global__ void __launch_bounds__(NT, GM ? kGmThreadsPerSm / NT : resident_ctas_per_sm<NT>())
     k_plane_segment_resident(const PlaneWorld* __restrict__ worlds,
                                                              const int* __restrict__ order,
-                                                             const int* __restrict__ meta, int cls, int CS,
+                                                             const int* __restrict__ meta, int cls,
                                                              int* counter, int* err,
                                                              unsigned long long* processed_cells) {
     extern __shared__ __align__(128) uint4 srows[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ int item;
-    namespace cg = cooperative_groups;
     const int n = meta[1 + cls], off = meta[1 + kAllClasses + cls];
-    if (!CL) CS = 1;
-    const int r = CL ? (int)cg::this_cluster().block_rank() : 0;
-    auto group_sync = [&]() {
-        if (CL)
-            cg::this_cluster().sync();
-        else
-            __syncthreads();
-    };
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
     const uint32_t tx_extra = g_inject_tx_extra;
     uint32_t phase = 0;
     const int lane = threadIdx.x & 31;
-    uint4* left = (CL && r > 0) ? cg::this_cluster().map_shared_rank(srows, r - 1) : nullptr;
     __shared__ unsigned long long s_processed;  // cell-steps evaluated (the rest were skipped as settled)
     __shared__ int s_count[2];                   // work-list length, by step parity
     constexpr int kKeys = 32;                    // step keys computed together, one per thread
@@ -541,29 +511,22 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
         s_count[0] = s_count[1] = 0;
     }
     for (;;) {
-        // after an error every group stops taking worlds (and all of a cluster stop together)
-        if (r == 0 && threadIdx.x == 0) item = *(volatile int*)err ? n : atomicAdd(counter, 1);
-        group_sync();
-        const int it = CL ? *cg::this_cluster().map_shared_rank(&item, 0) : item;
-        group_sync();
+        // after an error no CTA takes another world
+        if (threadIdx.x == 0) item = *(volatile int*)err ? n : atomicAdd(counter, 1);
+        __syncthreads();
+        const int it = item;
+        __syncthreads();
         if (it >= n) break;
         const PlaneWorld w = worlds[order[off + it]];
         if (w.steps <= 0) continue;
-        SlabView<CL> v;
-        v.lo = slab_lo(w.Y, r, CS);
-        v.hi = r == CS - 1 ? w.Y : slab_lo(w.Y, r + 1, CS);
-        v.left_lo = r > 0 ? slab_lo(w.Y, r - 1, CS) : 0;
-        const uint32_t row_bytes = (uint32_t)w.Z * (uint32_t)w.nw * 16u;
-        const uint32_t bytes = GM ? 0u : (uint32_t)(v.hi - v.lo) * row_bytes;  // bulk-copied bytes
-        uint4* gslab = w.rows + (int64_t)v.lo * w.Z * w.nw;
-        v.mine = GM ? gslab : srows;
-        v.left = left;
+        const uint32_t bytes = GM ? 0u : (uint32_t)w.Y * (uint32_t)w.Z * (uint32_t)w.nw * 16u;  // bulk-copied bytes
+        WorldView v;
+        v.rows = GM ? w.rows : srows;
         v.Z = w.Z;
         v.nw = w.nw;
-        v.fmine = reinterpret_cast<uint8_t*>(srows) + slab_flag_offset(bytes);
-        v.fleft = left ? reinterpret_cast<uint8_t*>(left) + slab_flag_offset((uint32_t)(v.lo - v.left_lo) * row_bytes)
-                       : nullptr;
-        if (threadIdx.x == 0 && bytes) bulk_load(srows, gslab, bytes, bytes + tx_extra, &bar);
+        v.flags = reinterpret_cast<uint8_t*>(srows) + slab_flag_offset(bytes);
+        v.stride = WorldView::flag_stride(w.Y);
+        if (threadIdx.x == 0 && bytes) bulk_load(srows, w.rows, bytes, bytes + tx_extra, &bar);
         if (threadIdx.x < 2) {
             s_nbz[threadIdx.x] = (uint32_t)nblocks(w.Z, (int)threadIdx.x);
             s_magic[threadIdx.x] = 0xFFFFFFFFu / (uint32_t)nblocks(w.Z, (int)threadIdx.x) + 1u;
@@ -572,13 +535,13 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
         // that changed the layer), or every layer changed at t0 - 1 and t0 - 2
         {
             const bool kept = w.lflags != nullptr && !w.lflags_fresh;
-            const uint32_t t0b = (uint32_t)w.t & 3u, fs = SlabView<CL>::flag_stride(v.hi - v.lo);
-            for (int i = threadIdx.x; i < v.hi - v.lo; i += NT) {
-                const uint32_t age = kept ? (((uint32_t)w.t - (uint32_t)w.lflags[v.lo + i]) & 0xFFu) : 0u;
-                v.fmine[((t0b + 3u) & 3u) * fs + i] = kept ? (age == 1u) : 1u;
-                v.fmine[((t0b + 2u) & 3u) * fs + i] = kept ? (age == 2u) : 1u;
-                v.fmine[t0b * fs + i] = 0u;
-                v.fmine[((t0b + 1u) & 3u) * fs + i] = 0u;
+            const uint32_t t0b = (uint32_t)w.t & 3u, fs = v.stride;
+            for (int i = threadIdx.x; i < w.Y; i += NT) {
+                const uint32_t age = kept ? (((uint32_t)w.t - (uint32_t)w.lflags[i]) & 0xFFu) : 0u;
+                v.flags[((t0b + 3u) & 3u) * fs + i] = kept ? (age == 1u) : 1u;
+                v.flags[((t0b + 2u) & 3u) * fs + i] = kept ? (age == 2u) : 1u;
+                v.flags[t0b * fs + i] = 0u;
+                v.flags[((t0b + 1u) & 3u) * fs + i] = 0u;
             }
         }
         bool ok = true;
@@ -594,12 +557,11 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
         const bool poisoned = __syncthreads_or(!ok) != 0;
         if (poisoned && threadIdx.x == 0 && atomicCAS(err, 0, 1) == 0)
             *reinterpret_cast<unsigned long long*>(err + 2) = (unsigned long long)w.t;
-        group_sync();  // every slab is loaded before a neighbour reads it
-        const int G = 1 << w.lg, per = NT >> w.lg;
+                const int G = 1 << w.lg, per = NT >> w.lg;
         const int gl = lane & (G - 1);
-        // layer pairs to evaluate in a step (16-bit offsets from j_lo), after the buffers
-        const uint32_t fs = SlabView<CL>::flag_stride(v.hi - v.lo);
-        uint16_t* jlist = reinterpret_cast<uint16_t*>(v.fmine + 4u * fs);
+        // layer pairs to evaluate in a step, after the buffers
+        const uint32_t fs = v.stride;
+        uint16_t* jlist = reinterpret_cast<uint16_t*>(v.flags + 4u * fs);
         for (int s = 0; s < w.steps; ++s) {
             if ((s & (kKeys - 1)) == 0) {
                 // the next kKeys steps' keys, one thread each (the previous step's
@@ -609,18 +571,17 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
                 __syncthreads();
             }
             if (poisoned) {
-                group_sync();
+                __syncthreads();
                 continue;
             }
             const uint64_t t = w.t + (uint64_t)s;
             const int o = (int)(t & 1u);
             const uint32_t sk = s_keys[s & (kKeys - 1)];
             const int NBZ = (int)s_nbz[o];
-            const int j_lo = v.lo / 2, j_hi = (r == CS - 1) ? nblocks(w.Y, o) : v.hi / 2;
-            const int nj = j_hi - j_lo;
+            const int nj = nblocks(w.Y, o);
             const uint32_t tb = (uint32_t)t & 3u;
             // the buffer the next step writes: read and written by no one in this step
-            for (int i = threadIdx.x; i < v.hi - v.lo; i += NT) v.fmine[((tb + 1u) & 3u) * fs + i] = 0u;
+            for (int i = threadIdx.x; i < w.Y; i += NT) v.flags[((tb + 1u) & 3u) * fs + i] = 0u;
             // dirty layer pairs: up to 96 as bit masks every warp computes for
             // itself (the buffers it reads are not written in this step), more
             // through the shared list
@@ -629,9 +590,9 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
             const bool masked = nj <= kMasked;
             uint8_t* list = s_list[threadIdx.x >> 5];
             if (masked) {
-                dm0 = __ballot_sync(0xFFFFFFFFu, lane < nj && layer_dirty(v, w, o, tb, j_lo + lane));
-                if (nj > 32) dm1 = __ballot_sync(0xFFFFFFFFu, lane + 32 < nj && layer_dirty(v, w, o, tb, j_lo + 32 + lane));
-                if (nj > 64) dm2 = __ballot_sync(0xFFFFFFFFu, lane + 64 < nj && layer_dirty(v, w, o, tb, j_lo + 64 + lane));
+                dm0 = __ballot_sync(0xFFFFFFFFu, lane < nj && layer_dirty(v, w, o, tb, lane));
+                if (nj > 32) dm1 = __ballot_sync(0xFFFFFFFFu, lane + 32 < nj && layer_dirty(v, w, o, tb, 32 + lane));
+                if (nj > 64) dm2 = __ballot_sync(0xFFFFFFFFu, lane + 64 < nj && layer_dirty(v, w, o, tb, 64 + lane));
                 n_layers = __popc(dm0) + __popc(dm1) + __popc(dm2);
                 if (kListed) {
                     __syncwarp();  // the last step's readers are done
@@ -648,7 +609,7 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
                 int* cnt = &s_count[s & 1];
                 for (int base = 0; base < nj; base += NT) {
                     const int i = base + (int)threadIdx.x;
-                    const bool add = i < nj && layer_dirty(v, w, o, tb, j_lo + i);
+                    const bool add = i < nj && layer_dirty(v, w, o, tb, i);
                     const uint32_t m = __ballot_sync(0xFFFFFFFFu, add);
                     if (m) {
                         int pos = 0;
@@ -665,8 +626,8 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
                 // cells evaluated: the rows of every dirty layer pair inside the world, X*Z cells each
                 int rows = 2 * n_layers;
                 if (n_layers) {
-                    if (2 * j_lo - o < 0 && layer_dirty(v, w, o, tb, j_lo)) --rows;
-                    if (2 * (j_hi - 1) - o + 1 >= w.Y && layer_dirty(v, w, o, tb, j_hi - 1)) --rows;
+                    if (o && layer_dirty(v, w, o, tb, 0)) --rows;
+                    if (2 * (nj - 1) - o + 1 >= w.Y && layer_dirty(v, w, o, tb, nj - 1)) --rows;
                 }
                 s_processed += (unsigned long long)rows * (unsigned long long)(w.X * w.Z);
             }
@@ -693,22 +654,22 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
                     else
                         jj = 64 + select_bit(dm2, jd - __popc(dm0) - __popc(dm1));
                 }
-                slab_rowpair(v, w, o, sk, tb, j_lo + jj, kk, valid, gl, G);
+                world_rowpair(v, w, o, sk, tb, jj, kk, valid, gl, G);
             }
-            group_sync();
+            __syncthreads();
         }
         if (w.lflags && !poisoned) {
             // kept for the next segment: the last of the final two steps that changed the layer
             const uint64_t te = w.t + (uint64_t)w.steps;
             const uint32_t b1 = (uint32_t)(te - 1u) & 3u, b2 = (uint32_t)(te - 2u) & 3u;
-            for (int i = threadIdx.x; i < v.hi - v.lo; i += NT)
-                w.lflags[v.lo + i] = (uint8_t)(v.fmine[b1 * fs + i] ? te - 1u : (v.fmine[b2 * fs + i] ? te - 2u : te - 3u));
+            for (int i = threadIdx.x; i < w.Y; i += NT)
+                w.lflags[i] = (uint8_t)(v.flags[b1 * fs + i] ? te - 1u : (v.flags[b2 * fs + i] ? te - 2u : te - 3u));
         }
         // make the threads' shared-memory writes visible to the bulk copy
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (threadIdx.x == 0 && bytes && !poisoned) bulk_store_wait(gslab, srows, bytes);
-        group_sync();  // the slab is free again (and no neighbour still reads it)
+        if (threadIdx.x == 0 && bytes && !poisoned) bulk_store_wait(w.rows, srows, bytes);
+        __syncthreads();  // the buffer is free again
     }
     __syncthreads();
     if (threadIdx.x == 0 && processed_cells && s_processed) atomicAdd(processed_cells, s_processed);
@@ -720,18 +681,18 @@ __global__ void __launch_bounds__(NT, CL ? 1 : (GM ? kGmThreadsPerSm / NT : resi
 namespace {
 
 struct ResidentCfg {
-    int threads, ctas_per_sm, cs;
+    int threads, ctas_per_sm;
     int smem;  // dynamic shared memory per CTA (bytes), 0 = class unavailable
     const void* fn;
 };
 
 // filled once per process (the first device the library is used on), from any thread
-ResidentCfg g_classes[kResidentClasses];
+ResidentCfg g_classes[kSingleCtaClasses];
 std::once_flag g_classes_once;
 
-template <int NT, bool CL>
+template <int NT>
 const void* resident_fn() {
-    return reinterpret_cast<const void*>(&k_plane_segment_resident<NT, CL>);
+    return reinterpret_cast<const void*>(&k_plane_segment_resident<NT>);
 }
 
 void fill_classes() {
@@ -741,14 +702,10 @@ void fill_classes() {
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
     const int kStatic = 256;  // the kernel's own shared variables, rounded up
-    const ResidentCfg base[kResidentClasses] = {
-        {128, resident_ctas_per_sm<128>(), 1, 0, resident_fn<128, false>()},
-        {256, resident_ctas_per_sm<256>(), 1, 0, resident_fn<256, false>()},
-        {768, resident_ctas_per_sm<768>(), 1, 0, resident_fn<768, false>()},
-        {512, 1, 2, 0, resident_fn<512, true>()},
-        {512, 1, 4, 0, resident_fn<512, true>()},
-        {512, 1, 8, 0, resident_fn<512, true>()}};
-    for (int c = 0; c < kResidentClasses; ++c) {
+    const ResidentCfg base[kSingleCtaClasses] = {{128, resident_ctas_per_sm<128>(), 0, resident_fn<128>()},
+                                                 {256, resident_ctas_per_sm<256>(), 0, resident_fn<256>()},
+                                                 {768, resident_ctas_per_sm<768>(), 0, resident_fn<768>()}};
+    for (int c = 0; c < kSingleCtaClasses; ++c) {
         ResidentCfg k = base[c];
         int stat = kStatic;
         cudaFuncAttributes fa;
@@ -775,18 +732,14 @@ void init_classes() { std::call_once(g_classes_once, fill_classes); }
 
 int resident_class(int X, int Y, int Z) {
     init_classes();
-    const int64_t row_bytes = (int64_t)Z * plane_nw(X) * 16;
-    for (int c = 0; c < kResidentClasses; ++c) {
-        const ResidentCfg& k = g_classes[c];
-        if (!k.smem) continue;
-        // every slab holds at most 2*ceil(NYP/CS) rows (NYP = row pairs); each
-        // slab must be non-empty so the row below a slab is in its neighbour
-        const int64_t nyp = (Y + 1) / 2;
-        const int64_t mx = k.cs == 1 ? Y : 2 * ((nyp + k.cs - 1) / k.cs);
+    const int64_t planes = (int64_t)Y * Z * plane_nw(X) * 16;
+    for (int c = 0; c < kSingleCtaClasses; ++c) {
         // planes, then the layer flags and the layer list
-        const int64_t need = ((mx * row_bytes + 15) & ~(int64_t)15) + (int64_t)slab_aux_bytes((uint32_t)mx);
-        if (need <= k.smem && (k.cs == 1 || nyp >= k.cs)) return c;
+        const int64_t need = ((planes + 15) & ~(int64_t)15) + (int64_t)slab_aux_bytes((uint32_t)Y);
+        if (g_classes[c].smem && need <= g_classes[c].smem) return c;
     }
+    for (int c = kSingleCtaClasses; c < kResidentClasses; ++c)
+        if (batch_slabs_fit(X, Y, Z, kClusterSizes[c - kSingleCtaClasses])) return c;
     return -1;
 }
 
@@ -834,8 +787,8 @@ static cudaError_t launch_gm(int cls, int grid, size_t smem, cudaStream_t st, co
     }
     lc.attrs = attr;
     lc.numAttrs = first ? 1 : 0;
-    return cudaLaunchKernelEx(&lc, k_plane_segment_resident<NT, false, true>, worlds, order, meta,
-                              kResidentClasses + cls, 1, counter, err, processed_cells);
+    return cudaLaunchKernelEx(&lc, k_plane_segment_resident<NT, true>, worlds, order, meta,
+                              kResidentClasses + cls, counter, err, processed_cells);
 }
 
 fs3d_status launch_plane_segment_gm(int cls, const PlaneWorld* worlds, const int* order, const int* meta,
@@ -844,11 +797,11 @@ fs3d_status launch_plane_segment_gm(int cls, const PlaneWorld* worlds, const int
     if (cls < 0 || cls >= kGmClasses) return set_error(FS3D_ERR_INVALID_ARG, "global-memory class out of range");
     std::call_once(g_gm_once, [] {
         // the planes are read through L1: leave most of the unified memory to it
-        const void* fns[kGmClasses] = {reinterpret_cast<const void*>(&k_plane_segment_resident<32, false, true>),
-                                       reinterpret_cast<const void*>(&k_plane_segment_resident<64, false, true>),
-                                       reinterpret_cast<const void*>(&k_plane_segment_resident<128, false, true>),
-                                       reinterpret_cast<const void*>(&k_plane_segment_resident<256, false, true>),
-                                       reinterpret_cast<const void*>(&k_plane_segment_resident<768, false, true>)};
+        const void* fns[kGmClasses] = {reinterpret_cast<const void*>(&k_plane_segment_resident<32, true>),
+                                       reinterpret_cast<const void*>(&k_plane_segment_resident<64, true>),
+                                       reinterpret_cast<const void*>(&k_plane_segment_resident<128, true>),
+                                       reinterpret_cast<const void*>(&k_plane_segment_resident<256, true>),
+                                       reinterpret_cast<const void*>(&k_plane_segment_resident<768, true>)};
         for (const void* fn : fns) cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 50);
         cudaGetLastError();
     });
@@ -873,7 +826,8 @@ fs3d_status launch_plane_segment_gm(int cls, const PlaneWorld* worlds, const int
 }
 
 fs3d_status set_inject_tx_extra(uint32_t bytes) {
-    set_slab_tx_extra(bytes);
+    const fs3d_status s = set_slab_tx_extra(bytes);
+    if (s != FS3D_OK) return s;
     FS3D_CUDA(cudaMemcpyToSymbol(g_inject_tx_extra, &bytes, sizeof(bytes)));
     return FS3D_OK;
 }
@@ -881,37 +835,16 @@ fs3d_status set_inject_tx_extra(uint32_t bytes) {
 fs3d_status launch_plane_segment_resident(int cls, const PlaneWorld* worlds, const int* order, const int* meta,
                                           int* counter, int* err, cudaStream_t st,
                                           unsigned long long* processed_cells) {
+    if (cls < 0 || cls >= kSingleCtaClasses) return set_error(FS3D_ERR_INVALID_ARG, "resident class out of range");
     init_classes();
     const ResidentCfg& k = g_classes[cls];
     if (!k.smem) return set_error(FS3D_ERR_CUDA, "resident segment kernel unavailable for this class");
     FS3D_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), st));
-    const int groups = sm_count_public() * k.ctas_per_sm / k.cs;
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)(groups * k.cs));
-    lc.blockDim = dim3((unsigned)k.threads);
-    lc.dynamicSmemBytes = (size_t)k.smem;
-    lc.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)k.cs;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    lc.attrs = attr;
-    lc.numAttrs = k.cs > 1 ? 1 : 0;
-    const int CS = k.cs;
-    cudaError_t e;
-    if (k.cs > 1)
-        e = cudaLaunchKernelEx(&lc, k_plane_segment_resident<512, true>, worlds, order, meta, cls, CS, counter, err,
-                               processed_cells);
-    else if (k.threads == 128)
-        e = cudaLaunchKernelEx(&lc, k_plane_segment_resident<128, false>, worlds, order, meta, cls, CS, counter, err,
-                               processed_cells);
-    else if (k.threads == 256)
-        e = cudaLaunchKernelEx(&lc, k_plane_segment_resident<256, false>, worlds, order, meta, cls, CS, counter, err,
-                               processed_cells);
-    else
-        e = cudaLaunchKernelEx(&lc, k_plane_segment_resident<768, false>, worlds, order, meta, cls, CS, counter, err,
-                               processed_cells);
+    const unsigned grid = (unsigned)(sm_count_public() * k.ctas_per_sm);
+    auto fn = k.threads == 128 ? &k_plane_segment_resident<128>
+                               : (k.threads == 256 ? &k_plane_segment_resident<256> : &k_plane_segment_resident<768>);
+    fn<<<grid, (unsigned)k.threads, (size_t)k.smem, st>>>(worlds, order, meta, cls, counter, err, processed_cells);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "resident segment launch");
     note_launch();
     return FS3D_OK;

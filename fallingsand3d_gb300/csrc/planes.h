@@ -37,9 +37,10 @@ constexpr int kPlaneMaxX = 2048;  // lane groups of at most 32 words
 // Resident segment classes: worlds whose planes fit in shared memory take
 // all their segment steps in one launch.  Classes 0..2 hold a world in one CTA
 // of 128 / 256 / 768 threads (6 / 3 / 1 CTAs per SM); classes 3..5 split a
-// world into y-slabs over a cluster of 2 / 4 / 8 CTAs of 512 threads.
+// world into z-slabs over a cluster of 2 / 4 / 8 CTAs.
 constexpr int kResidentClasses = 6;
 constexpr int kSingleCtaClasses = 3;  // classes 0..2 hold a world in one CTA
+constexpr int kClusterSizes[3] = {2, 4, 8};
 // Global-memory segment classes (the world stays in L2/HBM; one CTA of
 // 32/64/128/256 threads per world, by the work of one layer pair; -1 if the
 // world has too many layers), and kGmDense: one CTA of 768 threads per SM
@@ -60,8 +61,9 @@ constexpr int kErrInts = 4;  // size of the error record a resident launch is gi
 fs3d_status set_inject_tx_extra(uint32_t bytes);
 // test hook: the next n stream-ordered allocations of batch admissions fail as out of memory
 void set_inject_alloc_failures(int n);
-// One launch steps every world of class `cls` (order[meta[1+K+cls] ...],
-// meta[1+cls] of them) through its segment steps in shared memory.  err
+// One launch steps every world of the single-CTA class `cls`
+// (order[meta[1+K+cls] ...], meta[1+cls] of them) through its segment steps in
+// shared memory.  err
 // points to 4 ints (8-byte aligned): a bulk copy that does not complete
 // within the wait limit sets err[0] = 1 and err[2..3] = the failing world's
 // step at the start of the launch (first failure only); while err[0] is set,
@@ -192,7 +194,16 @@ bool prefer_slabs(int X, int Y, int Z, int n_steps, SlabPlan* out);
 // to call), err as for launch_plane_segment_resident
 fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_t* rflags, void* scratch, int* err,
                                cudaStream_t st);
-void set_slab_tx_extra(uint32_t bytes);  // test hook, as set_inject_tx_extra
+fs3d_status set_slab_tx_extra(uint32_t bytes);  // test hook, as set_inject_tx_extra
+// ---- a batch's worlds of a cluster class: CS CTAs a world, cut along z
+// (slab.cu).  Whether a world's slabs fit; the most words (Y * nw) of a layer
+// at a cut; the bytes of edge buffer a class needs; the launch, as
+// launch_plane_segment_resident.
+constexpr int kBatchSlabEdgeWords = 1024;
+bool batch_slabs_fit(int X, int Y, int Z, int CS);
+size_t batch_slab_edge_bytes(int CS);
+fs3d_status launch_batch_slabs(int cls, int CS, const PlaneWorld* worlds, const int* order, const int* meta, int* counter,
+                               int* err, void* edges, cudaStream_t st, unsigned long long* processed_cells);
 
 fs3d_status planes_hash_async(const uint4* rows, const uint8_t* statics, int X, int Y, int Z,
                               unsigned long long* out_dev, cudaStream_t st);

@@ -1,4 +1,5 @@
-// Many steps of one world in one launch over the whole GPU.
+// Many steps of one world by several CTAs: over the whole GPU (one world in one
+// launch) or by one thread-block cluster (a batch's large young worlds).
 //
 // The world is cut along y or z into slabs of whole layer pairs, one CTA per
 // slab, and each CTA keeps its slab's planes and row flags in shared memory
@@ -18,7 +19,8 @@
 // word is stored again by the lane that read it, so a word is never
 // overwritten before it was read.
 //
-// All CTAs are resident at once (cooperative launch).  Every wait is bounded
+// All CTAs of a world are resident at once (a cooperative launch, or a
+// cluster).  Every wait is bounded
 // in time; the planes and flags in global memory are written only once every
 // CTA has taken all the steps (one of the CTAs decides: the last to arrive
 // commits, one that gives up aborts, whichever is first), so a launch that
@@ -33,8 +35,9 @@
 // 12, 200^3 4.1 / 3.5 against 6.5 / 7.3, 256^3 4.9 / 3.7 against 7.1 / 8.2.
 #include <stdint.h>
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
-#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -48,6 +51,11 @@ namespace fs3d {
 namespace {
 
 constexpr int kSlabKeys = 32;  // step keys computed together
+constexpr int kBatchSlabThreads = 640;
+
+// Test hook (fs3d_test_inject), as the resident kernels': bytes announced on
+// the mbarrier beyond what the bulk copies deliver.  0 in normal operation.
+static __device__ uint32_t g_slab_tx_extra;
 
 // The launch's shared words, zeroed before it, at the start of the scratch;
 // the edge buffer follows at kSlabEdgeOff.
@@ -80,17 +88,18 @@ __device__ __forceinline__ bool edge_try(const unsigned long long* p, uint32_t s
 }
 
 // Waits for the edge words at p0 and p1 (each nullable) to have taken `step`
-// steps.  False if it gave up: the wait's limit, a verdict reached without
-// this CTA, or *dead set by another of its threads.
+// steps.  False if it gave up: the wait's limit, *stop set (a verdict reached
+// without this CTA, or an error recorded), or *dead set by another of its
+// threads.
 __device__ __forceinline__ bool edge_read(const unsigned long long* p0, const unsigned long long* p1, uint32_t step,
-                                          const SlabState* st, const volatile int* dead, uint4& q0, uint4& q1,
+                                          const int* stop, const volatile int* dead, uint4& q0, uint4& q1,
                                           bool& ch0, bool& ch1) {
     unsigned long long t0 = 0;
     for (uint32_t it = 0;; ++it) {
         const bool ok0 = !p0 || edge_try(p0, step, q0, ch0), ok1 = !p1 || edge_try(p1, step, q1, ch1);
         if (ok0 && ok1) return true;
         if ((it & 255u) == 255u) {
-            if (*dead || *(volatile const int*)&st->verdict) return false;
+            if (*dead || *(volatile const int*)stop) return false;
             const unsigned long long now = global_ns();
             if (!t0)
                 t0 = now;
@@ -117,57 +126,93 @@ struct SlabTask {
     bool cut;         // the pair's rows of one layer are the cut's
 };
 
-// ZS: the slabs are cut along z (else along y).  MAXT: the most threads.
-// READY: the draws of a row-pair are hashed before its cut's words are waited
-// for (few warps per SM: a step is one warp's chain of instructions and the
-// words' way through L2, and the hashing hides in the latter), else slot by
-// slot where needed (more warps: the instructions count).
+// What CTA r of C holds of a world cut along z (ZS) or y.
+template <bool ZS>
+struct SlabGeo {
+    int NO;          // the world's size along the other axis
+    bool first, last;
+    int lo, hi;      // its layers along the cut axis
+    int keep;        // layers lo .. keep-1 are held here, layer hi-1 of an inner slab in the edge buffer
+    int layers;
+    int row_ys, row_off;  // shared-memory row of (y, z): y * row_ys + z + row_off
+    int fl_ys, fl_off;    // row flag, of layers lo-1 .. hi-1 (the edge layers' too)
+    uint32_t bytes;       // of the planes held
+    __device__ __forceinline__ SlabGeo(const PlaneWorld& w, int r, int C) {
+        const int NS = ZS ? w.Z : w.Y, NP = (NS + 1) >> 1;
+        NO = ZS ? w.Y : w.Z;
+        first = r == 0;
+        last = r == C - 1;
+        lo = 2 * (int)((int64_t)r * NP / C);
+        hi = last ? NS : 2 * (int)((int64_t)(r + 1) * NP / C);
+        keep = last ? hi : hi - 1;
+        layers = keep - lo;
+        row_ys = ZS ? layers : w.Z;
+        row_off = ZS ? -lo : -lo * w.Z;
+        fl_ys = ZS ? hi - lo + 1 : w.Z;
+        fl_off = ZS ? 1 - lo : (1 - lo) * w.Z;
+        bytes = (uint32_t)layers * (uint32_t)NO * (uint32_t)w.nw * 16u;
+    }
+    // (y, z) of row flag i
+    __device__ __forceinline__ void flag_at(const PlaneWorld& w, int i, int& y, int& z) const {
+        y = ZS ? i / fl_ys : lo - 1 + i / w.Z;
+        z = ZS ? lo - 1 + i % fl_ys : i % w.Z;
+    }
+    __device__ __forceinline__ int flags() const { return (hi - lo + 1) * NO; }
+    // the planes into shared memory, as bulk copies on `bar` (told to expect them)
+    __device__ __forceinline__ void load(const PlaneWorld& w, uint4* srows, uint64_t* bar) const {
+        const int pieces = ZS ? w.Y : 1;
+        const uint32_t pb = bytes / (uint32_t)pieces;
+        for (int i = threadIdx.x; i < pieces; i += blockDim.x) {
+            const uint4* src = w.rows + (ZS ? ((int64_t)i * w.Z + lo) * w.nw : (int64_t)lo * w.Z * w.nw);
+            bulk_copy_in(reinterpret_cast<uint8_t*>(srows) + (size_t)i * pb, src, pb, bar);
+        }
+    }
+    // the edge layer this CTA took the last step of (-1: none); o: that step's phase
+    __device__ __forceinline__ int last_edge(int o) const { return o ? (first ? -1 : lo - 1) : (last ? -1 : hi - 1); }
+    // the planes back, and the edge layer el from the edge buffer (r: this CTA, o as above)
+    __device__ __forceinline__ void store(const PlaneWorld& w, const uint4* srows, const unsigned long long* edge, int r,
+                                          int o) const {
+        const int nw = w.nw, el = last_edge(o);
+        for (int i = threadIdx.x; i < layers * NO * nw; i += blockDim.x) {
+            const int row = i / nw, g = i - row * nw;
+            const int y = ZS ? row / layers : lo + row / w.Z, z = ZS ? lo + row % layers : row % w.Z;
+            w.rows[((int64_t)y * w.Z + z) * nw + g] = srows[i];
+        }
+        if (el < 0) return;
+        const unsigned long long* eb = edge + (size_t)(o ? r - 1 : r) * NO * nw * 4;
+        for (int i = threadIdx.x; i < NO * nw; i += blockDim.x) {
+            unsigned long long a, b, c, d;
+            ld_tagged(eb + 4 * (size_t)i, a, b);
+            ld_tagged(eb + 4 * (size_t)i + 2, c, d);
+            const int row = i / nw, g = i - row * nw;
+            const int y = ZS ? row : el, z = ZS ? el : row;
+            w.rows[((int64_t)y * w.Z + z) * nw + g] = make_uint4((uint32_t)a, (uint32_t)b, (uint32_t)c, (uint32_t)d);
+        }
+    }
+    // whether the row flag of (y, z) is this CTA's to report
+    __device__ __forceinline__ bool owns(int y, int z, int o) const {
+        const int sl = ZS ? z : y, el = last_edge(o);
+        return (sl >= lo && sl < keep) || (el >= 0 && sl == el);
+    }
+};
+
+// The steps of CTA r's slab (planes in srows, row flags in rf).  ZS, READY: the
+// draws of a row-pair are hashed before its cut's words are waited for (few
+// warps per SM: a step is one warp's chain of instructions and the words' way
+// through L2, and the hashing hides in the latter), else slot by slot where
+// needed (more warps: the instructions count).  True if it gave up (or came in
+// dead).  rows_done: the rows of the row-pairs this lane evaluated.
 // Threads work in lane groups of 1 << lg, one block row-pair at a time, as
 // the per-step kernel does; row-pairs none of whose rows changed in the two
 // previous steps are skipped (same argument, same row flags).
-template <bool ZS, int MAXT, bool READY>
-__global__ void __launch_bounds__(MAXT, 1)
-    k_plane_slabs(const PlaneWorld w, uint8_t* __restrict__ rflags, SlabState* st, unsigned long long* edge, int* err,
-                  uint32_t tx_extra) {
-    extern __shared__ __align__(128) uint4 srows[];
-    __shared__ __align__(8) uint64_t bar;
-    __shared__ uint32_t s_keys[kSlabKeys];
-    __shared__ int s_dead, s_verdict;  // s_dead: some thread gave up (a hint to the others' waits)
-    const int C = gridDim.x, r = blockIdx.x, NT = blockDim.x, tid = threadIdx.x;
-    const int NS = ZS ? w.Z : w.Y, NO = ZS ? w.Y : w.Z;  // along the cut axis, and the other one
-    const int NP = (NS + 1) >> 1;
-    const bool first = r == 0, last = r == C - 1;
-    const int lo = 2 * (int)((int64_t)r * NP / C), hi = last ? NS : 2 * (int)((int64_t)(r + 1) * NP / C);
-    const int keep = last ? hi : hi - 1;  // layers lo .. keep-1 are held here, layer hi-1 of an inner slab in `edge`
-    const int nw = w.nw, layers = keep - lo;
-    // shared-memory rows: y-cut (y - lo)*Z + z, z-cut y*layers + (z - lo)
-    const int row_ys = ZS ? layers : w.Z, row_off = ZS ? -lo : -lo * w.Z;
-    // row flags of layers lo-1 .. hi-1 (the edge layers' too)
-    const int fl_ys = ZS ? hi - lo + 1 : w.Z, fl_off = ZS ? 1 - lo : (1 - lo) * w.Z;
-    const uint32_t bytes = (uint32_t)layers * (uint32_t)NO * (uint32_t)nw * 16u;
-    uint8_t* rf = reinterpret_cast<uint8_t*>(srows) + bytes;
-    if (tid == 0) {
-        mbar_init(&bar, 1);
-        s_dead = 0;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&bar)), "r"(bytes + tx_extra)
-                     : "memory");
-    }
-    // an error recorded earlier: nothing is stepped (and every CTA's load is skipped or waited for)
-    bool dead = __syncthreads_or(tid == 0 && *(volatile int*)err != 0) != 0;
-    if (!dead) {
-        const int pieces = ZS ? w.Y : 1;
-        const uint32_t pb = bytes / (uint32_t)pieces;
-        for (int i = tid; i < pieces; i += NT) {
-            const uint4* src = w.rows + (ZS ? ((int64_t)i * w.Z + lo) * nw : (int64_t)lo * w.Z * nw);
-            bulk_copy_in(reinterpret_cast<uint8_t*>(srows) + (size_t)i * pb, src, pb, &bar);
-        }
-        for (int i = tid; i < (hi - lo + 1) * NO; i += NT) {
-            const int y = ZS ? i / fl_ys : lo - 1 + i / w.Z, z = ZS ? lo - 1 + i % fl_ys : i % w.Z;
-            rf[i] = (y >= 0 && z >= 0) ? rflags[(int64_t)y * w.Z + z] : 0;
-        }
-        const bool ok = mbar_wait(&bar, 0, tx_extra ? kCopyWaitInjectedNs : kCopyWaitNs);
-        dead = __syncthreads_or(!ok) != 0;
-    }
+template <bool ZS, bool READY>
+__device__ __forceinline__ bool slab_steps(const PlaneWorld& w, const SlabGeo<ZS>& geo, int r, uint4* srows, uint8_t* rf,
+                                           unsigned long long* edge, const int* stop, volatile int* s_dead,
+                                           uint32_t* s_keys, bool dead, uint32_t& rows_done) {
+    const int NO = geo.NO, lo = geo.lo, hi = geo.hi, row_ys = geo.row_ys, row_off = geo.row_off, fl_ys = geo.fl_ys,
+              fl_off = geo.fl_off;
+    const bool first = geo.first, last = geo.last;
+    const int tid = threadIdx.x, NT = blockDim.x, nw = w.nw;
     const int lane = tid & 31, lg = w.lg, G = 1 << lg, per = NT >> lg, gl = lane & (G - 1);
     const uint32_t gmask = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << (lane & ~(G - 1));
     const bool half_at_end = (w.X & 63) == 0;
@@ -238,7 +283,7 @@ __global__ void __launch_bounds__(MAXT, 1)
                 if (p1) q[E1] = at(k.c0 + 1);
             } else if ((p0 || p1) && !gave_up) {
                 bool ch0 = false, ch1 = false;
-                gave_up = !edge_read(p0, p1, (uint32_t)s, st, &s_dead, q[E0], q[E1], ch0, ch1);
+                gave_up = !edge_read(p0, p1, (uint32_t)s, stop, s_dead, q[E0], q[E1], ch0, ch1);
                 if (ch0) rf[flag(E0)] = (uint8_t)(tb - 1u);
                 if (ch1) rf[flag(E1)] = (uint8_t)(tb - 1u);
                 if ((ch0 || ch1) && !dirty) {
@@ -251,6 +296,7 @@ __global__ void __launch_bounds__(MAXT, 1)
             some = __any_sync(0xFFFFFFFFu, dirty);
             if (READY && some && !had) ready.fill(rk, (uint32_t)gl);
         }
+        if (dirty && gl == 0) rows_done += __popc(k.in);
         uint32_t chg = 0;  // bit a: row a changed in this lane's word
         if (some) {
             uint4 q0[4];
@@ -308,9 +354,43 @@ __global__ void __launch_bounds__(MAXT, 1)
                 for (int e = tid >> lg, n = tasks(0); e - (tid >> lg) < n; e += per)
                     evaluate(std::integral_constant<int, 0>(), task(0, e), s, tb, sk);
         }
-        if (gave_up) s_dead = 1;
+        if (gave_up) *s_dead = 1;
         dead = __syncthreads_or(gave_up) != 0;
     }
+    return dead;
+}
+
+// One world over the whole GPU.  MAXT: the most threads.
+template <bool ZS, int MAXT, bool READY>
+__global__ void __launch_bounds__(MAXT, 1)
+    k_plane_slabs(const PlaneWorld w, uint8_t* __restrict__ rflags, SlabState* st, unsigned long long* edge, int* err) {
+    extern __shared__ __align__(128) uint4 srows[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t s_keys[kSlabKeys];
+    __shared__ int s_dead, s_verdict;  // s_dead: some thread gave up (a hint to the others' waits)
+    const int C = gridDim.x, r = blockIdx.x, tid = threadIdx.x;
+    const SlabGeo<ZS> geo(w, r, C);
+    const uint32_t tx_extra = g_slab_tx_extra;
+    uint8_t* rf = reinterpret_cast<uint8_t*>(srows) + geo.bytes;
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        s_dead = 0;
+        mbar_expect(&bar, geo.bytes + tx_extra);
+    }
+    // an error recorded earlier: nothing is stepped (and every CTA's load is skipped or waited for)
+    bool dead = __syncthreads_or(tid == 0 && *(volatile int*)err != 0) != 0;
+    if (!dead) {
+        geo.load(w, srows, &bar);
+        for (int i = tid; i < geo.flags(); i += blockDim.x) {
+            int y, z;
+            geo.flag_at(w, i, y, z);
+            rf[i] = (y >= 0 && z >= 0) ? rflags[(int64_t)y * w.Z + z] : 0;
+        }
+        const bool ok = mbar_wait(&bar, 0, tx_extra ? kCopyWaitInjectedNs : kCopyWaitNs);
+        dead = __syncthreads_or(!ok) != 0;
+    }
+    uint32_t rows_done = 0;
+    dead = slab_steps<ZS, READY>(w, geo, r, srows, rf, edge, &st->verdict, &s_dead, s_keys, dead, rows_done);
     // the verdict: commit when every CTA has taken all the steps
     if (tid == 0) {
         if (dead)
@@ -331,31 +411,100 @@ __global__ void __launch_bounds__(MAXT, 1)
     }
     __syncthreads();
     if (s_verdict != 1) return;
-    for (int i = tid; i < layers * NO * nw; i += NT) {
-        const int row = i / nw, g = i - row * nw;
-        const int y = ZS ? row / layers : lo + row / w.Z, z = ZS ? lo + row % layers : row % w.Z;
-        w.rows[((int64_t)y * w.Z + z) * nw + g] = srows[i];
-    }
-    // an edge layer is written back by the CTA that took its last step
     const int lasto = (int)((w.t + (uint64_t)w.steps - 1u) & 1u);
-    const int el = lasto ? lo - 1 : hi - 1;
-    if (lasto ? !first : !last) {
-        const unsigned long long* eb = edge + (size_t)(lasto ? r - 1 : r) * NO * nw * 4;
-        for (int i = tid; i < NO * nw; i += NT) {
-            unsigned long long a, b, c, d;
-            ld_tagged(eb + 4 * (size_t)i, a, b);
-            ld_tagged(eb + 4 * (size_t)i + 2, c, d);
-            const int row = i / nw, g = i - row * nw;
-            const int y = ZS ? row : el, z = ZS ? el : row;
-            w.rows[((int64_t)y * w.Z + z) * nw + g] = make_uint4((uint32_t)a, (uint32_t)b, (uint32_t)c, (uint32_t)d);
+    geo.store(w, srows, edge, r, lasto);
+    for (int i = tid; i < geo.flags(); i += blockDim.x) {
+        int y, z;
+        geo.flag_at(w, i, y, z);
+        if (geo.owns(y, z, lasto)) rflags[(int64_t)y * w.Z + z] = rf[i];
+    }
+}
+
+// A batch's worlds of one cluster class: each cluster of CS CTAs takes worlds
+// of the class, largest first, from `counter`, and runs each through its
+// segment steps, cut along z.  One SM's 24 warps took 850 to 1020 us for the
+// 64 dense steps of a 128^3 world, which ended the segment of a batch of few
+// such worlds.
+__global__ void __launch_bounds__(kBatchSlabThreads, 1)
+    k_batch_slabs(const PlaneWorld* __restrict__ worlds, const int* __restrict__ order, const int* __restrict__ meta, int cls,
+                  int CS, int* counter, int* err, unsigned long long* processed_cells, unsigned long long* edges) {
+    extern __shared__ __align__(128) uint4 srows[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t s_keys[kSlabKeys];
+    __shared__ int s_dead, item;
+    __shared__ unsigned long long s_processed;
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cluster = cg::this_cluster();
+    const int r = (int)cluster.block_rank(), tid = threadIdx.x, NT = blockDim.x;
+    const int n = meta[1 + cls], off = meta[1 + kAllClasses + cls];
+    unsigned long long* edge = edges + (size_t)(blockIdx.x / CS) * (size_t)(CS - 1) * kBatchSlabEdgeWords * 4;
+    const uint32_t tx_extra = g_slab_tx_extra;
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        s_processed = 0;
+    }
+    __syncthreads();
+    uint32_t phase = 0;
+    for (;;) {
+        // after an error no cluster takes another world
+        if (r == 0 && tid == 0) item = *(volatile int*)err ? n : atomicAdd(counter, 1);
+        if (tid == 0) s_dead = 0;
+        cluster.sync();
+        const int it = *cluster.map_shared_rank(&item, 0);
+        cluster.sync();
+        if (it >= n) break;
+        const PlaneWorld w = worlds[order[off + it]];
+        if (w.steps <= 0) continue;
+        const SlabGeo<true> geo(w, r, CS);
+        uint8_t* rf = reinterpret_cast<uint8_t*>(srows) + geo.bytes;
+        if (tid == 0) mbar_expect(&bar, geo.bytes + tx_extra);
+        __syncthreads();
+        geo.load(w, srows, &bar);
+        // row flags from the layers', or every row changed just before
+        const bool kept = w.lflags != nullptr && !w.lflags_fresh;
+        for (int i = tid; i < geo.flags(); i += NT) {
+            int y, z;
+            geo.flag_at(w, i, y, z);
+            rf[i] = kept ? w.lflags[y] : (uint8_t)(w.t - 1u);
+        }
+        // this CTA's edge words: no tag of another world's left
+        if (!geo.last)
+            for (int i = tid; i < geo.NO * w.nw; i += NT) {
+                st_tagged(edge + ((size_t)r * geo.NO * w.nw + i) * 4, 0, 0);
+                st_tagged(edge + ((size_t)r * geo.NO * w.nw + i) * 4 + 2, 0, 0);
+            }
+        const bool ok = mbar_wait(&bar, phase, tx_extra ? kCopyWaitInjectedNs : kCopyWaitNs);
+        phase ^= 1u;
+        bool dead = __syncthreads_or(!ok) != 0;
+        cluster.sync();
+        uint32_t rows_done = 0;
+        dead = slab_steps<true, false>(w, geo, r, srows, rf, edge, err, &s_dead, s_keys, dead, rows_done);
+        if (dead && tid == 0 && atomicCAS(err, 0, 1) == 0)
+            *reinterpret_cast<unsigned long long*>(err + 2) = (unsigned long long)w.t;
+        rows_done = __reduce_add_sync(0xFFFFFFFFu, rows_done);
+        if ((tid & 31) == 0 && rows_done) atomicAdd(&s_processed, (unsigned long long)rows_done * (unsigned long long)w.X);
+        cluster.sync();
+        const bool write = *(volatile int*)err == 0;
+        const uint64_t te = w.t + (uint64_t)w.steps;
+        const int lasto = (int)((te - 1u) & 1u);
+        if (write) geo.store(w, srows, edge, r, lasto);
+        // layer flags: the last of the final two steps that changed one of the
+        // layer's rows, older ones first (each value by any CTA that has it)
+        if (w.lflags) {
+            if (write && r == 0)
+                for (int y = tid; y < w.Y; y += NT) w.lflags[y] = (uint8_t)(te - 3u);
+            for (uint32_t age = 2; age > 0; --age) {
+                cluster.sync();
+                for (int i = tid; write && i < geo.flags(); i += NT) {
+                    int y, z;
+                    geo.flag_at(w, i, y, z);
+                    if (rf[i] == (uint8_t)(te - age) && geo.owns(y, z, lasto)) w.lflags[y] = (uint8_t)(te - age);
+                }
+            }
         }
     }
-    for (int i = tid; i < (hi - lo + 1) * NO; i += NT) {
-        const int y = ZS ? i / fl_ys : lo - 1 + i / w.Z, z = ZS ? lo - 1 + i % fl_ys : i % w.Z;
-        const int sl = ZS ? z : y;
-        const bool mine = sl >= lo && sl < keep ? true : sl == el && (lasto ? !first : !last);
-        if (mine) rflags[(int64_t)y * w.Z + z] = rf[i];
-    }
+    __syncthreads();
+    if (tid == 0 && processed_cells && s_processed) atomicAdd(processed_cells, s_processed);
 }
 
 struct SlabLimits {
@@ -365,7 +514,7 @@ struct SlabLimits {
 
 constexpr int kSlabThreadsNarrow = 256, kSlabThreadsWide = 640;
 
-using SlabFn = void (*)(const PlaneWorld, uint8_t*, SlabState*, unsigned long long*, int*, uint32_t);
+using SlabFn = void (*)(const PlaneWorld, uint8_t*, SlabState*, unsigned long long*, int*);
 SlabFn slab_fn(bool zs, bool wide) {
     if (zs) return wide ? &k_plane_slabs<true, kSlabThreadsWide, false> : &k_plane_slabs<true, kSlabThreadsNarrow, true>;
     return wide ? &k_plane_slabs<false, kSlabThreadsWide, false> : &k_plane_slabs<false, kSlabThreadsNarrow, true>;
@@ -391,11 +540,57 @@ const SlabLimits& slab_limits() {
     return l;
 }
 
-std::atomic<uint32_t> g_slab_tx_extra{0};  // test hook, as the resident kernels'
-
 }  // namespace
 
-void set_slab_tx_extra(uint32_t bytes) { g_slab_tx_extra.store(bytes); }
+fs3d_status set_slab_tx_extra(uint32_t bytes) {
+    FS3D_CUDA(cudaMemcpyToSymbol(g_slab_tx_extra, &bytes, sizeof(bytes)));
+    return FS3D_OK;
+}
+
+bool batch_slabs_fit(int X, int Y, int Z, int CS) {
+    static const int smem = [] {
+        const int n = slab_limits().smem;
+        const bool ok = n > 0 && cudaFuncSetAttribute(k_batch_slabs, cudaFuncAttributeMaxDynamicSharedMemorySize, n) == cudaSuccess;
+        cudaGetLastError();
+        return ok ? n : 0;
+    }();
+    const int64_t nw = plane_nw(X), NP = (Z + 1) / 2, mp = (NP + CS - 1) / CS;
+    return X <= kPlaneMaxX && NP >= CS && Y * nw <= kBatchSlabEdgeWords && 2 * mp * Y * nw * 16 + (2 * mp + 1) * Y <= smem;
+}
+
+size_t batch_slab_edge_bytes(int CS) {
+    return (size_t)(sm_count_public() / CS) * (size_t)(CS - 1) * kBatchSlabEdgeWords * 32;
+}
+
+fs3d_status launch_batch_slabs(int cls, int CS, const PlaneWorld* worlds, const int* order, const int* meta, int* counter,
+                               int* err, void* edges, cudaStream_t st, unsigned long long* processed_cells) {
+    FS3D_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), st));
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)(sm_count_public() / CS * CS));
+    lc.blockDim = dim3(kBatchSlabThreads);
+    lc.dynamicSmemBytes = (size_t)slab_limits().smem;
+    lc.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)CS;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    // these worlds take the longest: their CTAs are placed before the other classes'
+    static const int greatest = [] {
+        int least = 0, g = 0;
+        if (cudaDeviceGetStreamPriorityRange(&least, &g) != cudaSuccess) g = 0;
+        return g;
+    }();
+    attr[1].id = cudaLaunchAttributePriority;
+    attr[1].val.priority = greatest;
+    lc.attrs = attr;
+    lc.numAttrs = 2;
+    const cudaError_t e = cudaLaunchKernelEx(&lc, k_batch_slabs, worlds, order, meta, cls, CS, counter, err, processed_cells,
+                                             static_cast<unsigned long long*>(edges));
+    if (e != cudaSuccess) return cuda_fail(e, "cluster segment launch");
+    note_launch();
+    return FS3D_OK;
+}
 
 // The cut: along z or y, and how many slabs.  A slab's work is its row-pairs'
 // lanes in a step.  Along z the moving layers of a settled world (a water
@@ -463,7 +658,7 @@ fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_
         lc.attrs = attr;
         lc.numAttrs = 1;
         const SlabFn fn = slab_fn(plan.zs != 0, plan.threads > kSlabThreadsNarrow);
-        const cudaError_t e = cudaLaunchKernelEx(&lc, fn, d, rflags, state, edge, err, g_slab_tx_extra.load());
+        const cudaError_t e = cudaLaunchKernelEx(&lc, fn, d, rflags, state, edge, err);
         if (e != cudaSuccess) return cuda_fail(e, "slab steps launch");
         note_launch();
     }

@@ -1,0 +1,44 @@
+"""A batch's few large young worlds, each stepped by a cluster of CTAs: bit-exact
+to the oracle at the sizes where the slabs' cuts change, over several segments
+(their last ones past the age where worlds leave the clusters)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# one world each: spread over 8 CTAs (or 4, or one, where 8 slabs do not fit)
+SIZES = [(128, 128, 128), (96, 97, 131), (128, 512, 16), (2048, 32, 40), (130, 120, 17), (64, 200, 99), (200, 90, 63)]
+
+
+@pytest.mark.parametrize("dims", SIZES, ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("segment,start", [(64, 0), (1, 3), (7, 120)])
+def test_spread_world_matches_oracle(fs3d, orc, dims, segment, start):
+    X, Y, Z = dims
+    seed, n = X + Y + Z + segment, 3 * segment + 1
+    r = np.random.default_rng(seed)
+    g = r.choice(np.array([0, 1, 2, 3, 9], np.uint8), (Y, Z, X), p=[0.5, 0.04, 0.25, 0.19, 0.02])
+    with fs3d.Batch(1 << 30, steps_per_segment=segment) as b:
+        t = b.admit(g, seed, n, start_step=start)
+        for _ in range(4):
+            b.run_segment()
+        b.sync()
+        c = b.counters()
+        assert 0 < c["processed_cell_steps"] <= c["dense_cell_steps"] == n * g.size
+        got = b.retire(t, g.shape)
+    orc.run(g, seed, start, n, nthreads=0)
+    assert (got == g).all()
+
+
+def test_mixed_young_batch_matches_oracle(fs3d, orc):
+    """Large worlds in clusters beside small ones in their own CTAs."""
+    dims = [(128, 128, 128), (16, 24, 32), (96, 128, 128), (48, 64, 64), (128, 96, 128), (64, 64, 64), (24, 16, 16)]
+    grids = [fs3d.gen_batch_world(7 + i, *d) for i, d in enumerate(dims)]
+    with fs3d.Batch(1 << 30) as b:
+        t = b.admit_many(grids, [7 + i for i in range(len(dims))], 192)
+        for _ in range(3):
+            b.run_segment()
+        outs = [np.empty_like(g) for g in grids]
+        b.retire_many(t, [o.ctypes.data for o in outs])
+    for i, (g, o) in enumerate(zip(grids, outs)):
+        orc.run(g, 7 + i, 0, 192, nthreads=0)
+        assert (o == g).all(), dims[i]
