@@ -26,6 +26,7 @@
 #include "fs3d_common.h"
 #include "pcg.h"
 #include "planes.h"
+#include "conv_device.cuh"
 #include "rule_device.cuh"
 #include "bulk_device.cuh"
 #include "bricks_device.cuh"
@@ -35,48 +36,54 @@ namespace fs3d {
 // ---------------------------------------------------------------------------
 // hashes
 // ---------------------------------------------------------------------------
-// the byte value of one cell of a plane word (static cells from `statics`, or stone)
-__device__ __forceinline__ uint32_t cell_value(const uint4& q, int m, int odd, const uint8_t* statics, int64_t idx) {
-    const uint32_t a = ((odd ? q.y : q.x) >> m) & 1u, b = ((odd ? q.w : q.z) >> m) & 1u;
-    if (a) return b ? 3u : 2u;
-    if (!b) return 0u;
-    return statics ? statics[idx] : 1u;
+// Sum of the hash terms of the chunk of row r at x = 64 w (plane word q).
+// Bound: the 64-bit finalizer's instructions (about 25 a cell), so the cells'
+// bytes come four at a time from the packed conversion.
+__device__ __forceinline__ uint64_t hash_chunk(const uint4& q, const uint8_t* statics, int X, int64_t r, int w) {
+    const int64_t idx = r * X + 64 * w;
+    const int n = min(64, X - 64 * w);
+    uint32_t p[4];
+    planes_to_pieces(q, p);
+    uint64_t h = 0;
+    for (int g = 0; g < 4; ++g) {
+        if (16 * g >= n) break;
+        const uint32_t pg = g == 0 ? p[0] : (g == 1 ? p[1] : (g == 2 ? p[2] : p[3]));
+#pragma unroll
+        for (int x = 0; x < 16; ++x) {
+            const int64_t i = idx + 16 * g + x;
+            uint32_t v = (pg >> (8 * (x & 3) + 2 * (x >> 2))) & 3u;
+            if (16 * g + x < n) {
+                if (statics && v == 1u) v = statics[i];
+                h += fmix64((uint64_t)i * 256u + v);
+            }
+        }
+    }
+    return h;
 }
 
 __global__ void k_hash_planes(const uint4* __restrict__ rows, const uint8_t* __restrict__ statics, int X, int Y,
                               int Z, int nw, unsigned long long* out) {
     const int64_t n = (int64_t)Y * Z * nw;
     uint64_t h = 0;
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-        const int w = (int)(u % nw);
-        const int64_t r = u / nw;
-        const uint4 q = rows[u];
-        for (int x = 64 * w; x < 64 * w + 64 && x < X; ++x) {
-            const int64_t idx = r * X + x;
-            h += fmix64((uint64_t)idx * 256u + cell_value(q, (x >> 1) & 31, x & 1, statics, idx));
-        }
-    }
+    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x)
+        h += hash_chunk(rows[u], statics, X, u / nw, (int)(u % nw));
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) h += __shfl_xor_sync(0xffffffffu, h, off);
     if ((threadIdx.x & 31) == 0 && h) atomicAdd(out, (unsigned long long)h);
 }
 
-// Whole-grid hashes of many worlds in one launch: CTA j hashes world j
-// (jobs[j]) and writes its sum to out[j].
+// Whole-grid hashes of many worlds in one launch: CTA (j, s) sums every
+// gridDim.y-th part of world j (jobs[j]) into out[j * gridDim.y + s].  (One CTA
+// a world left a poll waiting for its largest, up to 128^3 cells in 256 threads:
+// 393 worlds 857 us, in 32 parts each 130; the polls of 1000 served worlds 8.2
+// ms together, now 0.7.)
 __global__ void __launch_bounds__(256) k_hash_planes_many(const HashJob* __restrict__ jobs,
                                                          unsigned long long* __restrict__ out) {
     const HashJob jb = jobs[blockIdx.x];
     const int64_t n = (int64_t)jb.Y * jb.Z * jb.nw;
     uint64_t h = 0;
-    for (int64_t u = threadIdx.x; u < n; u += blockDim.x) {
-        const int w = (int)(u % jb.nw);
-        const int64_t r = u / jb.nw;
-        const uint4 q = jb.rows[u];
-        for (int x = 64 * w; x < 64 * w + 64 && x < jb.X; ++x) {
-            const int64_t idx = r * jb.X + x;
-            h += fmix64((uint64_t)idx * 256u + cell_value(q, (x >> 1) & 31, x & 1, jb.statics, idx));
-        }
-    }
+    for (int64_t u = blockIdx.y * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.y * blockDim.x)
+        h += hash_chunk(jb.rows[u], jb.statics, jb.X, u / jb.nw, (int)(u % jb.nw));
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) h += __shfl_xor_sync(0xffffffffu, h, off);
     __shared__ unsigned long long part[8];
@@ -85,7 +92,7 @@ __global__ void __launch_bounds__(256) k_hash_planes_many(const HashJob* __restr
     if (threadIdx.x == 0) {
         unsigned long long t = 0;
         for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += part[i];
-        out[blockIdx.x] = t;
+        out[(size_t)blockIdx.x * gridDim.y + blockIdx.y] = t;
     }
 }
 
@@ -105,39 +112,48 @@ __device__ __forceinline__ int find_job(const int64_t* __restrict__ unit_off, in
 // The mixed-size batch world generated straight into planes: stone at y < 2,
 // empty below Y/2, and above it one PCG32 draw per cell in index order; each
 // thread jumps its generator to the first draw of its 64-cell word.
-__global__ void k_gen_batch_planes(int X, int Y, int Z, int nw, BatchWorldGen p, uint4* __restrict__ rows) {
-    const int64_t n = (int64_t)Y * Z * nw;
-    const int yf = Y / 2;
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
-        const int w = (int)(u % nw);
-        const int64_t r = u / nw;
-        const int y = (int)(r / Z), z = (int)(r % Z);
-        uint32_t ae = 0, ao = 0, be = 0, bo = 0;
-        uint64_t st = 0;
-        if (y >= yf) st = pcg_jump(p.fill_state, ((uint64_t)(y - yf) * Z + z) * X + 64u * w, p.inc);
-        for (int m = 0; m < 64; ++m) {
-            const int x = 64 * w + m;
-            uint32_t v;
-            if (x >= X || y < 2) {
-                v = 1u;
-            } else if (y < yf) {
-                v = 0u;
-            } else {
-                const uint32_t d = pcg_output(st);
-                st = st * kPcgMult + p.inc;
-                v = d < p.sand_thr ? 2u : (d < p.water_thr ? 3u : 0u);
-            }
-            const uint32_t a = v >> 1, b = v & 1u;  // codes 0..3 are their own (A, B)
-            if (m & 1) {
-                ao |= a << (m >> 1);
-                bo |= b << (m >> 1);
-            } else {
-                ae |= a << (m >> 1);
-                be |= b << (m >> 1);
-            }
+__device__ __forceinline__ uint4 gen_word(const GenJob& g, int64_t r, int w) {
+    const int yf = g.Y / 2, y = (int)(r / g.Z), z = (int)(r % g.Z);
+    uint32_t ae = 0, ao = 0, be = 0, bo = 0;
+    uint64_t st = 0;
+    if (y >= yf) st = pcg_jump(g.p.fill_state, ((uint64_t)(y - yf) * g.Z + z) * g.X + 64u * w, g.p.inc);
+    for (int m = 0; m < 64; ++m) {
+        const int x = 64 * w + m;
+        uint32_t v;
+        if (x >= g.X || y < 2) {
+            v = 1u;
+        } else if (y < yf) {
+            v = 0u;
+        } else {
+            const uint32_t d = pcg_output(st);
+            st = st * kPcgMult + g.p.inc;
+            v = d < g.p.sand_thr ? 2u : (d < g.p.water_thr ? 3u : 0u);
         }
-        rows[u] = make_uint4(ae, ao, be, bo);
+        const uint32_t a = v >> 1, b = v & 1u;  // codes 0..3 are their own (A, B)
+        if (m & 1) {
+            ao |= a << (m >> 1);
+            bo |= b << (m >> 1);
+        } else {
+            ae |= a << (m >> 1);
+            be |= b << (m >> 1);
+        }
     }
+    return make_uint4(ae, ao, be, bo);
+}
+
+// many worlds per launch (blocks as the conversions'), or `one`
+__global__ void __launch_bounds__(kConvThreads) k_gen_batch_planes(const GenJob* __restrict__ jobs,
+                                                                   const ConvBlock* __restrict__ blocks, GenJob one) {
+    int64_t row0 = (int64_t)blockIdx.x * conv_rows(one.nw > 0 ? one.nw : 1, kConvChunks);
+    GenJob g = one;
+    if (blocks) {
+        const ConvBlock b = blocks[blockIdx.x];
+        g = jobs[b.job];
+        row0 = b.row0;
+    }
+    const int r = threadIdx.x / g.nw, w = threadIdx.x - r * g.nw;
+    if (r >= conv_rows(g.nw, kConvChunks) || row0 + r >= (int64_t)g.Y * g.Z) return;
+    g.rows[row0 * g.nw + threadIdx.x] = gen_word(g, row0 + r, w);
 }
 
 // ---------------------------------------------------------------------------
@@ -986,11 +1002,21 @@ bool alloc_range(const void* p, uintptr_t* start, size_t* bytes) {
     return true;
 }
 
+GenJob gen_job(uint64_t world_seed, int X, int Y, int Z, uint4* rows) {
+    return GenJob{rows, X, Y, Z, plane_nw(X), batch_world_gen(world_seed)};
+}
+
 fs3d_status planes_generate_batch_world(uint64_t world_seed, int X, int Y, int Z, uint4* rows, cudaStream_t st) {
-    const int nw = plane_nw(X);
-    k_gen_batch_planes<<<conv_grid((int64_t)Y * Z * nw), 256, 0, st>>>(X, Y, Z, nw, batch_world_gen(world_seed),
-                                                                       rows);
+    k_gen_batch_planes<<<(unsigned)conv_blocks(Y, Z, plane_nw(X), kConvChunks), kConvThreads, 0, st>>>(
+        nullptr, nullptr, gen_job(world_seed, X, Y, Z, rows));
     FS3D_CHECK_LAUNCH("generate batch world launch");
+    return FS3D_OK;
+}
+
+fs3d_status planes_generate_multi(const GenJob* jobs, const ConvBlock* blocks, int64_t nblocks, cudaStream_t st) {
+    if (nblocks <= 0) return FS3D_OK;
+    k_gen_batch_planes<<<(unsigned)nblocks, kConvThreads, 0, st>>>(jobs, blocks, GenJob{});
+    FS3D_CHECK_LAUNCH("generate batch worlds launch");
     return FS3D_OK;
 }
 
@@ -1003,9 +1029,9 @@ fs3d_status planes_hash_async(const uint4* rows, const uint8_t* statics, int X, 
     return FS3D_OK;
 }
 
-fs3d_status planes_hash_many(const HashJob* jobs, int njobs, unsigned long long* out_dev, cudaStream_t st) {
+fs3d_status planes_hash_many(const HashJob* jobs, int njobs, int parts, unsigned long long* out_dev, cudaStream_t st) {
     if (njobs <= 0) return FS3D_OK;
-    k_hash_planes_many<<<njobs, 256, 0, st>>>(jobs, out_dev);
+    k_hash_planes_many<<<dim3((unsigned)njobs, (unsigned)parts), 256, 0, st>>>(jobs, out_dev);
     FS3D_CHECK_LAUNCH("hash many worlds launch");
     return FS3D_OK;
 }

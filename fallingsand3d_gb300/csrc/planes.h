@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "fs3d_common.h"
+#include "pcg.h"
 
 namespace fs3d {
 
@@ -154,6 +155,14 @@ int plane_step_ctas_per_sm();
 fs3d_status planes_from_bytes(const uint8_t* g, int X, int Y, int Z, uint4* rows, cudaStream_t st);
 // the batch world of `world_seed` written straight into planes (needs Y >= 4)
 fs3d_status planes_generate_batch_world(uint64_t world_seed, int X, int Y, int Z, uint4* rows, cudaStream_t st);
+// the same for many worlds in one launch (blocks of kConvChunks chunks, as the admission conversion's)
+struct GenJob {
+    uint4* rows = nullptr;
+    int32_t X = 0, Y = 0, Z = 0, nw = 0;
+    BatchWorldGen p = {};
+};
+GenJob gen_job(uint64_t world_seed, int X, int Y, int Z, uint4* rows);
+fs3d_status planes_generate_multi(const GenJob* jobs, const ConvBlock* blocks, int64_t nblocks, cudaStream_t st);
 // skip_if_set (nullable): the conversion writes nothing when *skip_if_set is
 // non-zero (a drop-in run whose step kernel recorded a failure leaves the
 // caller's grid as it was)
@@ -207,13 +216,14 @@ fs3d_status launch_batch_slabs(int cls, int CS, const PlaneWorld* worlds, const 
 
 fs3d_status planes_hash_async(const uint4* rows, const uint8_t* statics, int X, int Y, int Z,
                               unsigned long long* out_dev, cudaStream_t st);
-// whole-grid hashes of njobs worlds in one launch: out_dev[j] for jobs[j]
+// whole-grid hashes of njobs worlds in one launch: the hash of jobs[j] is the
+// sum (mod 2^64) of out_dev[j * parts .. + parts)
 struct HashJob {
     const uint4* rows;
     const uint8_t* statics;  // nullable
     int32_t X, Y, Z, nw;
 };
-fs3d_status planes_hash_many(const HashJob* jobs, int njobs, unsigned long long* out_dev, cudaStream_t st);
+fs3d_status planes_hash_many(const HashJob* jobs, int njobs, int parts, unsigned long long* out_dev, cudaStream_t st);
 // One step of many worlds at once (the batch's worlds too large to be
 // resident).  brick_counts: nullable per-brick counts of non-empty cells of
 // world 0, kept exact as it steps.
@@ -244,5 +254,9 @@ fs3d_status launch_render_dda_planes(const uint4* rows, const uint8_t* statics, 
                                      uint8_t* bits, const fs3d_camera* cam, int W, int H, float* rgba_dev,
                                      cudaStream_t st, int* brick_counts = nullptr, bool recount = true);
 size_t brick_count_bytes(int X, int Y, int Z);
+
+// batch.cu: the admissions of a serving loop, many at once
+fs3d_status batch_admit_generated_many(fs3d_batch* b, int n, const fs3d_world_spec* specs, uint64_t* tickets,
+                                       int* n_admitted);
 
 }  // namespace fs3d

@@ -88,3 +88,35 @@ def test_serving_reports_a_device_wait_that_gave_up(fs3d):
         fs3d.inject(fs3d.INJECT_NONE, 0)
     stats, reqs = fs3d.serve(p)  # and serving works again
     assert stats["completed"] == len(reqs) > 0
+
+
+RAGGED = [(16, 4, 16), (1, 4, 1), (65, 5, 130), (63, 33, 7), (2048, 6, 20), (130, 96, 97), (128, 128, 128), (200, 200, 100),
+          (64, 4, 1024), (33, 1030, 2), (449, 9, 31)]
+
+
+@pytest.mark.parametrize("steps,kib", [(0, 0), (1, 0), (70, 0), (70, 4096)])
+def test_served_worlds_of_any_size_equal_the_oracle(fs3d, orc, steps, kib):
+    """Requests admitted together: rows of one to 32 plane words, the last
+    block of a world's generation part full, hashes in one to many parts; at
+    4 MiB the worlds are admitted in several groups."""
+    import ctypes as C
+    p = fs3d.serve_params(1e6, 1.0, master_seed=1, min_steps=1, max_steps=1, hbm_budget=kib << 10)
+    reqs = (fs3d.ServeRequest * (3 * len(RAGGED)))()
+    for i, r in enumerate(reqs):
+        r.X, r.Y, r.Z = RAGGED[i % len(RAGGED)]
+        r.seed, r.n_steps = 1000 + i, steps + i % 2
+    st = fs3d.ServeStats()
+    fs3d.check(fs3d.lib().fs3d_serve_run(C.byref(p), len(reqs), reqs, C.byref(st)))
+    assert st.completed == len(reqs)
+    assert [r.hash for r in reqs] == oracle_hashes(orc, reqs)
+
+
+def test_hashes_of_worlds_with_statics_in_many_parts(fs3d, orc):
+    dims = [(130, 96, 97), (17, 5, 9), (64, 64, 64), (1000, 20, 30)]
+    r = np.random.default_rng(3)
+    grids = [r.choice(np.array([0, 1, 2, 3, 5, 200, 255], np.uint8), (Y, Z, X)) for X, Y, Z in dims]
+    with fs3d.Batch(1 << 30) as b:
+        ts = b.admit_many(grids, list(range(len(dims))), 0)
+        done, hs = b.poll_many(ts)
+        assert done.all() and [int(h) for h in hs] == [orc.hash(g) for g in grids]
+        assert [b.poll(t)[1] for t in ts] == [int(h) for h in hs]
