@@ -209,9 +209,11 @@ struct fs3d_batch {
     uint32_t class_mask = ~0u, graph_mask = 0;
     int grid = 0;
     int promote = 0;  // single-CTA resident worlds run this many classes wider (autotuned)
-    // hybrid mode: young worlds of class `spread_from` or wider run in cluster
-    // class `spread` (0: none), chosen with the tables
+    // hybrid mode, chosen with the tables: young worlds of class `spread_from`
+    // or wider run in cluster class `spread` (0: none), settled worlds' CTAs
+    // are widened by level `widen` (choose_widen)
     int spread = 0, spread_from = 0;
+    int widen = 0;
     void* edges[kResidentClasses - kSingleCtaClasses] = {};  // the cluster classes' edge buffers (once needed)
     unsigned long long* hash_dev = nullptr;
     unsigned long long* processed_dev = nullptr;  // cell-steps the resident kernels evaluated
@@ -240,6 +242,12 @@ namespace {
 // from L2, which wins from age 128 on.)
 constexpr uint64_t kYoungSteps = 128;
 
+// Global-memory class of a settled world by its class for itself (0..3) and
+// the batch's level (choose_widen).
+constexpr int kWidenLevels = 4;
+constexpr int kWidened[kWidenLevels + 1][kGmDense] = {
+    {0, 1, 2, 3}, {0, 2, 3, 3}, {2, 3, 3, 3}, {3, 3, 3, 3}, {3, 3, 3, 4}};
+
 // Segment class of a running world (-1: the per-step kernel) under the
 // batch's mode: 1 shared-memory classes, 2 global-memory classes, 3 hybrid
 // (young worlds in shared memory when they fit, settled ones in global
@@ -257,7 +265,9 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
     auto gm = [&]() {
         if (w.cls_gm == -2) w.cls_gm = resident_class_gm(w.X, w.Y, w.Z);
         const int c = w.cls_gm;
-        return c < 0 ? -1 : kResidentClasses + std::min(c + b->promote, kGmDense - 1);
+        if (c < 0) return -1;
+        const int wide = mode == 3 ? kWidened[b->widen][c] : c;
+        return kResidentClasses + std::max(std::min(c + b->promote, kGmDense - 1), wide);
     };
     if (mode == 1) return smem();
     if (mode == 2) return gm();
@@ -317,6 +327,43 @@ void choose_spread(fs3d_batch* b) {
         spread(8, kSingleCtaClasses);
     else if (large > 0 && large * 4 + whole + rest / 3 <= 2 * sms)
         spread(4, kSingleCtaClasses);
+}
+
+// How far the hybrid mode widens the CTAs of settled worlds.  A world's class
+// by itself leaves no warp idle at a step's barrier, which is best while the
+// SMs are full; with fewer worlds than fill them, a segment takes as long as
+// its busiest world, whose step is shorter in a wider CTA.  So the widest level
+// whose CTAs all run at once is taken, and the first level (64 and 128 threads
+// doubled) up to 1.75 times that.  Settled 64-step segments, class for itself /
+// widened: 100 mixed worlds 326 / 262 us, 300 344 / 281, 600 410 / 365, 1200
+// 595 / 482 (2048: 745, and 769 with the first level); 64^3: 100 worlds 365 /
+// 237, 600 451 / 285; 16^3: 100 232 / 176, 600 280 / 194 (305 at 64 threads,
+// so the first level leaves one-warp worlds alone).
+void choose_widen(fs3d_batch* b) {
+    b->widen = 0;
+    if (b->cfg.use_smem != 3) return;
+    int64_t by_class[kGmDense] = {0, 0, 0, 0}, young = 0;
+    for (auto& kv : b->worlds) {
+        BWorld& w = kv.second;
+        if (w.done) continue;
+        if (w.t < kYoungSteps) {
+            if (w.cls_smem == -2) w.cls_smem = resident_class(w.X, w.Y, w.Z);
+            young += w.cls_smem == 0 || w.cls_smem == 1 ? 256 : 768;
+            continue;
+        }
+        if (w.cls_gm == -2) w.cls_gm = resident_class_gm(w.X, w.Y, w.Z);
+        if (w.cls_gm >= 0) ++by_class[w.cls_gm];
+    }
+    static const int threads[kGmClasses] = {32, 64, 128, 256, 768};
+    const int64_t fit = (int64_t)sm_count_public() * 768;
+    for (int l = kWidenLevels; l > 0; --l) {
+        int64_t need = young;
+        for (int c = 0; c < kGmDense; ++c) need += by_class[c] * threads[kWidened[l][c]];
+        if (need <= (l == 1 ? fit * 7 / 4 : fit)) {
+            b->widen = l;
+            return;
+        }
+    }
 }
 
 fs3d_status wait_stream(cudaStream_t st, int64_t timeout_ns) {
@@ -900,6 +947,7 @@ fs3d_status build_tables(fs3d_batch* b) {
     b->tn.select(b->tab_cur);
     b->to.select(b->tab_cur);
     choose_spread(b);
+    choose_widen(b);
     // resident class of every running world (-1: stepped by the per-step kernel)
     std::vector<std::pair<int, BWorld*>> run;
     size_t ni = 0, ns = 0;
