@@ -637,10 +637,6 @@ fs3d_status enqueue_segment(fs3d_batch* b, cudaStream_t a, bool fork, bool with_
 }
 
 fs3d_status capture_one(fs3d_batch* b, bool with_steps, cudaGraphExec_t* out) {
-    if (*out) {
-        cudaGraphExecDestroy(*out);
-        *out = nullptr;
-    }
     cudaStream_t cs;
     FS3D_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     cudaGraph_t g = nullptr;
@@ -658,9 +654,19 @@ fs3d_status capture_one(fs3d_batch* b, bool with_steps, cudaGraphExec_t* out) {
     return FS3D_OK;
 }
 
-fs3d_status capture_graph(fs3d_batch* b) {
-    fs3d_status s = capture_one(b, false, &b->graph);
-    if (s == FS3D_OK) s = capture_one(b, true, &b->graph_steps);
+// The graph that the next segment launches (with the per-step kernel's launches
+// where some world takes them: 64 more nodes, as long to capture as the rest),
+// unless it stands as captured.
+fs3d_status capture_graph(fs3d_batch* b, bool with_steps) {
+    if (b->graph_worlds != b->tw.d || b->graph_items != b->ti.d || b->graph_order != b->to.d ||
+        b->graph_mask != b->class_mask)
+        for (cudaGraphExec_t* g : {&b->graph, &b->graph_steps})
+            if (*g) {
+                cudaGraphExecDestroy(*g);
+                *g = nullptr;
+            }
+    if (with_steps ? b->graph_steps : b->graph) return FS3D_OK;
+    const fs3d_status s = capture_one(b, with_steps, with_steps ? &b->graph_steps : &b->graph);
     if (s != FS3D_OK) return s;
     b->graph_worlds = b->tw.d;
     b->graph_items = b->ti.d;
@@ -723,7 +729,7 @@ fs3d_status fs3d_batch_create(size_t budget, const fs3d_config* cfg, fs3d_batch*
     if (s == FS3D_OK) s = b->tw.reserve(4096);
     if (s == FS3D_OK) s = b->ti.reserve(1 << 16);
     if (s == FS3D_OK) s = b->to.reserve(4096);
-    if (s == FS3D_OK && b->cfg.use_graphs) s = capture_graph(b);
+    if (s == FS3D_OK && b->cfg.use_graphs) s = capture_graph(b, false);
     if (s != FS3D_OK) {
         fs3d_batch_destroy(b);
         return s;
@@ -1050,9 +1056,8 @@ fs3d_status build_tables(fs3d_batch* b) {
     if (si) FS3D_CUDA(b->to.upload(si, b->stream));
     FS3D_CUDA(b->tn.upload(kMetaInts, b->stream));
     FS3D_CUDA(cudaEventRecord(b->tables_free[b->tab_cur], b->stream));
-    if (b->cfg.use_graphs && (!b->graph || b->graph_worlds != b->tw.d || b->graph_items != b->ti.d ||
-                              b->graph_order != b->to.d || b->graph_mask != b->class_mask)) {
-        s = capture_graph(b);
+    if (b->cfg.use_graphs) {
+        s = capture_graph(b, ii > 0);
         if (s != FS3D_OK) {
             b->running.clear();
             return s;
@@ -1175,6 +1180,9 @@ fs3d_status fs3d_batch_poll_many(fs3d_batch* b, int n, const uint64_t* tickets, 
         return set_error(FS3D_ERR_INVALID_ARG, "fs3d_batch_poll_many: bad args");
     std::vector<BWorld*> need;
     std::vector<int> need_at;
+    // the worlds that finish in a segment share its event: asked once
+    const CUevent_st* asked = nullptr;
+    cudaError_t answer = cudaSuccess;
     for (int i = 0; i < n; ++i) {
         auto it = b->worlds.find(tickets[i]);
         if (it == b->worlds.end()) return set_error(FS3D_ERR_NOT_FOUND, "fs3d_batch_poll_many: unknown ticket");
@@ -1186,9 +1194,12 @@ fs3d_status fs3d_batch_poll_many(fs3d_batch* b, int n, const uint64_t* tickets, 
             if (f != FS3D_OK) return f;
         }
         if (w.finished) {
-            const cudaError_t q = cudaEventQuery(w.finished.get());
-            if (q == cudaErrorNotReady) continue;
-            if (q != cudaSuccess) return cuda_fail(q, "fs3d_batch_poll_many");
+            if (w.finished.get() != asked) {
+                asked = w.finished.get();
+                answer = cudaEventQuery(w.finished.get());
+            }
+            if (answer == cudaErrorNotReady) continue;
+            if (answer != cudaSuccess) return cuda_fail(answer, "fs3d_batch_poll_many");
         }
         done[i] = 1;
         if (!hashes) continue;
@@ -1918,7 +1929,8 @@ fs3d_status apply_tuning(fs3d_batch* b, const Tuning& t) {
     b->promote = t.promote;
     b->tables_stale = true;
     b->grid = sm_count_public() * t.ctas_per_sm;
-    return b->cfg.use_graphs ? capture_graph(b) : FS3D_OK;
+    b->graph_worlds = nullptr;  // no graph stands for another configuration
+    return b->cfg.use_graphs ? capture_graph(b, b->table_items > 0) : FS3D_OK;
 }
 
 // voxel-updates the next segment will perform
