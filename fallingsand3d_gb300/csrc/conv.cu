@@ -163,9 +163,9 @@ static ConvJob one_job(const uint4* rows, const uint8_t* statics, const uint8_t*
     return j;
 }
 
-fs3d_status planes_from_bytes(const uint8_t* g, int X, int Y, int Z, uint4* rows, cudaStream_t st) {
+fs3d_status planes_from_bytes(const uint8_t* g, int X, int Y, int Z, uint4* rows, cudaStream_t st, int* statics_flag) {
     k_bytes_to_planes<<<(unsigned)conv_blocks(Y, Z, plane_nw(X), kConvChunks), kConvThreads, 0, st>>>(
-        nullptr, nullptr, one_job(rows, nullptr, g, X, Y, Z), nullptr);
+        nullptr, nullptr, one_job(rows, nullptr, g, X, Y, Z), statics_flag);
     FS3D_CHECK_LAUNCH("bytes->planes launch");
     return FS3D_OK;
 }

@@ -152,7 +152,8 @@ int plane_lg(int nw);
 int plane_items_for(int Y, int Z, int nw);
 int plane_step_grid(int64_t n_items);
 int plane_step_ctas_per_sm();
-fs3d_status planes_from_bytes(const uint8_t* g, int X, int Y, int Z, uint4* rows, cudaStream_t st);
+fs3d_status planes_from_bytes(const uint8_t* g, int X, int Y, int Z, uint4* rows, cudaStream_t st,
+                              int* statics_flag = nullptr);
 // the batch world of `world_seed` written straight into planes (needs Y >= 4)
 fs3d_status planes_generate_batch_world(uint64_t world_seed, int X, int Y, int Z, uint4* rows, cudaStream_t st);
 // the same for many worlds in one launch (blocks of kConvChunks chunks, as the admission conversion's)

@@ -61,3 +61,25 @@ def test_admission_from_device_memory(fs3d, cuda, shift):
         t = b.admit_many(grids, [1] * len(grids), 0, ptrs=[d.data_ptr() + int(e) for e in ends[:-1]])
         b.retire_many(t, [out.data_ptr() + int(e) for e in ends[:-1]])
     assert (out.cpu().numpy() == flat).all()
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (64, 4, 64), (130, 33, 9), (2048, 3, 5)])
+def test_world_grids_with_and_without_statics(fs3d, orc, dims):
+    """A world's bytes are kept exactly while some cell (here the last one, or
+    any) is a static material: written grids alternate, each read back and
+    hashed after a step."""
+    X, Y, Z = dims
+    r = np.random.default_rng(X + Y)
+    plain = r.choice(np.array([0, 1, 2, 3], np.uint8), (Y, Z, X))
+    last, many = plain.copy(), r.integers(0, 256, (Y, Z, X), dtype=np.uint8)
+    last[-1, -1, -1] = 200
+    with fs3d.World(plain, 5) as w:
+        t = 0
+        for g in (plain, last, many, plain, many, last):
+            g = g.copy()
+            w.write(g)
+            assert (w.read() == g).all() and w.hash() == orc.hash(g)
+            w.step(1)
+            orc.run(g, 5, t, 1, nthreads=1)
+            t += 1
+            assert (w.read() == g).all() and w.hash() == orc.hash(g)
