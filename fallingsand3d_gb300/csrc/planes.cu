@@ -238,9 +238,17 @@ __device__ __forceinline__ bool rows_changed_recently(const uint8_t* __restrict_
     return d;
 }
 
-// three CTAs per SM (80 registers, a few bytes spilled): 24 warps hide the
+// LIST: more than two items a warp.  It then looks at the flags of its next G
+// items together, a row-pair a lane (one after another, the flags' loads took
+// most of a settled step), and takes the dirty ones of them (32 >> lg) at a
+// time.  1024^3 dunes, steps 60 / 420 / 960: 196 / 97 / 58 us item by item, 184
+// / 83 / 42 listed; 512^3 26.5 / 11 / 10.8 and 25.7 / 10 / 9.  With two items a
+// warp the list costs what it saves (400x300x350: 11.8 / 7.5 / 7.4 and 12.1 /
+// 7.5 / 7.3), with one 0.3 us (200^3: 6.2 and 6.6).
+// Three CTAs per SM (80 registers, a few bytes spilled): 24 warps hide the
 // rule's dependent chain better than 16 at 118 registers (1024^3 dunes:
 // 118 us per step against 133 us, 123 us at four CTAs)
+template <bool LIST>
 __global__ void __launch_bounds__(256, 3) k_plane_step_skip(const PlaneWorld w, uint8_t* __restrict__ rflags,
                                                         int* counts) {
     chain_wait();
@@ -253,44 +261,72 @@ __global__ void __launch_bounds__(256, 3) k_plane_step_skip(const PlaneWorld w, 
     const uint32_t gmask = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << (lane & ~(G - 1));
     const bool half_at_end = (w.X & 63) == 0;
     const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < n_items; it += warps) {
-        const int rp = it * per + (lane >> w.lg);
-        const bool valid = rp < nrp;
-        const int j = valid ? rp / NBZ : 0, k = valid ? rp - j * NBZ : 0;
-        const int y0 = 2 * j - o, z0 = 2 * k - o;
+    __shared__ int2 s_list[8][LIST ? 32 : 1];
+    int2* list = s_list[threadIdx.x >> 5];
+    for (int it0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it0 < n_items; it0 += LIST ? warps * G : warps) {
+        int n_dirty = 0, j = 0, k = 0;
         bool dirty = false;
-        if (valid && gl == 0) dirty = rows_changed_recently(rflags, w.Y, w.Z, y0, z0, tb);
-        dirty = __shfl_sync(0xFFFFFFFFu, dirty, lane & ~(G - 1));
-        if (!__any_sync(0xFFFFFFFFu, dirty)) continue;
-        const bool has = dirty && gl < w.nw;
-        uint4 q[4], q0[4];
-        uint4* ptr[4];
-        bool in[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int y = (a < 2) ? y0 + 1 : y0, z = z0 + (a & 1);
-            in[a] = has && y >= 0 && y < w.Y && z >= 0 && z < w.Z;
-            ptr[a] = in[a] ? w.rows + ((int64_t)y * w.Z + z) * w.nw + gl : w.rows;
-            q[a] = in[a] ? *ptr[a] : make_uint4(0u, 0u, 0xFFFFFFFFu, 0xFFFFFFFFu);
-            q0[a] = q[a];
-        }
-        rowpair_core(q, has, o, rowkey(sk, (uint32_t)j, (uint32_t)k), gl, G, w.nw, half_at_end);
-        bool any = false;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const bool chg =
-                in[a] && (q[a].x != q0[a].x || q[a].y != q0[a].y || q[a].z != q0[a].z || q[a].w != q0[a].w);
-            if (chg) {
-                *ptr[a] = q[a];
-                any = true;
+        if (LIST) {
+            const int it = it0 + (lane >> (5 - w.lg)) * warps, rp = it * per + (lane & (per - 1));
+            if (it < n_items && rp < nrp) {
+                j = rp / NBZ;
+                k = rp - j * NBZ;
+                dirty = rows_changed_recently(rflags, w.Y, w.Z, 2 * j - o, 2 * k - o, tb);
             }
-            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, chg);
-            if (gl == 0 && (bal & gmask)) {
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, dirty);
+            n_dirty = __popc(m);
+            if (dirty) list[__popc(m & ((1u << lane) - 1u))] = make_int2(j, k);
+            __syncwarp();
+        } else {
+            const int rp = it0 * per + (lane >> w.lg);
+            if (rp < nrp) {
+                j = rp / NBZ;
+                k = rp - j * NBZ;
+                if (gl == 0) dirty = rows_changed_recently(rflags, w.Y, w.Z, 2 * j - o, 2 * k - o, tb);
+            }
+            dirty = __shfl_sync(0xFFFFFFFFu, dirty, lane & ~(G - 1));
+            if (__any_sync(0xFFFFFFFFu, dirty)) n_dirty = 1;
+        }
+        for (int at = 0; at < n_dirty; at += per) {
+            if (LIST) {
+                const int me = at + (lane >> w.lg);
+                dirty = me < n_dirty;
+                const int2 jk = dirty ? list[me] : make_int2(0, 0);
+                j = jk.x;
+                k = jk.y;
+            }
+            const int y0 = 2 * j - o, z0 = 2 * k - o;
+            const bool has = dirty && gl < w.nw;
+            uint4 q[4], q0[4];
+            uint4* ptr[4];
+            bool in[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
                 const int y = (a < 2) ? y0 + 1 : y0, z = z0 + (a & 1);
-                rflags[(int64_t)y * w.Z + z] = (uint8_t)tb;
+                in[a] = has && y >= 0 && y < w.Y && z >= 0 && z < w.Z;
+                ptr[a] = in[a] ? w.rows + ((int64_t)y * w.Z + z) * w.nw + gl : w.rows;
+                q[a] = in[a] ? *ptr[a] : make_uint4(0u, 0u, 0xFFFFFFFFu, 0xFFFFFFFFu);
+                q0[a] = q[a];
             }
+            rowpair_core(q, has, o, rowkey(sk, (uint32_t)j, (uint32_t)k), gl, G, w.nw, half_at_end);
+            bool any = false;
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const bool chg =
+                    in[a] && (q[a].x != q0[a].x || q[a].y != q0[a].y || q[a].z != q0[a].z || q[a].w != q0[a].w);
+                if (chg) {
+                    *ptr[a] = q[a];
+                    any = true;
+                }
+                const uint32_t bal = __ballot_sync(0xFFFFFFFFu, chg);
+                if (gl == 0 && (bal & gmask)) {
+                    const int y = (a < 2) ? y0 + 1 : y0, z = z0 + (a & 1);
+                    rflags[(int64_t)y * w.Z + z] = (uint8_t)tb;
+                }
+            }
+            if (counts && any) count_bricks(counts, w, y0, z0, gl, q, q0, in);
         }
-        if (counts && any) count_bricks(counts, w, y0, z0, gl, q, q0, in);
+        if (LIST) __syncwarp();  // the list's readers are done
     }
     chain_go();
 }
@@ -1095,18 +1131,13 @@ fs3d_status layer_flags_from_cells(const uint4* rows, uint8_t* lflags, int X, in
 }
 
 fs3d_status launch_plane_step_skip(const PlaneWorld& w, uint8_t* rflags, int* counts, cudaStream_t st) {
-    static const int per_sm = [] {
-        int v = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_plane_step_skip, 256, 0) != cudaSuccess || v < 1) v = 1;
-        cudaGetLastError();
-        return v;
-    }();
     const int per = 32 >> w.lg;
     const int64_t nrp = (int64_t)nblocks(w.Y, 1) * nblocks(w.Z, 1);
     const int64_t need = ((nrp + per - 1) / per + 7) / 8;  // eight warps per CTA
-    const int64_t cap = (int64_t)sm_count_public() * per_sm;
+    const int64_t cap = (int64_t)sm_count_public() * 3;    // the kernel's launch bound
     const int grid = (int)(need < 1 ? 1 : (need < cap ? need : cap));
-    const cudaError_t e = launch_chained(k_plane_step_skip, (unsigned)grid, 256, st, w, rflags, counts);
+    const cudaError_t e = need > 2 * cap ? launch_chained(k_plane_step_skip<true>, (unsigned)grid, 256, st, w, rflags, counts)
+                                     : launch_chained(k_plane_step_skip<false>, (unsigned)grid, 256, st, w, rflags, counts);
     if (e != cudaSuccess) return cuda_fail(e, "plane step (settled skip) launch");
     note_launch();
     return FS3D_OK;

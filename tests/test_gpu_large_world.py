@@ -110,3 +110,23 @@ def test_render_counts_stay_exact(fs3d, orc):
             img = w.render(cam, 160, 90)
         exp = orc.render_dda(ref, oracle_lib.camera_from(cam), 160, 90)
         assert float(np.abs(img - exp).max()) <= 1e-5
+
+
+@pytest.mark.parametrize("dims", [(2048, 130, 235), (300, 281, 420), (130, 560, 421), (64, 1000, 941)], ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("start", [0, 251])
+def test_step_with_items_listed(fs3d, orc, dims, start):
+    """Just above the size where a warp looks at several items' flags at once:
+    rows of 32, 5, 3 and 1 words, a last item part full, settled and moving
+    parts (the lower half is stone and sand at rest) beside each other."""
+    X, Y, Z = dims
+    r = np.random.default_rng(X)
+    g = np.zeros((Y, Z, X), np.uint8)
+    g[: Y // 2] = 1
+    g[Y // 2 :] = r.choice(np.array([0, 1, 2, 3, 77], np.uint8), (Y - Y // 2, Z, X), p=[0.6, 0.05, 0.2, 0.13, 0.02])
+    g[:, : Z // 3] = np.where(g[:, : Z // 3] > 1, 0, g[:, : Z // 3])
+    with fs3d.World(g, 11, start_step=start) as w:
+        for _ in range(5):
+            w.step(2)
+        got = w.read()
+    orc.run(g, 11, start, 10, nthreads=0)
+    assert (got == g).all()
