@@ -66,6 +66,9 @@ void note_launch(uint64_t n = 1);
 // in another (after cudaDeviceReset, for example).
 bool current_context_id(unsigned long long* id);
 
+// device memory for a call's own duration, stream-ordered (scratch.cpp)
+cudaError_t scratch_alloc(void** p, size_t n, cudaStream_t st);
+
 // ---- chained launches: a kernel that begins with chain_wait() may be launched
 // with launch_chained(), so that its CTAs are placed and its first instructions
 // fetched while the kernel before it in the stream ends (programmatic

@@ -655,7 +655,7 @@ extern "C" fs3d_status fs3d_render_meshes(const fs3d_object_view* v, const fs3d_
     const size_t o_lut = (draws_b + 255) & ~(size_t)255, o_tris = (o_lut + lut_b + 255) & ~(size_t)255,
                  o_list = (o_tris + tris_b + 255) & ~(size_t)255, o_key = (o_list + list_b + 255) & ~(size_t)255;
     char* scratch = nullptr;
-    FS3D_CUDA(cudaMallocAsync((void**)&scratch, o_key + key_b + sizeof(uint32_t), st));
+    FS3D_CUDA(scratch_alloc((void**)&scratch, o_key + key_b + sizeof(uint32_t), st));
     uint32_t* list = reinterpret_cast<uint32_t*>(scratch + o_list);
     uint32_t* n_list = reinterpret_cast<uint32_t*>(scratch + o_key + key_b);
     MeshDrawDev* ddev = reinterpret_cast<MeshDrawDev*>(scratch);

@@ -76,7 +76,7 @@ extern "C" fs3d_status fs3d_run_device(uint8_t* grid_dev, int X, int Y, int Z, u
     // one block of scratch: the planes, the row flags, the slabs' scratch
     const size_t rows_b = (plane_bytes(X, Y, Z) + 255) & ~(size_t)255, flags_b = ((size_t)Y * Z + 255) & ~(size_t)255;
     char* scratch = nullptr;
-    FS3D_CUDA(cudaMallocAsync((void**)&scratch, rows_b + flags_b + (slabs ? plan.scratch : 0), st));
+    FS3D_CUDA(scratch_alloc((void**)&scratch, rows_b + flags_b + (slabs ? plan.scratch : 0), st));
     uint8_t* rflags = reinterpret_cast<uint8_t*>(scratch + rows_b);
     PlaneWorld d{};
     d.rows = reinterpret_cast<uint4*>(scratch);

@@ -578,7 +578,7 @@ fs3d_status fs3d_hash_device(const uint8_t* grid_dev, int64_t n, void* stream, u
     if (!grid_dev || n < 0 || !out) return set_error(FS3D_ERR_INVALID_ARG, "fs3d_hash_device: bad args");
     cudaStream_t st = (cudaStream_t)stream;
     unsigned long long* d = nullptr;
-    FS3D_CUDA(cudaMallocAsync((void**)&d, sizeof(*d), st));
+    FS3D_CUDA(scratch_alloc((void**)&d, sizeof(*d), st));
     fs3d_status s = hash_bytes_async(grid_dev, n, d, st);
     unsigned long long h = 0;
     if (s == FS3D_OK) {
@@ -595,7 +595,7 @@ fs3d_status fs3d_first_diff_device(const uint8_t* a, const uint8_t* b, int64_t n
     if (!a || !b || n < 0 || !out) return set_error(FS3D_ERR_INVALID_ARG, "fs3d_first_diff_device: bad args");
     cudaStream_t st = (cudaStream_t)stream;
     unsigned long long* d = nullptr;
-    FS3D_CUDA(cudaMallocAsync((void**)&d, sizeof(*d), st));
+    FS3D_CUDA(scratch_alloc((void**)&d, sizeof(*d), st));
     fs3d_status s = FS3D_OK;
     cudaError_t e = cudaMemsetAsync(d, 0xFF, sizeof(*d), st);
     if (e != cudaSuccess) s = cuda_fail(e, "first_diff memset");

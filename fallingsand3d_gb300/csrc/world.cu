@@ -90,7 +90,7 @@ fs3d_status upload(fs3d_world* w, const uint8_t* g) {
     // the conversion itself finds whether a cell holds a static material (a
     // host pass over 128x96x110 cells took 0.6 ms): only then are the bytes kept
     uint8_t* bytes = w->statics;
-    if (!bytes) FS3D_CUDA(cudaMallocAsync((void**)&bytes, (size_t)n, w->stream));
+    if (!bytes) FS3D_CUDA(scratch_alloc((void**)&bytes, (size_t)n, w->stream));
     int* flag = reinterpret_cast<int*>(w->hash_dev);
     int stat = 0;
     cudaError_t e = cudaMemcpyAsync(bytes, g, (size_t)n, cudaMemcpyHostToDevice, w->stream);
@@ -256,7 +256,7 @@ fs3d_status fs3d_world_read(fs3d_world* w, uint8_t* out) {
         return FS3D_OK;
     }
     uint8_t* staging = nullptr;
-    FS3D_CUDA(cudaMallocAsync((void**)&staging, n, w->stream));
+    FS3D_CUDA(scratch_alloc((void**)&staging, n, w->stream));
     fs3d_status s = planes_to_bytes(w->rows, w->statics, w->X, w->Y, w->Z, staging, w->stream);
     cudaError_t e = cudaSuccess;
     if (s == FS3D_OK) e = cudaMemcpyAsync(out, staging, n, cudaMemcpyDeviceToHost, w->stream);
@@ -380,7 +380,7 @@ fs3d_status fs3d_render(fs3d_world* w, const fs3d_camera* cam, int W, int H, int
     if (mode == FS3D_RENDER_DDA && w->layout == FS3D_LAYOUT_PLANES && !w->brick_counts &&
         plane_bytes(w->X, w->Y, w->Z) > kCountsPlaneBytes)
         FS3D_CUDA(cudaMalloc((void**)&w->brick_counts, brick_count_bytes(w->X, w->Y, w->Z)));
-    if (!out_on_device) FS3D_CUDA(cudaMallocAsync((void**)&dst, bytes, w->stream));
+    if (!out_on_device) FS3D_CUDA(scratch_alloc((void**)&dst, bytes, w->stream));
     fs3d_status s;
     if (mode == FS3D_RENDER_SDF_SPHERE)
         s = launch_render_sdf(cam, W, H, dst, w->stream);
