@@ -213,7 +213,7 @@ struct fs3d_batch {
     // or wider run in cluster class `spread` (0: none), settled worlds' CTAs
     // are widened by level `widen` (choose_widen)
     int spread = 0, spread_from = 0;
-    int widen = 0;
+    int widen = 1;
     void* edges[kResidentClasses - kSingleCtaClasses] = {};  // the cluster classes' edge buffers (once needed)
     unsigned long long* hash_dev = nullptr;
     unsigned long long* processed_dev = nullptr;  // cell-steps the resident kernels evaluated
@@ -244,9 +244,9 @@ constexpr uint64_t kYoungSteps = 128;
 
 // Global-memory class of a settled world by its class for itself (0..3) and
 // the batch's level (choose_widen).
-constexpr int kWidenLevels = 4;
-constexpr int kWidened[kWidenLevels + 1][kGmDense] = {
-    {0, 1, 2, 3}, {0, 2, 3, 3}, {2, 3, 3, 3}, {3, 3, 3, 3}, {3, 3, 3, 4}};
+constexpr int kPackedLevel = 0, kOwnLevel = 1, kWidestLevel = 5;
+constexpr int kWidened[kWidestLevel + 1][kGmDense] = {
+    {1, 1, 1, 3}, {0, 1, 2, 3}, {0, 2, 3, 3}, {2, 3, 3, 3}, {3, 3, 3, 3}, {3, 3, 3, 4}};
 
 // Segment class of a running world (-1: the per-step kernel) under the
 // batch's mode: 1 shared-memory classes, 2 global-memory classes, 3 hybrid
@@ -266,8 +266,8 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
         if (w.cls_gm == -2) w.cls_gm = resident_class_gm(w.X, w.Y, w.Z);
         const int c = w.cls_gm;
         if (c < 0) return -1;
-        const int wide = mode == 3 ? kWidened[b->widen][c] : c;
-        return kResidentClasses + std::max(std::min(c + b->promote, kGmDense - 1), wide);
+        const int leveled = mode == 3 ? kWidened[b->widen][c] : c;
+        return kResidentClasses + (b->promote ? std::max(std::min(c + b->promote, kGmDense - 1), leveled) : leveled);
     };
     if (mode == 1) return smem();
     if (mode == 2) return gm();
@@ -329,18 +329,22 @@ void choose_spread(fs3d_batch* b) {
         spread(4, kSingleCtaClasses);
 }
 
-// How far the hybrid mode widens the CTAs of settled worlds.  A world's class
-// by itself leaves no warp idle at a step's barrier, which is best while the
-// SMs are full; with fewer worlds than fill them, a segment takes as long as
-// its busiest world, whose step is shorter in a wider CTA.  So the widest level
-// whose CTAs all run at once is taken, and the first level (64 and 128 threads
-// doubled) up to 1.75 times that.  Settled 64-step segments, class for itself /
-// widened: 100 mixed worlds 326 / 262 us, 300 344 / 281, 600 410 / 365, 1200
-// 595 / 482 (2048: 745, and 769 with the first level); 64^3: 100 worlds 365 /
-// 237, 600 451 / 285; 16^3: 100 232 / 176, 600 280 / 194 (305 at 64 threads,
-// so the first level leaves one-warp worlds alone).
+// How wide the hybrid mode makes the CTAs of settled worlds.  A world's class
+// by itself leaves no warp idle at a step's barrier.  With fewer worlds than
+// fill the SMs, a segment takes as long as its busiest world, whose step is
+// shorter in a wider CTA: the widest level whose CTAs all run at once is taken,
+// and the first (64 and 128 threads doubled) up to 1.75 times that.  Settled
+// 64-step segments, class by itself / widened: 100 mixed worlds 326 / 262 us,
+// 300 344 / 281, 600 410 / 365, 1200 595 / 482; 64^3: 100 worlds 365 / 237, 600
+// 451 / 285; 16^3: 100 232 / 176, 600 280 / 194 (305 at 64 threads, so the
+// first level leaves one-warp worlds alone).  With many more worlds of mixed
+// classes (1.5 times what runs at once), CTAs of three widths beside each other
+// leave warps of an SM unused: all but the widest class take 64 threads (2048
+// mixed worlds 726 / 680 us, 3500 1066 / 977, 3500 ragged 1253 / 1204; 1400
+// ragged 694 / 781).  Worlds mostly of one class keep it (2048 of 16^3: 305 /
+// 358) up to 1.75 times (64x48x128: 1000 worlds 460 / 569, 2048 713 / 688).
 void choose_widen(fs3d_batch* b) {
-    b->widen = 0;
+    b->widen = kOwnLevel;
     if (b->cfg.use_smem != 3) return;
     int64_t by_class[kGmDense] = {0, 0, 0, 0}, young = 0;
     for (auto& kv : b->worlds) {
@@ -356,14 +360,28 @@ void choose_widen(fs3d_batch* b) {
     }
     static const int threads[kGmClasses] = {32, 64, 128, 256, 768};
     const int64_t fit = (int64_t)sm_count_public() * 768;
-    for (int l = kWidenLevels; l > 0; --l) {
+    int64_t own = 0, most = 0;  // threads with each class by itself, and those of the largest share
+    int largest = 0;
+    for (int l = kWidestLevel; l >= kOwnLevel; --l) {
         int64_t need = young;
-        for (int c = 0; c < kGmDense; ++c) need += by_class[c] * threads[kWidened[l][c]];
-        if (need <= (l == 1 ? fit * 7 / 4 : fit)) {
+        for (int c = 0; c < kGmDense; ++c) {
+            const int64_t t = by_class[c] * threads[kWidened[l][c]];
+            need += t;
+            if (l == kOwnLevel) {
+                own += t;
+                if (t > most) {
+                    most = t;
+                    largest = c;
+                }
+            }
+        }
+        if (l > kOwnLevel && need <= (l == kOwnLevel + 1 ? fit * 7 / 4 : fit)) {
             b->widen = l;
             return;
         }
     }
+    const bool one_class = 10 * most >= 7 * own;
+    if (one_class ? largest > 0 && own > fit * 7 / 4 : own > fit * 3 / 2) b->widen = kPackedLevel;
 }
 
 fs3d_status wait_stream(cudaStream_t st, int64_t timeout_ns) {
