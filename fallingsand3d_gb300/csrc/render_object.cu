@@ -284,13 +284,8 @@ __global__ void k_render_object(const __grid_constant__ ObjScene sc, int W, int 
 // restatement bit for bit (every float operation single-rounded, in the same
 // order).
 
-struct MeshDrawDev {
-    float mvp[16];
-    float color[4];
-    const float* verts;
-    const uint8_t* tex;
-    int tex_w, tex_h, material, n_tri;
-    long long prim0;
+struct Mat4 {
+    float m[16];
 };
 
 struct ScrTri {
@@ -345,11 +340,11 @@ __device__ __forceinline__ int top_left_dev(float ax, float ay, float bx, float 
 }
 
 // the draw holding primitive p: the last one whose first primitive is <= p
-__device__ __forceinline__ int find_draw(const MeshDrawDev* __restrict__ draws, int n_draws, long long p) {
+__device__ __forceinline__ int find_draw(const long long* __restrict__ prim0, int n_draws, long long p) {
     int lo = 0, hi = n_draws - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (draws[mid].prim0 <= p)
+        if (prim0[mid] <= p)
             lo = mid;
         else
             hi = mid - 1;
@@ -398,15 +393,27 @@ __device__ __forceinline__ bool screen_tri(const ClipVtx& v0, const ClipVtx& v1,
 // was clipped) go to slots 3p.. and their slots to `list` (any order: the
 // cover pass's keys decide).  A primitive wholly within the depth range is
 // its own polygon, so only the others go through the clipper's arrays.
-__global__ void __launch_bounds__(128) k_mesh_setup(const MeshDrawDev* __restrict__ draws, int n_draws, long long n_prims,
-                                                    int W, int H, ScrTri* __restrict__ tris, uint32_t* __restrict__ list,
+__global__ void __launch_bounds__(128) k_mesh_setup(const fs3d_mesh_draw* __restrict__ draws,
+                                                    const long long* __restrict__ prim0, int n_draws,
+                                                    long long n_prims, const Mat4 vp, int W, int H, ScrTri* __restrict__ tris, uint32_t* __restrict__ list,
                                                     uint32_t* __restrict__ n_list) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n_prims) return;
-    const int d = find_draw(draws, n_draws, p);
-    const MeshDrawDev& dr = draws[d];
-    const float* v = dr.verts + 15 * (p - dr.prim0);
-    const float* m = dr.mvp;
+    const int d = find_draw(prim0, n_draws, p);
+    const fs3d_mesh_draw& dr = draws[d];
+    const float* v = dr.vertices + 15 * (p - prim0[d]);
+    // the draw's matrix, as the host's product rounds it (on the host, 5202
+    // draws took 50 us, more than the frame's kernels beside it)
+    float m[16];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float* b = dr.model + 4 * c;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            m[4 * c + i] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(vp.m[i], b[0]), __fmul_rn(vp.m[4 + i], b[1])),
+                                               __fmul_rn(vp.m[8 + i], b[2])),
+                                     __fmul_rn(vp.m[12 + i], b[3]));
+    }
     ClipVtx a[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -491,7 +498,7 @@ __global__ void k_mesh_cover(const ScrTri* __restrict__ tris, const uint32_t* __
 
 __device__ __forceinline__ float clamp01_dev(float x) { return x < 0.0f ? 0.0f : (x > 1.0f ? 1.0f : x); }
 
-__global__ void k_mesh_resolve(const MeshDrawDev* __restrict__ draws, const ScrTri* __restrict__ tris,
+__global__ void k_mesh_resolve(const fs3d_mesh_draw* __restrict__ draws, const ScrTri* __restrict__ tris,
                                const unsigned long long* __restrict__ key, const float* __restrict__ lut, int W, int H,
                                float c0, float c1, float c2, float c3, float4* __restrict__ out) {
     const int px = blockIdx.x * blockDim.x + threadIdx.x;
@@ -506,7 +513,7 @@ __global__ void k_mesh_resolve(const MeshDrawDev* __restrict__ draws, const ScrT
     const long long prim = code >> 2;
     const int q = (int)(code & 3u);
     const ScrTri& s = tris[3 * prim + q];
-    const MeshDrawDev& dr = draws[s.draw];
+    const fs3d_mesh_draw& dr = draws[s.draw];
     float r = dr.color[0], g = dr.color[1], b = dr.color[2], a = dr.color[3];
     if (dr.material != FS3D_MAT_BASIC) {
         float l[3];
@@ -514,11 +521,11 @@ __global__ void k_mesh_resolve(const MeshDrawDev* __restrict__ draws, const ScrT
         const float den = lerp3(l[0], l[1], l[2], s.iw);
         const float u = __fdiv_rn(lerp3(l[0], l[1], l[2], s.uw), den);
         const float v = __fdiv_rn(lerp3(l[0], l[1], l[2], s.vw), den);
-        int ti = floor_to_int_dev(__fmul_rn(u, (float)dr.tex_w)) % dr.tex_w;
-        int tj = floor_to_int_dev(__fmul_rn(v, (float)dr.tex_h)) % dr.tex_h;
-        if (ti < 0) ti += dr.tex_w;
-        if (tj < 0) tj += dr.tex_h;
-        const uchar4 t = reinterpret_cast<const uchar4*>(dr.tex)[(size_t)tj * dr.tex_w + ti];
+        int ti = floor_to_int_dev(__fmul_rn(u, (float)dr.tex_width)) % dr.tex_width;
+        int tj = floor_to_int_dev(__fmul_rn(v, (float)dr.tex_height)) % dr.tex_height;
+        if (ti < 0) ti += dr.tex_width;
+        if (tj < 0) tj += dr.tex_height;
+        const uchar4 t = reinterpret_cast<const uchar4*>(dr.texture)[(size_t)tj * dr.tex_width + ti];
         const float tr = lut[t.x], tg = lut[t.y], tb = lut[t.z];
         if (dr.material == FS3D_MAT_TEXTURED) {
             r = __fadd_rn(r, tr);
@@ -588,9 +595,26 @@ extern "C" fs3d_status fs3d_render_meshes(const fs3d_object_view* v, const fs3d_
     cudaStream_t st = (cudaStream_t)stream;
     fs3d_object_view cam = *v;
     for (int i = 0; i < 16; ++i) cam.model[i] = (i % 5 == 0) ? 1.0f : 0.0f;
-    float vp[16];
-    object_mvp(&cam, vp);
-    std::vector<MeshDrawDev> dd((size_t)(n_draws > 0 ? n_draws : 1));
+    Mat4 vp;
+    object_mvp(&cam, vp.m);
+    // sRGB texels to linear, as the sampler of an _SRGB format does (built once)
+    static const std::vector<float> lut = [] {
+        std::vector<float> t(256);
+        for (int i = 0; i < 256; ++i) {
+            const double c = i / 255.0;
+            t[(size_t)i] = (float)(c <= 0.04045 ? c / 12.92 : pow((c + 0.055) / 1.055, 2.4));
+        }
+        return t;
+    }();
+    const size_t lut_b = sizeof(float) * 256;
+    // what goes up beside the draws: the table, then each draw's first primitive
+    std::vector<char> beside(lut_b + sizeof(long long) * (size_t)n_draws);
+    memcpy(beside.data(), lut.data(), lut_b);
+    long long* first = reinterpret_cast<long long*>(beside.data() + lut_b);
+    // the draws go up as they are, unless a buffer has another address on the
+    // device, or they could change before a copy of page-locked memory runs
+    std::vector<fs3d_mesh_draw> own;
+    if (n_draws > 0 && device_view(draws)) own.assign(draws, draws + n_draws);
     long long prims = 0;
     // draws usually share their buffers: look each distinct pointer up once
     const void* last_v = nullptr;
@@ -625,49 +649,38 @@ extern "C" fs3d_status fs3d_render_meshes(const fs3d_object_view* v, const fs3d_
             (m.material != FS3D_MAT_BASIC && (!tdev || (reinterpret_cast<uintptr_t>(tdev) & 3))))
             return set_error(FS3D_ERR_INVALID_ARG,
                              "fs3d_render_meshes: vertices and textures must be 4-byte aligned device or page-locked memory");
-        MeshDrawDev& x = dd[(size_t)d];
-        mat4_mul(vp, m.model, x.mvp);
-        memcpy(x.color, m.color, sizeof(x.color));
-        x.verts = reinterpret_cast<const float*>(vdev);
-        x.tex = tdev;
-        x.tex_w = m.tex_width;
-        x.tex_h = m.tex_height;
-        x.material = m.material;
-        x.n_tri = m.n_vertices / 3;
-        x.prim0 = prims;
-        prims += x.n_tri;
+        if ((vdev && vdev != reinterpret_cast<const uint8_t*>(m.vertices)) || (tdev && tdev != m.texture)) {
+            if (own.empty()) own.assign(draws, draws + n_draws);
+            if (vdev) own[(size_t)d].vertices = reinterpret_cast<const float*>(vdev);
+            if (tdev) own[(size_t)d].texture = tdev;
+        }
+        first[d] = prims;
+        prims += m.n_vertices / 3;
     }
     if (prims >= (1ll << 30)) return set_error(FS3D_ERR_INVALID_ARG, "fs3d_render_meshes: too many triangles");
-    // sRGB texels to linear, as the sampler of an _SRGB format does (built once)
-    static const std::vector<float> lut = [] {
-        std::vector<float> t(256);
-        for (int i = 0; i < 256; ++i) {
-            const double c = i / 255.0;
-            t[(size_t)i] = (float)(c <= 0.04045 ? c / 12.92 : pow((c + 0.055) / 1.055, 2.4));
-        }
-        return t;
-    }();
-    const size_t draws_b = sizeof(MeshDrawDev) * dd.size(), lut_b = sizeof(float) * 256;
+    const size_t draws_b = sizeof(fs3d_mesh_draw) * (size_t)n_draws;
     const size_t tris_b = sizeof(ScrTri) * 3 * (size_t)(prims > 0 ? prims : 1), key_b = sizeof(unsigned long long) * W * H;
-    // draws, table, triangles, their list, then the pixels' keys and the list's
+    // draws, what goes up beside them, triangles, their list, then the pixels' keys and the list's
     // counter (cleared together: all ones, so the counter starts at -1)
     const size_t list_b = sizeof(uint32_t) * 3 * (size_t)(prims > 0 ? prims : 1);
-    const size_t o_lut = (draws_b + 255) & ~(size_t)255, o_tris = (o_lut + lut_b + 255) & ~(size_t)255,
+    const size_t o_lut = (draws_b + 255) & ~(size_t)255, o_tris = (o_lut + beside.size() + 255) & ~(size_t)255,
                  o_list = (o_tris + tris_b + 255) & ~(size_t)255, o_key = (o_list + list_b + 255) & ~(size_t)255;
     char* scratch = nullptr;
     FS3D_CUDA(scratch_alloc((void**)&scratch, o_key + key_b + sizeof(uint32_t), st));
     uint32_t* list = reinterpret_cast<uint32_t*>(scratch + o_list);
     uint32_t* n_list = reinterpret_cast<uint32_t*>(scratch + o_key + key_b);
-    MeshDrawDev* ddev = reinterpret_cast<MeshDrawDev*>(scratch);
+    fs3d_mesh_draw* ddev = reinterpret_cast<fs3d_mesh_draw*>(scratch);
     float* lut_dev = reinterpret_cast<float*>(scratch + o_lut);
     ScrTri* tris = reinterpret_cast<ScrTri*>(scratch + o_tris);
     unsigned long long* key = reinterpret_cast<unsigned long long*>(scratch + o_key);
-    cudaError_t e = cudaMemcpyAsync(ddev, dd.data(), draws_b, cudaMemcpyHostToDevice, st);  // pageable: staged
-    if (e == cudaSuccess) e = cudaMemcpyAsync(lut_dev, lut.data(), lut_b, cudaMemcpyHostToDevice, st);
+    cudaError_t e = cudaMemcpyAsync(lut_dev, beside.data(), beside.size(), cudaMemcpyHostToDevice, st);  // pageable: staged
+    if (e == cudaSuccess && n_draws > 0)
+        e = cudaMemcpyAsync(ddev, own.empty() ? draws : own.data(), draws_b, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(key, 0xFF, key_b + sizeof(uint32_t), st);
     fs3d_status s = e == cudaSuccess ? FS3D_OK : cuda_fail(e, "fs3d_render_meshes upload");
     if (s == FS3D_OK && prims > 0) {
-        k_mesh_setup<<<(unsigned)((prims + 127) / 128), 128, 0, st>>>(ddev, n_draws, prims, W, H, tris, list, n_list);
+        k_mesh_setup<<<(unsigned)((prims + 127) / 128), 128, 0, st>>>(
+            ddev, reinterpret_cast<const long long*>(scratch + o_lut + lut_b), n_draws, prims, vp, W, H, tris, list, n_list);
         s = FS3D_OK;
         if (cudaGetLastError() != cudaSuccess) s = set_error(FS3D_ERR_CUDA, "mesh setup launch");
         if (s == FS3D_OK) {
