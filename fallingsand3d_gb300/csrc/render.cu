@@ -310,24 +310,32 @@ __device__ __forceinline__ bool key_before(float p, int pa, float q, int pb) {
 __device__ __forceinline__ float small_minus1(int k) { return __fsub_rn(__int_as_float(0x4B000000 + k), 8388609.0f); }
 __device__ __forceinline__ int small_int(float x) { return __float_as_int(__fadd_rn(x, 8388608.0f)) - 0x4B000000; }
 
-// Takes the steps of one axis (steps n.., at most k1 = k - 1 of them: its k-th
-// leaves the region) whose keys come before the leaving step's key ke of axis
-// ax.  r: about 1 / e, for the estimate of the first step not taken, which its
-// key and the one before it confirm or correct.
-__device__ __forceinline__ void advance_before(int& v, int s, float& n, float b, float e, float r, float& m, float k1, int pa,
-                                               float ke, int ax) {
+// Takes the steps of one axis at a crossing: of the axis that leaves the region
+// (ax) the k = k1 + 1 steps to its face, of another (steps n.., at most k1 of
+// them) those whose keys come before the leaving step's key ke.  r: about 1 / e,
+// for the estimate of the first step not taken, which its key and the one
+// before it confirm or correct.  All three axes run the same instructions, and
+// so does a cell's step below: branches by axis made the lanes of a warp wait
+// for each other (1024^3 at 1920x1080, young and settled 614 and 246 us a
+// frame, now 514 and 199; 395x179x418 at 436x245 483 and 92, now 388 and 74).
+__device__ __forceinline__ void take_steps(int& v, int s, float& n, float b, float e, float r, float& m, float k1, int pa,
+                                           float ke, int ax) {
+    const bool leaves = pa == ax;
     const float top = __fadd_rn(n, k1);
     float j = __fsub_rn(__fadd_rn(__fadd_rn(__fmul_rn(__fsub_rn(ke, b), r), 0.5f), 12582912.0f), 12582912.0f);
     j = fminf(fmaxf(j, n), top);
-    m = __fmaf_rn(j, e, b);
-    if ((j < top && key_before(m, pa, ke, ax)) ||
-        (j > n && !key_before(__fmaf_rn(__fsub_rn(j, 1.0f), e, b), pa, ke, ax))) {
+    if (leaves) j = __fadd_rn(top, 1.0f);
+    float at = __fmaf_rn(j, e, b);
+    if (!leaves && s &&
+        ((j < top && key_before(at, pa, ke, ax)) ||
+         (j > n && !key_before(__fmaf_rn(__fsub_rn(j, 1.0f), e, b), pa, ke, ax)))) {
         while (j < top && key_before(__fmaf_rn(j, e, b), pa, ke, ax)) j = __fadd_rn(j, 1.0f);
         while (j > n && !key_before(__fmaf_rn(__fsub_rn(j, 1.0f), e, b), pa, ke, ax)) j = __fsub_rn(j, 1.0f);
-        m = __fmaf_rn(j, e, b);
+        at = __fmaf_rn(j, e, b);
     }
     v += s * small_int(__fsub_rn(j, n));
     n = j;
+    m = s ? at : INFINITY;
 }
 
 // A warp takes 8 x 4 pixels (its rays stay together longer than a 16 x 2
@@ -439,91 +447,50 @@ __global__ void __launch_bounds__(64) k_render_dda(G grid, BrickMap bm, CamDev c
                 float ke = x0;
                 if (key_before(x1, 1, ke, ax)) { ax = 1; ke = x1; }
                 if (key_before(x2, 2, ke, ax)) { ax = 2; ke = x2; }
-                // the other axes take their steps that come before it (a prefix of their keys)
-                if (ax != 0 && s0) advance_before(v0, s0, n0, b0, e0, r0, m0, l0, 0, ke, ax);
-                if (ax != 1 && s1) advance_before(v1, s1, n1, b1, e1, r1, m1, l1, 1, ke, ax);
-                if (ax != 2 && s2) advance_before(v2, s2, n2, b2, e2, r2, m2, l2, 2, ke, ax);
+                // its k-th step, and the other axes' steps that come before it (a prefix of their keys)
+                take_steps(v0, s0, n0, b0, e0, r0, m0, l0, 0, ke, ax);
+                take_steps(v1, s1, n1, b1, e1, r1, m1, l1, 1, ke, ax);
+                take_steps(v2, s2, n2, b2, e2, r2, m2, l2, 2, ke, ax);
                 tcur = ke;
                 last = ax;
-                if (ax == 0) {
-                    if (k0 == g0) { left = 0; break; }
-                    v0 += s0 * k0;
-                    n0 = __fadd_rn(n0, __fadd_rn(l0, 1.0f));
-                    m0 = __fmaf_rn(n0, e0, b0);
-                } else if (ax == 1) {
-                    if (k1 == g1) { left = 0; break; }
-                    v1 += s1 * k1;
-                    n1 = __fadd_rn(n1, __fadd_rn(l1, 1.0f));
-                    m1 = __fmaf_rn(n1, e1, b1);
-                } else {
-                    if (k2 == g2) { left = 0; break; }
-                    v2 += s2 * k2;
-                    n2 = __fadd_rn(n2, __fadd_rn(l2, 1.0f));
-                    m2 = __fmaf_rn(n2, e2, b2);
-                }
+                if (ax == 0 ? k0 == g0 : (ax == 1 ? k1 == g1 : k2 == g2)) left = 0;
             }
             if (left <= 0) break;
-            // walk the brick's cells until one is not empty or the walk leaves it.
-            // Which cells it visits does not depend on what they hold, so kAhead
-            // of them are fetched at a time: a ray grazing a surface is a chain
-            // of hundreds of fetches, and the longest ray ends the frame
-            constexpr int kAhead = 4;
+            // walk the brick's cells until one is not empty or the walk leaves it
+            // (a cell's fetch runs while the next one is found)
+            const I dy = s1 > 0 ? ry : (s1 < 0 ? (I)0 - ry : (I)0), dz = s2 > 0 ? rz : (s2 < 0 ? (I)0 - rz : (I)0);
             I row = (I)v1 * ry + (I)v2 * rz;
             uint32_t m = 0;
             bool inside = true;
             while (inside && left > 0) {
-                typename G::Cell cell[kAhead];
-                I at_row[kAhead];
-                int at_x[kAhead], at_last[kAhead];
-                float at_t[kAhead];
-                int n = 0;
-#pragma unroll
-                for (int i = 0; i < kAhead; ++i) {
-                    if (!inside || left <= 0) continue;
-                    --left;
-                    cell[i] = grid.fetch(row, v0);
-                    at_row[i] = row;
-                    at_x[i] = v0;
-                    at_last[i] = last;
-                    at_t[i] = tcur;
-                    n = i + 1;
-                    // next cell: the axis whose boundary key comes first (equal keys: z, then y, then x)
-                    if (m0 < m1 ? m0 < m2 : false) {
-                        tcur = m0;
-                        const int u = v0;
-                        v0 += s0;
-                        inside = ((u ^ v0) & ~7) == 0;
-                        if ((unsigned)v0 >= (unsigned)NX) left = 0;
-                        m0 = __fmaf_rn(n0 = __fadd_rn(n0, 1.0f), e0, b0);
-                        last = 0;
-                    } else if (!(m0 < m1) && m1 < m2) {
-                        tcur = m1;
-                        const int u = v1;
-                        v1 += s1;
-                        inside = ((u ^ v1) & ~7) == 0;
-                        if ((unsigned)v1 >= (unsigned)NY) left = 0;
-                        m1 = __fmaf_rn(n1 = __fadd_rn(n1, 1.0f), e1, b1);
-                        row += s1 > 0 ? ry : (I)0 - ry;
-                        last = 1;
-                    } else {
-                        tcur = m2;
-                        const int u = v2;
-                        v2 += s2;
-                        inside = ((u ^ v2) & ~7) == 0;
-                        if ((unsigned)v2 >= (unsigned)NZ) left = 0;
-                        m2 = __fmaf_rn(n2 = __fadd_rn(n2, 1.0f), e2, b2);
-                        row += s2 > 0 ? rz : (s2 < 0 ? (I)0 - rz : (I)0);
-                        last = 2;
-                    }
+                --left;
+                const typename G::Cell cell = grid.fetch(row, v0);
+                const I at_row = row;
+                const int at_x = v0, at_last = last;
+                const float at_t = tcur;
+                // next cell: the axis whose boundary key comes first (equal keys: z, then y, then x)
+                const bool a0 = m0 < m1 && m0 < m2, a1 = !(m0 < m1) && m1 < m2, a2 = !a0 && !a1;
+                tcur = a0 ? m0 : (a1 ? m1 : m2);
+                last = a0 ? 0 : (a1 ? 1 : 2);
+                const int u0 = v0 + (a0 ? s0 : 0), u1 = v1 + (a1 ? s1 : 0), u2 = v2 + (a2 ? s2 : 0);
+                inside = (((u0 ^ v0) | (u1 ^ v1) | (u2 ^ v2)) & ~7) == 0;
+                if ((unsigned)u0 >= (unsigned)NX || (unsigned)u1 >= (unsigned)NY || (unsigned)u2 >= (unsigned)NZ) left = 0;
+                v0 = u0;
+                v1 = u1;
+                v2 = u2;
+                row += a1 ? dy : (a2 ? dz : (I)0);
+                n0 = __fadd_rn(n0, a0 ? 1.0f : 0.0f);
+                n1 = __fadd_rn(n1, a1 ? 1.0f : 0.0f);
+                n2 = __fadd_rn(n2, a2 ? 1.0f : 0.0f);
+                m0 = a0 ? __fmaf_rn(n0, e0, b0) : m0;
+                m1 = a1 ? __fmaf_rn(n1, e1, b1) : m1;
+                m2 = a2 ? __fmaf_rn(n2, e2, b2) : m2;
+                if (G::filled(cell)) {
+                    m = grid.material(cell, at_row, at_x);
+                    last = at_last;
+                    tcur = at_t;
+                    break;
                 }
-#pragma unroll
-                for (int i = kAhead - 1; i >= 0; --i)
-                    if (i < n && G::filled(cell[i])) {
-                        m = grid.material(cell[i], at_row[i], at_x[i]);
-                        last = at_last[i];
-                        tcur = at_t[i];
-                    }
-                if (m != 0u) break;
             }
             if (m != 0u) {
                 float n[3] = {0.0f, 0.0f, 0.0f};
