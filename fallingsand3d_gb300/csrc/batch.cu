@@ -111,7 +111,7 @@ struct PinnedArray {
         T *nh0 = nullptr, *nh1 = nullptr, *nd = nullptr;
         FS3D_CUDA(cudaMallocHost((void**)&nh0, sizeof(T) * c));
         cudaError_t e = cudaMallocHost((void**)&nh1, sizeof(T) * c);
-        if (e == cudaSuccess) e = cudaMalloc((void**)&nd, sizeof(T) * c);
+        if (e == cudaSuccess) e = device_alloc((void**)&nd, sizeof(T) * c);
         if (e != cudaSuccess) {
             cudaFreeHost(nh0);
             if (nh1) cudaFreeHost(nh1);
@@ -239,7 +239,8 @@ namespace {
 // mode keeps them in shared memory, where dense steps are cheap.
 // (2048 mixed worlds: 64-step segments at ages 0 / 64 / 128 / 192 take
 // 5.1 / 2.7 / 1.9 / 1.9 ms in shared memory and 8.5 / 3.4 / 1.6 / 1.3 ms
-// from L2, which wins from age 128 on.)
+// from L2, which wins from age 128 on; with today's kernels 1.37 and 0.75 ms at
+// age 192.)
 constexpr uint64_t kYoungSteps = 128;
 
 // Global-memory class of a settled world by its class for itself (0..3) and
@@ -420,7 +421,13 @@ void free_world(fs3d_batch* b, BWorld& w) {
 // cached: its release threshold is raised when a batch is created).
 template <class T>
 cudaError_t stream_alloc(T** p, size_t n, cudaStream_t st) {
-    return cudaMallocAsync(reinterpret_cast<void**>(p), n, st);
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(p), n, st);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        scratch_give_back();
+        e = cudaMallocAsync(reinterpret_cast<void**>(p), n, st);
+    }
+    return e;
 }
 
 // Test hook (fs3d_test_inject): admissions whose world memory allocation is
@@ -467,7 +474,7 @@ fs3d_batch::StagingSlot* take_slot(fs3d_batch::StagingSlot* ring, int& turn, siz
         if (sl.p) cudaFreeAsync(sl.p, st);
         sl.p = nullptr;
         sl.cap = 0;
-        *e = cudaMallocAsync(reinterpret_cast<void**>(&sl.p), n, st);
+        *e = stream_alloc(&sl.p, n, st);
         if (*e == cudaSuccess) sl.cap = n;
     }
     return &sl;
@@ -1056,7 +1063,7 @@ fs3d_status build_tables(fs3d_batch* b) {
         if (!by_class[c].empty()) mask |= 1u << c;
     for (int c = kSingleCtaClasses; c < kResidentClasses; ++c)
         if (((mask >> c) & 1u) && !b->edges[c - kSingleCtaClasses])
-            FS3D_CUDA(cudaMalloc(&b->edges[c - kSingleCtaClasses], batch_slab_edge_bytes(kClusterSizes[c - kSingleCtaClasses])));
+            FS3D_CUDA(device_alloc(&b->edges[c - kSingleCtaClasses], batch_slab_edge_bytes(kClusterSizes[c - kSingleCtaClasses])));
     b->class_mask = mask;
     // admissions complete before the segment reads their planes
     for (auto& ev : b->pending_ready) FS3D_CUDA(cudaStreamWaitEvent(b->stream, ev.get(), 0));

@@ -68,6 +68,10 @@ bool current_context_id(unsigned long long* id);
 
 // device memory for a call's own duration, stream-ordered (scratch.cpp)
 cudaError_t scratch_alloc(void** p, size_t n, cudaStream_t st);
+// unmaps what the scratch pool of the current device keeps unused
+void scratch_give_back();
+// cudaMalloc; out of memory, once more after scratch_give_back
+cudaError_t device_alloc(void** p, size_t n);
 
 // ---- chained launches: a kernel that begins with chain_wait() may be launched
 // with launch_chained(), so that its CTAs are placed and its first instructions

@@ -4,7 +4,8 @@
 // synchronisation, so a caller that waits for each result (a frame loop, a
 // script's run) paid for mapping it again: 115 to 145 us for the 37 MB of a
 // full-HD mesh frame.  This pool, one per device and context, keeps at most
-// kScratchKept bytes across a synchronisation.
+// kScratchKept bytes across a synchronisation, and gives those back when an
+// allocation of the library fails.
 #include <mutex>
 
 #include "fs3d_common.h"
@@ -58,9 +59,25 @@ cudaError_t scratch_alloc(void** p, size_t n, cudaStream_t st) {
         if (cudaMemPool_t pool = scratch_pool()) {
             if (cudaMallocFromPoolAsync(p, n, pool, st) == cudaSuccess) return cudaSuccess;
             cudaGetLastError();
-            cudaMemPoolTrimTo(pool, 0);
+            scratch_give_back();
         }
     return cudaMallocAsync(p, n, st);
+}
+
+void scratch_give_back() {
+    int dev = 0;
+    unsigned long long ctx = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices || !current_context_id(&ctx)) return;
+    std::lock_guard<std::mutex> lock(g_pools_mu);
+    if (g_pools[dev].pool && g_pools[dev].ctx == ctx) cudaMemPoolTrimTo(g_pools[dev].pool, 0);
+}
+
+cudaError_t device_alloc(void** p, size_t n) {
+    cudaError_t e = cudaMalloc(p, n);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    scratch_give_back();
+    return cudaMalloc(p, n);
 }
 
 }  // namespace fs3d

@@ -140,20 +140,20 @@ fs3d_status fs3d_world_create(const uint8_t* grid_host, int X, int Y, int Z, uin
     };
     cudaError_t e = cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return fail(e, "cudaStreamCreate");
-    e = cudaMalloc((void**)&w->hash_dev, sizeof(unsigned long long));
+    e = device_alloc((void**)&w->hash_dev, sizeof(unsigned long long));
     if (e != cudaSuccess) return fail(e, "cudaMalloc(hash)");
     if (layout == FS3D_LAYOUT_BYTES) {
-        e = cudaMalloc((void**)&w->bytes, (size_t)w->cells());
+        e = device_alloc((void**)&w->bytes, (size_t)w->cells());
         if (e != cudaSuccess) return fail(e, "cudaMalloc(grid)");
     } else {
-        e = cudaMalloc((void**)&w->rows, plane_bytes(X, Y, Z));
+        e = device_alloc((void**)&w->rows, plane_bytes(X, Y, Z));
         if (e != cudaSuccess) return fail(e, "cudaMalloc(planes)");
-        if (e == cudaSuccess) e = cudaMalloc((void**)&w->err, sizeof(int) * kErrInts);
+        if (e == cudaSuccess) e = device_alloc((void**)&w->err, sizeof(int) * kErrInts);
         if (e == cudaSuccess) e = cudaMemset(w->err, 0, sizeof(int) * kErrInts);
         if (e != cudaSuccess) return fail(e, "cudaMalloc(error record)");
         SlabPlan plan;
-        e = cudaMalloc((void**)&w->rflags, (size_t)Y * Z);
-        if (e == cudaSuccess && slab_plan(X, Y, Z, &plan)) e = cudaMalloc(&w->slab_scratch, plan.scratch);
+        e = device_alloc((void**)&w->rflags, (size_t)Y * Z);
+        if (e == cudaSuccess && slab_plan(X, Y, Z, &plan)) e = device_alloc(&w->slab_scratch, plan.scratch);
         if (e != cudaSuccess) return fail(e, "cudaMalloc(change flags)");
     }
     s = upload(w, grid_host);
@@ -373,13 +373,13 @@ fs3d_status fs3d_render(fs3d_world* w, const fs3d_camera* cam, int W, int H, int
     const size_t bytes = (size_t)W * H * 4 * sizeof(float);
     if (mode == FS3D_RENDER_DDA && !w->brickmap) {
         const size_t n = brickmap_bytes(w->X, w->Y, w->Z);
-        FS3D_CUDA(cudaMalloc((void**)&w->brickmap, n));
+        FS3D_CUDA(device_alloc((void**)&w->brickmap, n));
         FS3D_CUDA(cudaMemsetAsync(w->brickmap, 0, n, w->stream));  // (its counters)
     }
     // planes worlds stepped by the per-step kernel keep exact brick counts
     if (mode == FS3D_RENDER_DDA && w->layout == FS3D_LAYOUT_PLANES && !w->brick_counts &&
         plane_bytes(w->X, w->Y, w->Z) > kCountsPlaneBytes)
-        FS3D_CUDA(cudaMalloc((void**)&w->brick_counts, brick_count_bytes(w->X, w->Y, w->Z)));
+        FS3D_CUDA(device_alloc((void**)&w->brick_counts, brick_count_bytes(w->X, w->Y, w->Z)));
     if (!out_on_device) FS3D_CUDA(scratch_alloc((void**)&dst, bytes, w->stream));
     fs3d_status s;
     if (mode == FS3D_RENDER_SDF_SPHERE)
