@@ -214,6 +214,7 @@ struct fs3d_batch {
     // are widened by level `widen` (choose_widen)
     int spread = 0, spread_from = 0;
     int widen = 1;
+    bool widen_large = false;  // and those of the widest class by themselves to a whole SM's
     void* edges[kResidentClasses - kSingleCtaClasses] = {};  // the cluster classes' edge buffers (once needed)
     unsigned long long* hash_dev = nullptr;
     unsigned long long* processed_dev = nullptr;  // cell-steps the resident kernels evaluated
@@ -245,9 +246,9 @@ constexpr uint64_t kYoungSteps = 128;
 
 // Global-memory class of a settled world by its class for itself (0..3) and
 // the batch's level (choose_widen).
-constexpr int kPackedLevel = 0, kOwnLevel = 1, kWidestLevel = 5;
+constexpr int kPackedLevel = 0, kOwnLevel = 1, kWidestLevel = 4;
 constexpr int kWidened[kWidestLevel + 1][kGmDense] = {
-    {1, 1, 1, 3}, {0, 1, 2, 3}, {0, 2, 3, 3}, {2, 3, 3, 3}, {3, 3, 3, 3}, {3, 3, 3, 4}};
+    {1, 1, 1, 3}, {0, 1, 2, 3}, {0, 2, 3, 3}, {2, 3, 3, 3}, {3, 3, 3, 3}};
 
 // Segment class of a running world (-1: the per-step kernel) under the
 // batch's mode: 1 shared-memory classes, 2 global-memory classes, 3 hybrid
@@ -267,7 +268,7 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
         if (w.cls_gm == -2) w.cls_gm = resident_class_gm(w.X, w.Y, w.Z);
         const int c = w.cls_gm;
         if (c < 0) return -1;
-        const int leveled = mode == 3 ? kWidened[b->widen][c] : c;
+        const int leveled = mode == 3 ? (c == kGmDense - 1 && b->widen_large ? kGmDense : kWidened[b->widen][c]) : c;
         return kResidentClasses + (b->promote ? std::max(std::min(c + b->promote, kGmDense - 1), leveled) : leveled);
     };
     if (mode == 1) return smem();
@@ -334,7 +335,9 @@ void choose_spread(fs3d_batch* b) {
 // by itself leaves no warp idle at a step's barrier.  With fewer worlds than
 // fill the SMs, a segment takes as long as its busiest world, whose step is
 // shorter in a wider CTA: the widest level whose CTAs all run at once is taken,
-// and the first (64 and 128 threads doubled) up to 1.75 times that.  Settled
+// and the first (64 and 128 threads doubled) up to 1.75 times that; where they
+// still fit, the largest worlds' CTAs take a whole SM's threads (third segment
+// of 512 fresh mixed worlds: 673 us, 408 with them).  Settled
 // 64-step segments, class by itself / widened: 100 mixed worlds 326 / 262 us,
 // 300 344 / 281, 600 410 / 365, 1200 595 / 482; 64^3: 100 worlds 365 / 237, 600
 // 451 / 285; 16^3: 100 232 / 176, 600 280 / 194 (305 at 64 threads, so the
@@ -346,6 +349,7 @@ void choose_spread(fs3d_batch* b) {
 // 358) up to 1.75 times (64x48x128: 1000 worlds 460 / 569, 2048 713 / 688).
 void choose_widen(fs3d_batch* b) {
     b->widen = kOwnLevel;
+    b->widen_large = false;
     if (b->cfg.use_smem != 3) return;
     int64_t by_class[kGmDense] = {0, 0, 0, 0}, young = 0;
     for (auto& kv : b->worlds) {
@@ -378,6 +382,7 @@ void choose_widen(fs3d_batch* b) {
         }
         if (l > kOwnLevel && need <= (l == kOwnLevel + 1 ? fit * 7 / 4 : fit)) {
             b->widen = l;
+            b->widen_large = need + by_class[kGmDense - 1] * (threads[kGmDense] - threads[kGmDense - 1]) <= fit;
             return;
         }
     }
