@@ -638,11 +638,11 @@ def run_fs3d(args):
                 "hbm_frac": round(gbs / hbm, 3), "peak_gbs": hbm, "peak_source": src,
                 "note": "134 MB grid read+written per step, in place (comparable to the 126 MB L2): the "
                         "algorithmic figure counts 2 B per cell; dram_* are the DRAM bytes ncu measured"}
-        warm = profile_values("k_step_rows64_pillars512_warm", ("dram_bytes_per_launch", "duration_ns"))
+        warm = profile_values("k_step_rows_pillars512_warm", ("dram_bytes_per_launch", "duration_ns"))
         if warm:
             dram_gbs = warm["dram_bytes_per_launch"] / warm["duration_ns"]
             p512.update({"dram_gbs": round(dram_gbs, 1), "dram_frac": round(dram_gbs / hbm, 3),
-                         "dram_source": "ncu, 3 warm launches at steps ~990 (profiles/k_step_rows64_pillars512_warm.md)"})
+                         "dram_source": "ncu, 3 warm launches at steps ~990 (profiles/k_step_rows_pillars512_warm.md)"})
         # same world through the plane layout (the per-step kernel that skips settled row-pairs)
         with fs3d.World(g, 1, 0, fs3d.LAYOUT_PLANES) as w:
             w.step(8)
