@@ -24,3 +24,27 @@ def test_rows_of_any_length_and_alignment(fs3d, orc, cuda, X, shift):
     got = out[32 + shift:32 + shift + g.size].reshape(g.shape)
     assert (got == ref).all(), describe_diff(got, ref, n + 1)
     assert (out[:32 + shift] == buf[:32 + shift]).all() and (out[32 + shift + g.size:] == buf[32 + shift + g.size:]).all()
+
+
+@pytest.mark.parametrize("X", [64, 75, 2064])
+def test_captured_steps_replay(fs3d, orc, cuda, X):
+    """The chained launches of one call in a captured graph, between copies."""
+    Y, Z, n = 20, 33, 6
+    r = np.random.default_rng(X)
+    g = r.choice(np.array([0, 1, 2, 3, 9], np.uint8), (Y, Z, X), p=[0.5, 0.05, 0.25, 0.18, 0.02])
+    keep = cuda.from_numpy(g).cuda()
+    d, out = keep.clone(), cuda.empty_like(keep)
+    fs3d.step_device(d.data_ptr(), X, Y, Z, 7, 0, n, stream_ptr(cuda))
+    cuda.cuda.synchronize()
+    graph = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(graph):
+        d.copy_(keep)
+        fs3d.step_device(d.data_ptr(), X, Y, Z, 7, 0, n, stream_ptr(cuda))
+        out.copy_(d)
+    ref = g.copy()
+    orc.run(ref, 7, 0, n, nthreads=0)
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        cuda.cuda.synchronize()
+        assert (out.cpu().numpy() == ref).all()
