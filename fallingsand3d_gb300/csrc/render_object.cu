@@ -288,11 +288,16 @@ struct Mat4 {
     float m[16];
 };
 
-struct ScrTri {
-    float sx[3], sy[3], sz[3], iw[3], uw[3], vw[3];
-    float area;
+// (16-byte aligned: a thread of the set-up writes it in seven stores; in 4-byte
+// ones, each to 32 sectors, 62 k triangles took 15 us, now 11)
+struct __align__(16) ScrTri {
+    float sx[3], area;
+    float sy[3];
     int tl;
+    float sz[3];
     int draw;
+    int box[4];  // first and last column, first and last row of its pixels
+    float iw[3], uw[3], vw[3];
 };
 
 struct ClipVtx {
@@ -434,6 +439,10 @@ __global__ void __launch_bounds__(128) k_mesh_setup(const fs3d_mesh_draw* __rest
         const float ymin = fminf(fminf(s.sy[0], s.sy[1]), s.sy[2]), ymax = fmaxf(fmaxf(s.sy[0], s.sy[1]), s.sy[2]);
         if (xmax < -1.0f || ymax < -1.0f || xmin > (float)W + 1.0f || ymin > (float)H + 1.0f) return;
         s.draw = d;
+        s.box[0] = max(0, floor_to_int_dev(xmin));
+        s.box[1] = min(W - 1, floor_to_int_dev(ceilf(xmax)));
+        s.box[2] = max(0, floor_to_int_dev(ymin));
+        s.box[3] = min(H - 1, floor_to_int_dev(ceilf(ymax)));
         tris[3 * p + t] = s;
         list[atomicAdd(n_list, 1u) + 1u] = (uint32_t)(3 * p + t);  // (the counter starts at -1)
     };
@@ -464,7 +473,8 @@ __device__ __forceinline__ bool tri_cover_dev(const ScrTri& s, float fx, float f
 
 // One warp per listed screen triangle: it walks the box in 8 x 4 tiles (62 k
 // small triangles at 1920x1080: 98 us with a lane's pixel found by 64-bit
-// divisions and a warp for every possible slot).
+// divisions and a warp for every possible slot, 56 with the box found here and
+// not in the set-up, 48).  Bound: instructions, a third of them per triangle.
 __global__ void k_mesh_cover(const ScrTri* __restrict__ tris, const uint32_t* __restrict__ list,
                              const uint32_t* __restrict__ n_list, int W, int H, unsigned long long* __restrict__ key) {
     const int lane = threadIdx.x & 31;
@@ -476,10 +486,7 @@ __global__ void k_mesh_cover(const ScrTri* __restrict__ tris, const uint32_t* __
         const float x0 = g.sx[0], x1 = g.sx[1], x2 = g.sx[2], y0 = g.sy[0], y1 = g.sy[1], y2 = g.sy[2];
         const float area = g.area, z[3] = {g.sz[0], g.sz[1], g.sz[2]};
         const int tl = g.tl;
-        const float xmin = fminf(fminf(x0, x1), x2), xmax = fmaxf(fmaxf(x0, x1), x2);
-        const float ymin = fminf(fminf(y0, y1), y2), ymax = fmaxf(fmaxf(y0, y1), y2);
-        const int bx0 = max(0, floor_to_int_dev(xmin)), bx1 = min(W - 1, floor_to_int_dev(ceilf(xmax)));
-        const int by0 = max(0, floor_to_int_dev(ymin)), by1 = min(H - 1, floor_to_int_dev(ceilf(ymax)));
+        const int bx0 = g.box[0], bx1 = g.box[1], by0 = g.box[2], by1 = g.box[3];
         const uint32_t code = 0xFFFFFFFFu - sl / 3u * 4u - sl % 3u;
         for (int ty = by0; ty <= by1; ty += 4)
             for (int tx = bx0; tx <= bx1; tx += 8) {
