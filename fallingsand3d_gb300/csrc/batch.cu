@@ -210,9 +210,11 @@ struct fs3d_batch {
     int grid = 0;
     int promote = 0;  // single-CTA resident worlds run this many classes wider (autotuned)
     // hybrid mode, chosen with the tables: young worlds of class `spread_from`
-    // or wider run in cluster class `spread` (0: none), settled worlds' CTAs
+    // or wider, of at least `spread_lanes` lane tasks a step, run in cluster
+    // class `spread` (0: none), settled worlds' CTAs
     // are widened by level `widen` (choose_widen)
     int spread = 0, spread_from = 0;
+    int64_t spread_lanes = 0;
     int widen = 1;
     bool widen_large = false;  // and those of the widest class by themselves to a whole SM's
     void* edges[kResidentClasses - kSingleCtaClasses] = {};  // the cluster classes' edge buffers (once needed)
@@ -250,6 +252,9 @@ constexpr int kPackedLevel = 0, kOwnLevel = 1, kWidestLevel = 4;
 constexpr int kWidened[kWidestLevel + 1][kGmDense] = {
     {1, 1, 1, 3}, {0, 1, 2, 3}, {0, 2, 3, 3}, {2, 3, 3, 3}, {3, 3, 3, 3}};
 
+// lane tasks of a dense step
+int64_t step_lanes(const BWorld& w) { return (int64_t)nblocks(w.Y, 1) * nblocks(w.Z, 1) << plane_lg(w.nw); }
+
 // Segment class of a running world (-1: the per-step kernel) under the
 // batch's mode: 1 shared-memory classes, 2 global-memory classes, 3 hybrid
 // (young worlds in shared memory when they fit, settled ones in global
@@ -283,7 +288,7 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
             // against 3.02 ms in 128-thread CTAs; moving the 256-thread worlds
             // up to 768 threads too measured 3.09 ms)
             const int c = smem();
-            if (b->spread && (c < 0 || c >= b->spread_from) &&
+            if (b->spread && (c < 0 || c >= b->spread_from) && step_lanes(w) >= b->spread_lanes &&
                 batch_slabs_fit(w.X, w.Y, w.Z, kClusterSizes[b->spread - kSingleCtaClasses]))
                 return b->spread;
             if (c >= 0 && c < kSingleCtaClasses) return c == 0 ? 1 : c;
@@ -305,13 +310,20 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
 // segments of fresh mixed worlds, none spread / the larger ones / all: 32
 // worlds 1625 / 1076 / 969 us, 64 1482 / 1152 / 1249, 150 1837 / 1284 / 1855,
 // 350 2213 / 1704 / 1975, 512 2304 / 3317 (in clusters of 2) / -.
+// With still more worlds only those of 1.75 times an SM's average share of a
+// step are spread (over 8): 512 ragged worlds, whose few largest (130 cells a
+// side, 4 lanes a row pair) end each segment, 3452 us for two segments without
+// and 2126 with; 512 mixed 2009 and 1993; from 700 worlds on none is that large.
 void choose_spread(fs3d_batch* b) {
     b->spread = 0;
+    b->spread_lanes = 0;
     if (b->cfg.use_smem != 3) return;
     int large = 0, whole = 0, rest = 0;
+    int64_t lanes = 0;
     for (auto& kv : b->worlds) {
         BWorld& w = kv.second;
         if (w.done || w.t >= kYoungSteps) continue;
+        lanes += step_lanes(w);
         if (w.cls_smem == -2) w.cls_smem = resident_class(w.X, w.Y, w.Z);
         if (w.cls_smem < 0 || w.cls_smem >= kSingleCtaClasses) ++large;
         else if (w.cls_smem == kSingleCtaClasses - 1) ++whole;
@@ -329,6 +341,10 @@ void choose_spread(fs3d_batch* b) {
         spread(8, kSingleCtaClasses);
     else if (large > 0 && large * 4 + whole + rest / 3 <= 2 * sms)
         spread(4, kSingleCtaClasses);
+    else {
+        spread(8, kSingleCtaClasses - 1);
+        b->spread_lanes = lanes / sms * 7 / 4 + 1;
+    }
 }
 
 // How wide the hybrid mode makes the CTAs of settled worlds.  A world's class

@@ -42,3 +42,23 @@ def test_mixed_young_batch_matches_oracle(fs3d, orc):
     for i, (g, o) in enumerate(zip(grids, outs)):
         orc.run(g, 7 + i, 0, 192, nthreads=0)
         assert (o == g).all(), dims[i]
+
+
+@pytest.mark.parametrize("small,large", [(900, [(130, 128, 131), (128, 128, 128), (257, 64, 100)]), (1500, [(64, 200, 99)])])
+def test_few_largest_of_many_young_worlds(fs3d, orc, small, large):
+    """More young worlds than are spread by count: only those far above an
+    SM's share of a step take clusters, beside many that do not."""
+    dims = large + [(16 + 8 * (i % 4), 12 + i % 9, 20 + i % 13) for i in range(small)]
+    seeds = [50 + i % 40 for i in range(len(dims))]
+    grids = [fs3d.gen_batch_world(s, *d) for s, d in zip(seeds, dims)]
+    with fs3d.Batch(4 << 30, steps_per_segment=40) as b:
+        ts = b.admit_many(grids, seeds, 100)
+        for _ in range(3):
+            b.run_segment()
+        b.sync()
+        done, hs = b.poll_many(ts)
+    assert done.all()
+    for i, (g, s) in enumerate(zip(grids, seeds)):
+        if i < len(large) or i % 29 == 0:
+            orc.run(g, s, 0, 100, nthreads=0)
+            assert int(hs[i]) == orc.hash(g), dims[i]
