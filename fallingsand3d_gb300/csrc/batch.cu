@@ -301,19 +301,18 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
     return -1;
 }
 
-// How the hybrid mode spreads young worlds over clusters.  A large world's
-// dense steps are the segment's longest chain, so where SMs are left over it
-// is spread: every world of a whole SM's class and larger over 8 CTAs when the
-// batch then still fits the SMs, else those larger than one CTA's shared
-// memory over 8 or 4 while the batch fits the SMs twice over.  Beyond that,
-// and in clusters of 2, clusters only take SMs from the other worlds.  Two
-// segments of fresh mixed worlds, none spread / the larger ones / all: 32
-// worlds 1625 / 1076 / 969 us, 64 1482 / 1152 / 1249, 150 1837 / 1284 / 1855,
-// 350 2213 / 1704 / 1975, 512 2304 / 3317 (in clusters of 2) / -.
-// With still more worlds only those of 1.75 times an SM's average share of a
-// step are spread (over 8): 512 ragged worlds, whose few largest (130 cells a
-// side, 4 lanes a row pair) end each segment, 3452 us for two segments without
-// and 2126 with; 512 mixed 2009 and 1993; from 700 worlds on none is that large.
+// How the hybrid mode spreads young worlds over clusters of 8 CTAs.  A large
+// world's dense steps are the segment's longest chain, so where SMs are left
+// over it is spread: every world of a whole SM's class and larger when the
+// batch then still fits the SMs, else those larger than one CTA's shared memory
+// while the batch fits the SMs twice over.  Two segments of fresh mixed worlds,
+// none spread / the larger ones / all: 32 worlds 1625 / 1076 / 969 us, 64 1482 /
+// 1152 / 1249, 150 1837 / 1284 / 1855.  With still more worlds clusters take SMs
+// from the others, and only those far above an SM's average share of a step are
+// spread, 1.75 times it or, while a batch of half as many CTAs a world would fit
+// the SMs twice, 2 times: 400 mixed worlds (all larger ones over 4 CTAs, those)
+// 1835 / 1501 us, 220 ragged 1631 / 1493; 512 mixed (none, those) 2101 / 1528,
+// 300 ragged 1890 / 1611; from 700 worlds on none is that large.
 void choose_spread(fs3d_batch* b) {
     b->spread = 0;
     b->spread_lanes = 0;
@@ -330,20 +329,14 @@ void choose_spread(fs3d_batch* b) {
         else ++rest;  // three to an SM
     }
     const int sms = sm_count_public();
-    auto spread = [&](int cs, int from) {
-        for (int c = kSingleCtaClasses; c < kResidentClasses; ++c)
-            if (kClusterSizes[c - kSingleCtaClasses] == cs) b->spread = c;
-        b->spread_from = from;
-    };
-    if (large + whole > 0 && (large + whole) * 8 + rest / 3 <= sms)
-        spread(8, kSingleCtaClasses - 1);
-    else if (large > 0 && large * 8 + whole + rest / 3 <= 2 * sms)
-        spread(8, kSingleCtaClasses);
-    else if (large > 0 && large * 4 + whole + rest / 3 <= 2 * sms)
-        spread(4, kSingleCtaClasses);
-    else {
-        spread(8, kSingleCtaClasses - 1);
-        b->spread_lanes = lanes / sms * 7 / 4 + 1;
+    b->spread = kResidentClasses - 1;
+    static_assert(kClusterSizes[kResidentClasses - 1 - kSingleCtaClasses] == 8, "the widest cluster class");
+    b->spread_from = kSingleCtaClasses - 1;
+    const bool all = large + whole > 0 && (large + whole) * 8 + rest / 3 <= sms;
+    if (!all && large > 0 && large * 8 + whole + rest / 3 <= 2 * sms) {
+        b->spread_from = kSingleCtaClasses;
+    } else if (!all) {
+        b->spread_lanes = lanes / sms * (large * 4 + whole + rest / 3 <= 2 * sms ? 8 : 7) / 4 + 1;
     }
 }
 
