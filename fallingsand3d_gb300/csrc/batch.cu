@@ -1077,7 +1077,8 @@ fs3d_status build_tables(fs3d_batch* b) {
         if (!by_class[c].empty()) mask |= 1u << c;
     for (int c = kSingleCtaClasses; c < kResidentClasses; ++c)
         if (((mask >> c) & 1u) && !b->edges[c - kSingleCtaClasses])
-            FS3D_CUDA(device_alloc(&b->edges[c - kSingleCtaClasses], batch_slab_edge_bytes(kClusterSizes[c - kSingleCtaClasses])));
+            FS3D_CUDA(stream_alloc(&b->edges[c - kSingleCtaClasses], batch_slab_edge_bytes(kClusterSizes[c - kSingleCtaClasses]),
+                                   b->stream));
     b->class_mask = mask;
     // admissions complete before the segment reads their planes
     for (auto& ev : b->pending_ready) FS3D_CUDA(cudaStreamWaitEvent(b->stream, ev.get(), 0));
