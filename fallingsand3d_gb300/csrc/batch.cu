@@ -246,12 +246,6 @@ namespace {
 // age 192.)
 constexpr uint64_t kYoungSteps = 128;
 
-// Global-memory class of a settled world by its class for itself (0..3) and
-// the batch's level (choose_widen).
-constexpr int kPackedLevel = 0, kOwnLevel = 1, kWidestLevel = 4;
-constexpr int kWidened[kWidestLevel + 1][kGmDense] = {
-    {1, 1, 1, 3}, {0, 1, 2, 3}, {0, 2, 3, 3}, {2, 3, 3, 3}, {3, 3, 3, 3}};
-
 // lane tasks of a dense step
 int64_t step_lanes(const BWorld& w) { return (int64_t)nblocks(w.Y, 1) * nblocks(w.Z, 1) << plane_lg(w.nw); }
 
@@ -273,7 +267,7 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
         if (w.cls_gm == -2) w.cls_gm = resident_class_gm(w.X, w.Y, w.Z);
         const int c = w.cls_gm;
         if (c < 0) return -1;
-        const int leveled = mode == 3 ? (c == kGmDense - 1 && b->widen_large ? kGmDense : kWidened[b->widen][c]) : c;
+        const int leveled = mode == 3 ? (c == kGmDense - 1 && b->widen_large ? kGmDense : gm_class_at(b->widen, c, w.Y)) : c;
         return kResidentClasses + (b->promote ? std::max(std::min(c + b->promote, kGmDense - 1), leveled) : leveled);
     };
     if (mode == 1) return smem();
@@ -292,7 +286,7 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
                 batch_slabs_fit(w.X, w.Y, w.Z, kClusterSizes[b->spread - kSingleCtaClasses]))
                 return b->spread;
             if (c >= 0 && c < kSingleCtaClasses) return c == 0 ? 1 : c;
-            if (w.Y <= 4096) return kResidentClasses + kGmDense;
+            if (w.Y <= kGmMaxY[kGmDense]) return kResidentClasses + kGmDense;
             return c >= 0 ? c : gm();
         }
         const int first = gm();
@@ -360,7 +354,8 @@ void choose_widen(fs3d_batch* b) {
     b->widen = kOwnLevel;
     b->widen_large = false;
     if (b->cfg.use_smem != 3) return;
-    int64_t by_class[kGmDense] = {0, 0, 0, 0}, young = 0;
+    // settled worlds by their class for themselves and the first that holds their layers
+    int64_t count[kGmDense][kGmDense] = {}, young = 0;
     for (auto& kv : b->worlds) {
         BWorld& w = kv.second;
         if (w.done) continue;
@@ -370,16 +365,16 @@ void choose_widen(fs3d_batch* b) {
             continue;
         }
         if (w.cls_gm == -2) w.cls_gm = resident_class_gm(w.X, w.Y, w.Z);
-        if (w.cls_gm >= 0) ++by_class[w.cls_gm];
+        if (w.cls_gm >= 0) ++count[w.cls_gm][gm_class_holding(0, w.Y)];
     }
-    static const int threads[kGmClasses] = {32, 64, 128, 256, 768};
     const int64_t fit = (int64_t)sm_count_public() * 768;
     int64_t own = 0, most = 0;  // threads with each class by itself, and those of the largest share
     int largest = 0;
     for (int l = kWidestLevel; l >= kOwnLevel; --l) {
         int64_t need = young;
         for (int c = 0; c < kGmDense; ++c) {
-            const int64_t t = by_class[c] * threads[kWidened[l][c]];
+            int64_t t = 0;
+            for (int m = 0; m <= c; ++m) t += count[c][m] * kGmThreads[std::max(kWidened[l][c], m)];
             need += t;
             if (l == kOwnLevel) {
                 own += t;
@@ -391,7 +386,9 @@ void choose_widen(fs3d_batch* b) {
         }
         if (l > kOwnLevel && need <= (l == kOwnLevel + 1 ? fit * 7 / 4 : fit)) {
             b->widen = l;
-            b->widen_large = need + by_class[kGmDense - 1] * (threads[kGmDense] - threads[kGmDense - 1]) <= fit;
+            int64_t widest = 0;
+            for (int64_t n : count[kGmDense - 1]) widest += n;
+            b->widen_large = need + widest * (kGmThreads[kGmDense] - kGmThreads[kGmDense - 1]) <= fit;
             return;
         }
     }
@@ -999,7 +996,10 @@ fs3d_status build_tables(fs3d_batch* b) {
     for (auto& kv : b->worlds) {
         BWorld& w = kv.second;
         if (w.done) continue;
-        const int c = segment_class(b, w);
+        int c = segment_class(b, w);
+        // a class whose shared memory does not hold the world's layers is never
+        // launched on it, whatever the rules above come to
+        if (c >= kResidentClasses && w.Y > kGmMaxY[c - kResidentClasses]) c = -1;
         run.emplace_back(c, &w);
         if (c >= 0)
             ++ns;

@@ -804,15 +804,12 @@ int resident_class(int X, int Y, int Z) {
 // step's barrier.  Each class caps the layers it holds flags for so that its
 // CTAs per SM (24 warps in all) fit in shared memory.
 namespace {
-constexpr int kGmThreads[kGmClasses] = {32, 64, 128, 256, 768};
-constexpr int kGmMaxY[kGmClasses] = {1024, 1024, 2048, 4096, 4096};
 std::once_flag g_gm_once;
 }  // namespace
 
 int resident_class_gm(int X, int Y, int Z) {
     const int lanes = nblocks(Z, 1) << plane_lg(plane_nw(X));  // lane tasks of one layer pair
-    int c = lanes <= 16 ? 0 : (lanes <= 48 ? 1 : (lanes <= 96 ? 2 : 3));
-    while (c < kGmDense && Y > kGmMaxY[c]) ++c;
+    const int c = gm_class_holding(lanes <= 16 ? 0 : (lanes <= 48 ? 1 : (lanes <= 96 ? 2 : 3)), Y);
     return c < kGmDense ? c : -1;
 }
 

@@ -48,6 +48,21 @@ constexpr int kClusterSizes[3] = {2, 4, 8};
 // for a young (dense) world too large for one CTA's shared memory.
 constexpr int kGmClasses = 5;
 constexpr int kGmDense = 4;
+constexpr int kGmThreads[kGmClasses] = {32, 64, 128, 256, 768};
+// the most layers of a world in each: its CTAs have shared memory for the flags of so many
+constexpr int kGmMaxY[kGmClasses] = {1024, 1024, 2048, 4096, 4096};
+// the first class from c on that holds Y layers (kGmClasses: none does)
+inline int gm_class_holding(int c, int Y) {
+    while (c < kGmClasses && Y > kGmMaxY[c]) ++c;
+    return c;
+}
+// Classes of settled worlds at a batch's level (choose_widen), by their class
+// for themselves (`own`, 0..3).  A level may narrow a world's CTA only as far
+// as its layers still fit.
+constexpr int kPackedLevel = 0, kOwnLevel = 1, kWidestLevel = 4;
+constexpr int kWidened[kWidestLevel + 1][kGmDense] = {
+    {1, 1, 1, 3}, {0, 1, 2, 3}, {0, 2, 3, 3}, {2, 3, 3, 3}, {3, 3, 3, 3}};
+inline int gm_class_at(int level, int own, int Y) { return gm_class_holding(kWidened[level][own], Y); }
 int resident_class_gm(int X, int Y, int Z);
 // Class ids of a segment's tables: shared-memory classes 0..5, then the
 // global-memory classes 6..9.  meta = {per-step items, worlds per class,

@@ -25,3 +25,24 @@ def test_settled_worlds_match_oracle_at_every_level(fs3d, orc, copies):
     for g, s in zip(grids, seeds):
         orc.run(g, s, 128, n, nthreads=0)
     assert [int(h) for h in hs] == [orc.hash(g) for g in grids] * copies
+
+
+def test_tall_settled_worlds_among_many(fs3d, orc):
+    """Worlds of more layers than the narrow CTAs hold flags for, among so many
+    mixed ones that the others are packed into those."""
+    tall = [(16, 1024, 16), (16, 1025, 16), (16, 1500, 16), (20, 2048, 12), (16, 2049, 16), (70, 1100, 24)]
+    n, copies, seeds = 70, 250, [3 + i for i in range(len(DIMS) + len(tall))]
+    grids = [fs3d.gen_batch_world(s, *d) for s, d in zip(seeds, DIMS + tall)]
+    m = len(DIMS)
+    with fs3d.Batch(8 << 30, steps_per_segment=35) as b:
+        ts = b.admit_many(grids[:m] * copies + grids[m:], seeds[:m] * copies + seeds[m:], n,
+                          start_steps=[128] * (m * copies + len(tall)))
+        for _ in range(2):
+            b.run_segment()
+        b.sync()
+        done, hs = b.poll_many(ts)
+    assert done.all()
+    for g, s in zip(grids, seeds):
+        orc.run(g, s, 128, n, nthreads=0)
+    want = [orc.hash(g) for g in grids]
+    assert [int(h) for h in hs] == want[:m] * copies + want[m:]
