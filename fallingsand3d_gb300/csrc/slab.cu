@@ -446,6 +446,10 @@ __global__ void __launch_bounds__(kBatchSlabThreads, 1)
     __syncthreads();
     uint32_t phase = 0;
     for (;;) {
+        // the last world's planes and flags were written here with ordinary
+        // stores, and the next world's bulk copies write the same bytes through
+        // the async proxy: each thread orders its own before the barrier
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         // after an error no cluster takes another world
         if (r == 0 && tid == 0) item = *(volatile int*)err ? n : atomicAdd(counter, 1);
         if (tid == 0) s_dead = 0;

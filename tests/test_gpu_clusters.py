@@ -62,3 +62,25 @@ def test_few_largest_of_many_young_worlds(fs3d, orc, small, large):
         if i < len(large) or i % 29 == 0:
             orc.run(g, s, 0, 100, nthreads=0)
             assert int(hs[i]) == orc.hash(g), dims[i]
+
+
+def test_each_cluster_runs_several_worlds(fs3d, orc):
+    """More spread worlds than clusters, of different shapes: a cluster's shared
+    memory, its barrier's phase and the edge words pass from world to world."""
+    dims = [(128 - 7 * (i % 5), 128 - 9 * (i % 4), 128 - 5 * (i % 7)) for i in range(36)]
+    seeds = [300 + i for i in range(len(dims))]
+    grids = [fs3d.gen_batch_world(s, *d) for s, d in zip(seeds, dims)]
+    for mode in (3, 1):  # clusters of 8, and each world's smallest cluster
+        with fs3d.Batch(4 << 30, steps_per_segment=37, use_smem=mode) as b:
+            ts = b.admit_many(grids, seeds, 74)
+            for _ in range(2):
+                b.run_segment()
+            b.sync()
+            done, hs = b.poll_many(ts)
+        assert done.all()
+        if mode == 3:
+            for g, s in zip(grids, seeds):
+                orc.run(g, s, 0, 74, nthreads=0)
+            want = [orc.hash(g) for g in grids]
+            grids = [fs3d.gen_batch_world(s, *d) for s, d in zip(seeds, dims)]
+        assert [int(h) for h in hs] == want, mode
