@@ -85,9 +85,10 @@ fs3d_status fs3d_test_inject(int what, int count) {
     switch (what) {
         case FS3D_INJECT_NONE:
             fs3d::set_inject_alloc_failures(0);
-            return fs3d::set_inject_tx_extra(0u);
+            return fs3d::set_inject_tx_extra(fs3d::kStallNone);
         case FS3D_INJECT_COPY_STALL:
-            return fs3d::set_inject_tx_extra(count > 0 ? 16u : 0u);
+            return fs3d::set_inject_tx_extra(count <= 0 ? (uint32_t)fs3d::kStallNone
+                                                        : (count < (int)fs3d::kStallKinds ? (uint32_t)count : (uint32_t)fs3d::kStallAll));
         case FS3D_INJECT_ALLOC_FAIL:
             fs3d::set_inject_alloc_failures(count);
             return FS3D_OK;

@@ -73,8 +73,15 @@ constexpr int kMetaInts = kMetaWorlds + 1;
 // smallest class that holds a world of these dims, -1 if none does
 int resident_class(int X, int Y, int Z);
 constexpr int kErrInts = 4;  // size of the error record a resident launch is given
-// test hook: resident kernels announce `bytes` more than each bulk copy delivers
-fs3d_status set_inject_tx_extra(uint32_t bytes);
+// test hook: bulk copies announced with more bytes than they deliver
+enum CopyStall : uint32_t {
+    kStallNone = 0,
+    kStallAll = 1,        // every one
+    kStallOneCta = 2,     // those of worlds held by one CTA
+    kStallFirstSlab = 3,  // that of the first CTA of a world cut into slabs
+    kStallKinds = 4
+};
+fs3d_status set_inject_tx_extra(uint32_t stall);
 // test hook: the next n stream-ordered allocations of batch admissions fail as out of memory
 void set_inject_alloc_failures(int n);
 // One launch steps every world of the single-CTA class `cls`
@@ -219,7 +226,7 @@ bool prefer_slabs(int X, int Y, int Z, int n_steps, SlabPlan* out);
 // to call), err as for launch_plane_segment_resident
 fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_t* rflags, void* scratch, int* err,
                                cudaStream_t st);
-fs3d_status set_slab_tx_extra(uint32_t bytes);  // test hook, as set_inject_tx_extra
+fs3d_status set_slab_stall(uint32_t stall);  // test hook, as set_inject_tx_extra
 // ---- a batch's worlds of a cluster class: CS CTAs a world, cut along z
 // (slab.cu).  Whether a world's slabs fit; the most words (Y * nw) of a layer
 // at a cut; the bytes of edge buffer a class needs; the launch, as

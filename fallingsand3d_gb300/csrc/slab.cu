@@ -20,11 +20,12 @@
 // overwritten before it was read.
 //
 // All CTAs of a world are resident at once (a cooperative launch, or a
-// cluster).  Every wait is bounded
-// in time; the planes and flags in global memory are written only once every
-// CTA has taken all the steps (one of the CTAs decides: the last to arrive
-// commits, one that gives up aborts, whichever is first), so a launch that
-// fails leaves the world as it was.
+// cluster).  Every wait is bounded in time; the planes and flags in global
+// memory are written only once every CTA has taken all the steps, on one
+// decision for the whole world: in a whole-GPU launch the last CTA to arrive
+// commits and one that gives up aborts, whichever is first; in a cluster its
+// first CTA looks at the batch's error record once.  A world whose launch
+// fails is as it was.
 //
 // Bound: latency.  A step of a small world is a chain of a word's way through
 // L2 to the neighbour (about 1 us), the draws (hidden in that wait), the
@@ -53,9 +54,21 @@ namespace {
 constexpr int kSlabKeys = 32;  // step keys computed together
 constexpr int kBatchSlabThreads = 640;
 
-// Test hook (fs3d_test_inject), as the resident kernels': bytes announced on
-// the mbarrier beyond what the bulk copies deliver.  0 in normal operation.
-static __device__ uint32_t g_slab_tx_extra;
+// Test hook (fs3d_test_inject): which bulk copies are announced with more bytes
+// than they deliver (a CopyStall, planes.h).  0 in normal operation.
+static __device__ uint32_t g_slab_stall;
+constexpr uint32_t kStallBytes = 16;
+// bytes announced too many by CTA r, and the limits of its copy's wait and of
+// the waits for other CTAs: of the first CTA's stall, theirs run out first
+__device__ __forceinline__ uint32_t stall_bytes(uint32_t stall, int r) {
+    return stall == kStallAll || (stall == kStallFirstSlab && r == 0) ? kStallBytes : 0u;
+}
+__device__ __forceinline__ uint64_t copy_limit(uint32_t stall) {
+    return stall == 0 ? kCopyWaitNs : (stall == kStallAll ? 1u : 2u) * kCopyWaitInjectedNs;
+}
+__device__ __forceinline__ uint64_t peer_limit() {
+    return *(volatile uint32_t*)&g_slab_stall ? kCopyWaitInjectedNs : kCopyWaitNs;
+}
 
 // The launch's shared words, zeroed before it, at the start of the scratch;
 // the edge buffer follows at kSlabEdgeOff.
@@ -103,7 +116,7 @@ __device__ __forceinline__ bool edge_read(const unsigned long long* p0, const un
             const unsigned long long now = global_ns();
             if (!t0)
                 t0 = now;
-            else if (now - t0 > kCopyWaitNs)
+            else if (now - t0 > peer_limit())
                 return false;
         }
     }
@@ -370,12 +383,12 @@ __global__ void __launch_bounds__(MAXT, 1)
     __shared__ int s_dead, s_verdict;  // s_dead: some thread gave up (a hint to the others' waits)
     const int C = gridDim.x, r = blockIdx.x, tid = threadIdx.x;
     const SlabGeo<ZS> geo(w, r, C);
-    const uint32_t tx_extra = g_slab_tx_extra;
+    const uint32_t stall = g_slab_stall;
     uint8_t* rf = reinterpret_cast<uint8_t*>(srows) + geo.bytes;
     if (tid == 0) {
         mbar_init(&bar, 1);
         s_dead = 0;
-        mbar_expect(&bar, geo.bytes + tx_extra);
+        mbar_expect(&bar, geo.bytes + stall_bytes(stall, r));
     }
     // an error recorded earlier: nothing is stepped (and every CTA's load is skipped or waited for)
     bool dead = __syncthreads_or(tid == 0 && *(volatile int*)err != 0) != 0;
@@ -386,7 +399,7 @@ __global__ void __launch_bounds__(MAXT, 1)
             geo.flag_at(w, i, y, z);
             rf[i] = (y >= 0 && z >= 0) ? rflags[(int64_t)y * w.Z + z] : 0;
         }
-        const bool ok = mbar_wait(&bar, 0, tx_extra ? kCopyWaitInjectedNs : kCopyWaitNs);
+        const bool ok = mbar_wait(&bar, 0, copy_limit(stall));
         dead = __syncthreads_or(!ok) != 0;
     }
     uint32_t rows_done = 0;
@@ -400,7 +413,7 @@ __global__ void __launch_bounds__(MAXT, 1)
         const unsigned long long t0 = global_ns();
         int v;
         while ((v = *(volatile int*)&st->verdict) == 0) {
-            if (global_ns() - t0 > kCopyWaitNs) {
+            if (global_ns() - t0 > peer_limit()) {
                 v = atomicCAS(&st->verdict, 0, 2);
                 if (v == 0) v = 2;
                 break;
@@ -431,14 +444,14 @@ __global__ void __launch_bounds__(kBatchSlabThreads, 1)
     extern __shared__ __align__(128) uint4 srows[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t s_keys[kSlabKeys];
-    __shared__ int s_dead, item;
+    __shared__ int s_dead, s_write, item;
     __shared__ unsigned long long s_processed;
     namespace cg = cooperative_groups;
     const cg::cluster_group cluster = cg::this_cluster();
     const int r = (int)cluster.block_rank(), tid = threadIdx.x, NT = blockDim.x;
     const int n = meta[1 + cls], off = meta[1 + kAllClasses + cls];
     unsigned long long* edge = edges + (size_t)(blockIdx.x / CS) * (size_t)(CS - 1) * kBatchSlabEdgeWords * 4;
-    const uint32_t tx_extra = g_slab_tx_extra;
+    const uint32_t stall = g_slab_stall;
     if (tid == 0) {
         mbar_init(&bar, 1);
         s_processed = 0;
@@ -461,7 +474,7 @@ __global__ void __launch_bounds__(kBatchSlabThreads, 1)
         if (w.steps <= 0) continue;
         const SlabGeo<true> geo(w, r, CS);
         uint8_t* rf = reinterpret_cast<uint8_t*>(srows) + geo.bytes;
-        if (tid == 0) mbar_expect(&bar, geo.bytes + tx_extra);
+        if (tid == 0) mbar_expect(&bar, geo.bytes + stall_bytes(stall, r));
         __syncthreads();
         geo.load(w, srows, &bar);
         // row flags from the layers', or every row changed just before
@@ -477,7 +490,7 @@ __global__ void __launch_bounds__(kBatchSlabThreads, 1)
                 st_tagged(edge + ((size_t)r * geo.NO * w.nw + i) * 4, 0, 0);
                 st_tagged(edge + ((size_t)r * geo.NO * w.nw + i) * 4 + 2, 0, 0);
             }
-        const bool ok = mbar_wait(&bar, phase, tx_extra ? kCopyWaitInjectedNs : kCopyWaitNs);
+        const bool ok = mbar_wait(&bar, phase, copy_limit(stall));
         phase ^= 1u;
         bool dead = __syncthreads_or(!ok) != 0;
         cluster.sync();
@@ -487,8 +500,13 @@ __global__ void __launch_bounds__(kBatchSlabThreads, 1)
             *reinterpret_cast<unsigned long long*>(err + 2) = (unsigned long long)w.t;
         rows_done = __reduce_add_sync(0xFFFFFFFFu, rows_done);
         if ((tid & 31) == 0 && rows_done) atomicAdd(&s_processed, (unsigned long long)rows_done * (unsigned long long)w.X);
+        // Write back or not is one answer for the whole world: another class's
+        // kernel may record an error between two reads of the record, and a
+        // world written by some of its CTAs only would be torn.
+        cluster.sync();  // this cluster's own failures are recorded
+        if (r == 0 && tid == 0) s_write = *(volatile int*)err == 0;
         cluster.sync();
-        const bool write = *(volatile int*)err == 0;
+        const bool write = *cluster.map_shared_rank(&s_write, 0) != 0;
         const uint64_t te = w.t + (uint64_t)w.steps;
         const int lasto = (int)((te - 1u) & 1u);
         if (write) geo.store(w, srows, edge, r, lasto);
@@ -546,8 +564,8 @@ const SlabLimits& slab_limits() {
 
 }  // namespace
 
-fs3d_status set_slab_tx_extra(uint32_t bytes) {
-    FS3D_CUDA(cudaMemcpyToSymbol(g_slab_tx_extra, &bytes, sizeof(bytes)));
+fs3d_status set_slab_stall(uint32_t which) {
+    FS3D_CUDA(cudaMemcpyToSymbol(g_slab_stall, &which, sizeof(which)));
     return FS3D_OK;
 }
 
