@@ -248,10 +248,14 @@ __device__ __forceinline__ bool rows_changed_recently(const uint8_t* __restrict_
 // Three CTAs per SM (80 registers, a few bytes spilled): 24 warps hide the
 // rule's dependent chain better than 16 at 118 registers (1024^3 dunes:
 // 118 us per step against 133 us, 123 us at four CTAs)
+//
+// err: the world's error record (nullable); while it is set nothing is stepped.
+// Its load runs beside the flags' and is looked at with them.
 template <bool LIST>
 __global__ void __launch_bounds__(256, 3) k_plane_step_skip(const PlaneWorld w, uint8_t* __restrict__ rflags,
-                                                        int* counts) {
+                                                        int* counts, const int* err) {
     chain_wait();
+    const int failed = err ? *(volatile const int*)err : 0;
     const uint64_t t = w.t;
     const int o = (int)(t & 1u);
     const int lane = threadIdx.x & 31;
@@ -273,6 +277,7 @@ __global__ void __launch_bounds__(256, 3) k_plane_step_skip(const PlaneWorld w, 
                 k = rp - j * NBZ;
                 dirty = rows_changed_recently(rflags, w.Y, w.Z, 2 * j - o, 2 * k - o, tb);
             }
+            dirty = dirty && !failed;
             const uint32_t m = __ballot_sync(0xFFFFFFFFu, dirty);
             n_dirty = __popc(m);
             if (dirty) list[__popc(m & ((1u << lane) - 1u))] = make_int2(j, k);
@@ -284,7 +289,7 @@ __global__ void __launch_bounds__(256, 3) k_plane_step_skip(const PlaneWorld w, 
                 k = rp - j * NBZ;
                 if (gl == 0) dirty = rows_changed_recently(rflags, w.Y, w.Z, 2 * j - o, 2 * k - o, tb);
             }
-            dirty = __shfl_sync(0xFFFFFFFFu, dirty, lane & ~(G - 1));
+            dirty = __shfl_sync(0xFFFFFFFFu, dirty && !failed, lane & ~(G - 1));
             if (__any_sync(0xFFFFFFFFu, dirty)) n_dirty = 1;
         }
         for (int at = 0; at < n_dirty; at += per) {
@@ -1128,14 +1133,14 @@ fs3d_status layer_flags_from_cells(const uint4* rows, uint8_t* lflags, int X, in
     return FS3D_OK;
 }
 
-fs3d_status launch_plane_step_skip(const PlaneWorld& w, uint8_t* rflags, int* counts, cudaStream_t st) {
+fs3d_status launch_plane_step_skip(const PlaneWorld& w, uint8_t* rflags, int* counts, const int* err, cudaStream_t st) {
     const int per = 32 >> w.lg;
     const int64_t nrp = (int64_t)nblocks(w.Y, 1) * nblocks(w.Z, 1);
     const int64_t need = ((nrp + per - 1) / per + 7) / 8;  // eight warps per CTA
     const int64_t cap = (int64_t)sm_count_public() * 3;    // the kernel's launch bound
     const int grid = (int)(need < 1 ? 1 : (need < cap ? need : cap));
-    const cudaError_t e = need > 2 * cap ? launch_chained(k_plane_step_skip<true>, (unsigned)grid, 256, st, w, rflags, counts)
-                                     : launch_chained(k_plane_step_skip<false>, (unsigned)grid, 256, st, w, rflags, counts);
+    const auto fn = need > 2 * cap ? &k_plane_step_skip<true> : &k_plane_step_skip<false>;
+    const cudaError_t e = launch_chained(fn, (unsigned)grid, 256, st, w, rflags, counts, err);
     if (e != cudaSuccess) return cuda_fail(e, "plane step (settled skip) launch");
     note_launch();
     return FS3D_OK;

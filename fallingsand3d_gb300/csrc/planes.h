@@ -207,8 +207,9 @@ fs3d_status layer_flags_from_cells_multi(const ConvJob* jobs, int njobs, int max
 // the same for one world
 fs3d_status layer_flags_from_cells(const uint4* rows, uint8_t* lflags, int X, int Y, int Z, uint64_t t0,
                                    cudaStream_t st);
-// one step (w.t) of the world; counts as for launch_plane_step
-fs3d_status launch_plane_step_skip(const PlaneWorld& w, uint8_t* rflags, int* counts, cudaStream_t st);
+// one step (w.t) of the world; counts as for launch_plane_step; err (nullable):
+// while *err is set nothing is stepped
+fs3d_status launch_plane_step_skip(const PlaneWorld& w, uint8_t* rflags, int* counts, const int* err, cudaStream_t st);
 // ---- many steps of one world in one launch over the whole GPU (slab.cu)
 struct SlabPlan {
     int zs = 0;          // slabs cut along z (else along y)

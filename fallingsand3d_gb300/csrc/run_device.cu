@@ -95,7 +95,7 @@ extern "C" fs3d_status fs3d_run_device(uint8_t* grid_dev, int X, int Y, int Z, u
     } else {
         for (int a = 0; a < n_steps && s == FS3D_OK; ++a) {
             d.t = t0 + (uint64_t)a;
-            s = launch_plane_step_skip(d, rflags, nullptr, st);
+            s = launch_plane_step_skip(d, rflags, nullptr, nullptr, st);
         }
     }
     // a recorded failure (this run's or an earlier one's) leaves the grid as it was

@@ -131,7 +131,7 @@ extern "C" fs3d_status fs3d_run_device_noalloc(uint8_t* grid_dev, int X, int Y, 
     } else {
         for (int a = 0; a < n_steps && s == FS3D_OK; ++a) {
             d.t = t0 + (uint64_t)a;
-            s = launch_plane_step_skip(d, rflags, nullptr, st);
+            s = launch_plane_step_skip(d, rflags, nullptr, nullptr, st);
         }
     }
     // static cells never change: their values are read back from the grid

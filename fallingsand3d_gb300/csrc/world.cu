@@ -209,7 +209,7 @@ fs3d_status fs3d_world_step(fs3d_world* w, int n_steps) {
         int launched = 0;
         while (s == FS3D_OK && launched < n_steps) {
             d.t = w->step + (uint64_t)launched;
-            s = launch_plane_step_skip(d, w->rflags, counts, w->stream);
+            s = launch_plane_step_skip(d, w->rflags, counts, w->err, w->stream);
             if (s == FS3D_OK) ++launched;
         }
         w->step += (uint64_t)launched;  // the steps that went out before a failed launch still count
