@@ -207,6 +207,7 @@ struct fs3d_batch {
     void* graph_order = nullptr;
     // classes with worlds in the current tables (bit c), and those the graphs launch
     uint32_t class_mask = ~0u, graph_mask = 0;
+    ResidentLimits limits;  // the shared-memory classes', in the batch's context
     int grid = 0;
     int promote = 0;  // single-CTA resident worlds run this many classes wider (autotuned)
     // hybrid mode, chosen with the tables: young worlds of class `spread_from`
@@ -258,7 +259,7 @@ int64_t step_lanes(const BWorld& w) { return (int64_t)nblocks(w.Y, 1) * nblocks(
 int segment_class(const fs3d_batch* b, const BWorld& w) {
     const int mode = b->cfg.use_smem;
     auto smem = [&]() {
-        if (w.cls_smem == -2) w.cls_smem = resident_class(w.X, w.Y, w.Z);
+        if (w.cls_smem == -2) w.cls_smem = resident_class(b->limits, w.X, w.Y, w.Z);
         int c = w.cls_smem;
         if (mode == 1 && c >= 0 && c < kSingleCtaClasses) c = std::min(c + b->promote, kSingleCtaClasses - 1);
         return c;
@@ -283,7 +284,7 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
             // up to 768 threads too measured 3.09 ms)
             const int c = smem();
             if (b->spread && (c < 0 || c >= b->spread_from) && step_lanes(w) >= b->spread_lanes &&
-                batch_slabs_fit(w.X, w.Y, w.Z, kClusterSizes[b->spread - kSingleCtaClasses]))
+                batch_slabs_fit(b->limits, w.X, w.Y, w.Z, kClusterSizes[b->spread - kSingleCtaClasses]))
                 return b->spread;
             if (c >= 0 && c < kSingleCtaClasses) return c == 0 ? 1 : c;
             if (w.Y <= kGmMaxY[kGmDense]) return kResidentClasses + kGmDense;
@@ -317,7 +318,7 @@ void choose_spread(fs3d_batch* b) {
         BWorld& w = kv.second;
         if (w.done || w.t >= kYoungSteps) continue;
         lanes += step_lanes(w);
-        if (w.cls_smem == -2) w.cls_smem = resident_class(w.X, w.Y, w.Z);
+        if (w.cls_smem == -2) w.cls_smem = resident_class(b->limits, w.X, w.Y, w.Z);
         if (w.cls_smem < 0 || w.cls_smem >= kSingleCtaClasses) ++large;
         else if (w.cls_smem == kSingleCtaClasses - 1) ++whole;
         else ++rest;  // three to an SM
@@ -360,7 +361,7 @@ void choose_widen(fs3d_batch* b) {
         BWorld& w = kv.second;
         if (w.done) continue;
         if (w.t < kYoungSteps) {
-            if (w.cls_smem == -2) w.cls_smem = resident_class(w.X, w.Y, w.Z);
+            if (w.cls_smem == -2) w.cls_smem = resident_class(b->limits, w.X, w.Y, w.Z);
             young += w.cls_smem == 0 || w.cls_smem == 1 ? 256 : 768;
             continue;
         }
@@ -757,6 +758,7 @@ fs3d_status fs3d_batch_create(size_t budget, const fs3d_config* cfg, fs3d_batch*
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
         }
     }
+    b->limits = resident_limits();
     fs3d_status s = e == cudaSuccess ? FS3D_OK : cuda_fail(e, "fs3d_batch_create");
     if (s == FS3D_OK) s = b->tn.reserve(kMetaInts);
     // size the tables for a few thousand worlds and capture the segment graph
@@ -1955,7 +1957,7 @@ std::vector<int> batch_shape(const fs3d_batch* b) {
     std::vector<int> h(kResidentClasses + 1, 0);
     for (auto& kv : b->worlds) {
         if (kv.second.done) continue;
-        const int c = resident_class(kv.second.X, kv.second.Y, kv.second.Z);
+        const int c = resident_class(b->limits, kv.second.X, kv.second.Y, kv.second.Z);
         ++h[(size_t)(c < 0 ? kResidentClasses : c)];
     }
     return h;
@@ -2016,7 +2018,7 @@ fs3d_status fs3d_batch_autotune(fs3d_batch* b, int trial_segments, fs3d_tune_rep
     const int resident = plane_step_ctas_per_sm();
     bool stepped = false;
     for (auto& kv : b->worlds)
-        if (!kv.second.done && resident_class(kv.second.X, kv.second.Y, kv.second.Z) < 0 &&
+        if (!kv.second.done && resident_class(b->limits, kv.second.X, kv.second.Y, kv.second.Z) < 0 &&
             resident_class_gm(kv.second.X, kv.second.Y, kv.second.Z) < 0)
             stepped = true;
     // the hybrid mode picks a world's memory by its age itself; an explicit

@@ -9,6 +9,7 @@
 #include <string>
 
 #include "../../include/fs3d.h"
+#include "per_context.h"
 
 #define FS3D_HD __host__ __device__ __forceinline__
 
@@ -65,6 +66,22 @@ void note_launch(uint64_t n = 1);
 // the driver cannot tell.  A device address cached for one context is stale
 // in another (after cudaDeviceReset, for example).
 bool current_context_id(unsigned long long* id);
+// the value of `p` for the current device and context (make: its value there)
+template <class T, class Make>
+T of_current_context(PerContext<T>& p, Make make) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return T{};
+    }
+    return p.get(
+        dev,
+        [] {
+            unsigned long long id = 0;
+            return current_context_id(&id) ? id : 0ull;
+        },
+        make);
+}
 
 // device memory for a call's own duration, stream-ordered (scratch.cpp)
 cudaError_t scratch_alloc(void** p, size_t n, cudaStream_t st);

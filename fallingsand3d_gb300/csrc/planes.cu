@@ -21,7 +21,6 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "fs3d_common.h"
 #include "pcg.h"
@@ -743,16 +742,17 @@ struct ResidentCfg {
     const void* fn;
 };
 
-// filled once per process (the first device the library is used on), from any thread
-ResidentCfg g_classes[kSingleCtaClasses];
-std::once_flag g_classes_once;
+struct ResidentCfgs {
+    ResidentCfg c[kSingleCtaClasses] = {};
+};
 
 template <int NT>
 const void* resident_fn() {
     return reinterpret_cast<const void*>(&k_plane_segment_resident<NT>);
 }
 
-void fill_classes() {
+ResidentCfgs fill_classes() {
+    ResidentCfgs out;
     int dev = 0, per_sm = 0, optin = 0, reserved = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
@@ -778,25 +778,37 @@ void fill_classes() {
                      fit < k.ctas_per_sm))
             smem = 0;
         k.smem = smem;
-        g_classes[c] = k;
+        out.c[c] = k;
     }
     cudaGetLastError();  // a refused attribute leaves the class unused, not an error
+    return out;
 }
 
-void init_classes() { std::call_once(g_classes_once, fill_classes); }
+// those of the current device and context (the attribute belongs to them)
+ResidentCfgs resident_cfgs() {
+    static PerContext<ResidentCfgs> kept;
+    return of_current_context(kept, fill_classes);
+}
 
 }  // namespace
 
-int resident_class(int X, int Y, int Z) {
-    init_classes();
+ResidentLimits resident_limits() {
+    const ResidentCfgs k = resident_cfgs();
+    ResidentLimits l;
+    for (int c = 0; c < kSingleCtaClasses; ++c) l.one_cta[c] = k.c[c].smem;
+    l.cluster = batch_slabs_smem();
+    return l;
+}
+
+int resident_class(const ResidentLimits& l, int X, int Y, int Z) {
     const int64_t planes = (int64_t)Y * Z * plane_nw(X) * 16;
     for (int c = 0; c < kSingleCtaClasses; ++c) {
         // planes, then the layer flags and the layer list
         const int64_t need = ((planes + 15) & ~(int64_t)15) + (int64_t)slab_aux_bytes((uint32_t)Y);
-        if (g_classes[c].smem && need <= g_classes[c].smem) return c;
+        if (l.one_cta[c] && need <= l.one_cta[c]) return c;
     }
     for (int c = kSingleCtaClasses; c < kResidentClasses; ++c)
-        if (batch_slabs_fit(X, Y, Z, kClusterSizes[c - kSingleCtaClasses])) return c;
+        if (batch_slabs_fit(l, X, Y, Z, kClusterSizes[c - kSingleCtaClasses])) return c;
     return -1;
 }
 
@@ -808,10 +820,6 @@ int resident_class(int X, int Y, int Z) {
 // that layer work, not by the world's volume: idle warps would wait at every
 // step's barrier.  Each class caps the layers it holds flags for so that its
 // CTAs per SM (24 warps in all) fit in shared memory.
-namespace {
-std::once_flag g_gm_once;
-}  // namespace
-
 int resident_class_gm(int X, int Y, int Z) {
     const int lanes = nblocks(Z, 1) << plane_lg(plane_nw(X));  // lane tasks of one layer pair
     const int c = gm_class_holding(lanes <= 16 ? 0 : (lanes <= 48 ? 1 : (lanes <= 96 ? 2 : 3)), Y);
@@ -849,7 +857,8 @@ fs3d_status launch_plane_segment_gm(int cls, const PlaneWorld* worlds, const int
                                     int* counter, int* err, cudaStream_t st, unsigned long long* processed_cells,
                                     bool first) {
     if (cls < 0 || cls >= kGmClasses) return set_error(FS3D_ERR_INVALID_ARG, "global-memory class out of range");
-    std::call_once(g_gm_once, [] {
+    static PerContext<bool> carved;
+    of_current_context(carved, [] {
         // the planes are read through L1: leave most of the unified memory to it
         const void* fns[kGmClasses] = {reinterpret_cast<const void*>(&k_plane_segment_resident<32, true>),
                                        reinterpret_cast<const void*>(&k_plane_segment_resident<64, true>),
@@ -858,6 +867,7 @@ fs3d_status launch_plane_segment_gm(int cls, const PlaneWorld* worlds, const int
                                        reinterpret_cast<const void*>(&k_plane_segment_resident<768, true>)};
         for (const void* fn : fns) cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 50);
         cudaGetLastError();
+        return true;
     });
     FS3D_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), st));
     const int nt = kGmThreads[cls];
@@ -891,8 +901,7 @@ fs3d_status launch_plane_segment_resident(int cls, const PlaneWorld* worlds, con
                                           int* counter, int* err, cudaStream_t st,
                                           unsigned long long* processed_cells) {
     if (cls < 0 || cls >= kSingleCtaClasses) return set_error(FS3D_ERR_INVALID_ARG, "resident class out of range");
-    init_classes();
-    const ResidentCfg& k = g_classes[cls];
+    const ResidentCfg k = resident_cfgs().c[cls];
     if (!k.smem) return set_error(FS3D_ERR_CUDA, "resident segment kernel unavailable for this class");
     FS3D_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), st));
     const unsigned grid = (unsigned)(sm_count_public() * k.ctas_per_sm);

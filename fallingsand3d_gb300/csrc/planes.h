@@ -70,8 +70,15 @@ int resident_class_gm(int X, int Y, int Z);
 constexpr int kAllClasses = kResidentClasses + kGmClasses;
 constexpr int kMetaWorlds = 1 + 2 * kAllClasses;
 constexpr int kMetaInts = kMetaWorlds + 1;
+// Dynamic shared memory of a CTA of each shared-memory class (0: the class
+// cannot run) in the current device and context.
+struct ResidentLimits {
+    int one_cta[kSingleCtaClasses] = {};
+    int cluster = 0;
+};
+ResidentLimits resident_limits();
 // smallest class that holds a world of these dims, -1 if none does
-int resident_class(int X, int Y, int Z);
+int resident_class(const ResidentLimits& l, int X, int Y, int Z);
 constexpr int kErrInts = 4;  // size of the error record a resident launch is given
 // test hook: bulk copies announced with more bytes than they deliver
 enum CopyStall : uint32_t {
@@ -233,7 +240,8 @@ fs3d_status set_slab_stall(uint32_t stall);  // test hook, as set_inject_tx_extr
 // at a cut; the bytes of edge buffer a class needs; the launch, as
 // launch_plane_segment_resident.
 constexpr int kBatchSlabEdgeWords = 1024;
-bool batch_slabs_fit(int X, int Y, int Z, int CS);
+int batch_slabs_smem();  // ResidentLimits::cluster
+bool batch_slabs_fit(const ResidentLimits& l, int X, int Y, int Z, int CS);
 size_t batch_slab_edge_bytes(int CS);
 fs3d_status launch_batch_slabs(int cls, int CS, const PlaneWorld* worlds, const int* order, const int* meta, int* counter,
                                int* err, void* edges, cudaStream_t st, unsigned long long* processed_cells);

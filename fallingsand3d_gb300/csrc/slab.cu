@@ -531,7 +531,8 @@ __global__ void __launch_bounds__(kBatchSlabThreads, 1)
 
 struct SlabLimits {
     int sms = 0;
-    int smem = 0;  // dynamic shared memory a CTA may have (0: the kernels cannot run)
+    int smem = 0;        // dynamic shared memory a CTA may have (0: the kernels cannot run)
+    int batch_smem = 0;  // and one of a batch's clusters
 };
 
 constexpr int kSlabThreadsNarrow = 256, kSlabThreadsWide = 640;
@@ -542,24 +543,28 @@ SlabFn slab_fn(bool zs, bool wide) {
     return wide ? &k_plane_slabs<false, kSlabThreadsWide, false> : &k_plane_slabs<false, kSlabThreadsNarrow, true>;
 }
 
-const SlabLimits& slab_limits() {
-    static SlabLimits l;
-    static std::once_flag once;
-    std::call_once(once, [] {
+// The limits hold for the current device and context: the attribute that lets a
+// kernel have more than 48 KB belongs to them, so each is given it.
+SlabLimits slab_limits() {
+    static PerContext<SlabLimits> kept;
+    return of_current_context(kept, [] {
+        SlabLimits l;
         int dev = 0, optin = 0, coop = 0;
         cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&l.sms, cudaDevAttrMultiProcessorCount, dev);
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
         const int smem = (optin - 1024) / 16 * 16;  // room for the kernels' own variables
-        bool ok = coop && smem > 0;
+        bool ok = coop && smem > 0 && l.sms > 0;
         for (int i = 0; i < 4; ++i)
             ok = ok && cudaFuncSetAttribute(reinterpret_cast<const void*>(slab_fn(i & 1, i >> 1)),
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
-        cudaGetLastError();  // a refused attribute leaves the kernels unused, not an error
-        l.sms = sm_count_public();
         l.smem = ok ? smem : 0;
+        if (ok && cudaFuncSetAttribute(k_batch_slabs, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess)
+            l.batch_smem = smem;
+        cudaGetLastError();  // a refused attribute leaves the kernels unused, not an error
+        return l;
     });
-    return l;
 }
 
 }  // namespace
@@ -569,13 +574,10 @@ fs3d_status set_slab_stall(uint32_t which) {
     return FS3D_OK;
 }
 
-bool batch_slabs_fit(int X, int Y, int Z, int CS) {
-    static const int smem = [] {
-        const int n = slab_limits().smem;
-        const bool ok = n > 0 && cudaFuncSetAttribute(k_batch_slabs, cudaFuncAttributeMaxDynamicSharedMemorySize, n) == cudaSuccess;
-        cudaGetLastError();
-        return ok ? n : 0;
-    }();
+int batch_slabs_smem() { return slab_limits().batch_smem; }
+
+bool batch_slabs_fit(const ResidentLimits& l, int X, int Y, int Z, int CS) {
+    const int smem = l.cluster;
     const int64_t nw = plane_nw(X), NP = (Z + 1) / 2, mp = (NP + CS - 1) / CS;
     return X <= kPlaneMaxX && NP >= CS && Y * nw <= kBatchSlabEdgeWords && 2 * mp * Y * nw * 16 + (2 * mp + 1) * Y <= smem;
 }
@@ -590,7 +592,7 @@ fs3d_status launch_batch_slabs(int cls, int CS, const PlaneWorld* worlds, const 
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)(sm_count_public() / CS * CS));
     lc.blockDim = dim3(kBatchSlabThreads);
-    lc.dynamicSmemBytes = (size_t)slab_limits().smem;
+    lc.dynamicSmemBytes = (size_t)slab_limits().batch_smem;
     lc.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -627,7 +629,7 @@ fs3d_status launch_batch_slabs(int cls, int CS, const PlaneWorld* worlds, const 
 // 6.2, 8.6 and 8.3 there; 400x300x350 (2416) 11.7 and 16, 10.5 and 8.3 there.
 bool slab_plan(int X, int Y, int Z, SlabPlan* out) {
     constexpr double kSlabMaxLanes = 1280.0;
-    const SlabLimits& l = slab_limits();
+    const SlabLimits l = slab_limits();
     if (!l.smem || X > kPlaneMaxX) return false;
     const int64_t nw = plane_nw(X), G = (int64_t)1 << plane_lg((int)nw);
     double best = kSlabMaxLanes;
