@@ -890,7 +890,7 @@ fs3d_status launch_plane_segment_gm(int cls, const PlaneWorld* worlds, const int
 }
 
 fs3d_status set_inject_tx_extra(uint32_t stall) {
-    const fs3d_status s = set_slab_stall(stall == kStallAll || stall == kStallFirstSlab ? stall : kStallNone);
+    const fs3d_status s = set_slab_stall(stall == kStallOneCta ? (uint32_t)kStallNone : stall);
     if (s != FS3D_OK) return s;
     const uint32_t bytes = stall == kStallAll || stall == kStallOneCta ? 16u : 0u;
     FS3D_CUDA(cudaMemcpyToSymbol(g_inject_tx_extra, &bytes, sizeof(bytes)));

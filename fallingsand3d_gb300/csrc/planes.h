@@ -86,7 +86,8 @@ enum CopyStall : uint32_t {
     kStallAll = 1,        // every one
     kStallOneCta = 2,     // those of worlds held by one CTA
     kStallFirstSlab = 3,  // that of the first CTA of a world cut into slabs
-    kStallKinds = 4
+    kStallRefuse = 4,     // (none; multi-step launches are refused)
+    kStallKinds = 5
 };
 fs3d_status set_inject_tx_extra(uint32_t stall);
 // test hook: the next n stream-ordered allocations of batch admissions fail as out of memory
@@ -231,9 +232,10 @@ bool slab_plan(int X, int Y, int Z, SlabPlan* out);
 // launches of the per-step kernel
 bool prefer_slabs(int X, int Y, int Z, int n_steps, SlabPlan* out);
 // w.steps steps from w.t; rflags as for launch_plane_step_skip (kept from call
-// to call), err as for launch_plane_segment_resident
+// to call), err as for launch_plane_segment_resident.  *taken: the steps
+// launched, fewer than w.steps when the device refuses such a launch.
 fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_t* rflags, void* scratch, int* err,
-                               cudaStream_t st);
+                               cudaStream_t st, int* taken);
 fs3d_status set_slab_stall(uint32_t stall);  // test hook, as set_inject_tx_extra
 // ---- a batch's worlds of a cluster class: CS CTAs a world, cut along z
 // (slab.cu).  Whether a world's slabs fit; the most words (Y * nw) of a layer

@@ -90,13 +90,11 @@ extern "C" fs3d_status fs3d_run_device(uint8_t* grid_dev, int X, int Y, int Z, u
     d.lg = plane_lg(nw);
     fs3d_status s = planes_from_bytes(grid_dev, X, Y, Z, d.rows, st);
     if (s == FS3D_OK) s = init_row_flags(d.rows, rflags, X, Y, Z, t0, st);
-    if (s == FS3D_OK && slabs) {
-        s = launch_plane_slabs(d, plan, rflags, scratch + rows_b + flags_b, err, st);
-    } else {
-        for (int a = 0; a < n_steps && s == FS3D_OK; ++a) {
-            d.t = t0 + (uint64_t)a;
-            s = launch_plane_step_skip(d, rflags, nullptr, nullptr, st);
-        }
+    int taken = 0;
+    if (s == FS3D_OK && slabs) s = launch_plane_slabs(d, plan, rflags, scratch + rows_b + flags_b, err, st, &taken);
+    for (int a = taken; a < n_steps && s == FS3D_OK; ++a) {
+        d.t = t0 + (uint64_t)a;
+        s = launch_plane_step_skip(d, rflags, nullptr, nullptr, st);
     }
     // a recorded failure (this run's or an earlier one's) leaves the grid as it was
     if (s == FS3D_OK) s = planes_to_bytes(d.rows, grid_dev, X, Y, Z, grid_dev, st, err);

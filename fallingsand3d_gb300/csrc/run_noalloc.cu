@@ -126,13 +126,11 @@ extern "C" fs3d_status fs3d_run_device_noalloc(uint8_t* grid_dev, int X, int Y, 
     int* err = reinterpret_cast<int*>(base + kErrOff);
     s = planes_from_bytes(grid_dev, X, Y, Z, rows, st);
     if (s == FS3D_OK) s = init_row_flags(rows, rflags, X, Y, Z, t0, st);
-    if (s == FS3D_OK && slabs) {
-        s = launch_plane_slabs(d, plan, rflags, base + rows_b, err, st);
-    } else {
-        for (int a = 0; a < n_steps && s == FS3D_OK; ++a) {
-            d.t = t0 + (uint64_t)a;
-            s = launch_plane_step_skip(d, rflags, nullptr, nullptr, st);
-        }
+    int taken = 0;
+    if (s == FS3D_OK && slabs) s = launch_plane_slabs(d, plan, rflags, base + rows_b, err, st, &taken);
+    for (int a = taken; a < n_steps && s == FS3D_OK; ++a) {
+        d.t = t0 + (uint64_t)a;
+        s = launch_plane_step_skip(d, rflags, nullptr, nullptr, st);
     }
     // static cells never change: their values are read back from the grid
     // itself; a recorded failure leaves the grid as it was

@@ -39,6 +39,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -569,7 +570,12 @@ SlabLimits slab_limits() {
 
 }  // namespace
 
+// test hook: multi-step launches are refused as if the device could not hold them
+static std::atomic<bool> g_refuse_slabs{false};
+
 fs3d_status set_slab_stall(uint32_t which) {
+    g_refuse_slabs.store(which == kStallRefuse);
+    if (which == kStallRefuse) which = kStallNone;
     FS3D_CUDA(cudaMemcpyToSymbol(g_slab_stall, &which, sizeof(which)));
     return FS3D_OK;
 }
@@ -661,7 +667,8 @@ bool prefer_slabs(int X, int Y, int Z, int n_steps, SlabPlan* out) {
 }
 
 fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_t* rflags, void* scratch, int* err,
-                               cudaStream_t st) {
+                               cudaStream_t st, int* taken) {
+    *taken = 0;
     // steps are counted in 31 bits of a tag; a launch is kept to a fraction of a second
     constexpr int kMaxSteps = 1 << 15;
     PlaneWorld d = w;
@@ -682,9 +689,18 @@ fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_
         lc.attrs = attr;
         lc.numAttrs = 1;
         const SlabFn fn = slab_fn(plan.zs != 0, plan.threads > kSlabThreadsNarrow);
-        const cudaError_t e = cudaLaunchKernelEx(&lc, fn, d, rflags, state, edge, err);
+        const cudaError_t e = g_refuse_slabs.load() ? cudaErrorCooperativeLaunchTooLarge
+                                                    : cudaLaunchKernelEx(&lc, fn, d, rflags, state, edge, err);
+        // refused for what the device has free for this process (its SMs may be
+        // shared out), before anything ran: the caller takes the rest of the
+        // steps a launch at a time
+        if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
+            cudaGetLastError();
+            return FS3D_OK;
+        }
         if (e != cudaSuccess) return cuda_fail(e, "slab steps launch");
         note_launch();
+        *taken = done + d.steps;
     }
     return FS3D_OK;
 }

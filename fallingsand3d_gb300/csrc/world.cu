@@ -192,21 +192,14 @@ fs3d_status fs3d_world_step(fs3d_world* w, int n_steps) {
         }
         // one launch for all the steps, or one per-step launch per step (prefer_slabs)
         SlabPlan plan;
-        if (w->slab_scratch && prefer_slabs(w->X, w->Y, w->Z, n_steps, &plan)) {
-            if (s == FS3D_OK) s = launch_plane_slabs(d, plan, w->rflags, w->slab_scratch, w->err, w->stream);
-            w->counts_valid = false;  // the next frame recounts
-            if (s == FS3D_OK) {
-                w->step += (uint64_t)n_steps;
-                w->flags_t = w->step;
-            } else {
-                w->flags_ok = false;
-            }
-            return s;
+        int launched = 0;
+        if (s == FS3D_OK && w->slab_scratch && prefer_slabs(w->X, w->Y, w->Z, n_steps, &plan)) {
+            s = launch_plane_slabs(d, plan, w->rflags, w->slab_scratch, w->err, w->stream, &launched);
+            if (launched) w->counts_valid = false;  // the next frame recounts
         }
         // once a frame has counted the bricks, the per-step kernel keeps the
         // counts exact, so later frames read no pass over the planes
         int* counts = w->counts_valid ? w->brick_counts : nullptr;
-        int launched = 0;
         while (s == FS3D_OK && launched < n_steps) {
             d.t = w->step + (uint64_t)launched;
             s = launch_plane_step_skip(d, w->rflags, counts, w->err, w->stream);

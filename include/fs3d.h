@@ -399,7 +399,9 @@ fs3d_status fs3d_render_meshes(const fs3d_object_view* view, const fs3d_mesh_dra
  * in full, the barrier's phase never completes, and every such wait runs to
  * its limit (20 ms with the hook set) and reports a timeout.  count 1 stalls
  * every copy, 2 those of worlds held by one CTA, 3 the copy of the first CTA of
- * a world cut into slabs (the other CTAs' waits for its results run out).
+ * a world cut into slabs (the other CTAs' waits for its results run out); 4
+ * stalls none but has the device refuse multi-step launches (decided on the
+ * host).
  * ALLOC_FAIL: the next `count` world-memory allocations of batch admissions
  * fail as out of device memory (decided on the host; nothing is launched).
  * NONE clears both.  For tests only. */
