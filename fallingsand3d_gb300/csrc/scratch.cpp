@@ -19,20 +19,27 @@ constexpr int kMaxDevices = 64;
 
 struct ScratchPool {
     unsigned long long ctx = 0;  // the context it was made in (0: none)
-    cudaMemPool_t pool = nullptr;
+    cudaMemPool_t pool = nullptr, standard = nullptr;  // this pool, and the device's default one
 };
 ScratchPool g_pools[kMaxDevices];
 std::mutex g_pools_mu;
 
-// the current device's pool, null if it has none
+// The current device's pool; null if it has none, or while the caller has made
+// another pool than the default the device's current one: scratch then comes
+// from that, as every stream-ordered allocation does.
 cudaMemPool_t scratch_pool() {
     int dev = 0;
     unsigned long long ctx = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices || !current_context_id(&ctx) || !ctx)
         return nullptr;
+    cudaMemPool_t current = nullptr;
+    if (cudaDeviceGetMemPool(&current, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
     std::lock_guard<std::mutex> lock(g_pools_mu);
     ScratchPool& s = g_pools[dev];
-    if (s.ctx == ctx) return s.pool;
+    if (s.ctx == ctx) return current == s.standard ? s.pool : nullptr;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -44,9 +51,10 @@ cudaMemPool_t scratch_pool() {
     s.ctx = ctx;
     if (cudaMemPoolCreate(&s.pool, &props) != cudaSuccess) s.pool = nullptr;
     if (s.pool && cudaMemPoolSetAttribute(s.pool, cudaMemPoolAttrReleaseThreshold, &kept) != cudaSuccess) s.pool = nullptr;
+    if (s.pool && cudaDeviceGetDefaultMemPool(&s.standard, dev) != cudaSuccess) s.pool = nullptr;
     cudaThreadExchangeStreamCaptureMode(&mode);
     cudaGetLastError();
-    return s.pool;
+    return current == s.standard ? s.pool : nullptr;
 }
 
 }  // namespace
