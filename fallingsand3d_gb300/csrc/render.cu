@@ -16,6 +16,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "fs3d_common.h"
 #include "planes.h"
 
@@ -343,11 +345,11 @@ __device__ __forceinline__ void take_steps(int& v, int s, float& n, float b, flo
 // loops, one crossing empty regions and one walking the cells of an occupied
 // brick, so that the lanes of a warp run the same one of the two.
 template <class G>
-__global__ void __launch_bounds__(64) k_render_dda(G grid, BrickMap bm, CamDev cam, int W, int H,
+__global__ void __launch_bounds__(64) k_render_dda(G grid, BrickMap bm, CamDev cam, int W, int H, int row0,
                                                    float4* __restrict__ out) {
     chain_wait();
     const int px = blockIdx.x * 8 + (threadIdx.x & 7);
-    const int py = blockIdx.y * 8 + (threadIdx.x >> 3);
+    const int py = row0 + blockIdx.y * 8 + (threadIdx.x >> 3);
     if (px >= W || py >= H) return;
     const int NX = grid.X, NY = grid.Y, NZ = grid.Z;
     float ux, uy;
@@ -568,10 +570,14 @@ static cudaError_t launch_occupancy(void (*fn)(P...), int X, int Y, int Z, cudaS
 template <class G>
 static fs3d_status launch_dda(const G& grid, const BrickMap& bm, const fs3d_camera* cam, int W, int H, float* rgba_dev,
                               cudaStream_t st) {
-    const cudaError_t e = launch_chained(k_render_dda<G>, dim3((unsigned)((W + 7) / 8), (unsigned)((H + 7) / 8)), 64, st, grid,
-                                         bm, to_dev(cam), W, H, reinterpret_cast<float4*>(rgba_dev));
-    if (e != cudaSuccess) return cuda_fail(e, "render dda launch");
-    note_launch();
+    constexpr int kRows = 65535 * 8;  // of one launch: a grid counts 65535 tiles along y
+    for (int row0 = 0; row0 < H; row0 += std::min(kRows, H - row0)) {
+        const unsigned tiles = (unsigned)((std::min(kRows, H - row0) + 7) / 8);
+        const cudaError_t e = launch_chained(k_render_dda<G>, dim3((unsigned)((W + 7) / 8), tiles), 64, st, grid, bm,
+                                             to_dev(cam), W, H, row0, reinterpret_cast<float4*>(rgba_dev));
+        if (e != cudaSuccess) return cuda_fail(e, "render dda launch");
+        note_launch();
+    }
     return FS3D_OK;
 }
 
