@@ -94,7 +94,11 @@ cudaError_t device_alloc(void** p, size_t n);
 // with launch_chained(), so that its CTAs are placed and its first instructions
 // fetched while the kernel before it in the stream ends (programmatic
 // dependent launch).  chain_wait() returns once that kernel has run and its
-// writes are visible; nothing in global memory may be touched before it.
+// writes are visible; nothing in global memory may be touched before it.  What
+// the kernel before may have written is read with ordinary loads (no __ldg, no
+// const __restrict__ parameter): the read-only path takes for granted that the
+// data stand still while the kernel lives, which here begins before they do,
+// and such a load may be moved ahead of the wait.
 // chain_go() lets the next kernel's CTAs be placed; it stands at the end of
 // each CTA's work (the end of the kernel does the same): CTAs placed any
 // earlier hold registers that other streams' kernels could use (three 1024^3

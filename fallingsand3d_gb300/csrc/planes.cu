@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(256) k_plane_step(const PlaneWorld* __restrict
 // every byte at t0 - 1 (every row changed just before).  Warps take
 // (32 >> lg) row-pairs each in order; a warp whose row-pairs are all settled
 // loads nothing.
-__device__ __forceinline__ bool rows_changed_recently(const uint8_t* __restrict__ rf, int Y, int Z, int y0, int z0,
+__device__ __forceinline__ bool rows_changed_recently(const uint8_t* rf, int Y, int Z, int y0, int z0,
                                                       uint32_t tb) {
     bool d = false;
 #pragma unroll
