@@ -390,7 +390,8 @@ __global__ void __launch_bounds__(256) k_layer_flags_from_cells(const ConvJob* _
 // get the same value from both).
 __global__ void __launch_bounds__(256) k_row_flags_from_cells(const uint4* __restrict__ rows,
                                                               uint8_t* __restrict__ rflags, int X, int Y, int Z,
-                                                              int nw, uint32_t t0b) {
+                                                              int nw, uint32_t t0b, const int* err, int* own) {
+    if (own && blockIdx.x == 0 && threadIdx.x == 0) *own = *(volatile const int*)err;
     const int lane = threadIdx.x & 31, lg = lanes_lg(nw);
     const int G = 1 << lg, per = 32 >> lg, gl = lane & (G - 1), gi = lane >> lg;
     const uint32_t gmask = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << (lane & ~(G - 1));
@@ -1106,13 +1107,14 @@ fs3d_status launch_advance_worlds(PlaneWorld* worlds, const int* meta, cudaStrea
     return FS3D_OK;
 }
 
-fs3d_status init_row_flags(const uint4* rows, uint8_t* rflags, int X, int Y, int Z, uint64_t t0, cudaStream_t st) {
+fs3d_status init_row_flags(const uint4* rows, uint8_t* rflags, int X, int Y, int Z, uint64_t t0, cudaStream_t st,
+                           const int* err, int* own) {
     FS3D_CUDA(cudaMemsetAsync(rflags, (int)((t0 - 3u) & 0xFFu), (size_t)Y * (size_t)Z, st));
     const int nw = plane_nw(X), per = 32 >> plane_lg(nw);
     const int64_t items = (int64_t)nblocks(Y, 0) * ((nblocks(Z, 0) + per - 1) / per);  // the larger phase's
     const int64_t blocks = std::min<int64_t>((items + 7) / 8, (int64_t)sm_count_public() * 8);
     k_row_flags_from_cells<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(rows, rflags, X, Y, Z, nw,
-                                                                                   (uint32_t)t0 & 0xFFu);
+                                                                                   (uint32_t)t0 & 0xFFu, err, own);
     FS3D_CUDA(cudaGetLastError());
     note_launch();
     return FS3D_OK;

@@ -205,8 +205,10 @@ fs3d_status planes_to_bytes(const uint4* rows, const uint8_t* statics, int X, in
 // that changed it (Y*Z bytes).  init_row_flags: a world about to take step t0
 // with no history: a row is marked changed at t0 - 1 when a block row-pair of
 // either phase that covers it can change (the rule's activity mask on its
-// cells), else at t0 - 3.
-fs3d_status init_row_flags(const uint4* rows, uint8_t* rflags, int X, int Y, int Z, uint64_t t0, cudaStream_t st);
+// cells), else at t0 - 3.  own (nullable): set to *err on the way, the word that
+// decides about one drop-in run (see launch_plane_slabs).
+fs3d_status init_row_flags(const uint4* rows, uint8_t* rflags, int X, int Y, int Z, uint64_t t0, cudaStream_t st,
+                           const int* err = nullptr, int* own = nullptr);
 
 // Layer flags of newly admitted worlds (jobs with lflags set), the same way
 // per layer: marked changed at t0 - 1 when a block row-pair of either phase
@@ -232,9 +234,13 @@ bool slab_plan(int X, int Y, int Z, SlabPlan* out);
 // launches of the per-step kernel
 bool prefer_slabs(int X, int Y, int Z, int n_steps, SlabPlan* out);
 // w.steps steps from w.t; rflags as for launch_plane_step_skip (kept from call
-// to call), err as for launch_plane_segment_resident.  *taken: the steps
-// launched, fewer than w.steps when the device refuses such a launch.
-fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_t* rflags, void* scratch, int* err,
+// to call), err as for launch_plane_segment_resident.  own: the word whose being
+// set keeps the launch from stepping; a failure sets both.  It is err itself
+// where the launches of one stream share err, else a copy of it taken when the
+// run began: a failure on another stream that is recorded while this run goes
+// on must not change its mind half-way.  *taken: the steps launched, fewer than
+// w.steps when the device refuses such a launch.
+fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_t* rflags, void* scratch, int* err, int* own,
                                cudaStream_t st, int* taken);
 fs3d_status set_slab_stall(uint32_t stall);  // test hook, as set_inject_tx_extra
 // ---- a batch's worlds of a cluster class: CS CTAs a world, cut along z

@@ -73,11 +73,12 @@ extern "C" fs3d_status fs3d_run_device(uint8_t* grid_dev, int X, int Y, int Z, u
         const fs3d_status se = run_error_word(&err);
         if (se != FS3D_OK) return se;
     }
-    // one block of scratch: the planes, the row flags, the slabs' scratch
+    // one block of scratch: the planes, the row flags, the run's own error word, the slabs' scratch
     const size_t rows_b = (plane_bytes(X, Y, Z) + 255) & ~(size_t)255, flags_b = ((size_t)Y * Z + 255) & ~(size_t)255;
     char* scratch = nullptr;
-    FS3D_CUDA(scratch_alloc((void**)&scratch, rows_b + flags_b + (slabs ? plan.scratch : 0), st));
+    FS3D_CUDA(scratch_alloc((void**)&scratch, rows_b + flags_b + 256 + (slabs ? plan.scratch : 0), st));
     uint8_t* rflags = reinterpret_cast<uint8_t*>(scratch + rows_b);
+    int* own = reinterpret_cast<int*>(scratch + rows_b + flags_b);
     PlaneWorld d{};
     d.rows = reinterpret_cast<uint4*>(scratch);
     d.seed = seed;
@@ -89,15 +90,15 @@ extern "C" fs3d_status fs3d_run_device(uint8_t* grid_dev, int X, int Y, int Z, u
     d.steps = n_steps;
     d.lg = plane_lg(nw);
     fs3d_status s = planes_from_bytes(grid_dev, X, Y, Z, d.rows, st);
-    if (s == FS3D_OK) s = init_row_flags(d.rows, rflags, X, Y, Z, t0, st);
+    if (s == FS3D_OK) s = init_row_flags(d.rows, rflags, X, Y, Z, t0, st, err, own);
     int taken = 0;
-    if (s == FS3D_OK && slabs) s = launch_plane_slabs(d, plan, rflags, scratch + rows_b + flags_b, err, st, &taken);
+    if (s == FS3D_OK && slabs) s = launch_plane_slabs(d, plan, rflags, scratch + rows_b + flags_b + 256, err, own, st, &taken);
     for (int a = taken; a < n_steps && s == FS3D_OK; ++a) {
         d.t = t0 + (uint64_t)a;
         s = launch_plane_step_skip(d, rflags, nullptr, nullptr, st);
     }
-    // a recorded failure (this run's or an earlier one's) leaves the grid as it was
-    if (s == FS3D_OK) s = planes_to_bytes(d.rows, grid_dev, X, Y, Z, grid_dev, st, err);
+    // a failure (this run's, or one recorded before it began) leaves the grid as it was
+    if (s == FS3D_OK) s = planes_to_bytes(d.rows, grid_dev, X, Y, Z, grid_dev, st, own);
     cudaFreeAsync(scratch, st);
     return s;
 }

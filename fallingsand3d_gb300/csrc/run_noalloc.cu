@@ -42,6 +42,7 @@ constexpr int kMaxDevices = 64;
 
 // scratch layout: [planes, then the slabs' scratch where it fits][sticky error record][row flags]
 constexpr size_t kErrOff = kNoAllocPlaneBytes;  // set by a timed-out copy, cleared by fs3d_run_device_check only
+constexpr size_t kOwnErrOff = kErrOff + 64;     // the current run's own word, set anew by each run
 constexpr size_t kFlagsOff = kErrOff + 256;
 // one byte per row of the per-step kernel: a world of at most 64 MiB of
 // planes has at most 4 Mi rows (one 16-byte word each at the least)
@@ -124,16 +125,17 @@ extern "C" fs3d_status fs3d_run_device_noalloc(uint8_t* grid_dev, int X, int Y, 
     d.lg = plane_lg(d.nw);
     uint8_t* rflags = base + kFlagsOff;
     int* err = reinterpret_cast<int*>(base + kErrOff);
+    int* own = reinterpret_cast<int*>(base + kOwnErrOff);
     s = planes_from_bytes(grid_dev, X, Y, Z, rows, st);
-    if (s == FS3D_OK) s = init_row_flags(rows, rflags, X, Y, Z, t0, st);
+    if (s == FS3D_OK) s = init_row_flags(rows, rflags, X, Y, Z, t0, st, err, own);
     int taken = 0;
-    if (s == FS3D_OK && slabs) s = launch_plane_slabs(d, plan, rflags, base + rows_b, err, st, &taken);
+    if (s == FS3D_OK && slabs) s = launch_plane_slabs(d, plan, rflags, base + rows_b, err, own, st, &taken);
     for (int a = taken; a < n_steps && s == FS3D_OK; ++a) {
         d.t = t0 + (uint64_t)a;
         s = launch_plane_step_skip(d, rflags, nullptr, nullptr, st);
     }
     // static cells never change: their values are read back from the grid
-    // itself; a recorded failure leaves the grid as it was
-    if (s == FS3D_OK) s = planes_to_bytes(rows, grid_dev, X, Y, Z, grid_dev, st, err);
+    // itself; a failure recorded before the run or by it leaves the grid as it was
+    if (s == FS3D_OK) s = planes_to_bytes(rows, grid_dev, X, Y, Z, grid_dev, st, own);
     return s;
 }

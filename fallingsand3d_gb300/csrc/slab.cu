@@ -377,7 +377,8 @@ __device__ __forceinline__ bool slab_steps(const PlaneWorld& w, const SlabGeo<ZS
 // One world over the whole GPU.  MAXT: the most threads.
 template <bool ZS, int MAXT, bool READY>
 __global__ void __launch_bounds__(MAXT, 1)
-    k_plane_slabs(const PlaneWorld w, uint8_t* __restrict__ rflags, SlabState* st, unsigned long long* edge, int* err) {
+    k_plane_slabs(const PlaneWorld w, uint8_t* __restrict__ rflags, SlabState* st, unsigned long long* edge, int* err,
+                  int* own) {
     extern __shared__ __align__(128) uint4 srows[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t s_keys[kSlabKeys];
@@ -392,7 +393,7 @@ __global__ void __launch_bounds__(MAXT, 1)
         mbar_expect(&bar, geo.bytes + stall_bytes(stall, r));
     }
     // an error recorded earlier: nothing is stepped (and every CTA's load is skipped or waited for)
-    bool dead = __syncthreads_or(tid == 0 && *(volatile int*)err != 0) != 0;
+    bool dead = __syncthreads_or(tid == 0 && *(volatile int*)own != 0) != 0;
     if (!dead) {
         geo.load(w, srows, &bar);
         for (int i = tid; i < geo.flags(); i += blockDim.x) {
@@ -421,7 +422,10 @@ __global__ void __launch_bounds__(MAXT, 1)
             }
         }
         s_verdict = v;
-        if (v == 2 && atomicCAS(err, 0, 1) == 0) *reinterpret_cast<unsigned long long*>(err + 2) = (unsigned long long)w.t;
+        if (v == 2) {
+            if (atomicCAS(err, 0, 1) == 0) *reinterpret_cast<unsigned long long*>(err + 2) = (unsigned long long)w.t;
+            *(volatile int*)own = 1;
+        }
     }
     __syncthreads();
     if (s_verdict != 1) return;
@@ -538,7 +542,7 @@ struct SlabLimits {
 
 constexpr int kSlabThreadsNarrow = 256, kSlabThreadsWide = 640;
 
-using SlabFn = void (*)(const PlaneWorld, uint8_t*, SlabState*, unsigned long long*, int*);
+using SlabFn = void (*)(const PlaneWorld, uint8_t*, SlabState*, unsigned long long*, int*, int*);
 SlabFn slab_fn(bool zs, bool wide) {
     if (zs) return wide ? &k_plane_slabs<true, kSlabThreadsWide, false> : &k_plane_slabs<true, kSlabThreadsNarrow, true>;
     return wide ? &k_plane_slabs<false, kSlabThreadsWide, false> : &k_plane_slabs<false, kSlabThreadsNarrow, true>;
@@ -666,7 +670,7 @@ bool prefer_slabs(int X, int Y, int Z, int n_steps, SlabPlan* out) {
     return n_steps >= 4 && slab_plan(X, Y, Z, out);
 }
 
-fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_t* rflags, void* scratch, int* err,
+fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_t* rflags, void* scratch, int* err, int* own,
                                cudaStream_t st, int* taken) {
     *taken = 0;
     // steps are counted in 31 bits of a tag; a launch is kept to a fraction of a second
@@ -690,7 +694,7 @@ fs3d_status launch_plane_slabs(const PlaneWorld& w, const SlabPlan& plan, uint8_
         lc.numAttrs = 1;
         const SlabFn fn = slab_fn(plan.zs != 0, plan.threads > kSlabThreadsNarrow);
         const cudaError_t e = g_refuse_slabs.load() ? cudaErrorCooperativeLaunchTooLarge
-                                                    : cudaLaunchKernelEx(&lc, fn, d, rflags, state, edge, err);
+                                                    : cudaLaunchKernelEx(&lc, fn, d, rflags, state, edge, err, own);
         // refused for what the device has free for this process (its SMs may be
         // shared out), before anything ran: the caller takes the rest of the
         // steps a launch at a time

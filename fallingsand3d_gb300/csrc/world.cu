@@ -194,7 +194,7 @@ fs3d_status fs3d_world_step(fs3d_world* w, int n_steps) {
         SlabPlan plan;
         int launched = 0;
         if (s == FS3D_OK && w->slab_scratch && prefer_slabs(w->X, w->Y, w->Z, n_steps, &plan)) {
-            s = launch_plane_slabs(d, plan, w->rflags, w->slab_scratch, w->err, w->stream, &launched);
+            s = launch_plane_slabs(d, plan, w->rflags, w->slab_scratch, w->err, w->err, w->stream, &launched);
             if (launched) w->counts_valid = false;  // the next frame recounts
         }
         // once a frame has counted the bricks, the per-step kernel keeps the
