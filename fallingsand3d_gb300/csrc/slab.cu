@@ -53,7 +53,9 @@ namespace fs3d {
 namespace {
 
 constexpr int kSlabKeys = 32;  // step keys computed together
-constexpr int kBatchSlabThreads = 640;
+// 128 registers a thread, so nothing spills (640 threads: 5 to 10 % slower on
+// 128^3, 96^3 and 64x64x1024)
+constexpr int kBatchSlabThreads = 512;
 
 // Test hook (fs3d_test_inject): which bulk copies are announced with more bytes
 // than they deliver (a CopyStall, planes.h).  0 in normal operation.
@@ -219,7 +221,18 @@ struct SlabGeo {
 // Threads work in lane groups of 1 << lg, one block row-pair at a time, as
 // the per-step kernel does; row-pairs none of whose rows changed in the two
 // previous steps are skipped (same argument, same row flags).
-template <bool ZS, bool READY>
+//
+// ONCE: a slab's row-pairs may all have a lane group of their own, which is then
+// worked out once per phase (a whole-GPU launch's slabs).  A cluster's slabs take
+// several passes, and which row-pairs share a pass decides how long they take:
+// after the cut's layer pair (first, since the neighbour waits for it) come the
+// row-pairs of one place along the other axis, y, in all layer pairs, then the
+// next place's.  A young world falls from the top and rests at the bottom, so
+// layer pair by layer pair, with a whole number of them in a pass, the same
+// warps had the resting rows in every pass and others the falling ones: two
+// 64-step segments of one 128^3 world, 4 CTAs, 1530 us so and 905 now; 60 worlds
+// of 96^3 over 2 CTAs each 1365 and 1070; 64x64x1024 1362 and 733.
+template <bool ZS, bool READY, bool ONCE>
 __device__ __forceinline__ bool slab_steps(const PlaneWorld& w, const SlabGeo<ZS>& geo, int r, uint4* srows, uint8_t* rf,
                                            unsigned long long* edge, const int* stop, volatile int* s_dead,
                                            uint32_t* s_keys, bool dead, uint32_t& rows_done) {
@@ -238,7 +251,11 @@ __device__ __forceinline__ bool slab_steps(const PlaneWorld& w, const SlabGeo<ZS
         const int NB = (NO + o + 1) >> 1, n = tasks(o), np = n / NB;
         SlabTask t{};
         if (e >= n || gl >= nw) return t;
-        const int pi = e / NB, k = e - pi * NB;
+        int pi = e / NB, k = e - pi * NB;
+        if (!ONCE && e >= NB) {
+            k = (e - NB) / (np - 1);
+            pi = 1 + (e - NB) - k * (np - 1);
+        }
         const int p = o ? pi : np - 1 - pi;  // the cut's pair first: its result travels while the rest is done
         const int s0 = lo - o + 2 * p, c0 = 2 * k - o;
         const int y0 = ZS ? c0 : s0, z0 = ZS ? s0 : c0;
@@ -341,7 +358,7 @@ __device__ __forceinline__ bool slab_steps(const PlaneWorld& w, const SlabGeo<ZS
             }
         }
     };
-    const bool once = max(tasks(0), tasks(1)) <= per;  // a lane group for every row-pair of either phase
+    const bool once = ONCE && max(tasks(0), tasks(1)) <= per;  // a lane group for every row-pair of either phase
     SlabTask even{}, odd{};
     if (once) {
         even = task(0, tid >> lg);
@@ -405,7 +422,7 @@ __global__ void __launch_bounds__(MAXT, 1)
         dead = __syncthreads_or(!ok) != 0;
     }
     uint32_t rows_done = 0;
-    dead = slab_steps<ZS, READY>(w, geo, r, srows, rf, edge, &st->verdict, &s_dead, s_keys, dead, rows_done);
+    dead = slab_steps<ZS, READY, true>(w, geo, r, srows, rf, edge, &st->verdict, &s_dead, s_keys, dead, rows_done);
     // the verdict: commit when every CTA has taken all the steps
     if (tid == 0) {
         if (dead)
@@ -500,7 +517,7 @@ __global__ void __launch_bounds__(kBatchSlabThreads, 1)
         bool dead = __syncthreads_or(!ok) != 0;
         cluster.sync();
         uint32_t rows_done = 0;
-        dead = slab_steps<true, false>(w, geo, r, srows, rf, edge, err, &s_dead, s_keys, dead, rows_done);
+        dead = slab_steps<true, false, false>(w, geo, r, srows, rf, edge, err, &s_dead, s_keys, dead, rows_done);
         if (dead && tid == 0 && atomicCAS(err, 0, 1) == 0)
             *reinterpret_cast<unsigned long long*>(err + 2) = (unsigned long long)w.t;
         rows_done = __reduce_add_sync(0xFFFFFFFFu, rows_done);
