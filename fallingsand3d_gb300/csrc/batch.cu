@@ -21,6 +21,7 @@
 #include <atomic>
 #include <chrono>
 #include <deque>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -250,6 +251,8 @@ constexpr uint64_t kYoungSteps = 128;
 // lane tasks of a dense step
 int64_t step_lanes(const BWorld& w) { return (int64_t)nblocks(w.Y, 1) * nblocks(w.Z, 1) << plane_lg(w.nw); }
 
+bool is_spread(const fs3d_batch* b, const BWorld& w, int c);
+
 // Segment class of a running world (-1: the per-step kernel) under the
 // batch's mode: 1 shared-memory classes, 2 global-memory classes, 3 hybrid
 // (young worlds in shared memory when they fit, settled ones in global
@@ -283,9 +286,7 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
             // against 3.02 ms in 128-thread CTAs; moving the 256-thread worlds
             // up to 768 threads too measured 3.09 ms)
             const int c = smem();
-            if (b->spread && (c < 0 || c >= b->spread_from) && step_lanes(w) >= b->spread_lanes &&
-                batch_slabs_fit(b->limits, w.X, w.Y, w.Z, kClusterSizes[b->spread - kSingleCtaClasses]))
-                return b->spread;
+            if (is_spread(b, w, c)) return b->spread;
             if (c >= 0 && c < kSingleCtaClasses) return c == 0 ? 1 : c;
             if (w.Y <= kGmMaxY[kGmDense]) return kResidentClasses + kGmDense;
             return c >= 0 ? c : gm();
@@ -296,22 +297,36 @@ int segment_class(const fs3d_batch* b, const BWorld& w) {
     return -1;
 }
 
+// whether a young world of class c (its shared-memory class) is spread as chosen
+bool is_spread(const fs3d_batch* b, const BWorld& w, int c) {
+    return b->spread && (c < 0 || c >= b->spread_from) && step_lanes(w) >= b->spread_lanes &&
+           batch_slabs_fit(b->limits, w.X, w.Y, w.Z, kClusterSizes[b->spread - kSingleCtaClasses]);
+}
+
 // How the hybrid mode spreads young worlds over clusters of 8 CTAs.  A large
 // world's dense steps are the segment's longest chain, so where SMs are left
 // over it is spread: every world of a whole SM's class and larger when the
 // batch then still fits the SMs, else those larger than one CTA's shared memory
-// while the batch fits the SMs twice over.  Two segments of fresh mixed worlds,
-// none spread / the larger ones / all: 32 worlds 1625 / 1076 / 969 us, 64 1482 /
-// 1152 / 1249, 150 1837 / 1284 / 1855.  With still more worlds clusters take SMs
-// from the others, and only those far above an SM's average share of a step are
-// spread, 1.75 times it or, while a batch of half as many CTAs a world would fit
-// the SMs twice, 2 times: 400 mixed worlds (all larger ones over 4 CTAs, those)
-// 1835 / 1501 us, 220 ragged 1631 / 1493; 512 mixed (none, those) 2101 / 1528,
-// 300 ragged 1890 / 1611; from 700 worlds on none is that large.
+// while the batch fits the SMs twice over, else only those far above an SM's
+// average share of a step, since clusters take SMs from the others.  Two 64-step
+// segments of fresh mixed worlds, none spread / as here: 32 worlds 1684 / 653 us,
+// 64 1362 / 793, 150 1541 / 1120, 400 1584 / 1501, 512 (three mixes) 1546 /
+// 1547, 1354 / 1544 and 1887 / 1890; ragged 64 1408 / 977, 150 1876 / 1266, 220
+// 2255 / 1580, 300 1988 / 1665, 512 2116 / 2123.  What counts as far above, 1.75
+// times the share or, for batches with fewer large worlds, 2 times, has no reason
+// but such measurements: of the two the better one for a mix is up to a quarter
+// faster.
+//
+// And nothing is spread where the clusters would take longer than the largest of
+// its worlds by itself.  A world of L lane tasks takes about as long in a cluster
+// as 0.28 L + 600 lane tasks of one CTA (128^3 4.7 us a step and 12.9, 96^3 3.4
+// and 6.9), and as many clusters as run at once (16 on 152 SMs) share the worlds:
+// 60 worlds of 96^3 2040 us spread and 1210 not, 40 of 200x16x200 1083 and 740,
+// 19 of 128^3 1198 and 2465.
 void choose_spread(fs3d_batch* b) {
     b->spread = 0;
     b->spread_lanes = 0;
-    if (b->cfg.use_smem != 3) return;
+    if (b->cfg.use_smem != 3 || b->limits.clusters < 1) return;
     int large = 0, whole = 0, rest = 0;
     int64_t lanes = 0;
     for (auto& kv : b->worlds) {
@@ -333,6 +348,16 @@ void choose_spread(fs3d_batch* b) {
     } else if (!all) {
         b->spread_lanes = lanes / sms * (large * 4 + whole + rest / 3 <= 2 * sms ? 8 : 7) / 4 + 1;
     }
+    // the spread worlds, largest first, each to the cluster that is free first
+    std::vector<int64_t> spread;
+    for (const auto& kv : b->worlds) {
+        const BWorld& w = kv.second;
+        if (!w.done && w.t < kYoungSteps && is_spread(b, w, w.cls_smem)) spread.push_back(step_lanes(w));
+    }
+    std::sort(spread.begin(), spread.end(), std::greater<int64_t>());
+    std::vector<int64_t> busy((size_t)b->limits.clusters, 0);
+    for (int64_t l : spread) *std::min_element(busy.begin(), busy.end()) += l * 28 / 100 + 600;
+    if (!spread.empty() && *std::max_element(busy.begin(), busy.end()) > spread[0]) b->spread = 0;
 }
 
 // How wide the hybrid mode makes the CTAs of settled worlds.  A world's class

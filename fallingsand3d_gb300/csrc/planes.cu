@@ -797,7 +797,7 @@ ResidentLimits resident_limits() {
     const ResidentCfgs k = resident_cfgs();
     ResidentLimits l;
     for (int c = 0; c < kSingleCtaClasses; ++c) l.one_cta[c] = k.c[c].smem;
-    l.cluster = batch_slabs_smem();
+    batch_slabs_limits(&l);
     return l;
 }
 

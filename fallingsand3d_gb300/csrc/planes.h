@@ -75,6 +75,7 @@ constexpr int kMetaInts = kMetaWorlds + 1;
 struct ResidentLimits {
     int one_cta[kSingleCtaClasses] = {};
     int cluster = 0;
+    int clusters = 0;  // clusters of 8 CTAs that run at once
 };
 ResidentLimits resident_limits();
 // smallest class that holds a world of these dims, -1 if none does
@@ -248,7 +249,7 @@ fs3d_status set_slab_stall(uint32_t stall);  // test hook, as set_inject_tx_extr
 // at a cut; the bytes of edge buffer a class needs; the launch, as
 // launch_plane_segment_resident.
 constexpr int kBatchSlabEdgeWords = 1024;
-int batch_slabs_smem();  // ResidentLimits::cluster
+void batch_slabs_limits(ResidentLimits* out);  // its last two
 bool batch_slabs_fit(const ResidentLimits& l, int X, int Y, int Z, int CS);
 size_t batch_slab_edge_bytes(int CS);
 fs3d_status launch_batch_slabs(int cls, int CS, const PlaneWorld* worlds, const int* order, const int* meta, int* counter,

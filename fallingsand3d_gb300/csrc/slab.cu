@@ -555,6 +555,7 @@ struct SlabLimits {
     int sms = 0;
     int smem = 0;        // dynamic shared memory a CTA may have (0: the kernels cannot run)
     int batch_smem = 0;  // and one of a batch's clusters
+    int clusters = 0;    // clusters of 8 that run at once
 };
 
 constexpr int kSlabThreadsNarrow = 256, kSlabThreadsWide = 640;
@@ -584,6 +585,20 @@ SlabLimits slab_limits() {
         l.smem = ok ? smem : 0;
         if (ok && cudaFuncSetAttribute(k_batch_slabs, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess)
             l.batch_smem = smem;
+        if (l.batch_smem) {
+            cudaLaunchConfig_t lc = {};
+            lc.gridDim = dim3((unsigned)(l.sms / 8 * 8));
+            lc.blockDim = dim3(kBatchSlabThreads);
+            lc.dynamicSmemBytes = (size_t)smem;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 8;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            lc.attrs = attr;
+            lc.numAttrs = 1;
+            // (fewer than an eighth of the SMs: a cluster lies within a group of them)
+            if (cudaOccupancyMaxActiveClusters(&l.clusters, k_batch_slabs, &lc) != cudaSuccess) l.clusters = 0;
+        }
         cudaGetLastError();  // a refused attribute leaves the kernels unused, not an error
         return l;
     });
@@ -601,7 +616,11 @@ fs3d_status set_slab_stall(uint32_t which) {
     return FS3D_OK;
 }
 
-int batch_slabs_smem() { return slab_limits().batch_smem; }
+void batch_slabs_limits(ResidentLimits* out) {
+    const SlabLimits l = slab_limits();
+    out->cluster = l.batch_smem;
+    out->clusters = l.clusters;
+}
 
 bool batch_slabs_fit(const ResidentLimits& l, int X, int Y, int Z, int CS) {
     const int smem = l.cluster;
