@@ -309,20 +309,22 @@ bool is_spread(const fs3d_batch* b, const BWorld& w, int c) {
 // batch then still fits the SMs, else those larger than one CTA's shared memory
 // while the batch fits the SMs twice over, else only those far above an SM's
 // average share of a step, since clusters take SMs from the others.  Two 64-step
-// segments of fresh mixed worlds, none spread / as here: 32 worlds 1684 / 653 us,
-// 64 1362 / 793, 150 1541 / 1120, 400 1584 / 1501, 512 (three mixes) 1546 /
-// 1547, 1354 / 1544 and 1887 / 1890; ragged 64 1408 / 977, 150 1876 / 1266, 220
-// 2255 / 1580, 300 1988 / 1665, 512 2116 / 2123.  What counts as far above, 1.75
-// times the share or, for batches with fewer large worlds, 2 times, has no reason
-// but such measurements: of the two the better one for a mix is up to a quarter
-// faster.
+// segments of fresh mixed worlds, none spread / as here: 32 worlds 1684 / 952 us,
+// 64 1362 / 1018, 150 1541 / 1130, 400 1584 / 1597, 512 (two mixes) 1354 / 1573
+// and 1887 / 1919; ragged 64 1408 / 1032, 150 1876 / 1515, 220 2255 / 1600, 300
+// 1988 / 1733, 512 2116 / 2125.  What counts as far above, 1.75 times the share
+// or, for batches with fewer large worlds, 2 times, has no reason but such
+// measurements, and no mix of them is right for all: of the two the better one
+// is up to a quarter faster.
 //
 // And nothing is spread where the clusters would take longer than the largest of
 // its worlds by itself.  A world of L lane tasks takes about as long in a cluster
-// as 0.28 L + 600 lane tasks of one CTA (128^3 4.7 us a step and 12.9, 96^3 3.4
-// and 6.9), and as many clusters as run at once (16 on 152 SMs) share the worlds:
-// 60 worlds of 96^3 2040 us spread and 1210 not, 40 of 200x16x200 1083 and 740,
-// 19 of 128^3 1198 and 2465.
+// as 0.3 L + 1900 lane tasks of one CTA (128^3 7.2 us a step and 12.9, 96^3 4.8
+// and 6.9), as many clusters as run at once (16 on 152 SMs) share the worlds, and
+// beside others of its size a world by itself takes 1.25 times as long at the
+// least (19 of 128^3 2465 us, one 1647).  Spread and not: 60 worlds of 96^3 2741
+// us and 1206, 40 of 200x16x200 2016 and 739, 19 of 96^3 1220 and 1205, 19 of
+// 128^3 1763 and 2465.
 void choose_spread(fs3d_batch* b) {
     b->spread = 0;
     b->spread_lanes = 0;
@@ -356,8 +358,8 @@ void choose_spread(fs3d_batch* b) {
     }
     std::sort(spread.begin(), spread.end(), std::greater<int64_t>());
     std::vector<int64_t> busy((size_t)b->limits.clusters, 0);
-    for (int64_t l : spread) *std::min_element(busy.begin(), busy.end()) += l * 28 / 100 + 600;
-    if (!spread.empty() && *std::max_element(busy.begin(), busy.end()) > spread[0]) b->spread = 0;
+    for (int64_t l : spread) *std::min_element(busy.begin(), busy.end()) += l * 3 / 10 + 1900;
+    if (!spread.empty() && *std::max_element(busy.begin(), busy.end()) > spread[0] * 5 / 4) b->spread = 0;
 }
 
 // How wide the hybrid mode makes the CTAs of settled worlds.  A world's class
@@ -679,8 +681,10 @@ fs3d_status enqueue_segment(fs3d_batch* b, cudaStream_t a, bool fork, bool with_
             if (c >= kSingleCtaClasses) {
                 void* edges = b->edges[c - kSingleCtaClasses];
                 if (has(c) && edges)
+                    // (the shared-memory mode's worlds by place; the hybrid mode's
+                    // spread ones keep the order its choice of them was measured with)
                     s = launch_batch_slabs(c, kClusterSizes[c - kSingleCtaClasses], b->tw.d, b->to.d, b->tn.d, b->counter + c,
-                                           b->err, edges, fork ? b->branch[c] : a, b->processed_dev);
+                                           b->err, edges, fork ? b->branch[c] : a, b->processed_dev, mode == 1);
             } else if (has(c))
                 s = launch_plane_segment_resident(c, b->tw.d, b->to.d, b->tn.d, b->counter + c, b->err,
                                                   fork ? b->branch[c] : a, b->processed_dev);

@@ -247,13 +247,13 @@ fs3d_status set_slab_stall(uint32_t stall);  // test hook, as set_inject_tx_extr
 // ---- a batch's worlds of a cluster class: CS CTAs a world, cut along z
 // (slab.cu).  Whether a world's slabs fit; the most words (Y * nw) of a layer
 // at a cut; the bytes of edge buffer a class needs; the launch, as
-// launch_plane_segment_resident.
+// launch_plane_segment_resident (by_place: the order of a slab's row-pairs).
 constexpr int kBatchSlabEdgeWords = 1024;
 void batch_slabs_limits(ResidentLimits* out);  // its last two
 bool batch_slabs_fit(const ResidentLimits& l, int X, int Y, int Z, int CS);
 size_t batch_slab_edge_bytes(int CS);
 fs3d_status launch_batch_slabs(int cls, int CS, const PlaneWorld* worlds, const int* order, const int* meta, int* counter,
-                               int* err, void* edges, cudaStream_t st, unsigned long long* processed_cells);
+                               int* err, void* edges, cudaStream_t st, unsigned long long* processed_cells, bool by_place);
 
 fs3d_status planes_hash_async(const uint4* rows, const uint8_t* statics, int X, int Y, int Z,
                               unsigned long long* out_dev, cudaStream_t st);

@@ -53,9 +53,11 @@ namespace fs3d {
 namespace {
 
 constexpr int kSlabKeys = 32;  // step keys computed together
-// 128 registers a thread, so nothing spills (640 threads: 5 to 10 % slower on
-// 128^3, 96^3 and 64x64x1024)
-constexpr int kBatchSlabThreads = 512;
+// threads of a batch's cluster CTAs, by the order of their row-pairs (slab_steps).
+// By place, 512 threads of 128 registers, without spills, are 5 to 10 % faster
+// than 640 on 128^3, 96^3 and 64x64x1024.
+template <bool PLACE>
+constexpr int batch_slab_threads() { return PLACE ? 512 : 640; }
 
 // Test hook (fs3d_test_inject): which bulk copies are announced with more bytes
 // than they deliver (a CopyStall, planes.h).  0 in normal operation.
@@ -222,17 +224,17 @@ struct SlabGeo {
 // the per-step kernel does; row-pairs none of whose rows changed in the two
 // previous steps are skipped (same argument, same row flags).
 //
-// ONCE: a slab's row-pairs may all have a lane group of their own, which is then
-// worked out once per phase (a whole-GPU launch's slabs).  A cluster's slabs take
-// several passes, and which row-pairs share a pass decides how long they take:
-// after the cut's layer pair (first, since the neighbour waits for it) come the
-// row-pairs of one place along the other axis, y, in all layer pairs, then the
-// next place's.  A young world falls from the top and rests at the bottom, so
-// layer pair by layer pair, with a whole number of them in a pass, the same
-// warps had the resting rows in every pass and others the falling ones: two
-// 64-step segments of one 128^3 world, 4 CTAs, 1530 us so and 905 now; 60 worlds
-// of 96^3 over 2 CTAs each 1365 and 1070; 64x64x1024 1362 and 733.
-template <bool ZS, bool READY, bool ONCE>
+// The cut's layer pair comes first, since the neighbour waits for it, and the
+// others after it, one layer pair after another, or (PLACE) the row-pairs of one
+// place along the other axis, y, in all of them, then the next place's.  A young
+// world falls from the top and rests at the bottom, so with a whole number of
+// layer pairs in a pass the same warps have the resting rows in every pass and
+// others the falling ones: two 64-step segments of one 128^3 world, 4 CTAs, 1530
+// us layer pair by layer pair and 905 by place; 60 worlds of 96^3 over 2 CTAs
+// each 1365 and 1070; 64x64x1024 over 8 1362 and 733.  Where a slab's row-pairs
+// have a lane group each (most whole-GPU launches) there is but one pass, and
+// the row-pair of a group is worked out once per phase.
+template <bool ZS, bool READY, bool PLACE>
 __device__ __forceinline__ bool slab_steps(const PlaneWorld& w, const SlabGeo<ZS>& geo, int r, uint4* srows, uint8_t* rf,
                                            unsigned long long* edge, const int* stop, volatile int* s_dead,
                                            uint32_t* s_keys, bool dead, uint32_t& rows_done) {
@@ -252,7 +254,7 @@ __device__ __forceinline__ bool slab_steps(const PlaneWorld& w, const SlabGeo<ZS
         SlabTask t{};
         if (e >= n || gl >= nw) return t;
         int pi = e / NB, k = e - pi * NB;
-        if (!ONCE && e >= NB) {
+        if (PLACE && e >= NB) {
             k = (e - NB) / (np - 1);
             pi = 1 + (e - NB) - k * (np - 1);
         }
@@ -358,7 +360,7 @@ __device__ __forceinline__ bool slab_steps(const PlaneWorld& w, const SlabGeo<ZS
             }
         }
     };
-    const bool once = ONCE && max(tasks(0), tasks(1)) <= per;  // a lane group for every row-pair of either phase
+    const bool once = !PLACE && max(tasks(0), tasks(1)) <= per;  // a lane group for every row-pair of either phase
     SlabTask even{}, odd{};
     if (once) {
         even = task(0, tid >> lg);
@@ -422,7 +424,7 @@ __global__ void __launch_bounds__(MAXT, 1)
         dead = __syncthreads_or(!ok) != 0;
     }
     uint32_t rows_done = 0;
-    dead = slab_steps<ZS, READY, true>(w, geo, r, srows, rf, edge, &st->verdict, &s_dead, s_keys, dead, rows_done);
+    dead = slab_steps<ZS, READY, false>(w, geo, r, srows, rf, edge, &st->verdict, &s_dead, s_keys, dead, rows_done);
     // the verdict: commit when every CTA has taken all the steps
     if (tid == 0) {
         if (dead)
@@ -460,7 +462,8 @@ __global__ void __launch_bounds__(MAXT, 1)
 // segment steps, cut along z.  One SM's 24 warps took 850 to 1020 us for the
 // 64 dense steps of a 128^3 world, which ended the segment of a batch of few
 // such worlds.
-__global__ void __launch_bounds__(kBatchSlabThreads, 1)
+template <bool PLACE>
+__global__ void __launch_bounds__(batch_slab_threads<PLACE>(), 1)
     k_batch_slabs(const PlaneWorld* __restrict__ worlds, const int* __restrict__ order, const int* __restrict__ meta, int cls,
                   int CS, int* counter, int* err, unsigned long long* processed_cells, unsigned long long* edges) {
     extern __shared__ __align__(128) uint4 srows[];
@@ -517,7 +520,7 @@ __global__ void __launch_bounds__(kBatchSlabThreads, 1)
         bool dead = __syncthreads_or(!ok) != 0;
         cluster.sync();
         uint32_t rows_done = 0;
-        dead = slab_steps<true, false, false>(w, geo, r, srows, rf, edge, err, &s_dead, s_keys, dead, rows_done);
+        dead = slab_steps<true, false, PLACE>(w, geo, r, srows, rf, edge, err, &s_dead, s_keys, dead, rows_done);
         if (dead && tid == 0 && atomicCAS(err, 0, 1) == 0)
             *reinterpret_cast<unsigned long long*>(err + 2) = (unsigned long long)w.t;
         rows_done = __reduce_add_sync(0xFFFFFFFFu, rows_done);
@@ -583,12 +586,13 @@ SlabLimits slab_limits() {
             ok = ok && cudaFuncSetAttribute(reinterpret_cast<const void*>(slab_fn(i & 1, i >> 1)),
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
         l.smem = ok ? smem : 0;
-        if (ok && cudaFuncSetAttribute(k_batch_slabs, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess)
-            l.batch_smem = smem;
+        for (const void* fn : {reinterpret_cast<const void*>(&k_batch_slabs<false>), reinterpret_cast<const void*>(&k_batch_slabs<true>)})
+            ok = ok && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+        if (ok) l.batch_smem = smem;
         if (l.batch_smem) {
             cudaLaunchConfig_t lc = {};
             lc.gridDim = dim3((unsigned)(l.sms / 8 * 8));
-            lc.blockDim = dim3(kBatchSlabThreads);
+            lc.blockDim = dim3(batch_slab_threads<false>());
             lc.dynamicSmemBytes = (size_t)smem;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -597,7 +601,7 @@ SlabLimits slab_limits() {
             lc.attrs = attr;
             lc.numAttrs = 1;
             // (fewer than an eighth of the SMs: a cluster lies within a group of them)
-            if (cudaOccupancyMaxActiveClusters(&l.clusters, k_batch_slabs, &lc) != cudaSuccess) l.clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&l.clusters, k_batch_slabs<false>, &lc) != cudaSuccess) l.clusters = 0;
         }
         cudaGetLastError();  // a refused attribute leaves the kernels unused, not an error
         return l;
@@ -633,11 +637,11 @@ size_t batch_slab_edge_bytes(int CS) {
 }
 
 fs3d_status launch_batch_slabs(int cls, int CS, const PlaneWorld* worlds, const int* order, const int* meta, int* counter,
-                               int* err, void* edges, cudaStream_t st, unsigned long long* processed_cells) {
+                               int* err, void* edges, cudaStream_t st, unsigned long long* processed_cells, bool by_place) {
     FS3D_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), st));
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)(sm_count_public() / CS * CS));
-    lc.blockDim = dim3(kBatchSlabThreads);
+    lc.blockDim = dim3((unsigned)(by_place ? batch_slab_threads<true>() : batch_slab_threads<false>()));
     lc.dynamicSmemBytes = (size_t)slab_limits().batch_smem;
     lc.stream = st;
     cudaLaunchAttribute attr[2];
@@ -655,7 +659,8 @@ fs3d_status launch_batch_slabs(int cls, int CS, const PlaneWorld* worlds, const 
     attr[1].val.priority = greatest;
     lc.attrs = attr;
     lc.numAttrs = 2;
-    const cudaError_t e = cudaLaunchKernelEx(&lc, k_batch_slabs, worlds, order, meta, cls, CS, counter, err, processed_cells,
+    const auto fn = by_place ? &k_batch_slabs<true> : &k_batch_slabs<false>;
+    const cudaError_t e = cudaLaunchKernelEx(&lc, fn, worlds, order, meta, cls, CS, counter, err, processed_cells,
                                              static_cast<unsigned long long*>(edges));
     if (e != cudaSuccess) return cuda_fail(e, "cluster segment launch");
     note_launch();
