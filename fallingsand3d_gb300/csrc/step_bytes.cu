@@ -460,6 +460,11 @@ static bool rows_aligned(const void* grid, int X) {
 
 // most items per SM that k_step_ragged splits over four warps each (one wave of CTAs)
 constexpr int kSplitItemsPerSm = 4;
+// Rows of so few cells leave most of a lane's 64 cells empty.  While an item has
+// four warps that costs nothing; beyond, a thread a block is faster: a step of
+// 1x1000x1000 8.2 us so and 25.7 by k_step_ragged, 4x600x600 8.9 and 11.9,
+// 8x300x300 6.6 and 7.6, 12x300x300 8.1 and 8.0.
+constexpr int kThinRow = 8;
 
 static int rows_ctas_per_sm() {
     static const int n = [] {
@@ -487,6 +492,9 @@ fs3d_status launch_step_bytes(uint8_t* grid, int X, int Y, int Z, uint64_t seed,
         return FS3D_OK;
     }
     const int lg = plane_lg(plane_nw(X)), per = 32 >> lg;
+    const int64_t split_max = (int64_t)sm_count() * kSplitItemsPerSm;
+    if (X <= kThinRow && (int64_t)nblocks(Y, 1) * ((nblocks(Z, 1) + per - 1) / per) > split_max)
+        return launch_step_simple(grid, X, Y, Z, seed, t0, n_steps, st);
     for (int a = 0; a < n_steps; ++a) {
         const uint64_t t = t0 + (uint64_t)a;
         const int o = (int)(t & 1u);
@@ -497,7 +505,7 @@ fs3d_status launch_step_bytes(uint8_t* grid, int X, int Y, int Z, uint64_t seed,
                                stepkey(seed, t), lg, a & 1);
         } else {
             const int64_t items = (int64_t)nblocks(Y, o) * ((nblocks(Z, o) + per - 1) / per);
-            if (items <= (int64_t)sm_count() * kSplitItemsPerSm)
+            if (items <= split_max)
                 e = launch_chained(k_step_ragged<true>, (unsigned)items, 128, st, grid, X, Y, Z, o, stepkey(seed, t), lg);
             else
                 e = launch_chained(k_step_ragged<false>, grid_for(items * 32, 128, 5), 128, st, grid, X, Y, Z, o,
