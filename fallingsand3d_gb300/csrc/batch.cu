@@ -331,20 +331,25 @@ void choose_spread(fs3d_batch* b) {
     if (b->cfg.use_smem != 3 || b->limits.clusters < 1) return;
     int large = 0, whole = 0, rest = 0;
     int64_t lanes = 0;
+    std::vector<const BWorld*> wide;  // of a whole SM's class and larger
     for (auto& kv : b->worlds) {
         BWorld& w = kv.second;
         if (w.done || w.t >= kYoungSteps) continue;
         lanes += step_lanes(w);
         if (w.cls_smem == -2) w.cls_smem = resident_class(b->limits, w.X, w.Y, w.Z);
-        if (w.cls_smem < 0 || w.cls_smem >= kSingleCtaClasses) ++large;
-        else if (w.cls_smem == kSingleCtaClasses - 1) ++whole;
-        else ++rest;  // three to an SM
+        if (w.cls_smem >= 0 && w.cls_smem < kSingleCtaClasses - 1) {
+            ++rest;  // three to an SM
+            continue;
+        }
+        ++(w.cls_smem == kSingleCtaClasses - 1 ? whole : large);
+        wide.push_back(&w);
     }
+    if (wide.empty()) return;
     const int sms = sm_count_public();
     b->spread = kResidentClasses - 1;
     static_assert(kClusterSizes[kResidentClasses - 1 - kSingleCtaClasses] == 8, "the widest cluster class");
     b->spread_from = kSingleCtaClasses - 1;
-    const bool all = large + whole > 0 && (large + whole) * 8 + rest / 3 <= sms;
+    const bool all = (large + whole) * 8 + rest / 3 <= sms;
     if (!all && large > 0 && large * 8 + whole + rest / 3 <= 2 * sms) {
         b->spread_from = kSingleCtaClasses;
     } else if (!all) {
@@ -352,14 +357,16 @@ void choose_spread(fs3d_batch* b) {
     }
     // the spread worlds, largest first, each to the cluster that is free first
     std::vector<int64_t> spread;
-    for (const auto& kv : b->worlds) {
-        const BWorld& w = kv.second;
-        if (!w.done && w.t < kYoungSteps && is_spread(b, w, w.cls_smem)) spread.push_back(step_lanes(w));
+    for (const BWorld* w : wide)
+        if (is_spread(b, *w, w->cls_smem)) spread.push_back(step_lanes(*w));
+    if (spread.empty()) {
+        b->spread = 0;
+        return;
     }
     std::sort(spread.begin(), spread.end(), std::greater<int64_t>());
     std::vector<int64_t> busy((size_t)b->limits.clusters, 0);
     for (int64_t l : spread) *std::min_element(busy.begin(), busy.end()) += l * 3 / 10 + 1900;
-    if (!spread.empty() && *std::max_element(busy.begin(), busy.end()) > spread[0] * 5 / 4) b->spread = 0;
+    if (*std::max_element(busy.begin(), busy.end()) > spread[0] * 5 / 4) b->spread = 0;
 }
 
 // How wide the hybrid mode makes the CTAs of settled worlds.  A world's class
@@ -375,9 +382,10 @@ void choose_spread(fs3d_batch* b) {
 // first level leaves one-warp worlds alone).  With many more worlds of mixed
 // classes (1.5 times what runs at once), CTAs of three widths beside each other
 // leave warps of an SM unused: all but the widest class take 64 threads (2048
-// mixed worlds 726 / 680 us, 3500 1066 / 977, 3500 ragged 1253 / 1204; 1400
-// ragged 694 / 781).  Worlds mostly of one class keep it (2048 of 16^3: 305 /
-// 358) up to 1.75 times (64x48x128: 1000 worlds 460 / 569, 2048 713 / 688).
+// mixed worlds, host wait included, 734 / 650 us, 3500 985 / 888, 3500 ragged
+// 1175 / 1055; 1400 ragged 694 / 781, so not there).  Worlds mostly of one class
+// keep it (2048 of 16^3: 305 / 358) up to 1.75 times (64x48x128: 1000 worlds 460
+// / 569, 2048 700 / 660).
 void choose_widen(fs3d_batch* b) {
     b->widen = kOwnLevel;
     b->widen_large = false;

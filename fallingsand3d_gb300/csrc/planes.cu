@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kConvThreads) k_gen_batch_planes(const GenJob*
 // One block row-pair of one world; lane gl of a group of G lanes.  Every lane
 // of the warp calls this (valid = false for groups past the last row-pair).
 __device__ __forceinline__ void plane_rowpair(const PlaneWorld& w, int o, uint32_t sk, int rp, bool valid, int gl,
-                                              int G, int* counts) {
+                                              int G) {
     const int NBZ = nblocks(w.Z, o);
     const int j = valid ? rp / NBZ : 0, k = valid ? rp - j * NBZ : 0;
     const uint32_t rk = rowkey(sk, (uint32_t)j, (uint32_t)k);
@@ -179,14 +179,9 @@ __device__ __forceinline__ void plane_rowpair(const PlaneWorld& w, int o, uint32
         q0[a] = q[a];
     }
     rowpair_core(q, has, o, rk, gl, G, w.nw, (w.X & 63) == 0);
-    bool any = false;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
-        if (in[a] && (q[a].x != q0[a].x || q[a].y != q0[a].y || q[a].z != q0[a].z || q[a].w != q0[a].w)) {
-            *ptr[a] = q[a];
-            any = true;
-        }
-    if (counts && any) count_bricks(counts, w, y0, z0, gl, q, q0, in);
+        if (in[a] && (q[a].x != q0[a].x || q[a].y != q0[a].y || q[a].z != q0[a].z || q[a].w != q0[a].w)) *ptr[a] = q[a];
 }
 
 // One launch = one step (segment step s_seg) of every live world.  Work items
@@ -195,7 +190,7 @@ __device__ __forceinline__ void plane_rowpair(const PlaneWorld& w, int o, uint32
 // device memory so a captured graph keeps working as worlds come and go.
 __global__ void __launch_bounds__(256) k_plane_step(const PlaneWorld* __restrict__ worlds,
                                                    const PlaneItem* __restrict__ items,
-                                                   const int* __restrict__ n_items_p, int s_seg, int* counts) {
+                                                   const int* __restrict__ n_items_p, int s_seg) {
     const int n_items = *n_items_p;
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -209,7 +204,7 @@ __global__ void __launch_bounds__(256) k_plane_step(const PlaneWorld* __restrict
         const int gl = lane & (G - 1);
         const int rp = item.rp0 + (lane >> w.lg);
         const int nrp = nblocks(w.Y, o) * nblocks(w.Z, o);
-        plane_rowpair(w, o, stepkey(w.seed, t), rp, rp < nrp, gl, G, item.world == 0 ? counts : nullptr);
+        plane_rowpair(w, o, stepkey(w.seed, t), rp, rp < nrp, gl, G);
     }
 }
 
@@ -422,8 +417,8 @@ __global__ void __launch_bounds__(256) k_row_flags_from_cells(const uint4* __res
 // ---------------------------------------------------------------------------
 // shared-memory resident segment: one CTA steps one whole world
 // ---------------------------------------------------------------------------
-// Test hook (fs3d_test_inject): extra bytes every resident kernel announces
-// on its mbarrier beyond what its bulk copy delivers.  With it set, the copy
+// Test hook (fs3d_test_inject): extra bytes a single-CTA kernel announces on
+// its mbarrier beyond what its bulk copy delivers.  With it set, the copy
 // lands in full but the barrier's phase never completes, so each wait runs to
 // its iteration limit and reports a timeout; nothing else changes.  0 in
 // normal operation.
@@ -614,7 +609,7 @@ __global__ void __launch_bounds__(NT, GM ? kGmThreadsPerSm / NT : resident_ctas_
         const bool poisoned = __syncthreads_or(!ok) != 0;
         if (poisoned && threadIdx.x == 0 && atomicCAS(err, 0, 1) == 0)
             *reinterpret_cast<unsigned long long*>(err + 2) = (unsigned long long)w.t;
-                const int G = 1 << w.lg, per = NT >> w.lg;
+        const int G = 1 << w.lg, per = NT >> w.lg;
         const int gl = lane & (G - 1);
         // layer pairs to evaluate in a step, after the buffers
         const uint32_t fs = v.stride;
@@ -1086,8 +1081,8 @@ fs3d_status planes_hash_many(const HashJob* jobs, int njobs, int parts, unsigned
 }
 
 fs3d_status launch_plane_step(const PlaneWorld* worlds, const PlaneItem* items, const int* n_items_dev,
-                              int grid, int s_seg, cudaStream_t st, int* brick_counts) {
-    k_plane_step<<<grid, 256, 0, st>>>(worlds, items, n_items_dev, s_seg, brick_counts);
+                              int grid, int s_seg, cudaStream_t st) {
+    k_plane_step<<<grid, 256, 0, st>>>(worlds, items, n_items_dev, s_seg);
     FS3D_CHECK_LAUNCH("plane step launch");
     return FS3D_OK;
 }

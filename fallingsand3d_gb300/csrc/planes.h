@@ -218,8 +218,8 @@ fs3d_status layer_flags_from_cells_multi(const ConvJob* jobs, int njobs, int max
 // the same for one world
 fs3d_status layer_flags_from_cells(const uint4* rows, uint8_t* lflags, int X, int Y, int Z, uint64_t t0,
                                    cudaStream_t st);
-// one step (w.t) of the world; counts as for launch_plane_step; err (nullable):
-// while *err is set nothing is stepped
+// one step (w.t) of the world; counts (nullable): its per-brick counts of
+// non-empty cells, kept exact; err (nullable): while *err is set nothing is stepped
 fs3d_status launch_plane_step_skip(const PlaneWorld& w, uint8_t* rflags, int* counts, const int* err, cudaStream_t st);
 // ---- many steps of one world in one launch over the whole GPU (slab.cu)
 struct SlabPlan {
@@ -266,10 +266,9 @@ struct HashJob {
 };
 fs3d_status planes_hash_many(const HashJob* jobs, int njobs, int parts, unsigned long long* out_dev, cudaStream_t st);
 // One step of many worlds at once (the batch's worlds too large to be
-// resident).  brick_counts: nullable per-brick counts of non-empty cells of
-// world 0, kept exact as it steps.
+// resident).
 fs3d_status launch_plane_step(const PlaneWorld* worlds, const PlaneItem* items, const int* n_items_dev, int grid,
-                              int s_seg, cudaStream_t st, int* brick_counts = nullptr);
+                              int s_seg, cudaStream_t st);
 
 // After a segment: every world of the table (meta[kMetaWorlds] of them) moves
 // on by its segment steps, and its layer flags count as kept, so the next

@@ -28,8 +28,9 @@
 // fails is as it was.
 //
 // Bound: latency.  A step of a small world is a chain of a word's way through
-// L2 to the neighbour (about 1 us), the draws (hidden in that wait), the
-// slots' serial chain (0.5 us) and the loads, stores and barrier around it.
+// L2 to the neighbour (the draws hidden in that wait), the slots' serial chain
+// and the loads, stores and barrier around it; a warp spends half of its cycles
+// at the barrier, that is, waiting for the CTA's slowest one.
 // Measured per step (everything falling / settled), against the launch per
 // step and, where the world fitted, one CTA or cluster for the whole world:
 // 96x80x112 2.5 / 2.4 us against 6.6 and 6.9, 128^3 3.3 / 3.1 against 7.0 and
