@@ -386,7 +386,9 @@ __global__ void __launch_bounds__(256) k_layer_flags_from_cells(const ConvJob* _
 __global__ void __launch_bounds__(256) k_row_flags_from_cells(const uint4* __restrict__ rows,
                                                               uint8_t* __restrict__ rflags, int X, int Y, int Z,
                                                               int nw, uint32_t t0b, const int* err, int* own) {
-    if (own && blockIdx.x == 0 && threadIdx.x == 0) *own = *(volatile const int*)err;
+    // (loaded here, stored at the end: the warp does not wait for it)
+    const bool tells = own && blockIdx.x == 0 && threadIdx.x == 0;
+    const int was = tells ? *(volatile const int*)err : 0;
     const int lane = threadIdx.x & 31, lg = lanes_lg(nw);
     const int G = 1 << lg, per = 32 >> lg, gl = lane & (G - 1), gi = lane >> lg;
     const uint32_t gmask = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << (lane & ~(G - 1));
@@ -412,6 +414,7 @@ __global__ void __launch_bounds__(256) k_row_flags_from_cells(const uint4* __res
             }
         }
     }
+    if (tells) *own = was;
 }
 
 // ---------------------------------------------------------------------------
