@@ -111,13 +111,18 @@ fs3d_status fs3d_step_device(uint8_t* grid_dev, int X, int Y, int Z, uint64_t se
 fs3d_status fs3d_step_device_many(int n, uint8_t* const* grids_dev, const int* dims, const uint64_t* seeds,
                                   uint64_t t0, int n_steps, void* stream);
 /* Same contract as fs3d_step_device, through the bit-plane kernels: the grid is
- * converted into 2-bit planes held in device scratch taken from the
- * stream-ordered pool (about X*Y*Z/4 bytes, freed on `stream` when done), the
- * n steps run there (n >= 4 and a world whose slabs fit the SMs' shared memory,
- * up to about 300^3 cells: one launch for all of them; otherwise one launch
- * per step) and the planes are converted back.  Settled rows are skipped
- * exactly, starting from flags computed from the cells.
- * Asynchronous on `stream`. */
+ * converted into 2-bit planes held in device scratch (about X*Y*Z/4 bytes, freed
+ * on `stream` when done), the n steps run there (n >= 4 and a world whose slabs
+ * fit the SMs' shared memory, up to about 300^3 cells: one launch for all of
+ * them, if the device has room for it at once; otherwise one launch per step) and
+ * the planes are converted back.  Settled rows are skipped exactly, starting
+ * from flags computed from the cells.  Asynchronous on `stream`.
+ *
+ * Scratch of this and every other call comes from a stream-ordered pool of the
+ * library's own, one per device, which keeps up to 64 MB mapped between calls
+ * and gives them back when an allocation of the library fails; while the caller
+ * has made a pool other than the default the device's current one, and while
+ * `stream` is captured, it comes from the current pool. */
 fs3d_status fs3d_run_device(uint8_t* grid_dev, int X, int Y, int Z, uint64_t seed, uint64_t t0,
                             int n_steps, void* stream);
 /* fs3d_run_device for callers that cannot allocate device memory (an engine
@@ -135,11 +140,11 @@ fs3d_status fs3d_run_device_noalloc(uint8_t* grid_dev, int X, int Y, int Z, uint
                                     uint64_t t0, int n_steps, void* stream);
 /* Waits for `stream` (timeout_ns < 0: without limit; FS3D_ERR_TIMEOUT when
  * the limit passes first), then reports whether a drop-in run on the current
- * device (fs3d_run_device or fs3d_run_device_noalloc) met a bulk copy that
- * did not complete within its bounded wait since the last check:
- * FS3D_ERR_TIMEOUT if so, and the record is cleared.  Such a run leaves its
- * grid as it was, and so does every drop-in run on the device after it until
- * this check.  The runs are asynchronous, so this is where a caller learns of
+ * device (fs3d_run_device or fs3d_run_device_noalloc) gave up a bounded wait
+ * (for a bulk copy, or for another CTA's part of the world) since the last
+ * check: FS3D_ERR_TIMEOUT if so, and the record is cleared.  Such a run leaves
+ * its grid as it was, and so does every drop-in run on the device that begins
+ * after it until this check; one under way on another stream is not touched.  The runs are asynchronous, so this is where a caller learns of
  * it.  No counterpart in the upstream project (it has no step). */
 fs3d_status fs3d_run_device_check(void* stream, int64_t timeout_ns);
 /* Same contract, one thread per 2x2x2 block and byte loads: the plain
@@ -162,10 +167,10 @@ fs3d_status fs3d_world_create(const uint8_t* grid_host, int X, int Y, int Z, uin
  * one launch per step, and keeps its change flags from call to call */
 fs3d_status fs3d_world_step(fs3d_world* w, int n_steps);
 /* Bounded wait (timeout_ns < 0: without limit).  FS3D_ERR_TIMEOUT also when a
- * step launch of the world met a bulk copy that did not complete within its
- * bounded wait: that launch and the ones after it stepped nothing, so the
- * world's step counter is set back to the step its state holds, and the
- * world is usable again. */
+ * step launch of the world gave up a bounded wait (for a bulk copy, or for
+ * another CTA's part of the world): that launch and the ones after it, of many
+ * steps or one, stepped nothing, so the world's step counter is set back to the
+ * step its state holds, and the world is usable again. */
 fs3d_status fs3d_world_sync(fs3d_world* w, int64_t timeout_ns);
 fs3d_status fs3d_world_read(fs3d_world* w, uint8_t* grid_host_out); /* canonical layout */
 fs3d_status fs3d_world_write(fs3d_world* w, const uint8_t* grid_host); /* replace contents */
