@@ -34,6 +34,5 @@ def test_runs_beside_a_failing_run_leave_whole_grids(fs3d, orc, cuda):
     assert (failing.cpu().numpy() == small).all()
     start = orc.hash(g)
     states = [start] + [int(h) for h in orc.run(g.copy(), 8, 0, n * runs, nthreads=0, hashes=True)][n - 1::n]
-    at = [states.index(orc.hash(d.cpu().numpy())) for d in grids]  # (a torn grid has none of the states' hashes)
-    print("runs taken:", at)
-    assert 0 < min(at) <= runs
+    for d in grids:  # a torn grid has none of the states' hashes
+        assert orc.hash(d.cpu().numpy()) in states
